@@ -173,6 +173,11 @@ dyg_status check_device_errors(dyg_graph *G, cudaStream_t st) {
             set_error("a prefix scan tile timed out waiting for its predecessor");
             return DYG_ESTATE;
         }
+        if (err & kErrBarrier) {
+            DYG_CUDA(cudaMemset(ptr<unsigned long long>(G->ws.scalars) + S_BAR, 0, sizeof(unsigned long long)));
+            set_error("a block timed out waiting at a grid barrier; the graphs are no longer consistent");
+            return DYG_ESTATE;
+        }
         set_error("internal consistency check failed (device error bits " + std::to_string(err) + ")");
         return DYG_ESTATE;
     }
@@ -201,13 +206,11 @@ void free_graph(dyg_graph *G) {
     DeviceGuard dg(G->device);
     Workspace &ws = G->ws;
     Buf *bufs[] = {&ws.keys, &ws.flags, &ws.pos, &ws.f_src, &ws.f_dst, &ws.f_idx, &ws.f_uid,
-                   &ws.f_w, &ws.found, &ws.hx, &ws.hy, &ws.hw, &ws.path_v, &ws.path_s,
-                   &ws.path_len, &ws.cand_x, &ws.cand_y, &ws.cand_w, &ws.keep, &ws.htab_k,
-                   &ws.htab_v, &ws.nop, &ws.cub_tmp, &ws.scan_status, &ws.s_src, &ws.s_dst, &ws.s_w, &ws.s_o1,
-                   &ws.s_o2, &ws.s_o3, &ws.rx2, &ws.ry2, &ws.rk2, &ws.rank, &ws.lneed, &ws.dtmp,
-                   &ws.rowcnt, &ws.rowtmp, &ws.tmask, &ws.del_hx, &ws.del_hy,
-                   &ws.st_key, &ws.st_val, &ws.st_pos, &ws.st_wapp, &ws.big, &ws.s_uid, &ws.scalars,
-                   &ws.counts};
+                   &ws.f_w, &ws.found, &ws.path_v, &ws.path_s, &ws.path_len, &ws.cand_x, &ws.cand_y,
+                   &ws.cand_w, &ws.keep, &ws.htab_k, &ws.htab_v, &ws.cub_tmp, &ws.scan_status,
+                   &ws.s_src, &ws.s_dst, &ws.s_w, &ws.s_o1, &ws.s_o2, &ws.s_o3, &ws.rx2, &ws.ry2,
+                   &ws.rk2, &ws.nxt, &ws.dtmp, &ws.rowcnt, &ws.rowhead, &ws.blk, &ws.st_key,
+                   &ws.st_val, &ws.st_pos, &ws.st_wapp, &ws.big, &ws.s_uid, &ws.scalars, &ws.counts};
     for (Buf *b : bufs) free_buf(*b);
     if (ws.host_scalars) cudaFreeHost(ws.host_scalars);
     if (ws.host_counts) cudaFreeHost(ws.host_counts);
@@ -619,8 +622,8 @@ static dyg_status incremental_common(dyg_graph *H, dyg_graph *G, const uint32_t 
         return DYG_EINVAL;
     }
     DYG_TRY(check_params(p));
-    if (G && (G->g.n != H->g.n || G->device != H->device)) {
-        set_error("G and H must have the same vertex count and device");
+    if (G && (G == H || G->g.n != H->g.n || G->device != H->device)) {
+        set_error("G and H must be two handles with the same vertex count and device");
         return DYG_EINVAL;
     }
     if (n == 0) return DYG_OK;
@@ -707,8 +710,8 @@ static dyg_status decremental_common(dyg_graph *G, dyg_graph *H, const uint32_t 
         return DYG_EINVAL;
     }
     DYG_TRY(check_params(p));
-    if (G->g.n != H->g.n || G->device != H->device) {
-        set_error("G and H must have the same vertex count and device");
+    if (G == H || G->g.n != H->g.n || G->device != H->device) {
+        set_error("G and H must be two handles with the same vertex count and device");
         return DYG_EINVAL;
     }
     if (n_rec) *n_rec = 0;
@@ -861,8 +864,8 @@ dyg_status dyg_stream_file(dyg_graph *G, dyg_graph *H, uint32_t op, const uint32
         return DYG_EINVAL;
     }
     DYG_TRY(check_params(p));
-    if (G->g.n != H->g.n || G->device != H->device) {
-        set_error("G and H must have the same vertex count and device");
+    if (G == H || G->g.n != H->g.n || G->device != H->device) {
+        set_error("G and H must be two handles with the same vertex count and device");
         return DYG_EINVAL;
     }
     if (n_rec) *n_rec = 0;
@@ -904,6 +907,7 @@ dyg_status dyg_stream_file(dyg_graph *G, dyg_graph *H, uint32_t op, const uint32
                             &total, st, dev_in));
     if (!ins) G->last_rec = total;
     if (G->ws.host_scalars[S_ERR]) DYG_TRY(check_device_errors(G, st));
+    if (H->ws.host_scalars[S_ERR]) DYG_TRY(check_device_errors(H, st));
     bool host_out = false;
     if (status && o_st != status) DYG_TRY(copy_out(status, (const int32_t *)o_st, n, st, &host_out));
     if (conductance && o_cd != conductance)

@@ -40,6 +40,7 @@ constexpr uint32_t kErrPath = 2u;      // winner re-walk disagreed with its key
 constexpr uint32_t kErrArena = 4u;     // arena overflow in a commit
 constexpr uint32_t kErrWeight = 8u;    // weight not finite and > 0 in a batch
 constexpr uint32_t kErrScan = 16u;     // a scan tile gave up waiting for its predecessor
+constexpr uint32_t kErrBarrier = 32u;  // a block gave up waiting at a grid barrier
 
 struct DevGraph {
     uint2 *desc;
@@ -105,10 +106,10 @@ __device__ __forceinline__ unsigned long long mul_hi32(uint32_t r, unsigned long
 }
 
 // ------------------------------------------------------------- long rows
-// Rows longer than kBigRow are scanned, moved and edited by a whole block
-// (kBigThreads threads) instead of one thread or one small lane group: on
-// power-law graphs a hub row holds tens of thousands of slots, and a serial
-// scan of it would bound the whole launch.
+// Rows longer than kBigRow are scanned and moved by a whole block instead of
+// one thread, lane group or warp: on power-law graphs a hub row holds tens of
+// thousands of slots, and a serial scan of it would bound the whole launch.
+// kBigThreads: threads of the stream files' search blocks.
 constexpr uint32_t kBigRow = 256;
 constexpr uint32_t kBigThreads = 256;
 
@@ -153,18 +154,16 @@ struct Buf {
 
 struct Workspace {
     Buf keys;                                 // u64 per edge
-    Buf flags, pos;                           // u32 per edge
+    Buf flags, pos;                           // u32 per edge / per vertex (compaction)
     Buf f_src, f_dst, f_idx;                  // walk list (filtered deletions / new insertions)
     Buf f_uid;                                // u64 per walk-list entry
     Buf f_w;                                  // f32 per walk-list entry (insertions)
     Buf found;                                // u8 per half-edge
-    Buf hx, hy, hw;                           // half-edge lists (u32/f32)
     Buf path_v, path_s;                       // winner paths: vertices, taken slots
     Buf path_len;                             // i32 per filtered edge
     Buf cand_x, cand_y, cand_w;               // recovery candidates
     Buf keep;                                 // u32 per candidate
     Buf htab_k, htab_v;                       // dedup hash table
-    Buf nop;                                  // u32 no-path filtered indices
     Buf cub_tmp;
     Buf scan_status;                          // u64 per tile of the single-pass scan
     unsigned long long scan_tickets = 0;      // tile tickets handed out so far (S_SCAN)
@@ -172,14 +171,13 @@ struct Workspace {
     Buf s_src, s_dst, s_w, s_o1, s_o2, s_o3;  // whole-stream staging
     Buf rx2, ry2;                             // recovered edges of a whole stream
     Buf rk2;
-    Buf rank, lneed, dtmp;                    // row operations: per-entry rank / need / run
-    Buf rowcnt, rowtmp;                       // row operations: per-row counter / run base
-    Buf tmask;                                // dedup table size (device)
-    Buf del_hx, del_hy;                       // deletion half-edges
+    Buf nxt, dtmp;                            // row operations: per-entry chain link / ordered run
+    Buf rowcnt, rowhead;                      // row operations: per-row entries / last entry + 1
+    Buf blk;                                  // row operations: per-block words
     Buf st_key, st_val;                       // stream file: (min, max) keys and indices, sorted
     Buf st_pos;                               // stream file: uint4 slot positions in G and H
     Buf st_wapp;                              // stream file: G weight of each new edge
-    Buf big;                                  // uint4 per long-row item (block-cooperative pass)
+    Buf big;                                  // stream file: uint4 per long-row search
     Buf s_uid;                                // staged per-edge update ids
     Buf scalars;                              // u64 scalars (see Scalar)
     Buf counts;                               // u32 counts (see Count)
@@ -189,11 +187,11 @@ struct Workspace {
 
 // Indices into Workspace::scalars (u64, device) and Workspace::counts (u32).
 enum Scalar : int {
-    S_NEED = 0,       // arena slots a pending append needs (row moves)
-    S_CURSOR = 1,     // arena cursor of the moves of that append (follows S_NEED)
-    S_OPRAN = 2,      // set when an append took its row ranks
-    S_NBIG = 3,       // entries on the long-row list of the current row operation
-    S_TMPCUR = 4,     // scratch cursor of a delete (follows S_NBIG)
+    S_NEED = 0,       // arena slots a pending append needs (zero between appends)
+    S_CURSOR = 1,     // arena cursor of the moves of that append
+    S_KEPT = 2,       // recovery candidates kept so far (zero between recoveries)
+    S_NBIG = 3,       // stream file: entries on the long-row list
+    S_TMPCUR = 4,     // scratch cursor of a delete (zero between deletes)
     S_ERR = 5,        // device error bits (kErr*)
     S_MOVES = 6,      // walker moves (accumulating)
     S_WALKS = 7,      // walks finished (accumulating)
@@ -204,22 +202,15 @@ enum Scalar : int {
     S_RECCAP = 12,    // capacity of the record buffers (follows S_RECCNT)
     S_LONG = 13,      // set by an append that made a row longer than kBigRow
     S_SCAN = 14,      // tile tickets of the single-pass scan (accumulating)
-    S_BLOCKS = 15,    // blocks of an append's sizing pass that finished (the last resets it)
+    S_BAR = 15,       // grid barrier: arrivals (low word), generation (high word)
     S_NSCALARS = 16
 };
 enum Count : int {
     C_FILTERED = 0,   // decremental: edges to walk
-    C_CANDS = 1,      // recovery candidates
-    C_KEPT = 2,       // half-edges of the kept recovery candidates
-    C_NOPATH = 3,     // decremental: edges without a path
-    C_ACCEPTED = 4,   // incremental: accepted edges
-    C_CANDS2 = 5,     // fallback candidates
-    C_RANGE = 6,      // walk-list entries of the current range
-    C_WALKLIST = 7,   // stream file: new insertions to walk
-    C_GHALF = 8,      // stream file: half-edges of the new insertions (G append)
-    C_CANDS_ALL = 9,  // recovery candidates: path, then fallback
-    C_HHALF = 10,     // incremental: half-edges of the accepted edges (H append)
-    C_NCOUNTS = 12
+    C_CANDS = 1,      // path candidates of a recovery (fallback candidates follow)
+    C_CANDS_ALL = 2,  // all candidates of a recovery
+    C_WALKLIST = 3,   // stream file: new insertions to walk
+    C_NCOUNTS = 4
 };
 
 // Halt codes: (batch + 1) << 8 | kind << 4 | phase.
@@ -230,13 +221,6 @@ __host__ __device__ __forceinline__ unsigned long long halt_code(uint32_t batch,
                                                                  uint32_t phase) {
     return ((unsigned long long)(batch + 1) << 8) | (kind << 4) | phase;
 }
-
-struct AppendList {
-    const uint32_t *hx, *hy;
-    const float *hw;
-    const uint32_t *m_dev;   // device length, or null
-    uint32_t m_host;         // host length or upper bound
-};
 
 }  // namespace dyg
 
@@ -251,8 +235,8 @@ struct dyg_graph {
     // (as G); they stay in ws.rx2 / ry2 / rk2 until the next such call.
     uint64_t last_rec = 0;
     // The graph has (or may have) a row longer than kBigRow: row operations
-    // then send such rows to the block-cooperative kernels.  Without it every
-    // row takes the one-thread path (same results, no extra launches).
+    // then spread their entries over every SM, and stream files search such
+    // rows with whole blocks (the results do not depend on it).
     bool long_rows = false;
 };
 
@@ -298,26 +282,27 @@ struct WalkJob {
     const float *w;              // incremental: per-edge weight; else null
     const unsigned long long *uid;   // per-edge update id, or null -> uid0 + e
     unsigned long long uid0;
-    const uint32_t *n_dev;       // device edge count, or null -> n_host
-    uint32_t n_host;
+    const uint32_t *n_dev;       // device count of the whole list, or null -> n_host edges
+    uint32_t n_host;             // edges of this range at most
     uint32_t domain;
+    uint32_t f0;                 // this range's first entry in the list n_dev counts
 };
+// Edges of a job: those of [f0, f0 + n_host) the list has.
+__device__ __forceinline__ uint32_t job_count(const WalkJob &j) {
+    if (!j.n_dev) return j.n_host;
+    const uint32_t n = *j.n_dev;
+    return n > j.f0 ? min(n - j.f0, j.n_host) : 0u;
+}
+// counter_zero: the kernel's chunk counter is known to be zero (the commit
+// of the batch before reset it), so no memset precedes the launch.
 dyg_status launch_walk(dyg_graph *G, const WalkJob &job, const dyg_walk_params &p, bool incremental,
-                       unsigned long long *keys, cudaStream_t st);
+                       unsigned long long *keys, cudaStream_t st, bool counter_zero = false);
 dyg_status launch_walk_scalars(const DevGraph &g, const WalkJob &job, const dyg_walk_params &p,
                                bool incremental, unsigned long long *keys,
                                unsigned long long *scalars, cudaStream_t st);
 dyg_status launch_winner_paths(dyg_graph *G, const WalkJob &job, const dyg_walk_params &p,
                                const unsigned long long *keys, uint32_t n_max, uint32_t path_stride,
                                uint32_t *path_v, uint32_t *path_s, int32_t *path_len, cudaStream_t st);
-// Writes its candidates at cx/cy/cw + *base_dev.
-dyg_status launch_fallback_walks(dyg_graph *G, const unsigned long long *halt,
-                                 const uint32_t *f_src, const uint32_t *f_dst,
-                                 const unsigned long long *f_uid, const uint32_t *nop,
-                                 const uint32_t *n_nop_dev, uint32_t n_nop_max,
-                                 const dyg_walk_params &p, const uint32_t *base_dev, uint32_t *cx,
-                                 uint32_t *cy, float *cw, cudaStream_t st);
-
 // --- capi.cu
 // After a run: DYG_OK, or the error the kernels flagged in G's scalars (last
 // read by the run), which are cleared.
@@ -360,17 +345,19 @@ dyg_status decr_delete_enqueue(dyg_graph *G, dyg_graph *H, const uint32_t *src,
                                unsigned long long *halt, int32_t *status, float *cond,
                                cudaStream_t st);
 // keys_given (device, may be null): the walk list's winner keys, computed
-// elsewhere (a sharded batch); the walks are then skipped.
+// elsewhere (a sharded batch); the walks are then skipped.  walk_ready: the
+// handle's own keys and chunk counter are zero (the launch before left them so).
 dyg_status decr_walk_enqueue(dyg_graph *G, dyg_graph *H, uint32_t f0, uint32_t nf,
                              const uint32_t *F_dev, const dyg_walk_params &p,
                              unsigned long long *halt, uint32_t batch, uint32_t phase0,
-                             int32_t *status, float *cond, cudaStream_t st,
+                             int32_t *status, float *cond, cudaStream_t st, bool walk_ready,
                              const unsigned long long *keys_given = nullptr);
+// The commit reads keys; clear_keys zeroes them behind it for the next walk.
 dyg_status incr_commit_enqueue(dyg_graph *H, dyg_graph *G, const uint32_t *src,
                                const uint32_t *dst, const float *w, uint32_t n,
-                               const unsigned long long *keys, unsigned long long *halt,
-                               uint32_t batch, int32_t *found, float *cond, uint8_t *acc,
-                               cudaStream_t st);
+                               unsigned long long *keys, bool clear_keys,
+                               unsigned long long *halt, uint32_t batch, int32_t *found,
+                               float *cond, uint8_t *acc, cudaStream_t st);
 // Grows b to `bytes`, keeping its first `used` bytes.
 dyg_status grow_keep(Buf &b, size_t bytes, size_t used, cudaStream_t st);
 
@@ -384,13 +371,6 @@ dyg_status stream_file_run(dyg_graph *G, dyg_graph *H, uint32_t op, const uint32
 // --- graph.cu
 dyg_status upload_graph(dyg_graph *G, uint32_t n, const uint64_t *row_ptr, const uint32_t *col,
                         const float *w);
-dyg_status append_enqueue(dyg_graph *GA, const AppendList &A, dyg_graph *GB, const AppendList *B,
-                          unsigned long long *halt, unsigned long long code, cudaStream_t st);
-// Deletes list entries (hx[i], hy[i]) from G in list order (fG[i] = 1 when
-// found), then from H the entries G found on both sides of their edge (fH).
-dyg_status delete_pair_enqueue(dyg_graph *G, dyg_graph *H, const uint32_t *hx, const uint32_t *hy,
-                               uint32_t m, uint8_t *fG, uint8_t *fH, unsigned long long *halt,
-                               cudaStream_t st);
 // Copies both graphs' scalars and counts to the host with one synchronize.
 dyg_status read_scalars2(dyg_graph *A, dyg_graph *B, cudaStream_t st);
 // Exclusive scan of in[0, m) into out; with m_dev, of in[0, min(m, *m_dev)).

@@ -1,0 +1,755 @@
+// rowops.cuh -- device-driven row updates of the dynamic CSR, as phases of a
+// cooperative launch (gridsync.cuh).
+//
+// A list of edges e < n has half-edges i = 2e (the source's row gets the
+// target) and i = 2e + 1 (the target's row gets the source).  Both operations
+// apply the half-edges of a row in list order without sorting the list:
+//   link:    each half-edge pushes itself on its row's chain (one exchange on
+//            rowhead, one add on rowcnt); the one that found the chain empty
+//            is the row's leader.
+//   append:  leaders size their rows and the block that arrives last reserves
+//            the arena space of all moves, all or nothing (halting the stream
+//            when it does not fit); then each leader moves its row if it
+//            overflows, gathers its chain, puts it in list order and writes
+//            the tail.  Row order is therefore exactly the order the
+//            reference's host loop produces
+//            (random_walk_incremental/gpu_graph.cuh:297-329).
+//   delete:  each leader gathers its chain, puts it in list order and removes
+//            the entries one by one with swap-with-last
+//            (random_walk_decremental/gpu_graph.cuh:359-399).
+// The work of a row is done by its leader's lane, by the leader's warp, or --
+// hub rows and long chains -- by its block.  A chain of more than 32 entries
+// is not followed (each link is a dependent load): the block scans the list
+// for the row's entries instead, which meets them in order.
+// Nothing here needs a host-visible count, so a whole update stream is
+// enqueued with a single synchronize at its end.
+#pragma once
+
+#include "dyg_internal.cuh"
+#include "gridsync.cuh"
+
+namespace dyg {
+
+constexpr uint32_t kLaneRow = 32;     // rows up to this length are edited by one lane
+constexpr uint32_t kLaneChain = 4;    // ... with up to this many entries
+constexpr uint32_t kWarpChain = 32;   // entries a warp gathers
+constexpr uint32_t kWarpSearch = 4096;   // slots a warp looks at for one row's deletions
+constexpr uint32_t kTrackMax = 128;   // deletions of a hub row found in one pass over it
+
+// The chains of one graph's rows.
+struct Chains {
+    uint32_t *rowcnt, *rowhead;   // per row: entries, last entry + 1 (zero between operations)
+    uint32_t *nxt;                // per half-edge: previous entry + 1; 0 leader, ~0u not in the list
+};
+
+struct EdgeList {
+    const uint32_t *src, *dst;
+    const float *w;
+};
+
+struct AppSide {
+    DevGraph g;
+    Chains c;
+    EdgeList E;
+    uint32_t slack;
+    unsigned long long *sc;   // the graph's scalars
+};
+struct AppSides {
+    AppSide s[2];
+    uint32_t n;   // sides used
+};
+
+// A row left to a warp or to the block.
+struct RowItem {
+    uint32_t x, cnt, head, old_off, deg, off;
+};
+
+// Entries each thread looks at per tile of scan_entries.
+constexpr uint32_t kScanEdges = 8;
+
+// Shared memory of the row phases.  Items for the block fill `item` from the
+// front, items for one warp each from the back.
+struct RowShared {
+    RowItem item[kOpThreads];
+    uint32_t nbig, nwarp;
+    uint32_t warp[kOpThreads / 32 + 1];
+    uint32_t tile[kScanEdges * kOpThreads / 32 + 1];
+    // hub-row deletions
+    uint32_t best, ok, nlive;
+    uint32_t y[kTrackMax], pos[kTrackMax], occ[kTrackMax];
+    unsigned long long key[kTrackMax];
+};
+
+__device__ __forceinline__ void link_entry(const Chains &c, uint32_t i, uint32_t x, bool on) {
+    uint32_t nx = ~0u;
+    if (on) {
+        nx = atomicExch(c.rowhead + x, i + 1u);
+        atomicAdd(c.rowcnt + x, 1u);
+    }
+    c.nxt[i] = nx;
+}
+
+__device__ __forceinline__ uint32_t entry_row(const EdgeList &E, uint32_t i) {
+    return (i & 1u) ? E.dst[i >> 1] : E.src[i >> 1];
+}
+__device__ __forceinline__ uint32_t entry_col(const EdgeList &E, uint32_t i) {
+    return (i & 1u) ? E.src[i >> 1] : E.dst[i >> 1];
+}
+
+// Arena slots row x needs to take cnt more entries; 0 if they fit where it is.
+__device__ __forceinline__ uint32_t move_need(uint32_t deg, uint32_t cnt, uint32_t cap,
+                                              uint32_t slack) {
+    const uint32_t nd = deg + cnt;
+    if (nd <= cap) return 0u;
+    const uint32_t need = max(2u * nd, nd + slack);
+    return (need + 1u) & ~1u;
+}
+
+// ------------------------------------------------------------------ append
+
+// Leaders add up the arena slots their rows' moves need.
+__device__ __forceinline__ void app_need(const AppSide &a, uint32_t m,
+                                         unsigned long long *s_need) {
+    const uint2 r = block_range(m);
+    unsigned long long mine = 0ull;
+    for (uint32_t i = r.x + threadIdx.x; i < r.y; i += blockDim.x) {
+        if (a.c.nxt[i] != 0u) continue;
+        const uint32_t x = entry_row(a.E, i);
+        mine += move_need(a.g.desc[x].y, a.c.rowcnt[x], a.g.cap[x], a.slack);
+    }
+    if (threadIdx.x == 0) *s_need = 0ull;
+    __syncthreads();
+    if (mine) atomicAdd(s_need, mine);
+    __syncthreads();
+    if (threadIdx.x == 0 && *s_need) atomicAdd(a.sc + S_NEED, *s_need);
+}
+
+// Reserves the moves of all sides, all or nothing, or halts.  One thread.
+__device__ __forceinline__ bool reserve_moves(const AppSides &A, unsigned long long *halt,
+                                              unsigned long long code) {
+    bool ok = true;
+    for (uint32_t k = 0; k < A.n; ++k)
+        ok &= *A.s[k].g.top + __ldcg(A.s[k].sc + S_NEED) <= A.s[k].g.arena_cap;
+    for (uint32_t k = 0; k < A.n; ++k) {
+        unsigned long long *sc = A.s[k].sc;
+        const unsigned long long need = __ldcg(sc + S_NEED);
+        if (ok) {
+            sc[S_CURSOR] = *A.s[k].g.top;
+            *A.s[k].g.top += need;
+        }
+        sc[S_NEED] = 0ull;
+    }
+    if (!ok) *halt = code;
+    return ok;
+}
+
+// Slots [from, from + deg) to [to, to + deg) by `nt` threads of rank t.  The
+// ranges never overlap (a row moves to fresh arena space), so U slots per
+// thread are loaded before they are stored.
+template <uint32_t U>
+__device__ __forceinline__ void copy_row(const DevGraph &g, uint32_t from, uint32_t to,
+                                         uint32_t deg, uint32_t t, uint32_t nt) {
+    for (uint32_t j0 = 0; j0 < deg; j0 += U * nt) {
+        uint2 sv[U];
+        float wv[U];
+#pragma unroll
+        for (uint32_t u = 0; u < U; ++u) {
+            const uint32_t j = j0 + u * nt + t;
+            if (j < deg) {
+                sv[u] = g.slots[from + j];
+                wv[u] = g.wts[from + j];
+            }
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < U; ++u) {
+            const uint32_t j = j0 + u * nt + t;
+            if (j < deg) {
+                g.slots[to + j] = sv[u];
+                g.wts[to + j] = wv[u];
+            }
+        }
+    }
+}
+
+__device__ __forceinline__ void put_slot(const DevGraph &g, uint32_t at, uint32_t y, float w) {
+    g.slots[at] = make_uint2(y, __float_as_uint(__frcp_rn(w)));
+    g.wts[at] = w;
+}
+
+__device__ __forceinline__ void publish_row(const AppSide &a, uint32_t x, uint32_t off,
+                                            uint32_t deg, uint32_t cnt, uint32_t need) {
+    a.g.desc[x] = make_uint2(off, deg + cnt);
+    if (need) a.g.cap[x] = need;
+    if (deg + cnt > kBigRow && deg <= kBigRow) a.sc[S_LONG] = 1ull;
+}
+
+__device__ __forceinline__ void items_reset(RowShared &s) {
+    if (threadIdx.x == 0) {
+        s.nbig = 0u;
+        s.nwarp = 0u;
+    }
+    __syncthreads();
+}
+__device__ __forceinline__ void item_for_block(RowShared &s, const RowItem &it) {
+    s.item[atomicAdd(&s.nbig, 1u)] = it;
+}
+__device__ __forceinline__ void item_for_warp(RowShared &s, const RowItem &it) {
+    s.item[kOpThreads - 1u - atomicAdd(&s.nwarp, 1u)] = it;
+}
+
+// The whole block calls back(k, i) for the k-th entry i, in list order, of
+// row x.  The list is read kScanEdges edges per thread at a time, all loads
+// issued together (a 40 000-entry list: five tiles); rows(e) gives the rows
+// of edge e's two half-edges.
+template <class Rows, class Back>
+__device__ __forceinline__ void scan_entries(const Chains &c, uint32_t m, uint32_t x, uint32_t cnt,
+                                             RowShared &s, Rows rows, Back back) {
+    const uint32_t n = m >> 1, lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    const uint32_t nw = blockDim.x >> 5;
+    uint32_t run = 0;
+    for (uint32_t t0 = 0; t0 < n && run < cnt; t0 += kScanEdges * blockDim.x) {
+        uint32_t on = 0u;   // bits 2u, 2u + 1: the half-edges of edge u
+#pragma unroll
+        for (uint32_t u = 0; u < kScanEdges; ++u) {
+            const uint32_t e = t0 + u * blockDim.x + threadIdx.x;
+            if (e >= n) continue;
+            const uint2 nx = reinterpret_cast<const uint2 *>(c.nxt)[e];
+            const uint2 r = rows(e);
+            on |= ((nx.x != ~0u && r.x == x) ? 1u : 0u) << (2u * u);
+            on |= ((nx.y != ~0u && r.y == x) ? 1u : 0u) << (2u * u + 1u);
+        }
+        uint32_t before[kScanEdges];   // of this edge row, in this warp's earlier lanes
+#pragma unroll
+        for (uint32_t u = 0; u < kScanEdges; ++u) {
+            const uint32_t m0 = __ballot_sync(kFull, (on >> (2u * u)) & 1u);
+            const uint32_t m1 = __ballot_sync(kFull, (on >> (2u * u + 1u)) & 1u);
+            const uint32_t lt = (1u << lane) - 1u;
+            before[u] = __popc(m0 & lt) + __popc(m1 & lt);
+            if (lane == 0u) s.tile[u * nw + wid] = __popc(m0) + __popc(m1);
+        }
+        __syncthreads();
+        if (wid == 0u) {   // exclusive scan of the kScanEdges * nw counts
+            uint32_t carry = 0u;
+            for (uint32_t q = 0; q < kScanEdges * nw; q += 32u) {
+                const uint32_t v = q + lane < kScanEdges * nw ? s.tile[q + lane] : 0u;
+                uint32_t incl = v;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t t = __shfl_up_sync(kFull, incl, o);
+                    if (lane >= (uint32_t)o) incl += t;
+                }
+                if (q + lane < kScanEdges * nw) s.tile[q + lane] = carry + incl - v;
+                carry += __shfl_sync(kFull, incl, 31);
+            }
+            if (lane == 0u) s.tile[kScanEdges * nw] = carry;
+        }
+        __syncthreads();
+        if (on) {
+#pragma unroll
+            for (uint32_t u = 0; u < kScanEdges; ++u) {
+                const uint32_t e = t0 + u * blockDim.x + threadIdx.x;
+                uint32_t k = run + s.tile[u * nw + wid] + before[u];
+                if ((on >> (2u * u)) & 1u) back(k++, 2u * e);
+                if ((on >> (2u * u + 1u)) & 1u) back(k, 2u * e + 1u);
+            }
+        }
+        run += s.tile[kScanEdges * nw];
+        __syncthreads();   // s.tile is written again by the next tile
+    }
+}
+
+// Moves, fills and publishes the rows of this block's leaders (after a halt:
+// only clears their chains).  Every thread of the block calls it.
+__device__ __forceinline__ void app_rows(const AppSide &a, uint32_t m, bool halted, RowShared &s) {
+    const uint2 rg = block_range(m);
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t t = rg.x; t < rg.y; t += blockDim.x) {
+        items_reset(s);
+        const uint32_t i = t + threadIdx.x;
+        const bool lead = i < rg.y && a.c.nxt[i] == 0u;
+        uint32_t x = 0, cnt = 0, head = 0, need = 0, off = 0;
+        uint2 d = make_uint2(0u, 0u);
+        if (lead) {
+            x = entry_row(a.E, i);
+            cnt = a.c.rowcnt[x];
+            head = a.c.rowhead[x];
+            a.c.rowcnt[x] = 0u;
+            a.c.rowhead[x] = 0u;
+        }
+        if (halted) continue;
+        if (lead) {
+            d = a.g.desc[x];
+            need = move_need(d.y, cnt, a.g.cap[x], a.slack);
+            off = need ? (uint32_t)atomicAdd(a.sc + S_CURSOR, (unsigned long long)need) : d.x;
+        }
+        const bool by_lane = lead && cnt <= kLaneChain && (!need || d.y <= kLaneRow);
+        const bool by_warp = lead && !by_lane && cnt <= kWarpChain && (!need || d.y <= kBigRow);
+        if (by_lane) {
+            if (need) copy_row<4>(a.g, d.x, off, d.y, 0u, 1u);
+            // the chain at once, then each entry to its rank among the
+            // (distinct) list indices
+            uint32_t idx[kLaneChain], y[kLaneChain];
+            float w[kLaneChain];
+            uint32_t k = head;
+#pragma unroll
+            for (uint32_t u = 0; u < kLaneChain; ++u)
+                if (u < cnt) {
+                    idx[u] = k - 1u;
+                    k = a.c.nxt[k - 1u];
+                }
+#pragma unroll
+            for (uint32_t u = 0; u < kLaneChain; ++u)
+                if (u < cnt) {
+                    y[u] = entry_col(a.E, idx[u]);
+                    w[u] = a.E.w[idx[u] >> 1];
+                }
+#pragma unroll
+            for (uint32_t u = 0; u < kLaneChain; ++u)
+                if (u < cnt) {
+                    uint32_t r = 0;
+#pragma unroll
+                    for (uint32_t v = 0; v < kLaneChain; ++v)
+                        if (v < cnt) r += idx[v] < idx[u] ? 1u : 0u;
+                    put_slot(a.g, off + d.y + r, y[u], w[u]);
+                }
+            publish_row(a, x, off, d.y, cnt, need);
+        }
+        if (lead && !by_lane) {
+            const RowItem it{x, cnt, head, d.x, d.y, off};
+            if (by_warp) item_for_warp(s, it);
+            else item_for_block(s, it);
+        }
+        __syncthreads();
+        const uint32_t nwarp = s.nwarp;
+        for (uint32_t q = threadIdx.x >> 5; q < nwarp; q += blockDim.x >> 5) {
+            const RowItem it = s.item[kOpThreads - 1u - q];
+            const bool mv = it.off != it.old_off;
+            if (mv) copy_row<4>(a.g, it.old_off, it.off, it.deg, lane, 32u);
+            uint32_t mine = ~0u, k = it.head;
+            for (uint32_t u = 0; u < it.cnt; ++u) {   // the chain: one load for the whole warp each
+                if (lane == u) mine = k - 1u;
+                k = a.c.nxt[k - 1u];
+            }
+            uint32_t r = 0;
+            for (uint32_t u = 0; u < it.cnt; ++u) r += __shfl_sync(kFull, mine, u) < mine ? 1u : 0u;
+            if (lane < it.cnt)
+                put_slot(a.g, it.off + it.deg + r, entry_col(a.E, mine), a.E.w[mine >> 1]);
+            if (lane == 0u)
+                publish_row(a, it.x, it.off, it.deg, it.cnt,
+                            mv ? move_need(it.deg, it.cnt, a.g.cap[it.x], a.slack) : 0u);
+        }
+        const uint32_t nbig = s.nbig;
+        for (uint32_t q = 0; q < nbig; ++q) {
+            const RowItem it = s.item[q];
+            const bool mv = it.off != it.old_off;
+            if (mv) copy_row<4>(a.g, it.old_off, it.off, it.deg, threadIdx.x, blockDim.x);
+            scan_entries(
+                a.c, m, it.x, it.cnt, s, [&](uint32_t e) { return make_uint2(a.E.src[e], a.E.dst[e]); },
+                [&](uint32_t k, uint32_t j) {
+                    put_slot(a.g, it.off + it.deg + k, entry_col(a.E, j), a.E.w[j >> 1]);
+                });
+            if (threadIdx.x == 0)
+                publish_row(a, it.x, it.off, it.deg, it.cnt,
+                            mv ? move_need(it.deg, it.cnt, a.g.cap[it.x], a.slack) : 0u);
+        }
+        __syncthreads();
+    }
+}
+
+// Sizing, reservation and rows of an append whose m half-edges are linked.
+// on_reserve runs in one thread once the space is reserved.  False: the
+// barrier gave up.
+template <class F>
+__device__ __forceinline__ bool app_commit(const AppSides &A, uint32_t m, const GridBar &bar,
+                                           unsigned long long *halt, unsigned long long code,
+                                           RowShared &s, F on_reserve) {
+    __shared__ unsigned long long s_need;
+    for (uint32_t k = 0; k < A.n; ++k) {
+        app_need(A.s[k], m, &s_need);
+        __syncthreads();
+    }
+    if (!grid_sync(bar, [&] {
+            if (reserve_moves(A, halt, code)) on_reserve();
+        }))
+        return false;
+    const bool halted = *(volatile unsigned long long *)halt != 0ull;
+    for (uint32_t k = 0; k < A.n; ++k) app_rows(A.s[k], m, halted, s);
+    return true;
+}
+
+// ------------------------------------------------------------------ delete
+
+// Endpoints of deletion e: min -> max (random_walk_decremental/gpu_graph.cuh:340-343).
+__device__ __forceinline__ uint2 del_ends(const uint32_t *src, const uint32_t *dst, uint32_t e) {
+    const uint32_t a = src[e], b = dst[e];
+    return make_uint2(min(a, b), max(a, b));
+}
+
+struct DelList {
+    Chains c;
+    const uint32_t *src, *dst;   // as given
+    uint32_t *tmp;               // 4n words: ordered entries of hub rows, of G then of H
+    unsigned long long *cursor;  // next free word of tmp
+};
+
+__device__ __forceinline__ uint32_t del_row(const DelList &D, uint32_t i) {
+    const uint2 v = del_ends(D.src, D.dst, i >> 1);
+    return (i & 1u) ? v.y : v.x;
+}
+__device__ __forceinline__ uint32_t del_col(const DelList &D, uint32_t i) {
+    const uint2 v = del_ends(D.src, D.dst, i >> 1);
+    return (i & 1u) ? v.x : v.y;
+}
+
+// Whether entry k is to be applied: with a mask, only if its edge was found
+// on both sides of it.
+__device__ __forceinline__ bool del_on(const uint8_t *mask, uint32_t k) {
+    return !mask || (mask[k & ~1u] && mask[k | 1u]);
+}
+
+// The row's last slot into the hole at `pos`.
+__device__ __forceinline__ void del_swap(const DevGraph &g, uint32_t off, uint32_t pos,
+                                         uint32_t deg) {
+    g.slots[off + pos] = g.slots[off + deg - 1u];
+    g.wts[off + pos] = g.wts[off + deg - 1u];
+}
+
+// One block removes a hub row's entries (or a long chain's).  They are put in
+// list order in tmp, then taken kTrackMax at a time: when a group's columns
+// are distinct and each occurs at most once in the row, one pass over the row
+// finds every target's slot and one thread applies the swaps in order,
+// following the single slot each swap moves (the row's last); otherwise every
+// deletion of the group is a block-wide search.  Both give what removing them
+// one by one gives.
+__device__ inline void block_del_row(const DevGraph &g, const DelList &D, uint32_t m, uint32_t x,
+                              uint32_t cnt, uint32_t head, const uint8_t *mask, uint8_t *found,
+                              RowShared &s) {
+    if (threadIdx.x == 0) s.best = (uint32_t)atomicAdd(D.cursor, (unsigned long long)cnt);
+    __syncthreads();
+    uint32_t *sorted = D.tmp + s.best;
+    __syncthreads();
+    if (cnt <= kWarpChain) {
+        if (threadIdx.x < 32u) {
+            uint32_t mine = ~0u, k = head;
+            for (uint32_t u = 0; u < cnt; ++u) {
+                if (threadIdx.x == u) mine = k - 1u;
+                k = D.c.nxt[k - 1u];
+            }
+            uint32_t r = 0;
+            for (uint32_t u = 0; u < cnt; ++u) r += __shfl_sync(kFull, mine, u) < mine ? 1u : 0u;
+            if (threadIdx.x < cnt) sorted[r] = mine;
+        }
+    } else {
+        scan_entries(
+            D.c, m, x, cnt, s, [&](uint32_t e) { return del_ends(D.src, D.dst, e); },
+            [&](uint32_t k, uint32_t j) { sorted[k] = j; });
+    }
+    __syncthreads();
+    const uint2 d = g.desc[x];
+    uint32_t deg = d.y;
+    for (uint32_t g0 = 0; g0 < cnt; g0 += kTrackMax) {
+        const uint32_t gc = min(kTrackMax, cnt - g0);
+        const uint32_t *grp = sorted + g0;
+        if (threadIdx.x == 0) {
+            s.ok = 1u;
+            s.nlive = 0u;
+        }
+        __syncthreads();
+        for (uint32_t a = threadIdx.x; a < gc; a += blockDim.x) {
+            const bool on = del_on(mask, grp[a]);
+            s.y[a] = on ? del_col(D, grp[a]) : ~0u;
+            s.pos[a] = ~0u;
+            s.occ[a] = 0u;
+            if (on) atomicAdd(&s.nlive, 1u);
+        }
+        __syncthreads();
+        const uint32_t nlive = s.nlive;   // masked-off entries (column ~0u) sort last
+        // the group's columns sorted (rank by count, ties by index), so each
+        // slot of the row finds its deletion by binary search
+        for (uint32_t a = threadIdx.x; a < gc; a += blockDim.x) {
+            const unsigned long long ka = ((unsigned long long)s.y[a] << 8) | a;
+            uint32_t r = 0;
+            for (uint32_t c = 0; c < gc; ++c) {
+                const unsigned long long kc = ((unsigned long long)s.y[c] << 8) | c;
+                r += kc < ka;
+                if (c < a && s.y[a] != ~0u && s.y[c] == s.y[a]) s.ok = 0u;
+            }
+            s.key[r] = ka;
+        }
+        __syncthreads();
+        const uint32_t *cols = reinterpret_cast<const uint32_t *>(g.slots + d.x);
+        if (s.ok && nlive) {
+            for (uint32_t base = 0; base < deg; base += kFindUnroll * blockDim.x) {
+                uint32_t v[kFindUnroll];   // a tile's loads are issued before any search
+#pragma unroll
+                for (uint32_t u = 0; u < kFindUnroll; ++u) {
+                    const uint32_t j = base + u * blockDim.x + threadIdx.x;
+                    v[u] = j < deg ? cols[2u * j] : ~0u;
+                }
+#pragma unroll
+                for (uint32_t u = 0; u < kFindUnroll; ++u) {
+                    const uint32_t col = v[u];
+                    if (col == ~0u) continue;
+                    uint32_t lo = 0, hi = nlive;
+                    while (lo < hi) {
+                        const uint32_t mid = (lo + hi) >> 1;
+                        if ((uint32_t)(s.key[mid] >> 8) < col) lo = mid + 1u;
+                        else hi = mid;
+                    }
+                    if (lo < nlive && (uint32_t)(s.key[lo] >> 8) == col) {
+                        const uint32_t a = (uint32_t)(s.key[lo] & 0xFFu);
+                        atomicMin(&s.pos[a], base + u * blockDim.x + threadIdx.x);
+                        atomicAdd(&s.occ[a], 1u);
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        for (uint32_t a = threadIdx.x; a < gc; a += blockDim.x)
+            if (s.occ[a] > 1u) s.ok = 0u;
+        __syncthreads();
+        if (s.ok) {
+            if (threadIdx.x == 0) {
+                for (uint32_t a = 0; a < gc; ++a) {
+                    const uint32_t p = s.pos[a];
+                    if (s.y[a] == ~0u || p == ~0u) continue;
+                    const uint32_t last = deg - 1u;
+                    del_swap(g, d.x, p, deg);
+                    --deg;
+                    found[grp[a]] = 1;
+                    if (p != last)   // the slot from `last` now sits at p
+                        for (uint32_t c = a + 1; c < gc; ++c)
+                            if (s.pos[c] == last) s.pos[c] = p;
+                }
+                s.best = deg;
+            }
+            __syncthreads();
+            deg = s.best;
+            __syncthreads();   // block_find and the next group write s.best
+        } else {
+            for (uint32_t a = 0; a < gc; ++a) {
+                if (s.y[a] == ~0u) continue;
+                const uint32_t j = block_find(g.slots, d.x, deg, s.y[a], &s.best);
+                if (j != ~0u) {
+                    if (threadIdx.x == 0) {
+                        del_swap(g, d.x, j, deg);
+                        found[grp[a]] = 1;
+                    }
+                    --deg;
+                    __syncthreads();   // the moved slot is visible to the next search
+                }
+            }
+        }
+        __syncthreads();   // every thread is done with the group's shared words
+    }
+    if (threadIdx.x == 0) g.desc[x] = make_uint2(d.x, deg);
+    __syncthreads();
+}
+
+// One warp removes a row's entries (at most kWarpChain), searching the row
+// once per deletion, 256 slots at a time.
+__device__ __forceinline__ void warp_del_row(const DevGraph &g, const DelList &D, const RowItem &it,
+                                             const uint8_t *mask, uint8_t *found, uint32_t lane) {
+    uint32_t k = it.head, mine = ~0u;
+    for (uint32_t u = 0; u < it.cnt; ++u) {
+        if (lane == u) mine = k - 1u;
+        k = D.c.nxt[k - 1u];
+    }
+    uint32_t r = 0;
+    for (uint32_t u = 0; u < it.cnt; ++u) r += __shfl_sync(kFull, mine, u) < mine ? 1u : 0u;
+    if (lane >= it.cnt) r = ~0u;
+    const uint32_t my_y = lane < it.cnt ? del_col(D, mine) : 0u;
+    const bool my_on = lane < it.cnt && del_on(mask, mine);
+    const uint32_t off = it.old_off;
+    uint32_t deg = it.deg;
+    for (uint32_t a = 0; a < it.cnt; ++a) {
+        const uint32_t who = __ffs(__ballot_sync(kFull, r == a)) - 1u;
+        if (!__shfl_sync(kFull, my_on ? 1u : 0u, who)) continue;
+        const uint32_t y = __shfl_sync(kFull, my_y, who);
+        uint32_t pos = ~0u;
+        for (uint32_t j0 = 0; j0 < deg && pos == ~0u; j0 += 256u) {
+            uint32_t cv[8];
+#pragma unroll
+            for (uint32_t u = 0; u < 8u; ++u) {
+                const uint32_t j = j0 + 32u * u + lane;
+                cv[u] = j < deg ? g.slots[off + j].x : ~0u;   // vertex ids are never ~0u
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < 8u; ++u) {
+                const unsigned hit = __ballot_sync(kFull, cv[u] == y);
+                if (hit && pos == ~0u) pos = j0 + 32u * u + (uint32_t)(__ffs(hit) - 1);
+            }
+        }
+        if (pos != ~0u) {
+            if (lane == who) {
+                del_swap(g, off, pos, deg);
+                found[mine] = 1;
+            }
+            --deg;
+            __syncwarp();   // the moved slot is visible to the next search
+        }
+    }
+    if (lane == 0u && deg != it.deg) g.desc[it.x] = make_uint2(off, deg);
+    __syncwarp();
+}
+
+// Removes the entries of this block's leaders' rows from g in list order
+// (mask as in del_on); found[i] = 1 for each entry that was there.  `clear`
+// empties the chains.  Every thread of the block calls it.
+__device__ __forceinline__ void del_rows(const DevGraph &g, const DelList &D, uint32_t m,
+                                         const uint8_t *mask, uint8_t *found, bool clear,
+                                         RowShared &s) {
+    const uint2 rg = block_range(m);
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t t = rg.x; t < rg.y; t += blockDim.x) {
+        items_reset(s);
+        const uint32_t i = t + threadIdx.x;
+        const bool lead = i < rg.y && D.c.nxt[i] == 0u;
+        uint32_t x = 0, cnt = 0, head = 0;
+        uint2 d = make_uint2(0u, 0u);
+        if (lead) {
+            x = del_row(D, i);
+            cnt = D.c.rowcnt[x];
+            head = D.c.rowhead[x];
+            d = g.desc[x];
+        }
+        const bool by_lane = lead && cnt <= kLaneChain && d.y <= kLaneRow;
+        // a warp searches the row once per deletion: worth it up to kWarpSearch
+        // slots looked at in all
+        const bool by_warp = lead && !by_lane && cnt <= kWarpChain && (uint64_t)d.y * cnt <= kWarpSearch;
+        if (by_lane) {
+            uint32_t idx[kLaneChain];
+            uint32_t k = head;
+#pragma unroll
+            for (uint32_t u = 0; u < kLaneChain; ++u) {
+                idx[u] = ~0u;
+                if (u < cnt) {
+                    idx[u] = k - 1u;
+                    k = D.c.nxt[k - 1u];
+                }
+            }
+            uint32_t deg = d.y, from = 0u;
+            for (uint32_t a = 0; a < cnt; ++a) {
+                k = ~0u;   // the next entry in list order
+#pragma unroll
+                for (uint32_t u = 0; u < kLaneChain; ++u)
+                    if (idx[u] >= from) k = min(k, idx[u]);
+                from = k + 1u;
+                if (!del_on(mask, k)) continue;
+                const uint32_t y = del_col(D, k);
+                // first slot holding y, eight columns loaded before they are
+                // compared (vertex ids are never ~0u)
+                uint32_t pos = ~0u;
+                for (uint32_t j0 = 0; j0 < deg && pos == ~0u; j0 += 8u) {
+                    uint32_t cv[8];
+#pragma unroll
+                    for (uint32_t u = 0; u < 8u; ++u)
+                        cv[u] = j0 + u < deg ? g.slots[d.x + j0 + u].x : ~0u;
+#pragma unroll
+                    for (uint32_t u = 0; u < 8u; ++u)
+                        if (pos == ~0u && cv[u] == y) pos = j0 + u;
+                }
+                if (pos != ~0u) {
+                    del_swap(g, d.x, pos, deg);
+                    --deg;
+                    found[k] = 1;
+                }
+            }
+            if (deg != d.y) g.desc[x] = make_uint2(d.x, deg);
+        }
+        if (lead && !by_lane) {
+            const RowItem it{x, cnt, head, d.x, d.y, 0u};
+            if (by_warp) item_for_warp(s, it);
+            else item_for_block(s, it);
+        }
+        if (lead && clear) {
+            D.c.rowcnt[x] = 0u;
+            D.c.rowhead[x] = 0u;
+        }
+        __syncthreads();
+        const uint32_t nwarp = s.nwarp;
+        for (uint32_t q = threadIdx.x >> 5; q < nwarp; q += blockDim.x >> 5)
+            warp_del_row(g, D, s.item[kOpThreads - 1u - q], mask, found, lane);
+        const uint32_t nbig = s.nbig;
+        for (uint32_t q = 0; q < nbig; ++q) {
+            const RowItem it = s.item[q];
+            block_del_row(g, D, m, it.x, it.cnt, it.head, mask, found, s);
+        }
+        __syncthreads();
+    }
+}
+
+// ------------------------------------------------------------- append kernel
+
+// One launch per commit: op.take(e) decides edge e (and writes its results),
+// bit k of its value appending the edge to side k; edges whose op.listed(e)
+// holds go to op.list(e, q) in list order, op.total(n) getting their number.
+//   uint32_t count()                  edges (device or host count)
+//   uint32_t take(uint32_t e)
+//   static constexpr bool kList       whether take's bit 0 also lists the edge
+template <class Op>
+__global__ void __launch_bounds__(kOpThreads, 2)
+k_append(const Op op, const __grid_constant__ AppSides A, GridBar bar, uint32_t *blk, unsigned long long *work,
+         unsigned long long *halt, unsigned long long code) {
+    __shared__ RowShared s;
+    if (*halt) return;
+    const uint32_t n = op.count();
+    const uint2 rg = block_range(n);
+    uint32_t mine = 0u;
+    for (uint32_t e = rg.x + threadIdx.x; e < rg.y; e += blockDim.x) {
+        const uint32_t take = op.take(e);
+        mine += take & 1u;
+        for (uint32_t k = 0; k < A.n; ++k) {
+            const AppSide &a = A.s[k];
+            const uint32_t u = a.E.src[e], v = a.E.dst[e];
+            const bool on = (take >> k) & 1u;
+            link_entry(a.c, 2u * e, u, on && u < a.g.n);
+            link_entry(a.c, 2u * e + 1u, v, on && v < a.g.n);
+        }
+    }
+    if (work && blockIdx.x == 0 && threadIdx.x == 0) *work = 0ull;   // the next walk's chunk counter
+    if constexpr (Op::kList) {
+        const uint32_t sum = block_sum(mine, s.warp);
+        if (threadIdx.x == 0) blk[blockIdx.x] = sum;
+    }
+    if (!grid_sync(bar)) return;
+    if constexpr (Op::kList) {
+        uint32_t base = blocks_before(blk, s.warp).x;
+        for (uint32_t t = rg.x; t < rg.y; t += blockDim.x) {
+            const uint32_t e = t + threadIdx.x;
+            const uint32_t v = e < rg.y && op.listed(e) ? 1u : 0u;
+            uint32_t total;
+            const uint32_t q = base + block_excl(v, s.warp, &total);
+            if (v) op.list(e, q);
+            base += total;
+        }
+        if (blockIdx.x == gridDim.x - 1u && threadIdx.x == 0) op.total(base);
+    }
+    app_commit(A, 2u * n, bar, halt, code, s, [] {});
+}
+
+// Workspace of a row operation on up to m half-edges.
+dyg_status rowops_ensure(dyg_graph *G, uint64_t m);
+GridBar grid_bar(dyg_graph *G);
+AppSide append_side(dyg_graph *G, const uint32_t *src, const uint32_t *dst, const float *w);
+
+template <class Op>
+dyg_status append_enqueue(const Op &op, uint32_t n_host, dyg_graph *GA, const EdgeList &EA,
+                          dyg_graph *GB, const EdgeList &EB, unsigned long long *work,
+                          unsigned long long *halt, unsigned long long code, cudaStream_t st) {
+    if (n_host == 0) return DYG_OK;
+    DYG_TRY(rowops_ensure(GA, 2ull * n_host));
+    AppSides A{};
+    A.s[0] = append_side(GA, EA.src, EA.dst, EA.w);
+    A.n = 1;
+    if (GB) {
+        DYG_TRY(rowops_ensure(GB, 2ull * n_host));
+        A.s[1] = append_side(GB, EB.src, EB.dst, EB.w);
+        A.n = 2;
+    }
+    const bool hubs = GA->long_rows || (GB && GB->long_rows);
+    return launch_phases<k_append<Op>>(op_blocks(2ull * n_host, hubs), st, op, A, grid_bar(GA),
+                                       ptr<uint32_t>(GA->ws.blk), work, halt, code);
+}
+
+}  // namespace dyg

@@ -842,8 +842,8 @@ dyg_status dyg_server_create(dyg_graph *G, dyg_graph *H, uint32_t n_graphs,
     *out = nullptr;
     if (!G || !H || !vertex_offsets || n_graphs == 0)
         return fail(nullptr, DYG_EINVAL, "NULL graph or offsets, or no graphs");
-    if (G->g.n != H->g.n || G->device != H->device)
-        return fail(nullptr, DYG_EINVAL, "G and H must have the same vertex count and device");
+    if (G == H || G->g.n != H->g.n || G->device != H->device)
+        return fail(nullptr, DYG_EINVAL, "G and H must be two handles with the same vertex count and device");
     for (uint32_t k = 0; k < n_graphs; ++k)
         if (vertex_offsets[k] > vertex_offsets[k + 1])
             return fail(nullptr, DYG_EINVAL, "vertex offsets must ascend");

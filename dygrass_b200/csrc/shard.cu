@@ -125,8 +125,8 @@ dyg_status dyg_incremental_commit_keys(dyg_graph *H, dyg_graph *G, const uint32_
         set_error("NULL argument");
         return DYG_EINVAL;
     }
-    if (G && (G->g.n != H->g.n || G->device != H->device)) {
-        set_error("G and H must have the same vertex count and device");
+    if (G && (G == H || G->g.n != H->g.n || G->device != H->device)) {
+        set_error("G and H must be two handles with the same vertex count and device");
         return DYG_EINVAL;
     }
     if (n == 0) return DYG_OK;
@@ -155,8 +155,9 @@ dyg_status dyg_incremental_commit_keys(dyg_graph *H, dyg_graph *G, const uint32_
         if (round == 0)
             DYG_TRY(validate_enqueue(halt, ptr<unsigned long long>(ws.scalars) + S_ERR, d_src, d_dst,
                                      d_w, n, H->g.n, st));
-        DYG_TRY(incr_commit_enqueue(H, G, d_src, d_dst, d_w, n, (const unsigned long long *)keys,
-                                    halt, 0, found_at, conductance, accepted, st));
+        DYG_TRY(incr_commit_enqueue(H, G, d_src, d_dst, d_w, n,
+                                    (unsigned long long *)const_cast<uint64_t *>(keys), false, halt, 0,
+                                    found_at, conductance, accepted, st));
         DYG_TRY(read_scalars2(H, G, st));
         const unsigned long long h = H->ws.host_scalars[S_HALT];
         if (!h) return DYG_OK;
@@ -177,8 +178,8 @@ dyg_status dyg_decremental_delete(dyg_graph *G, dyg_graph *H, const uint32_t *sr
         set_error("NULL argument");
         return DYG_EINVAL;
     }
-    if (G->g.n != H->g.n || G->device != H->device) {
-        set_error("G and H must have the same vertex count and device");
+    if (G == H || G->g.n != H->g.n || G->device != H->device) {
+        set_error("G and H must be two handles with the same vertex count and device");
         return DYG_EINVAL;
     }
     *n_walk = 0;
@@ -291,7 +292,7 @@ dyg_status dyg_decremental_commit_keys(dyg_graph *G, dyg_graph *H, const dyg_wal
     for (; round < 64; ++round) {
         DYG_TRY(clear_halt_of(G, st));
         DYG_TRY(decr_walk_enqueue(G, H, 0, n_walk, nullptr, *p, halt, 0, phase, status,
-                                  conductance, st, (const unsigned long long *)keys));
+                                  conductance, st, false, (const unsigned long long *)keys));
         DYG_TRY(read_scalars2(G, H, st));
         const unsigned long long h = ws.host_scalars[S_HALT];
         if (!h) {

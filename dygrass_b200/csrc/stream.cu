@@ -24,7 +24,8 @@
 #include <cub/cub.cuh>
 
 #include "dyg_internal.cuh"
-#include "scan.cuh"
+#include "gridsync.cuh"
+#include "rowops.cuh"
 
 namespace dyg {
 
@@ -258,81 +259,50 @@ __global__ void k_st_merge(const unsigned long long *halt, DevGraph G, DevGraph 
     }
 }
 
-// New edges in file order: the walk list (file orientation, stream weight)
-// and G's half-edges (src gets dst, dst gets src; merged weight), at the
-// scanned positions of the new-edge flags.
-struct StCompactOp {
+// New edges in file order: G's half-edges (src gets dst, dst gets src; merged
+// weight) and the walk list (file orientation, stream weight).
+struct NewEdgeOp {
+    static constexpr bool kList = true;
     const uint32_t *nflag, *src, *dst;
-    const float *w, *wapp;
+    const float *w;
+    uint32_t n;
     unsigned long long uid0;
     uint32_t *f_src, *f_dst;
     float *f_w;
     unsigned long long *f_uid;
-    uint32_t *f_idx, *hx, *hy;
-    float *hw;
-    uint32_t *counts;
-    __device__ uint32_t load(uint32_t i) const { return nflag[i]; }
-    __device__ void store(uint32_t i, uint32_t q, uint32_t v) const {
-        if (!v) return;
-        const uint32_t u = src[i], x = dst[i];
-        f_src[q] = u;
-        f_dst[q] = x;
+    uint32_t *f_idx, *counts;
+    __device__ uint32_t count() const { return n; }
+    __device__ uint32_t take(uint32_t i) const { return nflag[i]; }
+    __device__ bool listed(uint32_t i) const { return nflag[i] != 0u; }
+    __device__ void list(uint32_t i, uint32_t q) const {
+        f_src[q] = src[i];
+        f_dst[q] = dst[i];
         f_w[q] = w[i];
         f_uid[q] = uid0 + i;
         f_idx[q] = i;
-        const float wa = wapp[i];
-        hx[2 * q] = u;
-        hy[2 * q] = x;
-        hw[2 * q] = wa;
-        hx[2 * q + 1] = x;
-        hy[2 * q + 1] = u;
-        hw[2 * q + 1] = wa;
     }
-    __device__ void last(uint32_t total) const {
-        counts[C_WALKLIST] = total;
-        counts[C_GHALF] = 2u * total;
-    }
+    __device__ void total(uint32_t n_new) const { counts[C_WALKLIST] = n_new; }
 };
 
-__global__ void k_st_range(const unsigned long long *halt, const uint32_t *F_dev, uint32_t f0,
-                           uint32_t nf, uint32_t *out) {
-    if (HALTED(halt)) return;
-    const uint32_t F = *F_dev;
-    *out = F > f0 ? min(F - f0, nf) : 0u;
-}
-
 // Chunk results: found_at / conductance by file index, and the accepted
-// edges (no walker connected them) to H's half-edge list in chunk order;
-// entries past the chunk's device count are not accepted.
+// edges (no walker connected them) to H in chunk order.  Keys are zeroed
+// behind the decode for the next chunk's walks.
 struct StAcceptOp {
-    const unsigned long long *keys;
-    const uint32_t *f_idx, *cnt, *f_src, *f_dst;
-    const float *f_w;
+    static constexpr bool kList = false;
+    WalkJob job;
+    unsigned long long *keys;
+    const uint32_t *f_idx;
     int32_t *status;
     float *cond;
-    uint32_t *hx, *hy;
-    float *hw;
-    uint32_t *counts;
-    __device__ uint32_t load(uint32_t f) const {
-        if (f >= *cnt) return 0u;
+    __device__ uint32_t count() const { return job_count(job); }
+    __device__ uint32_t take(uint32_t f) const {
         const unsigned long long k = keys[f];
+        if (k) keys[f] = 0ull;
         const uint32_t i = f_idx[f];
         status[i] = key_found(k);
         cond[i] = k ? __uint_as_float((uint32_t)(k >> 32)) : 0.f;
         return k ? 0u : 1u;
     }
-    __device__ void store(uint32_t f, uint32_t q, uint32_t v) const {
-        if (!v) return;
-        const uint32_t u = f_src[f], x = f_dst[f];
-        const float ww = f_w[f];
-        hx[2 * q] = u;
-        hy[2 * q] = x;
-        hw[2 * q] = ww;
-        hx[2 * q + 1] = x;
-        hy[2 * q + 1] = u;
-        hw[2 * q + 1] = ww;
-    }
-    __device__ void last(uint32_t total) const { counts[C_ACCEPTED] = 2u * total; }
 };
 
 // Files of up to kSortSmall edges are grouped by one block: a bitonic sort of
@@ -455,7 +425,7 @@ uint32_t key_bits(uint32_t nv) {
 
 // Probe, sort, merge and compact an insert file (no reservation: never halts).
 dyg_status insert_prep_enqueue(dyg_graph *G, dyg_graph *H, const uint32_t *src,
-                               const uint32_t *dst, const float *w, uint32_t n, uint64_t uid0,
+                               const uint32_t *dst, const float *w, uint32_t n,
                                unsigned long long *halt, int32_t *status, float *cond,
                                cudaStream_t st) {
     Workspace &ws = G->ws;
@@ -463,7 +433,6 @@ dyg_status insert_prep_enqueue(dyg_graph *G, dyg_graph *H, const uint32_t *src,
     unsigned long long *key = ptr<unsigned long long>(ws.st_key), *skey = key + n;
     uint32_t *val = ptr<uint32_t>(ws.st_val), *sval = val + n;
     uint32_t *nflag = ptr<uint32_t>(ws.flags);
-    uint32_t *counts = ptr<uint32_t>(ws.counts);
     unsigned long long *sc = ptr<unsigned long long>(ws.scalars);
     const bool big_ok = G->long_rows || H->long_rows;
     if (big_ok) DYG_CUDA(cudaMemsetAsync(sc + S_NBIG, 0, sizeof(unsigned long long), st));
@@ -494,48 +463,40 @@ dyg_status insert_prep_enqueue(dyg_graph *G, dyg_graph *H, const uint32_t *src,
                                                 ptr<uint4>(ws.st_pos), w, nflag,
                                                 ptr<float>(ws.st_wapp), status, cond);
     count_launch();
-    const StCompactOp op{nflag, src, dst, w, ptr<float>(ws.st_wapp), (unsigned long long)uid0,
-                         ptr<uint32_t>(ws.f_src), ptr<uint32_t>(ws.f_dst), ptr<float>(ws.f_w),
-                         ptr<unsigned long long>(ws.f_uid), ptr<uint32_t>(ws.f_idx),
-                         ptr<uint32_t>(ws.hx), ptr<uint32_t>(ws.hy), ptr<float>(ws.hw), counts};
-    DYG_TRY(scan_op(ws, op, n, nullptr, halt, st));
     DYG_CUDA(cudaGetLastError());
     return DYG_OK;
 }
 
-dyg_status insert_gappend_enqueue(dyg_graph *G, uint32_t n, unsigned long long *halt,
-                                  cudaStream_t st) {
+dyg_status insert_gappend_enqueue(dyg_graph *G, const uint32_t *src, const uint32_t *dst,
+                                  const float *w, uint32_t n, uint64_t uid0,
+                                  unsigned long long *halt, cudaStream_t st) {
     Workspace &ws = G->ws;
-    AppendList L{ptr<uint32_t>(ws.hx), ptr<uint32_t>(ws.hy), ptr<float>(ws.hw),
-                 ptr<uint32_t>(ws.counts) + C_GHALF, 2u * n};
-    return append_enqueue(G, L, nullptr, nullptr, halt, halt_code(0, (uint32_t)kHaltArena, 1), st);
+    const NewEdgeOp op{ptr<uint32_t>(ws.flags), src, dst, w, n, (unsigned long long)uid0,
+                       ptr<uint32_t>(ws.f_src), ptr<uint32_t>(ws.f_dst), ptr<float>(ws.f_w),
+                       ptr<unsigned long long>(ws.f_uid), ptr<uint32_t>(ws.f_idx),
+                       ptr<uint32_t>(ws.counts)};
+    return append_enqueue(op, n, G, EdgeList{src, dst, ptr<float>(ws.st_wapp)}, nullptr, EdgeList{},
+                          nullptr, halt, halt_code(0, (uint32_t)kHaltArena, 1), st);
 }
 
 // Walks chunk c (walk-list entries [c*chunk, c*chunk + nc)) on H and appends
-// its accepted edges to H.
+// its accepted edges to H.  walk_ready: the chunk before left H's keys and
+// chunk counter zero.
 dyg_status insert_chunk_enqueue(dyg_graph *G, dyg_graph *H, uint32_t c, uint32_t chunk,
                                 uint32_t nc, const dyg_walk_params &p, unsigned long long *halt,
-                                int32_t *status, float *cond, cudaStream_t st) {
+                                int32_t *status, float *cond, bool walk_ready, cudaStream_t st) {
     Workspace &wg = G->ws, &wh = H->ws;
     const uint32_t f0 = c * chunk;
-    uint32_t *gcounts = ptr<uint32_t>(wg.counts), *hcounts = ptr<uint32_t>(wh.counts);
-    k_st_range<<<1, 1, 0, st>>>(halt, gcounts + C_WALKLIST, f0, nc, gcounts + C_RANGE);
-    count_launch();
-    const uint32_t *cnt = gcounts + C_RANGE;
     const uint32_t *fsrc = ptr<uint32_t>(wg.f_src) + f0, *fdst = ptr<uint32_t>(wg.f_dst) + f0;
     const float *fw = ptr<float>(wg.f_w) + f0;
     unsigned long long *keys = ptr<unsigned long long>(wh.keys);
-    DYG_CUDA(cudaMemsetAsync(keys, 0, sizeof(unsigned long long) * nc, st));
-    WalkJob job{halt, fsrc, fdst, fw, ptr<unsigned long long>(wg.f_uid) + f0, 0ull, cnt, nc,
-                kDomainIncr};
-    DYG_TRY(launch_walk(H, job, p, true, keys, st));
-    const StAcceptOp op{keys, ptr<uint32_t>(wg.f_idx) + f0, cnt, fsrc, fdst, fw, status, cond,
-                        ptr<uint32_t>(wh.hx), ptr<uint32_t>(wh.hy), ptr<float>(wh.hw), hcounts};
-    DYG_TRY(scan_op(wh, op, nc, nullptr, halt, st));
-    DYG_CUDA(cudaGetLastError());
-    AppendList L{ptr<uint32_t>(wh.hx), ptr<uint32_t>(wh.hy), ptr<float>(wh.hw),
-                 hcounts + C_ACCEPTED, 2u * nc};
-    return append_enqueue(H, L, nullptr, nullptr, halt,
+    if (!walk_ready) DYG_CUDA(cudaMemsetAsync(keys, 0, sizeof(unsigned long long) * nc, st));
+    const WalkJob job{halt, fsrc, fdst, fw, ptr<unsigned long long>(wg.f_uid) + f0, 0ull,
+                      ptr<uint32_t>(wg.counts) + C_WALKLIST, nc, kDomainIncr, f0};
+    DYG_TRY(launch_walk(H, job, p, true, keys, st, walk_ready));
+    const StAcceptOp op{job, keys, ptr<uint32_t>(wg.f_idx) + f0, status, cond};
+    return append_enqueue(op, nc, H, EdgeList{fsrc, fdst, fw}, nullptr, EdgeList{},
+                          ptr<unsigned long long>(wh.scalars) + S_WORK, halt,
                           halt_code(c + 1, (uint32_t)kHaltArena, 0), st);
 }
 
@@ -565,38 +526,29 @@ dyg_status insert_file_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, cons
     DYG_TRY(ensure(wg.st_val, sizeof(uint32_t) * (size_t)n * 2));
     DYG_TRY(ensure(wg.st_pos, sizeof(uint4) * (size_t)n));
     DYG_TRY(ensure(wg.st_wapp, sizeof(float) * (size_t)n));
-    DYG_TRY(ensure(wg.big, sizeof(uint4) * (size_t)n * 2));   // probe, then the G append
-    DYG_TRY(ensure(wg.dtmp, sizeof(uint32_t) * (size_t)n * 4));
-    DYG_TRY(ensure(wg.rank, sizeof(uint32_t) * (size_t)n * 2));
-    DYG_TRY(ensure(wg.lneed, sizeof(uint32_t) * (size_t)n * 2));
+    DYG_TRY(ensure(wg.big, sizeof(uint4) * (size_t)n));
     DYG_TRY(ensure(wg.flags, sizeof(uint32_t) * (size_t)n));
-    DYG_TRY(ensure(wg.pos, sizeof(uint32_t) * (size_t)n));
     DYG_TRY(ensure(wg.f_src, sizeof(uint32_t) * (size_t)n));
     DYG_TRY(ensure(wg.f_dst, sizeof(uint32_t) * (size_t)n));
     DYG_TRY(ensure(wg.f_w, sizeof(float) * (size_t)n));
     DYG_TRY(ensure(wg.f_uid, sizeof(unsigned long long) * (size_t)n));
     DYG_TRY(ensure(wg.f_idx, sizeof(uint32_t) * (size_t)n));
-    DYG_TRY(ensure(wg.hx, sizeof(uint32_t) * (size_t)n * 2));
-    DYG_TRY(ensure(wg.hy, sizeof(uint32_t) * (size_t)n * 2));
-    DYG_TRY(ensure(wg.hw, sizeof(float) * (size_t)n * 2));
     DYG_TRY(ensure(wh.keys, sizeof(unsigned long long) * (size_t)nc_max));
-    DYG_TRY(ensure(wh.hx, sizeof(uint32_t) * (size_t)nc_max * 2));
-    DYG_TRY(ensure(wh.hy, sizeof(uint32_t) * (size_t)nc_max * 2));
-    DYG_TRY(ensure(wh.hw, sizeof(float) * (size_t)nc_max * 2));
     unsigned long long *halt = ptr<unsigned long long>(wg.scalars) + S_HALT;
     DYG_TRY(clear_halt(G, st));
     if (check_inputs)
         DYG_TRY(validate_enqueue(halt, ptr<unsigned long long>(wg.scalars) + S_ERR, src, dst, w, n,
                                  G->g.n, st));
-    DYG_TRY(insert_prep_enqueue(G, H, src, dst, w, n, uid0, halt, status, cond, st));
+    DYG_TRY(insert_prep_enqueue(G, H, src, dst, w, n, halt, status, cond, st));
     const uint32_t nchunks = (uint32_t)(((uint64_t)n + chunk - 1) / chunk);
     uint32_t start = 0;   // 0 = G append, c + 1 = chunk c
     for (int round = 0; round < 64; ++round) {
-        if (start == 0) DYG_TRY(insert_gappend_enqueue(G, n, halt, st));
-        for (uint32_t c = start ? start - 1 : 0; c < nchunks; ++c) {
+        if (start == 0) DYG_TRY(insert_gappend_enqueue(G, src, dst, w, n, uid0, halt, st));
+        const uint32_t c0 = start ? start - 1 : 0;
+        for (uint32_t c = c0; c < nchunks; ++c) {
             const uint32_t f0 = c * chunk;
             const uint32_t nc = n - f0 < chunk ? n - f0 : chunk;
-            DYG_TRY(insert_chunk_enqueue(G, H, c, chunk, nc, p, halt, status, cond, st));
+            DYG_TRY(insert_chunk_enqueue(G, H, c, chunk, nc, p, halt, status, cond, c > c0, st));
         }
         DYG_TRY(read_scalars2(G, H, st));
         const unsigned long long h = wg.host_scalars[S_HALT];
@@ -639,7 +591,7 @@ dyg_status delete_file_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, cons
             const uint32_t f0 = c * chunk;
             const uint32_t nc = n - f0 < chunk ? n - f0 : chunk;
             DYG_TRY(decr_walk_enqueue(G, H, f0, nc, ptr<uint32_t>(ws.counts) + C_FILTERED, p, halt,
-                                      c, c == c_start ? ph_start : 0, status, cond, st));
+                                      c, c == c_start ? ph_start : 0, status, cond, st, true));
         }
         DYG_TRY(read_scalars2(G, H, st));
         const unsigned long long h = ws.host_scalars[S_HALT];

@@ -442,7 +442,7 @@ __global__ void __launch_bounds__(kWalkThreads, WEIGHTED ? 3 : 6) k_walk(WalkArg
     if (a.job.halt && *a.job.halt) return;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lt_mask = (1u << lane) - 1u;
-    const uint32_t n = a.job.n_dev ? *a.job.n_dev : a.job.n_host;
+    const uint32_t n = job_count(a.job);
     const uint32_t CW = a.chunk;                // walkers per chunk (divides walkers)
     const uint32_t cpe = a.walkers / CW;        // chunks per edge
     const uint32_t cpe_sh = (cpe & (cpe - 1u)) ? 32u : (uint32_t)(__ffs(cpe) - 1);
@@ -619,7 +619,7 @@ __global__ void k_winner_paths(DevGraph g, WalkJob job, uint32_t max_steps, uint
                                uint32_t *ps, int32_t *plen, unsigned long long *scalars) {
     if (job.halt && *job.halt) return;
     const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t n = job.n_dev ? *job.n_dev : job.n_host;
+    const uint32_t n = job_count(job);
     if (f >= n) return;
     const unsigned long long k = keys[f];
     if (!k) {
@@ -673,7 +673,7 @@ k_winner_paths_weighted(DevGraph g, WalkJob job, uint32_t max_steps, uint2 key,
     if (job.halt && *job.halt) return;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t f = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t n = job.n_dev ? *job.n_dev : job.n_host;
+    const uint32_t n = job_count(job);
     if (f >= n) return;   // whole warps leave together
     const unsigned long long k = keys[f];
     if (!k) {
@@ -716,51 +716,6 @@ k_winner_paths_weighted(DevGraph g, WalkJob job, uint32_t max_steps, uint2 key,
         plen[f] = found;
         if (found != key_found(k)) atomicOr(scalars + S_ERR, (unsigned long long)kErrPath);
     }
-}
-
-// 2-step fallback walks from both endpoints of each edge that found no path
-// (random_walk_decremental/main.cu:243-290, with the second step reading the
-// row of the vertex the walker stands on).  Candidate pair 2i, 2i+1 of item
-// i = (q * 2 + side) * hw + j is (s0, x1), (x1, x2); x = ~0u marks none.
-__global__ void k_fallback(DevGraph g, const unsigned long long *halt, const uint32_t *f_src,
-                           const uint32_t *f_dst, const unsigned long long *f_uid,
-                           const uint32_t *nop, const uint32_t *n_nop_dev, uint32_t hw, uint2 key,
-                           const uint32_t *base_dev, uint32_t *cx, uint32_t *cy, float *cw) {
-    if (halt && *halt) return;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t per = 2u * hw;
-    if (i >= *n_nop_dev * per) return;
-    const uint32_t b = *base_dev;
-    cx += b;
-    cy += b;
-    cw += b;
-    const uint32_t q = i / per, rem = i - q * per, side = rem / hw, j = rem - side * hw;
-    const uint32_t f = nop[q];
-    const uint32_t s0 = side ? f_dst[f] : f_src[f];
-    const unsigned long long uid = f_uid[f];
-    const uint4 rb = philox4x32_10(make_uint4(0u, side * hw + j, (uint32_t)uid,
-                                              ctr3_of(uid, kDomainHeur)), key);
-    uint32_t x1 = ~0u, x2 = ~0u;
-    float w1 = 0.f, w2 = 0.f;
-    const uint2 d0 = __ldg(g.desc + s0);
-    if (d0.y != 0u) {
-        const uint32_t i0 = d0.x + rb.x % d0.y;
-        x1 = __ldg(&g.slots[i0].x);
-        w1 = __ldg(g.wts + i0);
-        const uint2 d1 = __ldg(g.desc + x1);
-        if (d1.y != 0u) {
-            uint32_t i1 = d1.x + rb.y % d1.y;
-            if (__ldg(&g.slots[i1].x) == s0) i1 = d1.x + d1.y - 1u;
-            x2 = __ldg(&g.slots[i1].x);
-            w2 = __ldg(g.wts + i1);
-        }
-    }
-    cx[2 * i] = (x1 == ~0u) ? ~0u : s0;
-    cy[2 * i] = x1;
-    cw[2 * i] = w1;
-    cx[2 * i + 1] = (x2 == ~0u) ? ~0u : x1;
-    cy[2 * i + 1] = x2;
-    cw[2 * i + 1] = w2;
 }
 
 // Walkers handed to a warp at a time: 32 by default, so that the 512 walks
@@ -847,7 +802,7 @@ static void launch_walk_any(const WalkArgs &a, bool incremental, bool wtd, cudaS
 }
 
 dyg_status launch_walk(dyg_graph *G, const WalkJob &job, const dyg_walk_params &p, bool incremental,
-                       unsigned long long *keys, cudaStream_t st) {
+                       unsigned long long *keys, cudaStream_t st, bool counter_zero) {
     WalkArgs a{};
     a.g = G->g;
     a.job = job;
@@ -860,7 +815,7 @@ dyg_status launch_walk(dyg_graph *G, const WalkJob &job, const dyg_walk_params &
     a.key = make_uint2((uint32_t)p.seed, (uint32_t)(p.seed >> 32));
     a.keys = keys;
     a.scalars = ptr<unsigned long long>(G->ws.scalars);
-    DYG_CUDA(cudaMemsetAsync(a.scalars + S_WORK, 0, sizeof(unsigned long long), st));
+    if (!counter_zero) DYG_CUDA(cudaMemsetAsync(a.scalars + S_WORK, 0, sizeof(unsigned long long), st));
     ProfScope prof(incremental ? 0 : 1, st);
     launch_walk_any(a, incremental, p.transition == DYG_TRANSITION_WEIGHTED, st);
     count_launch();
@@ -908,25 +863,6 @@ dyg_status launch_winner_paths(dyg_graph *G, const WalkJob &job, const dyg_walk_
     else
         k_winner_paths<false><<<grid, threads, 0, st>>>(G->g, job, p.max_steps, key, keys, stride,
                                                         path_v, path_s, path_len, sc);
-    count_launch();
-    DYG_CUDA(cudaGetLastError());
-    return DYG_OK;
-}
-
-dyg_status launch_fallback_walks(dyg_graph *G, const unsigned long long *halt,
-                                 const uint32_t *f_src, const uint32_t *f_dst,
-                                 const unsigned long long *f_uid, const uint32_t *nop,
-                                 const uint32_t *n_nop_dev, uint32_t n_nop_max,
-                                 const dyg_walk_params &p, const uint32_t *base_dev, uint32_t *cx,
-                                 uint32_t *cy, float *cw, cudaStream_t st) {
-    const uint64_t items = (uint64_t)n_nop_max * 2u * p.heuristic_walkers;
-    if (items == 0) return DYG_OK;
-    const uint2 key = make_uint2((uint32_t)p.seed, (uint32_t)(p.seed >> 32));
-    const int threads = 128;
-    ProfScope prof(2, st);
-    k_fallback<<<(unsigned)((items + threads - 1) / threads), threads, 0, st>>>(
-        G->g, halt, f_src, f_dst, f_uid, nop, n_nop_dev, p.heuristic_walkers, key, base_dev, cx, cy,
-        cw);
     count_launch();
     DYG_CUDA(cudaGetLastError());
     return DYG_OK;

@@ -1,0 +1,79 @@
+"""Row operations at the sizes where a row's work changes hands (one lane, a
+warp, the block; chains followed or scanned for; deletion groups of a hub
+row; lists over one block and over several), against the CPU oracle."""
+import numpy as np
+import pytest
+
+from test_gpu_parity import dyg, run_incr_both, same_graph  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+def star(n, leaves, rng):
+    """A path over all vertices and `leaves` edges from vertex 0, shuffled."""
+    s = np.concatenate([np.arange(n - 1), np.zeros(leaves, np.int64)]).astype(np.uint32)
+    d = np.concatenate([np.arange(1, n), 2 + np.arange(leaves)]).astype(np.uint32)
+    flip = rng.random(len(s)) < 0.5
+    s, d = np.where(flip, d, s), np.where(flip, s, d)
+    o = rng.permutation(len(s))
+    return s[o], d[o], rng.uniform(0.5, 2.0, len(s)).astype(np.float32)
+
+
+# entries one row gets in a batch: lane chains end at 4, warp chains at 32;
+# spread = further edges, one per row, so that the list needs several blocks
+@pytest.mark.parametrize("k,leaves,spread", [(1, 0, 0), (4, 40, 0), (5, 3, 0), (32, 300, 600), (33, 0, 0),
+                                             (33, 30, 3000), (257, 300, 0), (900, 20, 5000)])
+def test_append_chains(dyg, oracle, k, leaves, spread):  # noqa: F811
+    rng = np.random.default_rng(k + leaves + spread)
+    n = 1000 + 2 * spread
+    hs, hd, hw = star(n, leaves, rng)
+    e = np.concatenate([np.stack([np.zeros(k, np.int64), 2 + rng.integers(0, n - 2, k)], 1),
+                        np.stack([1000 + np.arange(spread), 1000 + spread + np.arange(spread)], 1)])
+    e = e[rng.permutation(len(e))]
+    flip = rng.random(len(e)) < 0.5
+    es = np.where(flip, e[:, 1], e[:, 0]).astype(np.uint32)
+    ed = np.where(flip, e[:, 0], e[:, 1]).astype(np.uint32)
+    ew = rng.uniform(0.5, 2.0, len(e)).astype(np.float32)
+    p = dyg.WalkParams.make(threshold=3.0, walkers=32, max_steps=8)
+    run_incr_both(dyg, oracle, n, hs, hd, hw, es, ed, ew, p, batch_size=len(e), with_g=(hs, hd, hw))
+
+
+# deletions of one row: lane rows end at 32 slots, warps look at 4096 slots in
+# all, hub rows take deletions in groups of 128 (repeats force single searches)
+@pytest.mark.parametrize("k,leaves,repeat,spread", [(1, 28, 0, 0), (4, 40, 1, 0), (5, 20, 0, 0), (32, 127, 0, 0),
+                                                    (32, 140, 2, 0), (33, 60, 0, 900), (128, 300, 0, 0),
+                                                    (129, 300, 3, 0), (500, 9000, 0, 2000)])
+def test_delete_chains(dyg, oracle, k, leaves, repeat, spread):  # noqa: F811
+    rng = np.random.default_rng(k + leaves + spread)
+    n = max(1000, leaves + 10) + 2 * spread
+    gs, gd, gw = star(n, leaves, rng)
+    hub = np.flatnonzero((gs == 0) | (gd == 0))
+    dele = rng.choice(hub, min(k, len(hub)), replace=False)
+    rest = rng.choice(np.setdiff1d(np.arange(len(gs)), hub), spread, replace=False)
+    dele = rng.permutation(np.concatenate([dele, dele[:repeat], rest]))
+    in_h = rng.random(len(gs)) < 0.7
+    hs, hd, hw = gs[in_h], gd[in_h], gw[in_h]
+    G, H = dyg.Graph.from_edges(n, gs, gd, gw), dyg.Graph.from_edges(n, hs, hd, hw)
+    Go, Ho = oracle.OGraph(n, gs, gd, gw), oracle.OGraph(n, hs, hd, hw)
+    p = dyg.WalkParams.make(walkers=32, max_steps=12, heuristic_walkers=3)
+    r = dyg.decremental_batch(G, H, gs[dele], gd[dele], p)
+    st, cd, rx, ry, rk, _ = oracle.decremental(Go, Ho, gs[dele], gd[dele], p, batch_size=len(dele))
+    assert np.array_equal(r.status, st)
+    assert np.array_equal(r.conductance.view(np.uint32), cd.view(np.uint32))
+    assert np.array_equal(r.rec_src, rx) and np.array_equal(r.rec_dst, ry)
+    assert np.array_equal(r.rec_kind, rk)
+    same_graph(G, Go)
+    same_graph(H, Ho)
+
+
+def test_one_handle_for_both_graphs_is_refused(dyg):  # noqa: F811
+    """The append keeps one set of chains per handle."""
+    g = dyg.Graph.from_edges(4, np.array([0, 1], np.uint32), np.array([1, 2], np.uint32),
+                             np.ones(2, np.float32))
+    one = (np.array([0], np.uint32), np.array([3], np.uint32))
+    p = dyg.WalkParams.make(walkers=32)
+    for call in (lambda: dyg.incremental_batch(g, *one, np.ones(1, np.float32), p, G=g),
+                 lambda: dyg.decremental_batch(g, g, *one, p),
+                 lambda: dyg.stream_file(g, g, 1, *one, None, p)):
+        with pytest.raises(dyg.DygError):
+            call()
