@@ -91,12 +91,17 @@ __host__ __device__ __forceinline__ int32_t key_found(unsigned long long k) {
 }
 
 // Fixed-point weight of the weight-proportional mode (exact w * 2^32,
-// truncated) so that prefix sums are associative and match the host.
+// truncated) so that prefix sums are associative and match the host: the
+// 24-bit significand shifted by the exponent.  Weights are positive; from
+// 2^32 on (infinity included) the value is all ones.
 __device__ __forceinline__ unsigned long long wq(float w) {
-    const double v = (double)w * 4294967296.0;
-    if (!(v > 0.0)) return 0ull;
-    if (v >= 18446744073709551615.0) return 0xFFFFFFFFFFFFFFFFull;
-    return (unsigned long long)v;
+    const uint32_t b = __float_as_uint(w);
+    const uint32_t ex = b >> 23;   // sign bit 0
+    const unsigned long long m = (b & 0x7FFFFFu) | 0x800000u;
+    // w = m * 2^(ex - 150), so w * 2^32 = m * 2^(ex - 118); below 2^-32 it is 0
+    if (ex < 95u || (int)b < 0) return 0ull;
+    if (ex >= 159u) return 0xFFFFFFFFFFFFFFFFull;
+    return ex >= 118u ? m << (ex - 118u) : m >> (118u - ex);
 }
 __device__ __forceinline__ unsigned long long mul_hi32(uint32_t r, unsigned long long total) {
     // floor(r * total / 2^32) for a 96-bit product
@@ -147,6 +152,16 @@ __device__ __forceinline__ uint32_t block_find(const uint2 *slots, uint32_t off,
 
 // ------------------------------------------------------------- workspace
 // Device scratch owned by a graph handle, grown on demand.
+// Lookup index of a graph's rows longer than kIdxRow for the weight-proportional
+// walks (k_index, walk.cu), rebuilt for every launch: rbase[v] is the word
+// offset of row v's region in `words`, 0 for a row without one.  A region is a
+// hash table of 2^k >= 2 deg words (position + 1 of a column, 0 empty) and the
+// row's deg inclusive prefix sums of wq (two words each).
+struct RowIndex {
+    const uint32_t *rbase;   // null: no row has an index
+    const uint32_t *words;
+};
+
 struct Buf {
     void *p = nullptr;
     size_t bytes = 0;
@@ -179,6 +194,7 @@ struct Workspace {
     Buf st_wapp;                              // stream file: G weight of each new edge
     Buf big;                                  // stream file: uint4 per long-row search
     Buf s_uid;                                // staged per-edge update ids
+    Buf ix_base, ix_list, ix_words;           // row index of the weighted walks
     Buf scalars;                              // u64 scalars (see Scalar)
     Buf counts;                               // u32 counts (see Count)
     unsigned long long *host_scalars = nullptr;   // pinned mirror
@@ -203,7 +219,9 @@ enum Scalar : int {
     S_LONG = 13,      // set by an append that made a row longer than kBigRow
     S_SCAN = 14,      // tile tickets of the single-pass scan (accumulating)
     S_BAR = 15,       // grid barrier: arrivals (low word), generation (high word)
-    S_NSCALARS = 16
+    S_IDX = 16,       // row index: next free word
+    S_IDXN = 17,      // row index: rows for a warp (low word), for a block (high word)
+    S_NSCALARS = 18
 };
 enum Count : int {
     C_FILTERED = 0,   // decremental: edges to walk
@@ -296,13 +314,19 @@ __device__ __forceinline__ uint32_t job_count(const WalkJob &j) {
 // counter_zero: the kernel's chunk counter is known to be zero (the commit
 // of the batch before reset it), so no memset precedes the launch.
 dyg_status launch_walk(dyg_graph *G, const WalkJob &job, const dyg_walk_params &p, bool incremental,
-                       unsigned long long *keys, cudaStream_t st, bool counter_zero = false);
+                       unsigned long long *keys, const RowIndex &ix, cudaStream_t st,
+                       bool counter_zero = false);
 dyg_status launch_walk_scalars(const DevGraph &g, const WalkJob &job, const dyg_walk_params &p,
                                bool incremental, unsigned long long *keys,
                                unsigned long long *scalars, cudaStream_t st);
+// The row index for weighted walks on G as it is now; empty for a uniform
+// transition or a graph without hub rows.
+dyg_status index_enqueue(dyg_graph *G, const dyg_walk_params &p, const unsigned long long *halt,
+                         RowIndex *out, cudaStream_t st);
 dyg_status launch_winner_paths(dyg_graph *G, const WalkJob &job, const dyg_walk_params &p,
                                const unsigned long long *keys, uint32_t n_max, uint32_t path_stride,
-                               uint32_t *path_v, uint32_t *path_s, int32_t *path_len, cudaStream_t st);
+                               uint32_t *path_v, uint32_t *path_s, int32_t *path_len, const RowIndex &ix,
+                               cudaStream_t st);
 // --- capi.cu
 // After a run: DYG_OK, or the error the kernels flagged in G's scalars (last
 // read by the run), which are cleared.

@@ -514,7 +514,9 @@ static dyg_status incr_enqueue(dyg_graph *H, dyg_graph *G, const uint32_t *src, 
     unsigned long long *keys = ptr<unsigned long long>(H->ws.keys);
     if (!walk_ready) DYG_CUDA(cudaMemsetAsync(keys, 0, sizeof(unsigned long long) * n, st));
     WalkJob job{halt, src, dst, w, uids, (unsigned long long)uid0, nullptr, n, kDomainIncr, 0u};
-    DYG_TRY(launch_walk(H, job, p, true, keys, st, walk_ready));
+    RowIndex ix{};
+    DYG_TRY(index_enqueue(H, p, halt, &ix, st));
+    DYG_TRY(launch_walk(H, job, p, true, keys, ix, st, walk_ready));
     return incr_commit_enqueue(H, G, src, dst, w, n, keys, true, halt, batch, found, cond, acc, st);
 }
 
@@ -638,12 +640,14 @@ dyg_status decr_walk_enqueue(dyg_graph *G, dyg_graph *H, uint32_t f0, uint32_t n
     a.code_arena = halt_code(batch, (uint32_t)kHaltArena, 1);
     if (phase0 == 0) {
         // walks on the updated G (main.cu:392, 420)
+        RowIndex ix{};   // of the walks, and of the replays of their winners
+        DYG_TRY(index_enqueue(G, p, halt, &ix, st));
         if (!keys_given) {
             if (!walk_ready) DYG_CUDA(cudaMemsetAsync(own, 0, sizeof(unsigned long long) * n, st));
-            DYG_TRY(launch_walk(G, job, p, false, own, st, walk_ready));
+            DYG_TRY(launch_walk(G, job, p, false, own, ix, st, walk_ready));
         }
         DYG_TRY(launch_winner_paths(G, job, p, a.keys, n, stride, ptr<uint32_t>(ws.path_v),
-                                    ptr<uint32_t>(ws.path_s), ptr<int32_t>(ws.path_len), st));
+                                    ptr<uint32_t>(ws.path_s), ptr<int32_t>(ws.path_len), ix, st));
     }
     // blocks for what a batch usually brings: a few candidates per deletion
     return launch_phases<k_recover>(op_blocks(4ull * n, H->long_rows), st, a, grid_bar(G));

@@ -109,7 +109,9 @@ dyg_status dyg_walk_keys(dyg_graph *X, const uint32_t *src, const uint32_t *dst,
                 d_ids ? (const unsigned long long *)d_ids + lo : nullptr,
                 (unsigned long long)(first_update_id + lo), nullptr, hi - lo,
                 incremental ? kDomainIncr : kDomainDecr};
-    DYG_TRY(launch_walk(X, job, *p, incremental != 0, k, st));
+    RowIndex ix{};
+    DYG_TRY(index_enqueue(X, *p, job.halt, &ix, st));
+    DYG_TRY(launch_walk(X, job, *p, incremental != 0, k, ix, st));
     DYG_TRY(read_scalars(X, st));
     if (ws.host_scalars[S_HALT]) return rejected_inputs(X, st);
     return DYG_OK;
@@ -244,7 +246,9 @@ dyg_status dyg_decremental_walk_keys(dyg_graph *G, uint32_t lo, uint32_t hi,
     DYG_CUDA(cudaMemsetAsync(k, 0, sizeof(unsigned long long) * (hi - lo), st));
     WalkJob job{nullptr, ptr<uint32_t>(ws.f_src) + lo, ptr<uint32_t>(ws.f_dst) + lo, nullptr,
                 ptr<unsigned long long>(ws.f_uid) + lo, 0ull, nullptr, hi - lo, kDomainDecr};
-    DYG_TRY(launch_walk(G, job, *p, false, k, st));
+    RowIndex ix{};
+    DYG_TRY(index_enqueue(G, *p, nullptr, &ix, st));
+    DYG_TRY(launch_walk(G, job, *p, false, k, ix, st));
     DYG_CUDA(cudaStreamSynchronize(st));
     return DYG_OK;
 }

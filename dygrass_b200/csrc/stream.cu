@@ -493,7 +493,9 @@ dyg_status insert_chunk_enqueue(dyg_graph *G, dyg_graph *H, uint32_t c, uint32_t
     if (!walk_ready) DYG_CUDA(cudaMemsetAsync(keys, 0, sizeof(unsigned long long) * nc, st));
     const WalkJob job{halt, fsrc, fdst, fw, ptr<unsigned long long>(wg.f_uid) + f0, 0ull,
                       ptr<uint32_t>(wg.counts) + C_WALKLIST, nc, kDomainIncr, f0};
-    DYG_TRY(launch_walk(H, job, p, true, keys, st, walk_ready));
+    RowIndex ix{};
+    DYG_TRY(index_enqueue(H, p, halt, &ix, st));
+    DYG_TRY(launch_walk(H, job, p, true, keys, ix, st, walk_ready));
     const StAcceptOp op{job, keys, ptr<uint32_t>(wg.f_idx) + f0, status, cond};
     return append_enqueue(op, nc, H, EdgeList{fsrc, fdst, fw}, nullptr, EdgeList{},
                           ptr<unsigned long long>(wh.scalars) + S_WORK, halt,

@@ -25,6 +25,7 @@
 #include <atomic>
 
 #include "dyg_internal.cuh"
+#include "gridsync.cuh"
 
 namespace dyg {
 
@@ -84,6 +85,7 @@ constexpr int kWalkThreads = 256;
 struct WalkArgs {
     DevGraph g;
     WalkJob job;
+    RowIndex ix;      // weighted walks
     uint32_t walkers, max_steps;
     uint32_t prune;
     uint32_t prune_every;   // iterations between reads of the edge's best (a power of two)
@@ -139,55 +141,71 @@ __device__ __forceinline__ int finish_move(Walker &s, uint2 sl, uint32_t at, boo
 // whose inclusive prefix of fixed-point weights wq(w) exceeds
 // floor(r * total / 2^32).  ~0u when total is 0; *picked receives the chosen
 // slot.  The row is read kPickGroup slots at a time with the group's loads
-// issued together (the second pass reads the groups again, from L1 mostly),
-// so a row of up to kPickGroup slots costs two rounds of loads, not 2 deg.
-constexpr uint32_t kPickGroup = 4;
+// issued together.  A row of one group (every lattice row) is read once, its
+// weights staying in registers for the choice; a longer row is read again.
+// (8,000 insertions and 12,000 deletions on a 40^3 mesh: 8.99 -> 7.68 ms with
+// this and wq in integers, against groups of four read twice and wq in FP64.)
+constexpr uint32_t kPickGroup = 8;
+
+struct PickGroup {
+    uint2 c[kPickGroup];
+    unsigned long long q[kPickGroup];   // 0 outside the row and for `ex`
+};
+__device__ __forceinline__ void pick_load(PickGroup &p, const uint2 *__restrict__ slots,
+                                          const float *__restrict__ wts, uint32_t lo,
+                                          uint32_t left, uint32_t ex, bool has_ex) {
+    float w[kPickGroup];
+#pragma unroll
+    for (uint32_t u = 0; u < kPickGroup; ++u) {
+        p.c[u] = u < left ? __ldg(slots + lo + u) : make_uint2(0u, 0u);
+        w[u] = u < left ? __ldg(wts + lo + u) : 0.f;
+    }
+#pragma unroll
+    for (uint32_t u = 0; u < kPickGroup; ++u)
+        p.q[u] = (u >= left || (has_ex && p.c[u].x == ex)) ? 0ull : wq(w[u]);
+}
+// The group's first slot whose prefix exceeds target (~0u: none); *acc is
+// carried over the groups.
+__device__ __forceinline__ uint32_t pick_in_group(const PickGroup &p, unsigned long long target,
+                                                  unsigned long long *acc, uint2 *picked) {
+    uint32_t at = ~0u;
+#pragma unroll
+    for (uint32_t u = 0; u < kPickGroup; ++u) {
+        *acc += p.q[u];
+        // a slot of weight 0 never is the first: the prefix did not grow
+        // (after a wrap past 2^64 it could still exceed the target, and the
+        // slots that count as absent are skipped)
+        if (at == ~0u && p.q[u] != 0ull && *acc > target) {
+            at = u;
+            *picked = p.c[u];
+        }
+    }
+    return at;
+}
+
 __device__ __forceinline__ uint32_t lane_pick_weighted(const uint2 *__restrict__ slots,
                                                        const float *__restrict__ wts, uint32_t lo,
                                                        uint32_t deg, uint32_t ex, bool has_ex,
                                                        uint32_t r, uint2 *picked) {
+    PickGroup p;
+    pick_load(p, slots, wts, lo, deg, ex, has_ex);
     unsigned long long total = 0ull;
-    for (uint32_t j0 = 0; j0 < deg; j0 += kPickGroup) {
-        uint2 c[kPickGroup];
-        float w[kPickGroup];
 #pragma unroll
-        for (uint32_t u = 0; u < kPickGroup; ++u) {
-            const bool in = j0 + u < deg;
-            c[u] = in ? __ldg(slots + lo + j0 + u) : make_uint2(0u, 0u);
-            w[u] = in ? __ldg(wts + lo + j0 + u) : 0.f;
-        }
+    for (uint32_t u = 0; u < kPickGroup; ++u) total += p.q[u];
+    for (uint32_t j0 = kPickGroup; j0 < deg; j0 += kPickGroup) {
+        pick_load(p, slots, wts, lo + j0, deg - j0, ex, has_ex);
 #pragma unroll
-        for (uint32_t u = 0; u < kPickGroup; ++u)
-            if (j0 + u < deg && !(has_ex && c[u].x == ex)) total += wq(w[u]);
+        for (uint32_t u = 0; u < kPickGroup; ++u) total += p.q[u];
     }
     if (total == 0ull) return ~0u;
     const unsigned long long target = mul_hi32(r, total);
     unsigned long long acc = 0ull;
-    uint32_t last = deg;
-    uint2 last_sl = make_uint2(0u, 0u);
     for (uint32_t j0 = 0; j0 < deg; j0 += kPickGroup) {
-        uint2 c[kPickGroup];
-        float w[kPickGroup];
-#pragma unroll
-        for (uint32_t u = 0; u < kPickGroup; ++u) {
-            const bool in = j0 + u < deg;
-            c[u] = in ? __ldg(slots + lo + j0 + u) : make_uint2(0u, 0u);
-            w[u] = in ? __ldg(wts + lo + j0 + u) : 0.f;
-        }
-#pragma unroll
-        for (uint32_t u = 0; u < kPickGroup; ++u) {
-            if (j0 + u >= deg || (has_ex && c[u].x == ex)) continue;
-            acc += wq(w[u]);
-            last = j0 + u;
-            last_sl = c[u];
-            if (acc > target) {
-                *picked = last_sl;
-                return lo + last;
-            }
-        }
+        if (deg > kPickGroup) pick_load(p, slots, wts, lo + j0, deg - j0, ex, has_ex);
+        const uint32_t u = pick_in_group(p, target, &acc, picked);
+        if (u != ~0u) return lo + j0 + u;
     }
-    *picked = last_sl;
-    return lo + last;
+    return ~0u;
 }
 
 // The uniform move from row d (deg = d.y, past the dead-end test) with draw r.
@@ -382,12 +400,204 @@ __device__ __forceinline__ uint32_t warp_pick_weighted(const uint2 *__restrict__
     return ~0u;
 }
 
+// ------------------------------------------------------------ row index
+// On a graph with hub rows nearly every weighted move is at one, and a warp
+// reading such a row for one lane after another bounds the walk: 9.87 ms for
+// the deletion walks of a 1,000-edge R-MAT file (scale 13).  A walker needs
+// two things of the row: the position and weight of the column it came from,
+// and the first prefix sum above its target.  k_index tabulates both for
+// every row longer than kIdxRow, once per launch of walks (the rows do not
+// change while they walk), and each lane then chooses by itself: one hash
+// lookup and one binary search.  Its cost is a pass over the long rows (40 us
+// a launch there, of which the walk was 9.87 ms and is 1.15 ms; the whole six
+// files 15.2 -> 4.4 ms).  It is built whenever the graph has hub rows (over
+// kBigRow slots): even a single edge's walkers scan more than it costs.  Rows with a repeated column, or whose sum
+// wraps past 2^64, get no index and are searched by the warp as before.
+constexpr uint32_t kIdxRow = 32;        // longer rows are indexed (kCoopRow: the lane scans up to it)
+constexpr uint32_t kIdxBlockRow = 1024; // ... by a whole block from here on
+constexpr uint32_t kIdxTile = 8;        // slots per thread of a block's tile
+
+__device__ __forceinline__ uint32_t idx_bits(uint32_t deg) { return 32u - __clz(2u * deg - 1u); }
+__device__ __forceinline__ uint32_t idx_hash(uint32_t col, uint32_t bits) {
+    return (col * 0x9E3779B1u) >> (32u - bits);
+}
+
+// The choice of lane_pick_weighted from row v's index region.
+__device__ __forceinline__ uint32_t index_pick(const uint2 *__restrict__ slots,
+                                               const float *__restrict__ wts,
+                                               const uint32_t *__restrict__ region, uint32_t lo,
+                                               uint32_t deg, uint32_t ex, bool has_ex, uint32_t r) {
+    const uint32_t bits = idx_bits(deg);
+    const unsigned long long *pre = reinterpret_cast<const unsigned long long *>(region + (1u << bits));
+    unsigned long long total = __ldg(pre + deg - 1u), e = 0ull;
+    uint32_t pos = deg;
+    if (has_ex) {
+        uint32_t h = idx_hash(ex, bits);
+        while (true) {
+            const uint32_t t = __ldg(region + h);
+            if (t == 0u) break;
+            if (__ldg(&slots[lo + t - 1u].x) == ex) {
+                pos = t - 1u;
+                e = wq(__ldg(wts + lo + pos));
+                break;
+            }
+            h = (h + 1u) & ((1u << bits) - 1u);
+        }
+    }
+    total -= e;
+    if (total == 0ull) return ~0u;
+    const unsigned long long target = mul_hi32(r, total);
+    // first slot whose prefix without `ex` exceeds the target; the slot of
+    // `ex` itself leaves that prefix as it was, so it is never the first
+    uint32_t a = 0u, b = deg - 1u;
+    while (a < b) {
+        const uint32_t mid = (a + b) >> 1;
+        const unsigned long long v = __ldg(pre + mid) - (mid >= pos ? e : 0ull);
+        if (v > target) b = mid;
+        else a = mid + 1u;
+    }
+    return lo + a;
+}
+
+struct IndexArgs {
+    DevGraph g;
+    uint32_t *rbase, *list, *words;
+    uint32_t cap;                    // words
+    unsigned long long *cursor;      // next free word (from 2 on: 0 means no region)
+    unsigned long long *counts;      // S_IDXN
+    const unsigned long long *halt;
+};
+
+// Hash insert of slot j's column; true if the column is there already.
+__device__ __forceinline__ bool idx_insert(const IndexArgs &a, uint32_t *tab, uint32_t bits,
+                                           uint32_t lo, uint32_t j, uint32_t col) {
+    uint32_t h = idx_hash(col, bits);
+    while (true) {
+        const uint32_t old = atomicCAS(tab + h, 0u, j + 1u);
+        if (old == 0u) return false;
+        if (a.g.slots[lo + old - 1u].x == col) return true;
+        h = (h + 1u) & ((1u << bits) - 1u);
+    }
+}
+
+__global__ void __launch_bounds__(kOpThreads, 2) k_index(const __grid_constant__ IndexArgs a, GridBar bar) {
+    __shared__ unsigned long long s_sum[kOpThreads / 32];
+    __shared__ uint32_t s_bad;
+    if (a.halt && *a.halt) return;
+    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    // regions, and the lists of rows: for a warp from the front, for a block
+    // from the back
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < a.g.n; v += gridDim.x * blockDim.x) {
+        const uint32_t deg = a.g.desc[v].y;
+        uint32_t base = 0u;
+        if (deg > kIdxRow) {
+            const unsigned long long want = (1ull << idx_bits(deg)) + 2ull * deg;
+            const unsigned long long at = atomicAdd(a.cursor, want) + 2ull;
+            if (at + want <= a.cap) {
+                base = (uint32_t)at;
+                if (deg <= kIdxBlockRow) a.list[(uint32_t)atomicAdd(a.counts, 1ull)] = v;
+                else a.list[a.g.n - 1u - (uint32_t)(atomicAdd(a.counts, 1ull << 32) >> 32)] = v;
+            }
+        }
+        a.rbase[v] = base;
+    }
+    if (!grid_sync(bar)) return;
+    const unsigned long long both = __ldcg(a.counts);
+    const uint32_t n_warp = (uint32_t)both, n_block = (uint32_t)(both >> 32);
+    for (uint32_t q = blockIdx.x; q < n_block; q += gridDim.x) {
+        const uint32_t v = a.list[a.g.n - 1u - q];
+        const uint2 d = a.g.desc[v];
+        const uint32_t bits = idx_bits(d.y);
+        uint32_t *tab = a.words + a.rbase[v];
+        unsigned long long *pre = reinterpret_cast<unsigned long long *>(tab + (1u << bits));
+        for (uint32_t h = threadIdx.x; h < (1u << bits); h += blockDim.x) tab[h] = 0u;
+        if (threadIdx.x == 0) s_bad = 0u;
+        __syncthreads();
+        bool bad = false;
+        unsigned long long carry = 0ull;
+        for (uint32_t t0 = 0; t0 < d.y; t0 += kIdxTile * blockDim.x) {
+            const uint32_t j0 = t0 + kIdxTile * threadIdx.x;
+            unsigned long long q8[kIdxTile], run = 0ull;
+#pragma unroll
+            for (uint32_t u = 0; u < kIdxTile; ++u) {
+                q8[u] = j0 + u < d.y ? wq(a.g.wts[d.x + j0 + u]) : 0ull;
+                if (j0 + u < d.y) bad |= idx_insert(a, tab, bits, d.x, j0 + u, a.g.slots[d.x + j0 + u].x);
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < kIdxTile; ++u) {
+                run += q8[u];
+                bad |= run < q8[u];
+                q8[u] = run;
+            }
+            unsigned long long incl = run;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned long long x = __shfl_up_sync(kFull, incl, o);
+                if (lane >= (uint32_t)o) {
+                    incl += x;
+                    bad |= incl < x;
+                }
+            }
+            if (lane == 31u) s_sum[wid] = incl;
+            __syncthreads();
+            unsigned long long before = carry, all = carry;
+            for (uint32_t k = 0; k < blockDim.x >> 5; ++k) {
+                const unsigned long long x = s_sum[k];
+                all += x;
+                bad |= all < x;
+                if (k < wid) before += x;
+            }
+            before += incl - run;
+#pragma unroll
+            for (uint32_t u = 0; u < kIdxTile; ++u)
+                if (j0 + u < d.y) pre[j0 + u] = before + q8[u];
+            carry = all;
+            __syncthreads();
+        }
+        if (bad) s_bad = 1u;
+        __syncthreads();
+        if (threadIdx.x == 0 && s_bad) a.rbase[v] = 0u;
+        __syncthreads();
+    }
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < n_warp; q += warps) {
+        const uint32_t v = a.list[q];
+        const uint2 d = a.g.desc[v];
+        const uint32_t bits = idx_bits(d.y);
+        uint32_t *tab = a.words + a.rbase[v];
+        unsigned long long *pre = reinterpret_cast<unsigned long long *>(tab + (1u << bits));
+        for (uint32_t h = lane; h < (1u << bits); h += 32u) tab[h] = 0u;
+        __syncwarp();
+        bool bad = false;
+        unsigned long long carry = 0ull;
+        for (uint32_t j0 = 0; j0 < d.y; j0 += 32u) {
+            const uint32_t j = j0 + lane;
+            unsigned long long incl = j < d.y ? wq(a.g.wts[d.x + j]) : 0ull;
+            if (j < d.y) bad |= idx_insert(a, tab, bits, d.x, j, a.g.slots[d.x + j].x);
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned long long x = __shfl_up_sync(kFull, incl, o);
+                if (lane >= (uint32_t)o) {
+                    incl += x;
+                    bad |= incl < x;
+                }
+            }
+            const unsigned long long at = carry + incl;
+            bad |= at < carry;
+            if (j < d.y) pre[j] = at;
+            carry = __shfl_sync(kFull, at, 31);
+        }
+        bad = __any_sync(kFull, bad);
+        if (lane == 0u && bad) a.rbase[v] = 0u;
+    }
+}
+
 // One move of every active lane's walker, with rows longer than kCoopRow
-// searched by the whole warp (all 32 lanes call this).  Returns the move's
-// result for active lanes.
+// chosen through their index or, without one, searched by the whole warp (all
+// 32 lanes call this).  Returns the move's result for active lanes.
 template <bool INCR>
 __device__ __forceinline__ int step_weighted_warp(Walker &s, bool active, const DevGraph &g,
-                                                  uint32_t max_steps, float thr, uint2 key,
+                                                  const RowIndex &ix, uint32_t max_steps, float thr, uint2 key,
                                                   unsigned long long *seg, uint32_t lane,
                                                   bool *moved, uint2 *taken, uint32_t *taken_at) {
     *moved = false;
@@ -406,7 +616,10 @@ __device__ __forceinline__ int step_weighted_warp(Walker &s, bool active, const 
     uint2 sl = make_uint2(0u, 0u);
     const bool own_row = pick && d.y <= kCoopRow;   // chosen by this lane, slot in hand
     if (own_row) at = lane_pick_weighted(g.slots, g.wts, d.x, d.y, s.prev, !first, r, &sl);
-    unsigned coop = __ballot_sync(kFull, pick && d.y > kCoopRow);
+    uint32_t base = 0u;
+    if (pick && !own_row && ix.rbase) base = __ldg(ix.rbase + s.cur);
+    if (base) at = index_pick(g.slots, g.wts, ix.words + base, d.x, d.y, s.prev, !first, r);
+    unsigned coop = __ballot_sync(kFull, pick && !own_row && !base);
     while (coop) {
         const uint32_t L = __ffs(coop) - 1u;
         coop &= coop - 1u;
@@ -547,7 +760,7 @@ __global__ void __launch_bounds__(kWalkThreads, WEIGHTED ? 3 : 6) k_walk(WalkArg
             uint2 taken;
             uint32_t taken_at;
             if constexpr (WEIGHTED) {
-                r = step_weighted_warp<INCR>(s, active, a.g, a.max_steps, a.threshold, a.key,
+                r = step_weighted_warp<INCR>(s, active, a.g, a.ix, a.max_steps, a.threshold, a.key,
                                              s_seg + (threadIdx.x >> 5) * kSegs, lane, &moved,
                                              &taken, &taken_at);
             } else if (MOVES == 4 && active) {
@@ -666,7 +879,7 @@ __global__ void k_winner_paths(DevGraph g, WalkJob job, uint32_t max_steps, uint
 // time).
 constexpr int kReplayThreads = 128;
 __global__ void __launch_bounds__(kReplayThreads)
-k_winner_paths_weighted(DevGraph g, WalkJob job, uint32_t max_steps, uint2 key,
+k_winner_paths_weighted(DevGraph g, WalkJob job, RowIndex ix, uint32_t max_steps, uint2 key,
                         const unsigned long long *keys, uint32_t stride, uint32_t *pv, uint32_t *ps,
                         int32_t *plen, unsigned long long *scalars) {
     __shared__ unsigned long long s_seg[(kReplayThreads / 32) * kSegs];
@@ -703,7 +916,7 @@ k_winner_paths_weighted(DevGraph g, WalkJob job, uint32_t max_steps, uint2 key,
         bool moved;
         uint2 taken;
         uint32_t taken_at;
-        r = step_weighted_warp<false>(s, lane == 0u, g, max_steps, 0.f, key, seg, lane, &moved,
+        r = step_weighted_warp<false>(s, lane == 0u, g, ix, max_steps, 0.f, key, seg, lane, &moved,
                                       &taken, &taken_at);
         r = __shfl_sync(kFull, r, 0);
         if (lane == 0u && moved && at < stride) {
@@ -801,10 +1014,46 @@ static void launch_walk_any(const WalkArgs &a, bool incremental, bool wtd, cudaS
     }
 }
 
+// Words the index may take: what rows filling the whole arena would need
+// (fewer than 4 deg table words and 2 deg prefix words each), at most 2 GB;
+// rows that do not fit stay without an index.
+constexpr uint64_t kIdxWordsMax = 1ull << 29;
+
+dyg_status index_enqueue(dyg_graph *G, const dyg_walk_params &p, const unsigned long long *halt,
+                         RowIndex *out, cudaStream_t st) {
+    *out = RowIndex{};
+    if (p.transition != DYG_TRANSITION_WEIGHTED || !G->long_rows) return DYG_OK;
+    Workspace &ws = G->ws;
+    const uint32_t n = G->g.n;
+    uint64_t words = 6ull * G->g.arena_cap + 2ull;
+    if (words > kIdxWordsMax) words = kIdxWordsMax;
+    DYG_TRY(ensure(ws.ix_base, sizeof(uint32_t) * (size_t)n));
+    DYG_TRY(ensure(ws.ix_list, sizeof(uint32_t) * (size_t)n));
+    DYG_TRY(ensure(ws.ix_words, sizeof(uint32_t) * (size_t)words));
+    unsigned long long *sc = ptr<unsigned long long>(ws.scalars);
+    DYG_CUDA(cudaMemsetAsync(sc + S_IDX, 0, 2 * sizeof(unsigned long long), st));
+    IndexArgs a{};
+    a.g = G->g;
+    a.rbase = ptr<uint32_t>(ws.ix_base);
+    a.list = ptr<uint32_t>(ws.ix_list);
+    a.words = ptr<uint32_t>(ws.ix_words);
+    a.cap = (uint32_t)words;
+    a.cursor = sc + S_IDX;
+    a.counts = sc + S_IDXN;
+    a.halt = halt;
+    uint32_t *bw = reinterpret_cast<uint32_t *>(sc + S_BAR);
+    const GridBar bar{bw, bw + 1, sc + S_ERR};
+    DYG_TRY(launch_phases<k_index>(2u * (uint32_t)num_sms(), st, a, bar));
+    *out = RowIndex{a.rbase, a.words};
+    return DYG_OK;
+}
+
 dyg_status launch_walk(dyg_graph *G, const WalkJob &job, const dyg_walk_params &p, bool incremental,
-                       unsigned long long *keys, cudaStream_t st, bool counter_zero) {
+                       unsigned long long *keys, const RowIndex &ix, cudaStream_t st,
+                       bool counter_zero) {
     WalkArgs a{};
     a.g = G->g;
+    a.ix = ix;
     a.job = job;
     a.walkers = p.walkers;
     a.max_steps = p.max_steps;
@@ -849,7 +1098,8 @@ dyg_status launch_walk_scalars(const DevGraph &g, const WalkJob &job, const dyg_
 
 dyg_status launch_winner_paths(dyg_graph *G, const WalkJob &job, const dyg_walk_params &p,
                                const unsigned long long *keys, uint32_t n_max, uint32_t stride,
-                               uint32_t *path_v, uint32_t *path_s, int32_t *path_len, cudaStream_t st) {
+                               uint32_t *path_v, uint32_t *path_s, int32_t *path_len, const RowIndex &ix,
+                               cudaStream_t st) {
     if (n_max == 0) return DYG_OK;
     const uint2 key = make_uint2((uint32_t)p.seed, (uint32_t)(p.seed >> 32));
     const int threads = 128;
@@ -858,7 +1108,7 @@ dyg_status launch_winner_paths(dyg_graph *G, const WalkJob &job, const dyg_walk_
     ProfScope prof(2, st);
     if (p.transition == DYG_TRANSITION_WEIGHTED)
         k_winner_paths_weighted<<<(unsigned)(((uint64_t)n_max * 32 + kReplayThreads - 1) / kReplayThreads),
-                                  kReplayThreads, 0, st>>>(G->g, job, p.max_steps, key, keys, stride,
+                                  kReplayThreads, 0, st>>>(G->g, job, ix, p.max_steps, key, keys, stride,
                                                            path_v, path_s, path_len, sc);
     else
         k_winner_paths<false><<<grid, threads, 0, st>>>(G->g, job, p.max_steps, key, keys, stride,

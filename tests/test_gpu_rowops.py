@@ -77,3 +77,37 @@ def test_one_handle_for_both_graphs_is_refused(dyg):  # noqa: F811
                  lambda: dyg.stream_file(g, g, 1, *one, None, p)):
         with pytest.raises(dyg.DygError):
             call()
+
+
+# weighted walks on graphs with hub rows: rows indexed by a warp (33..1024
+# slots) and by a block, a tile of a block's prefix pass (4096 slots), and
+# rows that must not be indexed (a repeated column, sums past 2^64)
+@pytest.mark.parametrize("leaves,repeat,huge", [(256, 0, 0), (1021, 0, 0), (1022, 0, 0), (1023, 2, 0), (4094, 0, 0),
+                                                (4095, 0, 0), (9000, 0, 0), (5000, 3, 0), (700, 0, 4), (5000, 0, 4)])
+def test_weighted_hub_rows(dyg, oracle, leaves, repeat, huge):  # noqa: F811
+    rng = np.random.default_rng(leaves + repeat + huge)
+    n = leaves + 40
+    hs, hd, hw = star(n, leaves, rng)
+    # a second row between the lane's and the block's lengths
+    far = 20 + rng.choice(n - 30, 33, replace=False)
+    far = far[far != 10]
+    more = rng.choice(np.flatnonzero((hs == 0) | (hd == 0)), repeat, replace=False)
+    hs = np.concatenate([hs, np.full(len(far), 10, np.uint32), hs[more]]).astype(np.uint32)
+    hd = np.concatenate([hd, far, hd[more]]).astype(np.uint32)
+    hw = np.concatenate([hw, rng.uniform(0.5, 2.0, len(far) + repeat)]).astype(np.float32)
+    hw[rng.choice(np.flatnonzero((hs == 0) | (hd == 0)), huge, replace=False)] = 3e9
+    es = rng.integers(0, n, 24).astype(np.uint32)
+    ed = ((es + 1 + rng.integers(0, n - 1, 24)) % n).astype(np.uint32)
+    ew = rng.uniform(0.01, 0.05, 24).astype(np.float32)
+    p = dyg.WalkParams.make(threshold=100.0, walkers=64, max_steps=30, transition=1)
+    run_incr_both(dyg, oracle, n, hs, hd, hw, es, ed, ew, p, batch_size=12)
+    G, H = dyg.Graph.from_edges(n, hs, hd, hw), dyg.Graph.from_edges(n, hs, hd, hw)
+    Go, Ho = oracle.OGraph(n, hs, hd, hw), oracle.OGraph(n, hs, hd, hw)
+    dele = rng.choice(len(hs), 40, replace=False)
+    r = dyg.decremental_batch(G, H, hs[dele], hd[dele], p)
+    st, cd, rx, ry, rk, _ = oracle.decremental(Go, Ho, hs[dele], hd[dele], p, batch_size=40)
+    assert np.array_equal(r.status, st)
+    assert np.array_equal(r.conductance.view(np.uint32), cd.view(np.uint32))
+    assert np.array_equal(r.rec_src, rx) and np.array_equal(r.rec_dst, ry)
+    same_graph(G, Go)
+    same_graph(H, Ho)
