@@ -188,6 +188,7 @@ struct Workspace {
     Buf rk2;
     Buf nxt, dtmp;                            // row operations: per-entry chain link / ordered run
     Buf rowcnt, rowhead;                      // row operations: per-row entries / last entry + 1
+    Buf rowlist;                              // row operations: rows for warps and blocks
     Buf blk;                                  // row operations: per-block words
     Buf st_key, st_val;                       // stream file: (min, max) keys and indices, sorted
     Buf st_pos;                               // stream file: uint4 slot positions in G and H
@@ -219,9 +220,10 @@ enum Scalar : int {
     S_LONG = 13,      // set by an append that made a row longer than kBigRow
     S_SCAN = 14,      // tile tickets of the single-pass scan (accumulating)
     S_BAR = 15,       // grid barrier: arrivals (low word), generation (high word)
+    S_ITEMS = 18,     // row operations: rows for a block (low word), for a warp (high word)
     S_IDX = 16,       // row index: next free word
     S_IDXN = 17,      // row index: rows for a warp (low word), for a block (high word)
-    S_NSCALARS = 18
+    S_NSCALARS = 19
 };
 enum Count : int {
     C_FILTERED = 0,   // decremental: edges to walk

@@ -90,7 +90,8 @@ struct IncrOp {
 //           the rows of G and H have the same entries, so one set of chains
 //           serves both
 //   G, H    rows edited in list order, H's entries only where G found the
-//           edge on both sides
+//           edge on both sides; the rows of G that are not for a lane are
+//           listed first and get a phase of their own when there are any
 //   list    deletion e found in G and in H goes to the walk list at its
 //           position in input order: min -> max, or with file_orient in file
 //           orientation; every deletion gets its status code
@@ -127,10 +128,19 @@ __global__ void __launch_bounds__(kOpThreads, 2) k_delete(const __grid_constant_
         a.keys[e] = 0ull;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) *a.work = 0ull;
+    if (!grid_sync(bar, [&] { *a.D.c.items = *a.D.items_h = 0ull; })) return;
+    const uint32_t m = 2u * a.n;
+    del_list(a.G, a.H, a.D, m);
+    __syncthreads();   // the marks of this block's entries are set
+    del_lane_rows(a.G, a.D, m, 1u, nullptr, a.fG, false);
     if (!grid_sync(bar)) return;
-    del_rows(a.G, a.D, 2u * a.n, nullptr, a.fG, false, s);
-    if (!grid_sync(bar)) return;
-    del_rows(a.H, a.D, 2u * a.n, a.fG, a.fH, true, s);
+    const unsigned long long items_g = __ldcg(a.D.c.items), items_h = __ldcg(a.D.items_h);
+    if (items_g) {
+        del_listed_rows(a.G, a.D, a.D.c.list, items_g, m, nullptr, a.fG, false, s);
+        if (!grid_sync(bar)) return;
+    }
+    del_lane_rows(a.H, a.D, m, 2u, a.fG, a.fH, true);
+    del_listed_rows(a.H, a.D, a.D.list_h, items_h, m, a.fG, a.fH, true, s);
     if (!grid_sync(bar, [&] { *a.D.cursor = 0ull; })) return;
     uint32_t mine = 0u;
     for (uint32_t e = rg.x + threadIdx.x; e < rg.y; e += blockDim.x) {
@@ -381,13 +391,14 @@ __global__ void __launch_bounds__(kOpThreads, 2) k_recover(const __grid_constant
     const uint2 rg = block_range(M);
     uint32_t kept = 0u;
     for (uint32_t t = rg.x; t < rg.y; t += blockDim.x) {
-        items_reset(s);
+        if (threadIdx.x == 0) s.nbig = 0u;
+        __syncthreads();
         const uint32_t i = t + threadIdx.x;
         bool kp = false;
         if (i < rg.y) {
             RowItem b;
             kp = cand_keep(a, i, mask, &b);
-            if (b.cnt) item_for_block(s, b);
+            if (b.cnt) s.item[atomicAdd(&s.nbig, 1u)] = b;
             a.keep[i] = kp ? 1u : 0u;
         }
         __syncthreads();
@@ -412,6 +423,7 @@ __global__ void __launch_bounds__(kOpThreads, 2) k_recover(const __grid_constant
     if (!grid_sync(bar, [&] {
             const unsigned long long k = __ldcg(a.sc + S_KEPT);
             a.sc[S_KEPT] = 0ull;
+            *a.A.s[0].c.items = 0ull;
             if (a.sc[S_RECCNT] + k > a.sc[S_RECCAP]) *a.halt = a.code_records;
         }))
         return;
@@ -534,6 +546,7 @@ dyg_status decr_delete_enqueue(dyg_graph *G, dyg_graph *H, const uint32_t *src,
     Workspace &ws = G->ws;
     const uint64_t m = 2ull * n;
     DYG_TRY(rowops_ensure(G, m));
+    DYG_TRY(rowops_ensure(H, m));
     DYG_TRY(ensure(ws.dtmp, sizeof(uint32_t) * (size_t)m * 2));
     DYG_TRY(ensure(ws.found, (size_t)m * 2));
     DYG_TRY(ensure(ws.keys, sizeof(unsigned long long) * n));
@@ -545,7 +558,8 @@ dyg_status decr_delete_enqueue(dyg_graph *G, dyg_graph *H, const uint32_t *src,
     DeleteArgs a{};
     a.G = G->g;
     a.H = H->g;
-    a.D = DelList{append_side(G, src, dst, nullptr).c, src, dst, ptr<uint32_t>(ws.dtmp), sc + S_TMPCUR};
+    a.D = DelList{append_side(G, src, dst, nullptr).c, src, dst, ptr<uint32_t>(ws.dtmp), sc + S_TMPCUR,
+                  ptr<uint32_t>(H->ws.rowlist), ptr<unsigned long long>(H->ws.scalars) + S_ITEMS};
     a.n = n;
     a.file_orient = file_orient;
     a.uid0 = uid0;

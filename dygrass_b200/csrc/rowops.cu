@@ -6,6 +6,7 @@ namespace dyg {
 dyg_status rowops_ensure(dyg_graph *G, uint64_t m) {
     Workspace &ws = G->ws;
     DYG_TRY(ensure(ws.nxt, sizeof(uint32_t) * (size_t)(m ? m : 1)));
+    DYG_TRY(ensure(ws.rowlist, sizeof(uint32_t) * (size_t)(m ? m : 1)));
     DYG_TRY(ensure(ws.blk, sizeof(uint32_t) * kOpBlocksMax * 2));
     if (!ws.rowcnt.p || !ws.rowhead.p) {
         const size_t bytes = sizeof(uint32_t) * (size_t)(G->g.n ? G->g.n : 1);
@@ -25,8 +26,11 @@ GridBar grid_bar(dyg_graph *G) {
 
 AppSide append_side(dyg_graph *G, const uint32_t *src, const uint32_t *dst, const float *w) {
     Workspace &ws = G->ws;
-    return AppSide{G->g, Chains{ptr<uint32_t>(ws.rowcnt), ptr<uint32_t>(ws.rowhead), ptr<uint32_t>(ws.nxt)},
-                   EdgeList{src, dst, w}, G->slack, ptr<unsigned long long>(ws.scalars)};
+    unsigned long long *sc = ptr<unsigned long long>(ws.scalars);
+    return AppSide{G->g,
+                   Chains{ptr<uint32_t>(ws.rowcnt), ptr<uint32_t>(ws.rowhead), ptr<uint32_t>(ws.nxt),
+                          ptr<uint32_t>(ws.rowlist), sc + S_ITEMS},
+                   EdgeList{src, dst, w}, G->slack, sc};
 }
 
 }  // namespace dyg

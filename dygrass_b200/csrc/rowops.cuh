@@ -17,10 +17,14 @@
 //   delete:  each leader gathers its chain, puts it in list order and removes
 //            the entries one by one with swap-with-last
 //            (random_walk_decremental/gpu_graph.cuh:359-399).
-// The work of a row is done by its leader's lane, by the leader's warp, or --
-// hub rows and long chains -- by its block.  A chain of more than 32 entries
-// is not followed (each link is a dependent load): the block scans the list
-// for the row's entries instead, which meets them in order.
+// The work of a row is done by its leader's lane, by a warp, or -- hub rows
+// and long chains -- by a block.  Leaders put the rows that are not for their
+// lane on a list, which the warps and blocks of the whole grid share out: the
+// leaders of hub rows are whichever blocks linked first, so a block keeping
+// its own leaders' rows could get most of them (725 us instead of 250 for the
+// recoveries of a 4,096-edge R-MAT file).  A chain of more than 32 entries is
+// not followed (each link is a dependent load): the block scans the edges for
+// the row's entries instead, which meets them in order.
 // Nothing here needs a host-visible count, so a whole update stream is
 // enqueued with a single synchronize at its end.
 #pragma once
@@ -39,8 +43,20 @@ constexpr uint32_t kTrackMax = 128;   // deletions of a hub row found in one pas
 // The chains of one graph's rows.
 struct Chains {
     uint32_t *rowcnt, *rowhead;   // per row: entries, last entry + 1 (zero between operations)
-    uint32_t *nxt;                // per half-edge: previous entry + 1; 0 leader, ~0u not in the list
+    uint32_t *nxt;                // per half-edge: previous entry + 1; ~0u not in the list; a leader:
+                                  // 0, or kItem with bits for the graphs whose row is on a list
+    uint32_t *list;               // leaders of rows for a block (from the front) and a warp (back)
+    unsigned long long *items;    // their numbers: low word, high word
 };
+constexpr uint32_t kItem = 0xFFFFFFF0u;
+
+__device__ __forceinline__ bool is_leader(uint32_t nx) { return nx == 0u || (nx >= kItem && nx != ~0u); }
+
+__device__ __forceinline__ void list_row(uint32_t *list, unsigned long long *items, uint32_t m,
+                                         uint32_t i, bool warp) {
+    if (warp) list[m - 1u - (uint32_t)(atomicAdd(items, 1ull << 32) >> 32)] = i;
+    else list[(uint32_t)atomicAdd(items, 1ull)] = i;
+}
 
 struct EdgeList {
     const uint32_t *src, *dst;
@@ -59,19 +75,17 @@ struct AppSides {
     uint32_t n;   // sides used
 };
 
-// A row left to a warp or to the block.
 struct RowItem {
     uint32_t x, cnt, head, old_off, deg, off;
 };
 
-// Entries each thread looks at per tile of scan_entries.
+// Edges each thread looks at per tile of scan_entries.
 constexpr uint32_t kScanEdges = 8;
 
-// Shared memory of the row phases.  Items for the block fill `item` from the
-// front, items for one warp each from the back.
+// Shared memory of the row phases.
 struct RowShared {
-    RowItem item[kOpThreads];
-    uint32_t nbig, nwarp;
+    RowItem item[kOpThreads];   // candidates whose rows the block searches (k_recover)
+    uint32_t nbig;
     uint32_t warp[kOpThreads / 32 + 1];
     uint32_t tile[kScanEdges * kOpThreads / 32 + 1];
     // hub-row deletions
@@ -107,7 +121,8 @@ __device__ __forceinline__ uint32_t move_need(uint32_t deg, uint32_t cnt, uint32
 
 // ------------------------------------------------------------------ append
 
-// Leaders add up the arena slots their rows' moves need.
+// Leaders add up the arena slots their rows' moves need and list the rows
+// that are not for their lane.
 __device__ __forceinline__ void app_need(const AppSide &a, uint32_t m,
                                          unsigned long long *s_need) {
     const uint2 r = block_range(m);
@@ -115,7 +130,13 @@ __device__ __forceinline__ void app_need(const AppSide &a, uint32_t m,
     for (uint32_t i = r.x + threadIdx.x; i < r.y; i += blockDim.x) {
         if (a.c.nxt[i] != 0u) continue;
         const uint32_t x = entry_row(a.E, i);
-        mine += move_need(a.g.desc[x].y, a.c.rowcnt[x], a.g.cap[x], a.slack);
+        const uint32_t deg = a.g.desc[x].y, cnt = a.c.rowcnt[x];
+        const uint32_t need = move_need(deg, cnt, a.g.cap[x], a.slack);
+        mine += need;
+        if (cnt > kLaneChain || (need && deg > kLaneRow)) {
+            a.c.nxt[i] = kItem;
+            list_row(a.c.list, a.c.items, m, i, cnt <= kWarpChain && (!need || deg <= kBigRow));
+        }
     }
     if (threadIdx.x == 0) *s_need = 0ull;
     __syncthreads();
@@ -183,20 +204,6 @@ __device__ __forceinline__ void publish_row(const AppSide &a, uint32_t x, uint32
     if (deg + cnt > kBigRow && deg <= kBigRow) a.sc[S_LONG] = 1ull;
 }
 
-__device__ __forceinline__ void items_reset(RowShared &s) {
-    if (threadIdx.x == 0) {
-        s.nbig = 0u;
-        s.nwarp = 0u;
-    }
-    __syncthreads();
-}
-__device__ __forceinline__ void item_for_block(RowShared &s, const RowItem &it) {
-    s.item[atomicAdd(&s.nbig, 1u)] = it;
-}
-__device__ __forceinline__ void item_for_warp(RowShared &s, const RowItem &it) {
-    s.item[kOpThreads - 1u - atomicAdd(&s.nwarp, 1u)] = it;
-}
-
 // The whole block calls back(k, i) for the k-th entry i, in list order, of
 // row x.  The list is read kScanEdges edges per thread at a time, all loads
 // issued together (a 40 000-entry list: five tiles); rows(e) gives the rows
@@ -258,107 +265,114 @@ __device__ __forceinline__ void scan_entries(const Chains &c, uint32_t m, uint32
     }
 }
 
-// Moves, fills and publishes the rows of this block's leaders (after a halt:
-// only clears their chains).  Every thread of the block calls it.
+// Row of leader i with its chain taken off, its space allocated.
+__device__ __forceinline__ RowItem app_take(const AppSide &a, uint32_t i, uint32_t *need) {
+    RowItem it{};
+    it.x = entry_row(a.E, i);
+    it.cnt = a.c.rowcnt[it.x];
+    it.head = a.c.rowhead[it.x];
+    const uint2 d = a.g.desc[it.x];
+    *need = move_need(d.y, it.cnt, a.g.cap[it.x], a.slack);
+    it.old_off = d.x;
+    it.deg = d.y;
+    it.off = *need ? (uint32_t)atomicAdd(a.sc + S_CURSOR, (unsigned long long)*need) : d.x;
+    a.c.rowcnt[it.x] = 0u;
+    a.c.rowhead[it.x] = 0u;
+    return it;
+}
+
+// Moves, fills and publishes every row of the list (after a halt: only clears
+// the chains).  Every thread of the grid calls it.
 __device__ __forceinline__ void app_rows(const AppSide &a, uint32_t m, bool halted, RowShared &s) {
     const uint2 rg = block_range(m);
     const uint32_t lane = threadIdx.x & 31u;
-    for (uint32_t t = rg.x; t < rg.y; t += blockDim.x) {
-        items_reset(s);
-        const uint32_t i = t + threadIdx.x;
-        const bool lead = i < rg.y && a.c.nxt[i] == 0u;
-        uint32_t x = 0, cnt = 0, head = 0, need = 0, off = 0;
-        uint2 d = make_uint2(0u, 0u);
-        if (lead) {
-            x = entry_row(a.E, i);
-            cnt = a.c.rowcnt[x];
-            head = a.c.rowhead[x];
-            a.c.rowcnt[x] = 0u;
-            a.c.rowhead[x] = 0u;
+    for (uint32_t i = rg.x + threadIdx.x; i < rg.y; i += blockDim.x) {
+        const uint32_t nx = a.c.nxt[i];
+        if (halted) {
+            if (is_leader(nx)) {
+                const uint32_t x = entry_row(a.E, i);
+                a.c.rowcnt[x] = 0u;
+                a.c.rowhead[x] = 0u;
+            }
+            continue;
         }
-        if (halted) continue;
-        if (lead) {
-            d = a.g.desc[x];
-            need = move_need(d.y, cnt, a.g.cap[x], a.slack);
-            off = need ? (uint32_t)atomicAdd(a.sc + S_CURSOR, (unsigned long long)need) : d.x;
-        }
-        const bool by_lane = lead && cnt <= kLaneChain && (!need || d.y <= kLaneRow);
-        const bool by_warp = lead && !by_lane && cnt <= kWarpChain && (!need || d.y <= kBigRow);
-        if (by_lane) {
-            if (need) copy_row<4>(a.g, d.x, off, d.y, 0u, 1u);
-            // the chain at once, then each entry to its rank among the
-            // (distinct) list indices
-            uint32_t idx[kLaneChain], y[kLaneChain];
-            float w[kLaneChain];
-            uint32_t k = head;
+        if (nx != 0u) continue;
+        uint32_t need;
+        const RowItem it = app_take(a, i, &need);
+        if (need) copy_row<4>(a.g, it.old_off, it.off, it.deg, 0u, 1u);
+        // the chain at once, then each entry to its rank among the (distinct)
+        // list indices
+        uint32_t idx[kLaneChain], y[kLaneChain];
+        float w[kLaneChain];
+        uint32_t k = it.head;
 #pragma unroll
-            for (uint32_t u = 0; u < kLaneChain; ++u)
-                if (u < cnt) {
-                    idx[u] = k - 1u;
-                    k = a.c.nxt[k - 1u];
-                }
-#pragma unroll
-            for (uint32_t u = 0; u < kLaneChain; ++u)
-                if (u < cnt) {
-                    y[u] = entry_col(a.E, idx[u]);
-                    w[u] = a.E.w[idx[u] >> 1];
-                }
-#pragma unroll
-            for (uint32_t u = 0; u < kLaneChain; ++u)
-                if (u < cnt) {
-                    uint32_t r = 0;
-#pragma unroll
-                    for (uint32_t v = 0; v < kLaneChain; ++v)
-                        if (v < cnt) r += idx[v] < idx[u] ? 1u : 0u;
-                    put_slot(a.g, off + d.y + r, y[u], w[u]);
-                }
-            publish_row(a, x, off, d.y, cnt, need);
-        }
-        if (lead && !by_lane) {
-            const RowItem it{x, cnt, head, d.x, d.y, off};
-            if (by_warp) item_for_warp(s, it);
-            else item_for_block(s, it);
-        }
-        __syncthreads();
-        const uint32_t nwarp = s.nwarp;
-        for (uint32_t q = threadIdx.x >> 5; q < nwarp; q += blockDim.x >> 5) {
-            const RowItem it = s.item[kOpThreads - 1u - q];
-            const bool mv = it.off != it.old_off;
-            if (mv) copy_row<4>(a.g, it.old_off, it.off, it.deg, lane, 32u);
-            uint32_t mine = ~0u, k = it.head;
-            for (uint32_t u = 0; u < it.cnt; ++u) {   // the chain: one load for the whole warp each
-                if (lane == u) mine = k - 1u;
+        for (uint32_t u = 0; u < kLaneChain; ++u)
+            if (u < it.cnt) {
+                idx[u] = k - 1u;
                 k = a.c.nxt[k - 1u];
             }
-            uint32_t r = 0;
-            for (uint32_t u = 0; u < it.cnt; ++u) r += __shfl_sync(kFull, mine, u) < mine ? 1u : 0u;
-            if (lane < it.cnt)
-                put_slot(a.g, it.off + it.deg + r, entry_col(a.E, mine), a.E.w[mine >> 1]);
-            if (lane == 0u)
-                publish_row(a, it.x, it.off, it.deg, it.cnt,
-                            mv ? move_need(it.deg, it.cnt, a.g.cap[it.x], a.slack) : 0u);
+#pragma unroll
+        for (uint32_t u = 0; u < kLaneChain; ++u)
+            if (u < it.cnt) {
+                y[u] = entry_col(a.E, idx[u]);
+                w[u] = a.E.w[idx[u] >> 1];
+            }
+#pragma unroll
+        for (uint32_t u = 0; u < kLaneChain; ++u)
+            if (u < it.cnt) {
+                uint32_t r = 0;
+#pragma unroll
+                for (uint32_t v = 0; v < kLaneChain; ++v)
+                    if (v < it.cnt) r += idx[v] < idx[u] ? 1u : 0u;
+                put_slot(a.g, it.off + it.deg + r, y[u], w[u]);
+            }
+        publish_row(a, it.x, it.off, it.deg, it.cnt, need);
+    }
+    if (halted) return;
+    const unsigned long long both = __ldcg(a.c.items);
+    const uint32_t n_block = (uint32_t)both, n_warp = (uint32_t)(both >> 32);
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    // warp q of block 0, then of block 1, ...: a short list still spreads
+    for (uint32_t q = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; q < n_warp; q += warps) {
+        uint32_t need = 0u;
+        RowItem it{};
+        if (lane == 0u) it = app_take(a, a.c.list[m - 1u - q], &need);
+        it.x = __shfl_sync(kFull, it.x, 0);
+        it.cnt = __shfl_sync(kFull, it.cnt, 0);
+        it.old_off = __shfl_sync(kFull, it.old_off, 0);
+        it.deg = __shfl_sync(kFull, it.deg, 0);
+        it.off = __shfl_sync(kFull, it.off, 0);
+        if (it.off != it.old_off) copy_row<4>(a.g, it.old_off, it.off, it.deg, lane, 32u);
+        uint32_t mine = ~0u, k = __shfl_sync(kFull, it.head, 0);
+        for (uint32_t u = 0; u < it.cnt; ++u) {   // the chain: one load for the whole warp each
+            if (lane == u) mine = k - 1u;
+            k = a.c.nxt[k - 1u];
         }
-        const uint32_t nbig = s.nbig;
-        for (uint32_t q = 0; q < nbig; ++q) {
-            const RowItem it = s.item[q];
-            const bool mv = it.off != it.old_off;
-            if (mv) copy_row<4>(a.g, it.old_off, it.off, it.deg, threadIdx.x, blockDim.x);
-            scan_entries(
-                a.c, m, it.x, it.cnt, s, [&](uint32_t e) { return make_uint2(a.E.src[e], a.E.dst[e]); },
-                [&](uint32_t k, uint32_t j) {
-                    put_slot(a.g, it.off + it.deg + k, entry_col(a.E, j), a.E.w[j >> 1]);
-                });
-            if (threadIdx.x == 0)
-                publish_row(a, it.x, it.off, it.deg, it.cnt,
-                            mv ? move_need(it.deg, it.cnt, a.g.cap[it.x], a.slack) : 0u);
-        }
+        uint32_t r = 0;
+        for (uint32_t u = 0; u < it.cnt; ++u) r += __shfl_sync(kFull, mine, u) < mine ? 1u : 0u;
+        if (lane < it.cnt)
+            put_slot(a.g, it.off + it.deg + r, entry_col(a.E, mine), a.E.w[mine >> 1]);
+        if (lane == 0u) publish_row(a, it.x, it.off, it.deg, it.cnt, need);
+    }
+    for (uint32_t q = blockIdx.x; q < n_block; q += gridDim.x) {
+        __syncthreads();   // the item before is done with s.item
+        uint32_t need = 0u;
+        if (threadIdx.x == 0) s.item[0] = app_take(a, a.c.list[q], &need);
         __syncthreads();
+        const RowItem it = s.item[0];
+        if (it.off != it.old_off) copy_row<4>(a.g, it.old_off, it.off, it.deg, threadIdx.x, blockDim.x);
+        scan_entries(
+            a.c, m, it.x, it.cnt, s, [&](uint32_t e) { return make_uint2(a.E.src[e], a.E.dst[e]); },
+            [&](uint32_t k, uint32_t j) {
+                put_slot(a.g, it.off + it.deg + k, entry_col(a.E, j), a.E.w[j >> 1]);
+            });
+        if (threadIdx.x == 0) publish_row(a, it.x, it.off, it.deg, it.cnt, need);
     }
 }
 
-// Sizing, reservation and rows of an append whose m half-edges are linked.
-// on_reserve runs in one thread once the space is reserved.  False: the
-// barrier gave up.
+// Sizing, reservation and rows of an append whose m half-edges are linked and
+// whose row lists are empty.  on_reserve runs in one thread once the space is
+// reserved.  False: the barrier gave up.
 template <class F>
 __device__ __forceinline__ bool app_commit(const AppSides &A, uint32_t m, const GridBar &bar,
                                            unsigned long long *halt, unsigned long long code,
@@ -390,6 +404,8 @@ struct DelList {
     const uint32_t *src, *dst;   // as given
     uint32_t *tmp;               // 4n words: ordered entries of hub rows, of G then of H
     unsigned long long *cursor;  // next free word of tmp
+    uint32_t *list_h;            // listed rows of H (c.list, c.items: of G)
+    unsigned long long *items_h;
 };
 
 __device__ __forceinline__ uint32_t del_row(const DelList &D, uint32_t i) {
@@ -593,89 +609,121 @@ __device__ __forceinline__ void warp_del_row(const DevGraph &g, const DelList &D
     __syncwarp();
 }
 
-// Removes the entries of this block's leaders' rows from g in list order
-// (mask as in del_on); found[i] = 1 for each entry that was there.  `clear`
-// empties the chains.  Every thread of the block calls it.
-__device__ __forceinline__ void del_rows(const DevGraph &g, const DelList &D, uint32_t m,
-                                         const uint8_t *mask, uint8_t *found, bool clear,
-                                         RowShared &s) {
+// How a row's cnt deletions are done.  A warp searches the row once per
+// deletion: worth it up to kWarpSearch slots looked at in all.
+__device__ __forceinline__ bool del_by_lane(uint32_t deg, uint32_t cnt) {
+    return cnt <= kLaneChain && deg <= kLaneRow;
+}
+__device__ __forceinline__ bool del_by_warp(uint32_t deg, uint32_t cnt) {
+    return cnt <= kWarpChain && (uint64_t)deg * cnt <= kWarpSearch;
+}
+
+// Leaders list the rows of G (bit 1 of the mark) and of H (bit 2) that are
+// not for their lane.
+__device__ __forceinline__ void del_list(const DevGraph &G, const DevGraph &H, const DelList &D,
+                                         uint32_t m) {
     const uint2 rg = block_range(m);
-    const uint32_t lane = threadIdx.x & 31u;
-    for (uint32_t t = rg.x; t < rg.y; t += blockDim.x) {
-        items_reset(s);
-        const uint32_t i = t + threadIdx.x;
-        const bool lead = i < rg.y && D.c.nxt[i] == 0u;
-        uint32_t x = 0, cnt = 0, head = 0;
-        uint2 d = make_uint2(0u, 0u);
-        if (lead) {
-            x = del_row(D, i);
-            cnt = D.c.rowcnt[x];
-            head = D.c.rowhead[x];
-            d = g.desc[x];
+    for (uint32_t i = rg.x + threadIdx.x; i < rg.y; i += blockDim.x) {
+        if (D.c.nxt[i] != 0u) continue;
+        const uint32_t x = del_row(D, i), cnt = D.c.rowcnt[x];
+        const uint32_t dg = G.desc[x].y, dh = H.desc[x].y;
+        uint32_t mark = 0u;
+        if (!del_by_lane(dg, cnt)) {
+            mark |= 1u;
+            list_row(D.c.list, D.c.items, m, i, del_by_warp(dg, cnt));
         }
-        const bool by_lane = lead && cnt <= kLaneChain && d.y <= kLaneRow;
-        // a warp searches the row once per deletion: worth it up to kWarpSearch
-        // slots looked at in all
-        const bool by_warp = lead && !by_lane && cnt <= kWarpChain && (uint64_t)d.y * cnt <= kWarpSearch;
-        if (by_lane) {
-            uint32_t idx[kLaneChain];
-            uint32_t k = head;
+        if (!del_by_lane(dh, cnt)) {
+            mark |= 2u;
+            list_row(D.list_h, D.items_h, m, i, del_by_warp(dh, cnt));
+        }
+        if (mark) D.c.nxt[i] = kItem | mark;
+    }
+}
+
+// The rows of g that are for their leader's lane: entries removed in list
+// order (mask as in del_on); found[i] = 1 for each entry that was there.
+// `bit`: the graph's mark.
+__device__ __forceinline__ void del_lane_rows(const DevGraph &g, const DelList &D, uint32_t m,
+                                              uint32_t bit, const uint8_t *mask, uint8_t *found,
+                                              bool clear) {
+    const uint2 rg = block_range(m);
+    for (uint32_t i = rg.x + threadIdx.x; i < rg.y; i += blockDim.x) {
+        const uint32_t nx = D.c.nxt[i];
+        if (!is_leader(nx) || (nx & bit)) continue;
+        const uint32_t x = del_row(D, i), cnt = D.c.rowcnt[x], head = D.c.rowhead[x];
+        const uint2 d = g.desc[x];
+        uint32_t idx[kLaneChain];
+        uint32_t k = head;
 #pragma unroll
-            for (uint32_t u = 0; u < kLaneChain; ++u) {
-                idx[u] = ~0u;
-                if (u < cnt) {
-                    idx[u] = k - 1u;
-                    k = D.c.nxt[k - 1u];
-                }
+        for (uint32_t u = 0; u < kLaneChain; ++u) {
+            idx[u] = ~0u;
+            if (u < cnt) {
+                idx[u] = k - 1u;
+                k = D.c.nxt[k - 1u];
             }
-            uint32_t deg = d.y, from = 0u;
-            for (uint32_t a = 0; a < cnt; ++a) {
-                k = ~0u;   // the next entry in list order
+        }
+        uint32_t deg = d.y, from = 0u;
+        for (uint32_t a = 0; a < cnt; ++a) {
+            k = ~0u;   // the next entry in list order
 #pragma unroll
-                for (uint32_t u = 0; u < kLaneChain; ++u)
-                    if (idx[u] >= from) k = min(k, idx[u]);
-                from = k + 1u;
-                if (!del_on(mask, k)) continue;
-                const uint32_t y = del_col(D, k);
-                // first slot holding y, eight columns loaded before they are
-                // compared (vertex ids are never ~0u)
-                uint32_t pos = ~0u;
-                for (uint32_t j0 = 0; j0 < deg && pos == ~0u; j0 += 8u) {
-                    uint32_t cv[8];
+            for (uint32_t u = 0; u < kLaneChain; ++u)
+                if (idx[u] >= from) k = min(k, idx[u]);
+            from = k + 1u;
+            if (!del_on(mask, k)) continue;
+            const uint32_t y = del_col(D, k);
+            // first slot holding y, eight columns loaded before they are
+            // compared (vertex ids are never ~0u)
+            uint32_t pos = ~0u;
+            for (uint32_t j0 = 0; j0 < deg && pos == ~0u; j0 += 8u) {
+                uint32_t cv[8];
 #pragma unroll
-                    for (uint32_t u = 0; u < 8u; ++u)
-                        cv[u] = j0 + u < deg ? g.slots[d.x + j0 + u].x : ~0u;
+                for (uint32_t u = 0; u < 8u; ++u)
+                    cv[u] = j0 + u < deg ? g.slots[d.x + j0 + u].x : ~0u;
 #pragma unroll
-                    for (uint32_t u = 0; u < 8u; ++u)
-                        if (pos == ~0u && cv[u] == y) pos = j0 + u;
-                }
-                if (pos != ~0u) {
-                    del_swap(g, d.x, pos, deg);
-                    --deg;
-                    found[k] = 1;
-                }
+                for (uint32_t u = 0; u < 8u; ++u)
+                    if (pos == ~0u && cv[u] == y) pos = j0 + u;
             }
-            if (deg != d.y) g.desc[x] = make_uint2(d.x, deg);
+            if (pos != ~0u) {
+                del_swap(g, d.x, pos, deg);
+                --deg;
+                found[k] = 1;
+            }
         }
-        if (lead && !by_lane) {
-            const RowItem it{x, cnt, head, d.x, d.y, 0u};
-            if (by_warp) item_for_warp(s, it);
-            else item_for_block(s, it);
-        }
-        if (lead && clear) {
+        if (deg != d.y) g.desc[x] = make_uint2(d.x, deg);
+        if (clear) {
             D.c.rowcnt[x] = 0u;
             D.c.rowhead[x] = 0u;
         }
-        __syncthreads();
-        const uint32_t nwarp = s.nwarp;
-        for (uint32_t q = threadIdx.x >> 5; q < nwarp; q += blockDim.x >> 5)
-            warp_del_row(g, D, s.item[kOpThreads - 1u - q], mask, found, lane);
-        const uint32_t nbig = s.nbig;
-        for (uint32_t q = 0; q < nbig; ++q) {
-            const RowItem it = s.item[q];
-            block_del_row(g, D, m, it.x, it.cnt, it.head, mask, found, s);
+    }
+}
+
+// The listed rows of g, shared out over the grid's warps and blocks.
+__device__ __forceinline__ void del_listed_rows(const DevGraph &g, const DelList &D,
+                                                const uint32_t *list, unsigned long long items,
+                                                uint32_t m, const uint8_t *mask, uint8_t *found,
+                                                bool clear, RowShared &s) {
+    const uint32_t n_block = (uint32_t)items, n_warp = (uint32_t)(items >> 32);
+    const uint32_t lane = threadIdx.x & 31u, warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t q = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; q < n_warp; q += warps) {
+        const uint32_t x = del_row(D, list[m - 1u - q]);
+        const uint2 d = g.desc[x];
+        const RowItem it{x, D.c.rowcnt[x], D.c.rowhead[x], d.x, d.y, 0u};
+        __syncwarp();
+        if (lane == 0u && clear) {
+            D.c.rowcnt[x] = 0u;
+            D.c.rowhead[x] = 0u;
         }
+        warp_del_row(g, D, it, mask, found, lane);
+    }
+    for (uint32_t q = blockIdx.x; q < n_block; q += gridDim.x) {
+        const uint32_t x = del_row(D, list[q]);
+        const uint32_t cnt = D.c.rowcnt[x], head = D.c.rowhead[x];
         __syncthreads();
+        if (threadIdx.x == 0 && clear) {
+            D.c.rowcnt[x] = 0u;
+            D.c.rowhead[x] = 0u;
+        }
+        block_del_row(g, D, m, x, cnt, head, mask, found, s);
     }
 }
 
@@ -712,7 +760,10 @@ k_append(const Op op, const __grid_constant__ AppSides A, GridBar bar, uint32_t 
         const uint32_t sum = block_sum(mine, s.warp);
         if (threadIdx.x == 0) blk[blockIdx.x] = sum;
     }
-    if (!grid_sync(bar)) return;
+    if (!grid_sync(bar, [&] {
+            for (uint32_t k = 0; k < A.n; ++k) *A.s[k].c.items = 0ull;
+        }))
+        return;
     if constexpr (Op::kList) {
         uint32_t base = blocks_before(blk, s.warp).x;
         for (uint32_t t = rg.x; t < rg.y; t += blockDim.x) {
