@@ -427,36 +427,28 @@ dyg_status dyg_graph_copy_from(dyg_graph *dst, const dyg_graph *src, dyg_stream_
     }
     DeviceGuard dg(dst->device);
     cudaStream_t st = (cudaStream_t)stream;
-    dyg_graph *s = const_cast<dyg_graph *>(src);
-    DYG_TRY(read_scalars(s, st));
-    const unsigned long long top = s->ws.host_scalars[S_TOP];
-    if (dst->g.arena_cap < top) {
-        uint2 *ns = nullptr;
-        float *nw = nullptr;
-        if (cudaMalloc(&ns, sizeof(uint2) * (size_t)src->g.arena_cap) != cudaSuccess ||
-            cudaMalloc(&nw, sizeof(float) * (size_t)src->g.arena_cap) != cudaSuccess) {
-            cudaGetLastError();
-            if (ns) cudaFree(ns);
-            set_error("cudaMalloc in copy_from failed");
-            return DYG_ENOMEM;
+    if (dst->g.arena_cap < src->g.arena_cap) {
+        // the host needs src's top only when dst's arena might not hold it
+        dyg_graph *s = const_cast<dyg_graph *>(src);
+        DYG_TRY(read_scalars(s, st));
+        if (dst->g.arena_cap < s->ws.host_scalars[S_TOP]) {
+            uint2 *ns = nullptr;
+            float *nw = nullptr;
+            if (cudaMalloc(&ns, sizeof(uint2) * (size_t)src->g.arena_cap) != cudaSuccess ||
+                cudaMalloc(&nw, sizeof(float) * (size_t)src->g.arena_cap) != cudaSuccess) {
+                cudaGetLastError();
+                if (ns) cudaFree(ns);
+                set_error("cudaMalloc in copy_from failed");
+                return DYG_ENOMEM;
+            }
+            DYG_CUDA(cudaFree(dst->g.slots));
+            DYG_CUDA(cudaFree(dst->g.wts));
+            dst->g.slots = ns;
+            dst->g.wts = nw;
+            dst->g.arena_cap = src->g.arena_cap;
         }
-        DYG_CUDA(cudaFree(dst->g.slots));
-        DYG_CUDA(cudaFree(dst->g.wts));
-        dst->g.slots = ns;
-        dst->g.wts = nw;
-        dst->g.arena_cap = src->g.arena_cap;
     }
-    const uint32_t n = src->g.n;
-    DYG_CUDA(cudaMemcpyAsync(dst->g.desc, src->g.desc, sizeof(uint2) * n, cudaMemcpyDeviceToDevice, st));
-    DYG_CUDA(cudaMemcpyAsync(dst->g.cap, src->g.cap, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, st));
-    DYG_CUDA(cudaMemcpyAsync(dst->g.slots, src->g.slots, sizeof(uint2) * (size_t)top,
-                             cudaMemcpyDeviceToDevice, st));
-    DYG_CUDA(cudaMemcpyAsync(dst->g.wts, src->g.wts, sizeof(float) * (size_t)top,
-                             cudaMemcpyDeviceToDevice, st));
-    DYG_CUDA(cudaMemcpyAsync(dst->g.top, src->g.top, sizeof(unsigned long long),
-                             cudaMemcpyDeviceToDevice, st));
-    DYG_CUDA(cudaMemsetAsync(ptr<unsigned long long>(dst->ws.scalars) + S_LONG, 0,
-                             sizeof(unsigned long long), st));
+    if (dst != src) DYG_TRY(copy_graph_enqueue(dst, src, st));
     dst->slack = src->slack;
     dst->headroom = src->headroom;
     dst->long_rows = src->long_rows;

@@ -403,6 +403,8 @@ dyg_status read_scalars2(dyg_graph *A, dyg_graph *B, cudaStream_t st);
 dyg_status exclusive_scan_u32(Workspace &ws, const uint32_t *in, uint32_t *out, uint32_t m,
                               cudaStream_t st, const uint32_t *m_dev = nullptr);
 dyg_status compact_graph(dyg_graph *G, cudaStream_t st);
+// src's rows, capacities and arena top into dst, whose arena holds them.
+dyg_status copy_graph_enqueue(dyg_graph *dst, const dyg_graph *src, cudaStream_t st);
 dyg_status grow_arena(dyg_graph *G, uint64_t min_cap, cudaStream_t st);
 dyg_status read_scalars(dyg_graph *G, cudaStream_t st);
 // Rows of local graph [v0, v0 + n) of a pool graph: load places them at the

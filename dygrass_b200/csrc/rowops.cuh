@@ -21,7 +21,7 @@
 // and long chains -- by a block.  Leaders put the rows that are not for their
 // lane on a list, which the warps and blocks of the whole grid share out: the
 // leaders of hub rows are whichever blocks linked first, so a block keeping
-// its own leaders' rows could get most of them (725 us instead of 250 for the
+// its own leaders' rows could get most of them (725 us instead of 134 for the
 // recoveries of a 4,096-edge R-MAT file).  A chain of more than 32 entries is
 // not followed (each link is a dependent load): the block scans the edges for
 // the row's entries instead, which meets them in order.
