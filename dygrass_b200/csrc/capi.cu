@@ -11,6 +11,7 @@
 //   in H, append the rest in order -> 2-step fallback walks for the edges
 //   without a path, same dedup and append.
 #include <math.h>
+#include <string.h>
 
 #include <string>
 
@@ -78,30 +79,186 @@ bool on_device(const void *p) {
     return at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged;
 }
 
-template <typename T>
-dyg_status stage_in(Buf &b, const T *p, size_t n, cudaStream_t st, const T **out) {
-    if (!p) {
-        *out = nullptr;
-        return DYG_OK;
-    }
-    if (on_device(p)) {
-        *out = p;
-        return DYG_OK;
-    }
-    DYG_TRY(ensure(b, sizeof(T) * n));
-    DYG_CUDA(cudaMemcpyAsync(b.p, p, sizeof(T) * n, cudaMemcpyHostToDevice, st));
-    *out = ptr<T>(b);
+// The arrays of one call.  Where each lives is asked once.  Host inputs of up
+// to kPackMax bytes together go to the device in one copy from pinned memory,
+// and host results come back in one that the call's own wait covers: three
+// pageable copies in and three out, each waited for by itself, were 45 of the
+// 130 us of a 32-edge batch.  Larger arrays are copied one by one (staging
+// them would cost the host a pass over memory that the copies overlap).
+constexpr size_t kPackMax = 1u << 20;
+
+struct InArray {
+    const char *name;
+    const void *p;
+    size_t bytes;
+    Buf *own;                   // device copy of a large array
+    const void *dev = nullptr;  // where the kernels read it
+    bool host = false;
+};
+struct OutArray {
+    const char *name;
+    void *p;
+    size_t bytes;               // 0: not wanted by anyone
+    Buf *own;
+    void *dev = nullptr;
+    bool host = false;          // the caller's array is host memory
+    size_t at = 0;              // in the packed block
+};
+
+size_t align16(size_t b) { return (b + 15) & ~(size_t)15; }
+
+dyg_status ensure_pinned(Buf &b, size_t bytes) {
+    if (b.bytes >= bytes) return DYG_OK;
+    if (b.p) cudaFreeHost(b.p);
+    b = Buf{};
+    size_t want = 4096;
+    while (want < bytes) want *= 2;
+    DYG_CUDA(cudaMallocHost(&b.p, want));
+    b.bytes = want;
     return DYG_OK;
 }
 
-template <typename T>
-dyg_status copy_out(T *dst, const T *src_dev, size_t n, cudaStream_t st, bool *host_out) {
-    if (!dst || n == 0) return DYG_OK;
-    const bool dev = on_device(dst);
-    if (!dev) *host_out = true;
-    DYG_CUDA(cudaMemcpyAsync(dst, src_dev, sizeof(T) * n,
-                             dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
+dyg_status check_places(int device, InArray *in, int nin, OutArray *out, int nout) {
+    auto place = [&](const void *p, const char *name, bool *host) {
+        const PtrPlace w = ptr_place(p, device);
+        *host = p && w == kOnHost;
+        if (w != kOnOtherDevice) return DYG_OK;
+        set_error(std::string(name) + " is device memory of another GPU than the graph's (device " +
+                  std::to_string(device) + ")");
+        return DYG_EINVAL;
+    };
+    for (int i = 0; i < nin; ++i) DYG_TRY(place(in[i].p, in[i].name, &in[i].host));
+    for (int i = 0; i < nout; ++i) DYG_TRY(place(out[i].p, out[i].name, &out[i].host));
     return DYG_OK;
+}
+
+dyg_status stage_inputs(Workspace &ws, InArray *in, int nin, cudaStream_t st) {
+    size_t total = 0;
+    for (int i = 0; i < nin; ++i) {
+        in[i].dev = in[i].p;
+        if (in[i].host) total += align16(in[i].bytes);
+    }
+    if (total == 0) return DYG_OK;
+    if (total > kPackMax) {
+        for (int i = 0; i < nin; ++i) {
+            if (!in[i].host) continue;
+            DYG_TRY(ensure(*in[i].own, in[i].bytes));
+            DYG_CUDA(cudaMemcpyAsync(in[i].own->p, in[i].p, in[i].bytes, cudaMemcpyHostToDevice, st));
+            in[i].dev = in[i].own->p;
+        }
+        return DYG_OK;
+    }
+    // every call waits for its copies, so the pinned block is free again
+    DYG_TRY(ensure_pinned(ws.pin_in, total));
+    DYG_TRY(ensure(ws.io_in, total));
+    size_t at = 0;
+    for (int i = 0; i < nin; ++i) {
+        if (!in[i].host) continue;
+        memcpy(static_cast<char *>(ws.pin_in.p) + at, in[i].p, in[i].bytes);
+        in[i].dev = static_cast<char *>(ws.io_in.p) + at;
+        at += align16(in[i].bytes);
+    }
+    DYG_CUDA(cudaMemcpyAsync(ws.io_in.p, ws.pin_in.p, total, cudaMemcpyHostToDevice, st));
+    return DYG_OK;
+}
+
+// Device places for the results: the caller's own where it is device memory.
+// *packed gets the bytes of the block the others share, 0 if they are large.
+dyg_status place_outputs(Workspace &ws, OutArray *out, int nout, size_t *packed) {
+    size_t total = 0;
+    for (int i = 0; i < nout; ++i) {
+        out[i].dev = out[i].p && !out[i].host ? out[i].p : nullptr;
+        if (out[i].dev || !out[i].bytes) continue;
+        out[i].at = total;
+        total += align16(out[i].bytes);
+    }
+    *packed = total <= kPackMax ? total : 0;
+    if (*packed) DYG_TRY(ensure(ws.io_out, total));
+    for (int i = 0; i < nout; ++i) {
+        if (out[i].dev || !out[i].bytes) continue;
+        if (*packed) {
+            out[i].dev = static_cast<char *>(ws.io_out.p) + out[i].at;
+        } else {
+            DYG_TRY(ensure(*out[i].own, out[i].bytes));
+            out[i].dev = out[i].own->p;
+        }
+    }
+    return DYG_OK;
+}
+
+bool any_host(const OutArray *out, int nout) {
+    for (int i = 0; i < nout; ++i)
+        if (out[i].host) return true;
+    return false;
+}
+
+// Host results to the caller: from the pinned block the call fetched, or by
+// one copy each (*wait is set: the stream is to be waited for).
+dyg_status deliver(Workspace &ws, const OutArray *out, int nout, size_t packed, cudaStream_t st,
+                   bool *wait) {
+    for (int i = 0; i < nout; ++i) {
+        if (!out[i].host) continue;
+        if (packed) {
+            memcpy(out[i].p, static_cast<char *>(ws.pin_out.p) + out[i].at, out[i].bytes);
+        } else {
+            DYG_CUDA(cudaMemcpyAsync(out[i].p, out[i].dev, out[i].bytes, cudaMemcpyDeviceToHost, st));
+            *wait = true;
+        }
+    }
+    return DYG_OK;
+}
+
+// The recovered edges of a deletion call.  They are fetched with the other
+// results as far as a call usually brings them (four per deletion); how many
+// there are is only known after the wait.
+struct RecordsOut {
+    uint32_t *src, *dst;
+    uint8_t *kind;
+    uint64_t cap;
+    bool host, any_host;        // all wanted arrays, any of them, are host memory
+    uint64_t fetched = 0;
+    size_t at = 0;              // of the fetched records in the pinned block
+    bool wanted() const { return src || dst || kind; }
+    dyg_status fetch(Workspace &ws, cudaStream_t st) {
+        if (!fetched) return DYG_OK;
+        char *pin = static_cast<char *>(ws.pin_out.p) + at;
+        if (src) DYG_CUDA(cudaMemcpyAsync(pin, ws.rx2.p, 4 * fetched, cudaMemcpyDeviceToHost, st));
+        if (dst) DYG_CUDA(cudaMemcpyAsync(pin + 4 * fetched, ws.ry2.p, 4 * fetched, cudaMemcpyDeviceToHost, st));
+        if (kind) DYG_CUDA(cudaMemcpyAsync(pin + 8 * fetched, ws.rk2.p, fetched, cudaMemcpyDeviceToHost, st));
+        return DYG_OK;
+    }
+    dyg_status deliver(Workspace &ws, uint64_t total, cudaStream_t st, bool *wait) {
+        const uint64_t n = total < cap ? total : cap;
+        if (!n || !wanted()) return DYG_OK;
+        if (n <= fetched) {
+            const char *pin = static_cast<const char *>(ws.pin_out.p) + at;
+            if (src) memcpy(src, pin, 4 * n);
+            if (dst) memcpy(dst, pin + 4 * fetched, 4 * n);
+            if (kind) memcpy(kind, pin + 8 * fetched, n);
+            return DYG_OK;
+        }
+        if (src) DYG_CUDA(cudaMemcpyAsync(src, ws.rx2.p, 4 * n, cudaMemcpyDefault, st));
+        if (dst) DYG_CUDA(cudaMemcpyAsync(dst, ws.ry2.p, 4 * n, cudaMemcpyDefault, st));
+        if (kind) DYG_CUDA(cudaMemcpyAsync(kind, ws.rk2.p, n, cudaMemcpyDefault, st));
+        *wait |= any_host;
+        return DYG_OK;
+    }
+};
+
+// Pinned room for the packed results and the records to fetch: at most what
+// the record buffers hold to begin with (four per deletion).
+dyg_status prepare_fetch(Workspace &ws, size_t packed, RecordsOut *rec, uint64_t n) {
+    size_t bytes = packed;
+    if (rec && rec->wanted() && rec->host && packed) {
+        uint64_t f = 4 * n + 64;
+        if (f > rec->cap) f = rec->cap;
+        if (9 * f <= kPackMax) {
+            rec->fetched = f;
+            rec->at = align16(packed);
+            bytes = rec->at + 9 * f;
+        }
+    }
+    return bytes ? ensure_pinned(ws.pin_out, bytes) : DYG_OK;
 }
 
 dyg_status check_params(const dyg_walk_params *p) {
@@ -128,8 +285,7 @@ dyg_status check_params(const dyg_walk_params *p) {
     return DYG_OK;
 }
 
-dyg_status check_host_ids(const uint32_t *v, size_t n, uint32_t nv, const char *what) {
-    if (!v || on_device(v)) return DYG_OK;
+dyg_status check_ids(const uint32_t *v, size_t n, uint32_t nv, const char *what) {
     for (size_t i = 0; i < n; ++i)
         if (v[i] >= nv) {
             set_error(std::string(what) + "[" + std::to_string(i) + "] = " + std::to_string(v[i]) +
@@ -139,14 +295,21 @@ dyg_status check_host_ids(const uint32_t *v, size_t n, uint32_t nv, const char *
     return DYG_OK;
 }
 
-dyg_status check_host_weights(const float *w, size_t n) {
-    if (!w || on_device(w)) return DYG_OK;
+dyg_status check_weights(const float *w, size_t n) {
     for (size_t i = 0; i < n; ++i)
         if (!(w[i] > 0.0f) || !isfinite(w[i])) {
             set_error("weight[" + std::to_string(i) + "] is not finite and > 0");
             return DYG_EINVAL;
         }
     return DYG_OK;
+}
+
+dyg_status check_host_ids(const uint32_t *v, size_t n, uint32_t nv, const char *what) {
+    return !v || on_device(v) ? DYG_OK : check_ids(v, n, nv, what);
+}
+
+dyg_status check_host_weights(const float *w, size_t n) {
+    return !w || on_device(w) ? DYG_OK : check_weights(w, n);
 }
 
 // Host batches up to this size are checked on the host (the message names
@@ -185,12 +348,13 @@ dyg_status check_device_errors(dyg_graph *G, cudaStream_t st) {
 }
 
 dyg_status graph_alloc_scalars(dyg_graph *G) {
-    DYG_TRY(ensure(G->ws.scalars, sizeof(unsigned long long) * S_NSCALARS));
-    DYG_TRY(ensure(G->ws.counts, sizeof(uint32_t) * C_NCOUNTS));
-    DYG_CUDA(cudaMemset(G->ws.scalars.p, 0, sizeof(unsigned long long) * S_NSCALARS));
-    DYG_CUDA(cudaMemset(G->ws.counts.p, 0, sizeof(uint32_t) * C_NCOUNTS));
-    DYG_CUDA(cudaMallocHost(&G->ws.host_scalars, sizeof(unsigned long long) * S_NSCALARS));
-    DYG_CUDA(cudaMallocHost(&G->ws.host_counts, sizeof(uint32_t) * C_NCOUNTS));
+    // counts follow the scalars, on the device and in the pinned mirror, so
+    // that one copy reads both
+    DYG_TRY(ensure(G->ws.scalars, kScalarBytes));
+    DYG_CUDA(cudaMemset(G->ws.scalars.p, 0, kScalarBytes));
+    G->ws.counts.p = ptr<unsigned long long>(G->ws.scalars) + S_NSCALARS;
+    DYG_CUDA(cudaMallocHost(&G->ws.host_scalars, kScalarBytes));
+    G->ws.host_counts = reinterpret_cast<uint32_t *>(G->ws.host_scalars + S_NSCALARS);
     G->g.top = ptr<unsigned long long>(G->ws.scalars) + S_TOP;
     return DYG_OK;
 }
@@ -211,10 +375,11 @@ void free_graph(dyg_graph *G) {
                    &ws.s_src, &ws.s_dst, &ws.s_w, &ws.s_o1, &ws.s_o2, &ws.s_o3, &ws.rx2, &ws.ry2,
                    &ws.rk2, &ws.nxt, &ws.dtmp, &ws.rowcnt, &ws.rowhead, &ws.rowlist, &ws.blk, &ws.st_key,
                    &ws.st_val, &ws.st_pos, &ws.st_wapp, &ws.big, &ws.s_uid, &ws.ix_base,
-                   &ws.ix_list, &ws.ix_words, &ws.scalars, &ws.counts};
+                   &ws.ix_list, &ws.ix_words, &ws.scalars, &ws.io_in, &ws.io_out};
     for (Buf *b : bufs) free_buf(*b);
     if (ws.host_scalars) cudaFreeHost(ws.host_scalars);
-    if (ws.host_counts) cudaFreeHost(ws.host_counts);
+    if (ws.pin_in.p) cudaFreeHost(ws.pin_in.p);
+    if (ws.pin_out.p) cudaFreeHost(ws.pin_out.p);
     if (G->g.desc) cudaFree(G->g.desc);
     if (G->g.cap) cudaFree(G->g.cap);
     if (G->g.slots) cudaFree(G->g.slots);
@@ -622,53 +787,41 @@ static dyg_status incremental_common(dyg_graph *H, dyg_graph *G, const uint32_t 
     if (n == 0) return DYG_OK;
     DeviceGuard dg(H->device);
     cudaStream_t st = (cudaStream_t)stream;
-    {
-        const void *ps[] = {src, dst, w, uids, found_at, conductance, accepted};
-        const char *nm[] = {"src", "dst", "w", "update_ids", "found_at", "conductance", "accepted"};
-        DYG_TRY(check_same_device(H->device, ps, nm, 7));
-    }
+    Workspace &ws = H->ws;
+    InArray in[] = {{"src", src, sizeof(uint32_t) * (size_t)n, &ws.s_src},
+                    {"dst", dst, sizeof(uint32_t) * (size_t)n, &ws.s_dst},
+                    {"w", w, sizeof(float) * (size_t)n, &ws.s_w},
+                    {"update_ids", uids, sizeof(uint64_t) * (size_t)n, &ws.s_uid}};
+    OutArray out[] = {{"found_at", found_at, found_at ? sizeof(int32_t) * (size_t)n : 0, &ws.s_o1},
+                      {"conductance", conductance, conductance ? sizeof(float) * (size_t)n : 0, &ws.s_o2},
+                      {"accepted", accepted, accepted ? (size_t)n : 0, &ws.s_o3}};
+    DYG_TRY(check_places(H->device, in, 4, out, 3));
     const bool host_check = n <= kHostCheckMax;
     if (host_check) {
-        DYG_TRY(check_host_ids(src, n, H->g.n, "src"));
-        DYG_TRY(check_host_ids(dst, n, H->g.n, "dst"));
-        DYG_TRY(check_host_weights(w, n));
+        if (in[0].host) DYG_TRY(check_ids(src, n, H->g.n, "src"));
+        if (in[1].host) DYG_TRY(check_ids(dst, n, H->g.n, "dst"));
+        if (in[2].host) DYG_TRY(check_weights(w, n));
     }
-    Workspace &ws = H->ws;
-    const uint32_t *d_src, *d_dst;
-    const float *d_w;
-    DYG_TRY(stage_in(ws.s_src, src, n, st, &d_src));
-    DYG_TRY(stage_in(ws.s_dst, dst, n, st, &d_dst));
-    DYG_TRY(stage_in(ws.s_w, w, n, st, &d_w));
-    const uint64_t *d_uid = nullptr;
-    DYG_TRY(stage_in(ws.s_uid, uids, n, st, &d_uid));
-    // device outputs are written in place; host outputs go through staging
-    int32_t *o_found = found_at && on_device(found_at) ? found_at : nullptr;
-    float *o_cond = conductance && on_device(conductance) ? conductance : nullptr;
-    uint8_t *o_acc = accepted && on_device(accepted) ? accepted : nullptr;
-    if (found_at && !o_found) {
-        DYG_TRY(ensure(ws.s_o1, sizeof(int32_t) * n));
-        o_found = ptr<int32_t>(ws.s_o1);
-    }
-    if (conductance && !o_cond) {
-        DYG_TRY(ensure(ws.s_o2, sizeof(float) * n));
-        o_cond = ptr<float>(ws.s_o2);
-    }
-    if (accepted && !o_acc) {
-        DYG_TRY(ensure(ws.s_o3, sizeof(uint8_t) * n));
-        o_acc = ptr<uint8_t>(ws.s_o3);
-    }
+    size_t packed = 0;
+    DYG_TRY(stage_inputs(ws, in, 4, st));
+    DYG_TRY(place_outputs(ws, out, 3, &packed));
+    if (!any_host(out, 3)) packed = 0;
+    DYG_TRY(prepare_fetch(ws, packed, nullptr, n));
+    const std::function<dyg_status()> fetch = [&]() -> dyg_status {
+        if (packed) DYG_CUDA(cudaMemcpyAsync(ws.pin_out.p, ws.io_out.p, packed, cudaMemcpyDeviceToHost, st));
+        return DYG_OK;
+    };
     const uint32_t B = batch_size ? batch_size : dyg_reference_batch_size(n);
     // inputs read in place from device memory were not checked on the host
-    const bool dev_in = !host_check || d_src == src || d_dst == dst || d_w == w;
-    DYG_TRY(incremental_run(H, G, d_src, d_dst, d_w, n, B, uid_base,
-                            (const unsigned long long *)d_uid, *p, o_found, o_cond, o_acc,
-                            st, dev_in));
+    const bool dev_in = !host_check || !in[0].host || !in[1].host || !in[2].host;
+    DYG_TRY(incremental_run(H, G, (const uint32_t *)in[0].dev, (const uint32_t *)in[1].dev,
+                            (const float *)in[2].dev, n, B, uid_base,
+                            (const unsigned long long *)in[3].dev, *p, (int32_t *)out[0].dev,
+                            (float *)out[1].dev, (uint8_t *)out[2].dev, st, dev_in, nullptr, &fetch));
     if (H->ws.host_scalars[S_ERR]) DYG_TRY(check_device_errors(H, st));
-    bool host_out = false;
-    if (found_at && o_found != found_at) DYG_TRY(copy_out(found_at, (const int32_t *)o_found, n, st, &host_out));
-    if (conductance && o_cond != conductance) DYG_TRY(copy_out(conductance, (const float *)o_cond, n, st, &host_out));
-    if (accepted && o_acc != accepted) DYG_TRY(copy_out(accepted, (const uint8_t *)o_acc, n, st, &host_out));
-    if (host_out) DYG_CUDA(cudaStreamSynchronize(st));
+    bool wait = false;
+    DYG_TRY(deliver(ws, out, 3, packed, st, &wait));
+    if (wait) DYG_CUDA(cudaStreamSynchronize(st));
     return DYG_OK;
 }
 
@@ -711,49 +864,48 @@ static dyg_status decremental_common(dyg_graph *G, dyg_graph *H, const uint32_t 
     if (n == 0) return DYG_OK;
     DeviceGuard dg(G->device);
     cudaStream_t st = (cudaStream_t)stream;
-    {
-        const void *ps[] = {src, dst, uids, status, conductance, rec_src, rec_dst, rec_kind};
-        const char *nm[] = {"src", "dst", "update_ids", "status", "conductance",
-                            "rec_src", "rec_dst", "rec_kind"};
-        DYG_TRY(check_same_device(G->device, ps, nm, 8));
-    }
+    Workspace &ws = G->ws;
+    InArray in[] = {{"src", src, sizeof(uint32_t) * (size_t)n, &ws.s_src},
+                    {"dst", dst, sizeof(uint32_t) * (size_t)n, &ws.s_dst},
+                    {"update_ids", uids, sizeof(uint64_t) * (size_t)n, &ws.s_uid}};
+    // statuses and conductances are needed on the device even if not asked for
+    OutArray out[] = {{"status", status, sizeof(int32_t) * (size_t)n, &ws.s_o1},
+                      {"conductance", conductance, sizeof(float) * (size_t)n, &ws.s_o2}};
+    OutArray recs[] = {{"rec_src", rec_src, 0, nullptr},
+                       {"rec_dst", rec_dst, 0, nullptr},
+                       {"rec_kind", rec_kind, 0, nullptr}};
+    DYG_TRY(check_places(G->device, in, 3, out, 2));
+    DYG_TRY(check_places(G->device, nullptr, 0, recs, 3));
     const bool host_check = n <= kHostCheckMax;
     if (host_check) {
-        DYG_TRY(check_host_ids(src, n, G->g.n, "src"));
-        DYG_TRY(check_host_ids(dst, n, G->g.n, "dst"));
+        if (in[0].host) DYG_TRY(check_ids(src, n, G->g.n, "src"));
+        if (in[1].host) DYG_TRY(check_ids(dst, n, G->g.n, "dst"));
     }
-    Workspace &ws = G->ws;
-    const uint32_t *d_src, *d_dst;
-    DYG_TRY(stage_in(ws.s_src, src, n, st, &d_src));
-    DYG_TRY(stage_in(ws.s_dst, dst, n, st, &d_dst));
-    const uint64_t *d_uid = nullptr;
-    DYG_TRY(stage_in(ws.s_uid, uids, n, st, &d_uid));
-    int32_t *o_st = status && on_device(status) ? status : nullptr;
-    float *o_cd = conductance && on_device(conductance) ? conductance : nullptr;
-    if (!o_st) {
-        DYG_TRY(ensure(ws.s_o1, sizeof(int32_t) * n));
-        o_st = ptr<int32_t>(ws.s_o1);
-    }
-    if (!o_cd) {
-        DYG_TRY(ensure(ws.s_o2, sizeof(float) * n));
-        o_cd = ptr<float>(ws.s_o2);
-    }
+    RecordsOut rec{rec_src, rec_dst, rec_kind, rec_cap,
+                   (!rec_src || recs[0].host) && (!rec_dst || recs[1].host) && (!rec_kind || recs[2].host),
+                   any_host(recs, 3)};
+    size_t packed = 0;
+    DYG_TRY(stage_inputs(ws, in, 3, st));
+    DYG_TRY(place_outputs(ws, out, 2, &packed));
+    if (!any_host(out, 2)) packed = 0;
+    DYG_TRY(prepare_fetch(ws, packed, &rec, n));
+    const std::function<dyg_status()> fetch = [&]() -> dyg_status {
+        if (packed) DYG_CUDA(cudaMemcpyAsync(ws.pin_out.p, ws.io_out.p, packed, cudaMemcpyDeviceToHost, st));
+        return rec.fetch(ws, st);
+    };
     const uint32_t B = batch_size ? batch_size : dyg_reference_batch_size(n);
     uint64_t total = 0;
-    const bool dev_in = !host_check || d_src == src || d_dst == dst;
+    const bool dev_in = !host_check || !in[0].host || !in[1].host;
     G->last_rec = 0;
-    DYG_TRY(decremental_run(G, H, d_src, d_dst, n, B, uid_base, (const unsigned long long *)d_uid,
-                            *p, o_st, o_cd, &total, st, dev_in));
+    DYG_TRY(decremental_run(G, H, (const uint32_t *)in[0].dev, (const uint32_t *)in[1].dev, n, B,
+                            uid_base, (const unsigned long long *)in[2].dev, *p, (int32_t *)out[0].dev,
+                            (float *)out[1].dev, &total, st, dev_in, nullptr, &fetch));
     G->last_rec = total;
     if (G->ws.host_scalars[S_ERR]) DYG_TRY(check_device_errors(G, st));
-    bool host_out = false;
-    if (status && o_st != status) DYG_TRY(copy_out(status, (const int32_t *)o_st, n, st, &host_out));
-    if (conductance && o_cd != conductance) DYG_TRY(copy_out(conductance, (const float *)o_cd, n, st, &host_out));
-    const uint64_t nout = total < rec_cap ? total : rec_cap;
-    DYG_TRY(copy_out(rec_src, (const uint32_t *)ptr<uint32_t>(ws.rx2), nout, st, &host_out));
-    DYG_TRY(copy_out(rec_dst, (const uint32_t *)ptr<uint32_t>(ws.ry2), nout, st, &host_out));
-    DYG_TRY(copy_out(rec_kind, (const uint8_t *)ptr<uint8_t>(ws.rk2), nout, st, &host_out));
-    if (host_out) DYG_CUDA(cudaStreamSynchronize(st));
+    bool wait = false;
+    DYG_TRY(deliver(ws, out, 2, packed, st, &wait));
+    DYG_TRY(rec.deliver(ws, total, st, &wait));
+    if (wait) DYG_CUDA(cudaStreamSynchronize(st));
     if (n_rec) *n_rec = total;
     if (total > rec_cap && (rec_src || rec_dst || rec_kind)) {
         set_error("more recovered edges than rec_cap");
@@ -865,53 +1017,51 @@ dyg_status dyg_stream_file(dyg_graph *G, dyg_graph *H, uint32_t op, const uint32
     if (n == 0) return DYG_OK;
     DeviceGuard dg(G->device);
     cudaStream_t st = (cudaStream_t)stream;
-    {
-        const void *ps[] = {src, dst, w, status, conductance, rec_src, rec_dst, rec_kind};
-        const char *nm[] = {"src", "dst", "w", "status", "conductance", "rec_src", "rec_dst",
-                            "rec_kind"};
-        DYG_TRY(check_same_device(G->device, ps, nm, 8));
-    }
+    Workspace &ws = G->ws;
+    InArray in[] = {{"src", src, sizeof(uint32_t) * (size_t)n, &ws.s_src},
+                    {"dst", dst, sizeof(uint32_t) * (size_t)n, &ws.s_dst},
+                    {"w", w, sizeof(float) * (size_t)n, &ws.s_w}};
+    // statuses and conductances are needed on the device even if not asked for
+    OutArray out[] = {{"status", status, sizeof(int32_t) * (size_t)n, &ws.s_o1},
+                      {"conductance", conductance, sizeof(float) * (size_t)n, &ws.s_o2}};
+    OutArray recs[] = {{"rec_src", rec_src, 0, nullptr},
+                       {"rec_dst", rec_dst, 0, nullptr},
+                       {"rec_kind", rec_kind, 0, nullptr}};
+    // a deletion file's weights are not read, an insertion file has no records
+    const int nin = ins ? 3 : 2;
+    DYG_TRY(check_places(G->device, in, 3, out, 2));
+    DYG_TRY(check_places(G->device, nullptr, 0, recs, 3));
     const bool host_check = n <= kHostCheckMax;
     if (host_check) {
-        DYG_TRY(check_host_ids(src, n, G->g.n, "src"));
-        DYG_TRY(check_host_ids(dst, n, G->g.n, "dst"));
-        if (ins) DYG_TRY(check_host_weights(w, n));
+        if (in[0].host) DYG_TRY(check_ids(src, n, G->g.n, "src"));
+        if (in[1].host) DYG_TRY(check_ids(dst, n, G->g.n, "dst"));
+        if (ins && in[2].host) DYG_TRY(check_weights(w, n));
     }
-    Workspace &ws = G->ws;
-    const uint32_t *d_src, *d_dst;
-    const float *d_w = nullptr;
-    DYG_TRY(stage_in(ws.s_src, src, n, st, &d_src));
-    DYG_TRY(stage_in(ws.s_dst, dst, n, st, &d_dst));
-    if (ins) DYG_TRY(stage_in(ws.s_w, w, n, st, &d_w));
-    int32_t *o_st = status && on_device(status) ? status : nullptr;
-    float *o_cd = conductance && on_device(conductance) ? conductance : nullptr;
-    if (!o_st) {
-        DYG_TRY(ensure(ws.s_o1, sizeof(int32_t) * n));
-        o_st = ptr<int32_t>(ws.s_o1);
-    }
-    if (!o_cd) {
-        DYG_TRY(ensure(ws.s_o2, sizeof(float) * n));
-        o_cd = ptr<float>(ws.s_o2);
-    }
+    RecordsOut rec{rec_src, rec_dst, rec_kind, rec_cap,
+                   (!rec_src || recs[0].host) && (!rec_dst || recs[1].host) && (!rec_kind || recs[2].host),
+                   any_host(recs, 3)};
+    size_t packed = 0;
+    DYG_TRY(stage_inputs(ws, in, nin, st));
+    DYG_TRY(place_outputs(ws, out, 2, &packed));
+    if (!any_host(out, 2)) packed = 0;
+    DYG_TRY(prepare_fetch(ws, packed, ins ? nullptr : &rec, n));
+    const std::function<dyg_status()> fetch = [&]() -> dyg_status {
+        if (packed) DYG_CUDA(cudaMemcpyAsync(ws.pin_out.p, ws.io_out.p, packed, cudaMemcpyDeviceToHost, st));
+        return rec.fetch(ws, st);
+    };
     uint64_t total = 0;
-    const bool dev_in = !host_check || d_src == src || d_dst == dst || (ins && d_w == w);
+    const bool dev_in = !host_check || !in[0].host || !in[1].host || (ins && !in[2].host);
     if (!ins) G->last_rec = 0;
-    DYG_TRY(stream_file_run(G, H, op, d_src, d_dst, d_w, n, first_update_id, chunk, *p, o_st, o_cd,
-                            &total, st, dev_in));
+    DYG_TRY(stream_file_run(G, H, op, (const uint32_t *)in[0].dev, (const uint32_t *)in[1].dev,
+                            ins ? (const float *)in[2].dev : nullptr, n, first_update_id, chunk, *p,
+                            (int32_t *)out[0].dev, (float *)out[1].dev, &total, st, dev_in, &fetch));
     if (!ins) G->last_rec = total;
     if (G->ws.host_scalars[S_ERR]) DYG_TRY(check_device_errors(G, st));
     if (H->ws.host_scalars[S_ERR]) DYG_TRY(check_device_errors(H, st));
-    bool host_out = false;
-    if (status && o_st != status) DYG_TRY(copy_out(status, (const int32_t *)o_st, n, st, &host_out));
-    if (conductance && o_cd != conductance)
-        DYG_TRY(copy_out(conductance, (const float *)o_cd, n, st, &host_out));
-    const uint64_t nout = total < rec_cap ? total : rec_cap;
-    if (!ins) {
-        DYG_TRY(copy_out(rec_src, (const uint32_t *)ptr<uint32_t>(ws.rx2), nout, st, &host_out));
-        DYG_TRY(copy_out(rec_dst, (const uint32_t *)ptr<uint32_t>(ws.ry2), nout, st, &host_out));
-        DYG_TRY(copy_out(rec_kind, (const uint8_t *)ptr<uint8_t>(ws.rk2), nout, st, &host_out));
-    }
-    if (host_out) DYG_CUDA(cudaStreamSynchronize(st));
+    bool wait = false;
+    DYG_TRY(deliver(ws, out, 2, packed, st, &wait));
+    if (!ins) DYG_TRY(rec.deliver(ws, total, st, &wait));
+    if (wait) DYG_CUDA(cudaStreamSynchronize(st));
     if (n_rec) *n_rec = total;
     if (total > rec_cap && (rec_src || rec_dst || rec_kind)) {
         set_error("more recovered edges than rec_cap");

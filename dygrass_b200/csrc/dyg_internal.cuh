@@ -197,9 +197,11 @@ struct Workspace {
     Buf s_uid;                                // staged per-edge update ids
     Buf ix_base, ix_list, ix_words;           // row index of the weighted walks
     Buf scalars;                              // u64 scalars (see Scalar)
-    Buf counts;                               // u32 counts (see Count)
-    unsigned long long *host_scalars = nullptr;   // pinned mirror
-    uint32_t *host_counts = nullptr;              // pinned mirror
+    Buf counts;                               // u32 counts (see Count), behind the scalars
+    unsigned long long *host_scalars = nullptr;   // pinned mirror of scalars and counts
+    uint32_t *host_counts = nullptr;
+    Buf io_in, io_out;                        // a call's host arrays, packed
+    Buf pin_in, pin_out;                      // pinned host memory beside them
 };
 
 // Indices into Workspace::scalars (u64, device) and Workspace::counts (u32).
@@ -232,6 +234,8 @@ enum Count : int {
     C_WALKLIST = 3,   // stream file: new insertions to walk
     C_NCOUNTS = 4
 };
+
+constexpr size_t kScalarBytes = sizeof(unsigned long long) * S_NSCALARS + sizeof(uint32_t) * C_NCOUNTS;
 
 // Halt codes: (batch + 1) << 8 | kind << 4 | phase.
 constexpr unsigned long long kHaltArena = 1;    // an arena reservation did not fit
@@ -352,18 +356,21 @@ dyg_status rejected_inputs(dyg_graph *D, cudaStream_t st);
 // uids (device, may be null): per-edge update ids instead of uid_base + e.
 // `during`, if given, runs on the host once the first pass of batches is
 // enqueued and before the call waits for them: host work that overlaps the
-// device work.
+// device work.  `fetch`, if given, runs before every wait and enqueues copies
+// of the results, so that the last wait covers them.
 dyg_status incremental_run(dyg_graph *H, dyg_graph *G, const uint32_t *src, const uint32_t *dst,
                            const float *w, uint32_t n, uint32_t B, uint64_t uid_base,
                            const unsigned long long *uids, const dyg_walk_params &p, int32_t *found, float *cond, uint8_t *acc,
                            cudaStream_t st, bool check_inputs = false,
-                           const std::function<void()> *during = nullptr);
+                           const std::function<void()> *during = nullptr,
+                           const std::function<dyg_status()> *fetch = nullptr);
 dyg_status decremental_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, const uint32_t *dst,
                            uint32_t n, uint32_t B, uint64_t uid_base,
                            const unsigned long long *uids, const dyg_walk_params &p,
                            int32_t *status, float *cond, uint64_t *n_rec, cudaStream_t st,
                            bool check_inputs = false,
-                           const std::function<void()> *during = nullptr);
+                           const std::function<void()> *during = nullptr,
+                           const std::function<dyg_status()> *fetch = nullptr);
 
 dyg_status decr_delete_enqueue(dyg_graph *G, dyg_graph *H, const uint32_t *src,
                                const uint32_t *dst, uint32_t n, uint64_t uid0,
@@ -392,7 +399,8 @@ uint32_t stream_default_chunk(uint32_t n_vertices);
 dyg_status stream_file_run(dyg_graph *G, dyg_graph *H, uint32_t op, const uint32_t *src,
                            const uint32_t *dst, const float *w, uint32_t n, uint64_t uid0,
                            uint32_t chunk, const dyg_walk_params &p, int32_t *status, float *cond,
-                           uint64_t *n_rec, cudaStream_t st, bool check_inputs = false);
+                           uint64_t *n_rec, cudaStream_t st, bool check_inputs = false,
+                           const std::function<dyg_status()> *fetch = nullptr);
 
 // --- graph.cu
 dyg_status upload_graph(dyg_graph *G, uint32_t n, const uint64_t *row_ptr, const uint32_t *col,

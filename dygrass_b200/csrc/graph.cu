@@ -49,29 +49,17 @@ dyg_status ensure(Buf &b, size_t bytes) {
     return DYG_OK;
 }
 
-dyg_status read_scalars(dyg_graph *G, cudaStream_t st) {
-    Workspace &ws = G->ws;
-    DYG_CUDA(cudaMemcpyAsync(ws.host_scalars, ws.scalars.p, S_NSCALARS * sizeof(unsigned long long),
-                             cudaMemcpyDeviceToHost, st));
-    DYG_CUDA(cudaMemcpyAsync(ws.host_counts, ws.counts.p, C_NCOUNTS * sizeof(uint32_t),
-                             cudaMemcpyDeviceToHost, st));
-    DYG_CUDA(cudaStreamSynchronize(st));
-    if (ws.host_scalars[S_LONG]) G->long_rows = true;
-    return DYG_OK;
-}
+dyg_status read_scalars(dyg_graph *G, cudaStream_t st) { return read_scalars2(G, nullptr, st); }
 
 dyg_status read_scalars2(dyg_graph *A, dyg_graph *B, cudaStream_t st) {
-    if (!B || B == A) return read_scalars(A, st);
-    for (dyg_graph *G : {A, B}) {
-        Workspace &ws = G->ws;
-        DYG_CUDA(cudaMemcpyAsync(ws.host_scalars, ws.scalars.p,
-                                 S_NSCALARS * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-        DYG_CUDA(cudaMemcpyAsync(ws.host_counts, ws.counts.p, C_NCOUNTS * sizeof(uint32_t),
-                                 cudaMemcpyDeviceToHost, st));
-    }
+    if (B == A) B = nullptr;
+    for (dyg_graph *G : {A, B})
+        if (G)
+            DYG_CUDA(cudaMemcpyAsync(G->ws.host_scalars, G->ws.scalars.p, kScalarBytes,
+                                     cudaMemcpyDeviceToHost, st));
     DYG_CUDA(cudaStreamSynchronize(st));
     for (dyg_graph *G : {A, B})
-        if (G->ws.host_scalars[S_LONG]) G->long_rows = true;
+        if (G && G->ws.host_scalars[S_LONG]) G->long_rows = true;
     return DYG_OK;
 }
 

@@ -710,7 +710,8 @@ dyg_status incremental_run(dyg_graph *H, dyg_graph *G, const uint32_t *src, cons
                            const float *w, uint32_t n, uint32_t B, uint64_t uid_base,
                            const unsigned long long *uids, const dyg_walk_params &p, int32_t *found, float *cond, uint8_t *acc,
                            cudaStream_t st, bool check_inputs,
-                           const std::function<void()> *during) {
+                           const std::function<void()> *during,
+                           const std::function<dyg_status()> *fetch) {
     unsigned long long *sc = ptr<unsigned long long>(H->ws.scalars);
     unsigned long long *halt = sc + S_HALT;
     DYG_TRY(clear_halt(H, st));
@@ -728,6 +729,7 @@ dyg_status incremental_run(dyg_graph *H, dyg_graph *G, const uint32_t *src, cons
                                  acc ? acc + b0 : nullptr, st, b > b_start));
         }
         if (during && round == 0) (*during)();
+        if (fetch) DYG_TRY((*fetch)());
         DYG_TRY(read_scalars2(H, G, st));
         const unsigned long long h = H->ws.host_scalars[S_HALT];
         if (!h) return DYG_OK;
@@ -745,7 +747,8 @@ dyg_status decremental_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, cons
                            uint32_t n, uint32_t B, uint64_t uid_base,
                            const unsigned long long *uids, const dyg_walk_params &p,
                            int32_t *status, float *cond, uint64_t *n_rec, cudaStream_t st,
-                           bool check_inputs, const std::function<void()> *during) {
+                           bool check_inputs, const std::function<void()> *during,
+                           const std::function<dyg_status()> *fetch) {
     Workspace &ws = G->ws;
     unsigned long long *sc = ptr<unsigned long long>(ws.scalars);
     unsigned long long *halt = sc + S_HALT;
@@ -770,6 +773,7 @@ dyg_status decremental_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, cons
                                  b == b_start ? ph_start : 0, status + b0, cond + b0, st));
         }
         if (during && round == 0) (*during)();
+        if (fetch) DYG_TRY((*fetch)());
         DYG_TRY(read_scalars2(G, H, st));
         const unsigned long long h = ws.host_scalars[S_HALT];
         if (!h) {

@@ -519,7 +519,8 @@ dyg_status clear_halt(dyg_graph *D, cudaStream_t st) {
 dyg_status insert_file_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, const uint32_t *dst,
                            const float *w, uint32_t n, uint64_t uid0, uint32_t chunk,
                            const dyg_walk_params &p, int32_t *status, float *cond,
-                           cudaStream_t st, bool check_inputs) {
+                           cudaStream_t st, bool check_inputs,
+                           const std::function<dyg_status()> *fetch) {
     Workspace &wg = G->ws, &wh = H->ws;
     const uint32_t nc_max = n < chunk ? n : chunk;
     // every buffer at its final size before anything is enqueued: a resumed
@@ -552,6 +553,7 @@ dyg_status insert_file_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, cons
             const uint32_t nc = n - f0 < chunk ? n - f0 : chunk;
             DYG_TRY(insert_chunk_enqueue(G, H, c, chunk, nc, p, halt, status, cond, c > c0, st));
         }
+        if (fetch) DYG_TRY((*fetch)());
         DYG_TRY(read_scalars2(G, H, st));
         const unsigned long long h = wg.host_scalars[S_HALT];
         if (!h) return DYG_OK;
@@ -569,7 +571,7 @@ dyg_status insert_file_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, cons
 dyg_status delete_file_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, const uint32_t *dst,
                            uint32_t n, uint64_t uid0, uint32_t chunk, const dyg_walk_params &p,
                            int32_t *status, float *cond, uint64_t *n_rec, cudaStream_t st,
-                           bool check_inputs) {
+                           bool check_inputs, const std::function<dyg_status()> *fetch) {
     Workspace &ws = G->ws;
     unsigned long long *sc = ptr<unsigned long long>(ws.scalars);
     unsigned long long *halt = sc + S_HALT;
@@ -595,6 +597,7 @@ dyg_status delete_file_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, cons
             DYG_TRY(decr_walk_enqueue(G, H, f0, nc, ptr<uint32_t>(ws.counts) + C_FILTERED, p, halt,
                                       c, c == c_start ? ph_start : 0, status, cond, st, true));
         }
+        if (fetch) DYG_TRY((*fetch)());
         DYG_TRY(read_scalars2(G, H, st));
         const unsigned long long h = ws.host_scalars[S_HALT];
         if (!h) {
@@ -633,14 +636,15 @@ uint32_t stream_default_chunk(uint32_t n_vertices) {
 dyg_status stream_file_run(dyg_graph *G, dyg_graph *H, uint32_t op, const uint32_t *src,
                            const uint32_t *dst, const float *w, uint32_t n, uint64_t uid0,
                            uint32_t chunk, const dyg_walk_params &p, int32_t *status, float *cond,
-                           uint64_t *n_rec, cudaStream_t st, bool check_inputs) {
+                           uint64_t *n_rec, cudaStream_t st, bool check_inputs,
+                           const std::function<dyg_status()> *fetch) {
     *n_rec = 0;
     if (chunk == 0) chunk = stream_default_chunk(G->g.n);
     if (op == DYG_STREAM_INSERT)
         return insert_file_run(G, H, src, dst, w, n, uid0, chunk, p, status, cond, st,
-                               check_inputs);
+                               check_inputs, fetch);
     return delete_file_run(G, H, src, dst, n, uid0, chunk, p, status, cond, n_rec, st,
-                           check_inputs);
+                           check_inputs, fetch);
 }
 
 }  // namespace dyg

@@ -111,3 +111,34 @@ def test_weighted_hub_rows(dyg, oracle, leaves, repeat, huge):  # noqa: F811
     assert np.array_equal(r.rec_src, rx) and np.array_equal(r.rec_dst, ry)
     same_graph(G, Go)
     same_graph(H, Ho)
+
+
+@pytest.mark.parametrize("k", [1, 3, 40])
+@pytest.mark.parametrize("room", [10_000, 100])
+def test_records_beyond_those_fetched_ahead(dyg, oracle, k, room):  # noqa: F811
+    """k deletions that recover 89 edges each, into host buffers with and
+    without room for them."""
+    L = 90
+    base = np.repeat(np.arange(k) * L, L)
+    i = np.tile(np.arange(L), k)
+    gs, gd = (base + i).astype(np.uint32), (base + (i + 1) % L).astype(np.uint32)
+    gw = np.linspace(0.5, 2.0, k * L).astype(np.float32)
+    first = np.arange(k) * L
+    G = dyg.Graph.from_edges(k * L, gs, gd, gw)
+    H = dyg.Graph.from_edges(k * L, gs[first], gd[first], gw[first])
+    Go, Ho = oracle.OGraph(k * L, gs, gd, gw), oracle.OGraph(k * L, gs[first], gd[first], gw[first])
+    p = dyg.WalkParams.make(walkers=32)
+    st, cd, rx, ry, rk, _ = oracle.decremental(Go, Ho, gs[first], gd[first], p, batch_size=k)
+    assert len(rx) == 89 * k
+    out = (np.empty(k, np.int32), np.empty(k, np.float32), np.zeros(room, np.uint32), np.zeros(room, np.uint32),
+           np.zeros(room, np.uint8))
+    if len(rx) > room:
+        with pytest.raises(dyg.DygError):
+            dyg.decremental_stream_into(G, H, gs[first], gd[first], p, *out, room, batch_size=k)
+    else:
+        assert dyg.decremental_stream_into(G, H, gs[first], gd[first], p, *out, room, batch_size=k) == len(rx)
+    m = min(room, len(rx))
+    assert np.array_equal(out[0], st) and np.array_equal(out[1].view(np.uint32), cd.view(np.uint32))
+    assert np.array_equal(out[2][:m], rx[:m]) and np.array_equal(out[3][:m], ry[:m]) and np.array_equal(out[4][:m], rk[:m])
+    same_graph(G, Go)
+    same_graph(H, Ho)
