@@ -7,11 +7,11 @@
 // max_steps walks), so instead of the reference's one-block-per-edge with a
 // 512-thread barrier tree, each warp of a persistent grid keeps its 32 lanes
 // busy: a lane whose walker ends takes the next walker of the warp's current
-// edge, and the warp pulls a new edge from a global counter when the current
-// one is handed out.  The per-edge winner (max 1/R, lowest walker id) is a
-// 64-bit key reduced with atomicMax, so no barrier and no global scratch
-// arrays are needed.  Lanes refill in step with one another (every fourth
-// warp iteration), so the random-number blocks are drawn by whole warps.
+// chunk, and the warp pulls a new chunk (32 walkers of an edge) from a global
+// counter when that is handed out.  The per-edge winner (max 1/R, lowest
+// walker id) is a 64-bit key reduced with atomicMax, so no barrier and no
+// global scratch arrays are needed.  Lanes refill in step with one another
+// (every four moves), so the random-number blocks are drawn by whole warps.
 //
 // Draw d of walker k of update u is word d&3 of
 // Philox4x32-10({d>>2, k, u_lo, u_hi | domain<<24}, seed): any walker can be
@@ -646,181 +646,247 @@ __device__ __forceinline__ bool below_best(float R, float c) {
     return __frcp_rn(R) < c;
 }
 
-// Resident blocks per SM the register budget is sized for: 6 (40 registers)
-// for the uniform walks, 3 for the weighted ones (shared-memory segment sums).
-template <bool INCR, bool WEIGHTED, int MOVES>
-__global__ void __launch_bounds__(kWalkThreads, WEIGHTED ? 3 : 6) k_walk(WalkArgs a) {
-    // per-warp segment sums of the cooperative weighted search
-    __shared__ unsigned long long s_seg[WEIGHTED ? (kWalkThreads / 32) * kSegs : 1];
-    if (a.job.halt && *a.job.halt) return;
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t lt_mask = (1u << lane) - 1u;
-    const uint32_t n = job_count(a.job);
-    const uint32_t CW = a.chunk;                // walkers per chunk (divides walkers)
-    const uint32_t cpe = a.walkers / CW;        // chunks per edge
-    const uint32_t cpe_sh = (cpe & (cpe - 1u)) ? 32u : (uint32_t)(__ffs(cpe) - 1);
-    const unsigned long long n_chunks = (unsigned long long)n * cpe;
-    unsigned long long *work = a.scalars + S_WORK;
+// ---------------------------------------------------------- uniform walks
+// r mod d for d below kDivTab by a table of floor((2^32 - 1) / d): the high
+// word of r times it is the quotient or one less, so one correction makes the
+// remainder exact.  A shared-memory lookup and two multiplies take the place
+// of the general division's conversions and its reciprocal.
+constexpr uint32_t kDivTab = 256;
+__device__ __forceinline__ uint32_t rem_small(uint32_t r, uint32_t d, const uint32_t *s_div) {
+    if (d >= kDivTab) return r % d;
+    const uint32_t m = r - __umulhi(r, s_div[d]) * d;
+    return m >= d ? m - d : m;
+}
 
-    // warp-uniform: the edge and walker range of the current chunk
-    uint32_t ce = 0xFFFFFFFFu, c_next = 0u, c_end = 0u;
+// ------------------------------------------------------- handing out walkers
+// Edge of a warp's current chunk of walkers.
+struct ChunkEdge {
+    uint32_t src, tgt, e;
+    float we;
+    uint32_t c2, c3;
+};
+// Warp-uniform: the walkers left of the current chunk.
+struct Chunk {
+    uint32_t next = 0u, end = 0u;
     bool exhausted = false;
-    // best conductance bits seen in this warp for the current chunk's edge and
-    // the previous one (warp-uniform)
-    uint32_t ce_best = 0u, pe = 0xFFFFFFFFu, pe_best = 0u;
+};
 
+// Starts walkers in the warp's free lanes.  One lane takes a chunk from the
+// global counter and reads its edge into shared memory, from where the lanes
+// that start its walkers take it; it also counts the chunk's walks (a walker
+// that started ends before the kernel does).  `start(edge, walker)` runs in
+// each lane that takes a walker.
+template <bool INCR, class Start>
+__device__ __forceinline__ void refill(const WalkArgs &a, unsigned long long n_chunks, Chunk &c,
+                                       ChunkEdge *ce, uint32_t lane, uint32_t free_mask,
+                                       uint32_t *walks, Start start) {
+    while (free_mask != 0u && !c.exhausted) {
+        if (c.next >= c.end) {
+            __syncwarp();   // the lanes that took the last chunk's walkers have read its edge
+            uint32_t first = 0u, have = 0u;
+            if (lane == 0u) {
+                const uint32_t cpe = a.walkers / a.chunk;   // chunks per edge
+                const unsigned long long t = atomicAdd(a.scalars + S_WORK, 1ull);
+                if (t < n_chunks) {
+                    // chunk t = edge e, part t mod cpe
+                    const uint32_t e = (t >> 32) ? (uint32_t)(t / cpe) : (uint32_t)t / cpe;
+                    first = (uint32_t)(t - (unsigned long long)e * cpe) * a.chunk;
+                    const unsigned long long uid = a.job.uid ? a.job.uid[e] : a.job.uid0 + e;
+                    const ChunkEdge x{a.job.src[e], a.job.dst[e], e, INCR ? a.job.w[e] : 0.f,
+                                      (uint32_t)uid, ctr3_of(uid, a.job.domain)};
+                    *ce = x;
+                    *walks += a.chunk;
+                    have = 1u;
+                    if (x.src >= a.g.n || x.tgt >= a.g.n) {
+                        atomicOr(a.scalars + S_ERR, (unsigned long long)kErrVertex);
+                        have = 2u;
+                    }
+                }
+            }
+            __syncwarp();
+            have = __shfl_sync(kFull, have, 0);
+            if (have == 0u) {
+                c.exhausted = true;
+                break;
+            }
+            if (have == 2u) continue;   // not walked
+            c.next = __shfl_sync(kFull, first, 0);
+            c.end = c.next + a.chunk;
+        }
+        const uint32_t take = min((uint32_t)__popc(free_mask), c.end - c.next);
+        const uint32_t rank = __popc(free_mask & ((1u << lane) - 1u));
+        const bool mine = ((free_mask >> lane) & 1u) && rank < take;
+        if (mine) start(*ce, c.next + rank);
+        free_mask &= ~__ballot_sync(kFull, mine);
+        c.next += take;
+    }
+}
+
+__device__ __forceinline__ void count_moves(const WalkArgs &a, uint32_t moves, uint32_t walks,
+                                            uint32_t lane) {
+    const uint32_t wm = __reduce_add_sync(kFull, moves);
+    if (lane == 0u) {
+        if (wm) atomicAdd(a.scalars + S_MOVES, (unsigned long long)wm);
+        if (walks) atomicAdd(a.scalars + S_WALKS, (unsigned long long)walks);
+    }
+}
+
+// Conductance bits of the best walk an edge has so far.
+__device__ __forceinline__ uint32_t best_bits(const WalkArgs &a, uint32_t e) {
+    return *(reinterpret_cast<const volatile uint32_t *>(a.keys + e) + 1);
+}
+
+// The uniform transition's walks.  Walks are short (5.8 moves on the mesh's
+// sparsifier: most end in a leaf), so the cost is shared between the moves and
+// what surrounds them; every iteration starts walkers in the free lanes and
+// then moves each walker four times, so that a walker enters every iteration
+// at a step 1 mod 4 and draws one Philox block for it, and the step counter
+// advances once per iteration.  The edge's best is read once per iteration,
+// after the moves, by the walkers still alive: R only grows along a walk and
+// 1/R is monotone, so a walker whose 1/R is below it can neither win nor tie,
+// and stopping it leaves every result unchanged.
+// 40 registers: six blocks (48 warps) per SM; eight blocks spill (insertions
+// of the 100^3 mesh 4.43 -> 6.43 ms).  Bound by instruction issue on a
+// sparsifier (65-70 % of cycles) and by gather latency and the L1's
+// throughput (70 %) on the dense graph.  Against one lane-private edge read
+// and best per walker and the general remainder: insertions of the 100^3 mesh
+// 5.27 -> 4.43 ms, 24 random geometric graphs 1.14 -> 0.96 ms, deletions of
+// the mesh 2.28 -> 2.25 ms.
+template <bool INCR>
+__global__ void __launch_bounds__(kWalkThreads, 6) k_walk_uniform(WalkArgs a) {
+    __shared__ uint32_t s_div[kDivTab];
+    __shared__ ChunkEdge s_edge[kWalkThreads / 32];
+    if (a.job.halt && *a.job.halt) return;
+    for (uint32_t d = threadIdx.x; d < kDivTab; d += kWalkThreads) s_div[d] = d ? 0xFFFFFFFFu / d : 0u;
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31u;
+    ChunkEdge *ce = s_edge + (threadIdx.x >> 5);
+    const unsigned long long n_chunks = (unsigned long long)job_count(a.job) * (a.walkers / a.chunk);
+    Chunk chunk;
     bool active = false;
-    uint32_t my_e = 0xFFFFFFFFu;
-    uint32_t gbest = 0u;  // lane: last read of the edge's global best (cond bits)
-    Walker s;
-    s.cur = s.prev = s.step = s.tgt = s.walker = s.c2 = s.c3 = 0u;
-    s.rblk = 0xFFFFFFFFu;
-    s.rbuf = make_uint4(0u, 0u, 0u, 0u);
-    s.R = 0.f;
-    s.we = 0.f;
+    uint32_t cur = 0u, prev = 0u, step = 0u, tgt = 0u, walker = 0u, c2 = 0u, c3 = 0u, my_e = 0u;
+    float R = 0.f, we = 0.f;
     uint32_t moves = 0u, walks = 0u;
-
-    // Walkers start only on warp iterations that keep every walker of the
-    // warp aligned to its 4-draw Philox blocks (each walker moves MOVES times
-    // per iteration): then all of them draw their next block at the same
-    // move, so the block (a quarter of the kernel's instructions when
-    // computed) runs for the whole warp at once instead of for a few lanes at
-    // a time, and refills are batched.  An empty warp refills at once.
-    uint32_t T = 0u;
-    while (true) {
-        uint32_t free_mask = __ballot_sync(kFull, !active);
-        if (free_mask == kFull) T = 0u;
-        // walkers start when their steps stay aligned to the 4-draw Philox
-        // blocks: every fourth iteration with one move per iteration, every
-        // second with two, every iteration with four
-        constexpr uint32_t kAlign = MOVES >= 4 ? 0u : (MOVES == 2 ? 1u : 3u);
-        const bool refill = (T & kAlign) == 0u;
-        while (free_mask != 0u && !exhausted && refill) {
-            if (c_next >= c_end) {
-                unsigned long long c = 0ull;
-                if (lane == 0u) c = atomicAdd(work, 1ull);
-                c = __shfl_sync(kFull, c, 0);
-                if (c >= n_chunks) {
-                    exhausted = true;
+    for (uint32_t T = 0u;; ++T) {
+        refill<INCR>(a, n_chunks, chunk, ce, lane, __ballot_sync(kFull, !active), &walks,
+                     [&](const ChunkEdge &x, uint32_t k) {
+                         walker = k;
+                         cur = x.src;
+                         tgt = x.tgt;
+                         my_e = x.e;
+                         we = x.we;
+                         c2 = x.c2;
+                         c3 = x.c3;
+                         step = 1u;
+                         R = 0.f;
+                         active = true;
+                     });
+        if (!__any_sync(kFull, active)) break;
+        if (active) {
+            const uint4 blk = philox4x32_10(make_uint4((step - 1u) >> 2, walker, c2, c3), a.key);
+            const uint32_t left = a.max_steps - step;   // the walk ends when its step reaches max_steps
+#pragma unroll
+            for (uint32_t mv = 0; mv < 4u; ++mv) {
+                if (!active) break;
+                const uint2 d = __ldg(a.g.desc + cur);
+                const bool first = mv == 0u && step == 1u;
+                // step 1: any neighbour; later: dead end if deg == 1, else
+                // r % (deg - 1) and the last slot when the draw lands on the
+                // previous vertex (main.cu:99-137)
+                const uint32_t deg = first ? d.y : d.y - 1u;
+                if ((int)deg <= 0) {
+                    active = false;
                     break;
                 }
-                // chunk c = edge e, part c mod cpe (cpe is a power of two
-                // whenever the walker count is one)
-                const uint32_t e = (c >> 32) ? (uint32_t)(c / cpe)
-                                             : (cpe_sh < 32u ? (uint32_t)c >> cpe_sh
-                                                             : (uint32_t)c / cpe);
-                if (e != ce) {
-                    pe = ce;
-                    pe_best = ce_best;
-                    ce = e;
-                    ce_best = 0u;
+                const uint32_t r = mv == 0u ? blk.x : (mv == 1u ? blk.y : (mv == 2u ? blk.z : blk.w));
+                const uint2 *row = a.g.slots + d.x;
+                uint2 sl = __ldg(row + rem_small(r, deg, s_div));
+                if (!first) {
+                    // loaded beside the drawn slot: some lane lands on its
+                    // previous vertex in almost every move
+                    const uint2 last = __ldg(row + deg);
+                    if (sl.x == prev) sl = last;
                 }
-                c_next = (uint32_t)(c - (unsigned long long)e * cpe) * CW;
-                c_end = c_next + CW;
-            }
-            const uint32_t take = min((uint32_t)__popc(free_mask), c_end - c_next);
-            const uint32_t rank = __popc(free_mask & lt_mask);
-            if (((free_mask >> lane) & 1u) && rank < take) {
-                const uint32_t e = ce;
-                my_e = e;
-                s.walker = c_next + rank;
-                s.cur = a.job.src[e];
-                s.tgt = a.job.dst[e];
-                s.we = INCR ? a.job.w[e] : 0.f;
-                const unsigned long long uid = a.job.uid ? a.job.uid[e] : a.job.uid0 + e;
-                s.c2 = (uint32_t)uid;
-                s.c3 = ctr3_of(uid, a.job.domain);
-                s.rblk = 0xFFFFFFFFu;
-                s.step = 1u;
-                s.R = 0.f;
-                s.prev = 0u;
-                gbest = a.prune ? (uint32_t)(*(volatile unsigned long long *)(a.keys + e) >> 32) : 0u;
-                if (s.cur >= a.g.n || s.tgt >= a.g.n) {
-                    atomicOr(a.scalars + S_ERR, (unsigned long long)kErrVertex);
-                    ++walks;
-                } else {
-                    active = true;
+                ++moves;
+                R = __fadd_rn(R, __uint_as_float(sl.y));
+                if (INCR && !first && __fmul_rn(R, we) >= a.threshold) {
+                    active = false;
+                } else if (sl.x == tgt) {
+                    // published at once, so the edge's other walkers can stop early
+                    atomicMax(a.keys + my_e, pack_key(__frcp_rn(R), walker, step + mv));
+                    active = false;
+                } else if (mv + 1u >= left) {
+                    active = false;
                 }
+                prev = cur;
+                cur = sl.x;
             }
-            // the lanes that took a walker leave the free mask
-            free_mask = __ballot_sync(kFull, ((free_mask >> lane) & 1u) && rank >= take);
-            c_next += take;
+            step += 4u;
+            if (active && a.prune && (T & (a.prune_every - 1u)) == a.prune_every - 1u) {
+                const uint32_t known = best_bits(a, my_e);
+                if (known && below_best(R, __uint_as_float(known))) active = false;
+            }
         }
+    }
+    count_moves(a, moves, walks, lane);
+}
+
+// The weighted transition's walks: as the uniform ones, but a move costs a
+// look at the whole row (or its index), so the bound is applied after every
+// move, and read again after every fourth.  Three blocks per SM.
+template <bool INCR>
+__global__ void __launch_bounds__(kWalkThreads, 3) k_walk_weighted(WalkArgs a) {
+    __shared__ unsigned long long s_seg[(kWalkThreads / 32) * kSegs];
+    __shared__ ChunkEdge s_edge[kWalkThreads / 32];
+    if (a.job.halt && *a.job.halt) return;
+    const uint32_t lane = threadIdx.x & 31u;
+    ChunkEdge *ce = s_edge + (threadIdx.x >> 5);
+    unsigned long long *seg = s_seg + (threadIdx.x >> 5) * kSegs;
+    const unsigned long long n_chunks = (unsigned long long)job_count(a.job) * (a.walkers / a.chunk);
+    Chunk chunk;
+    bool active = false;
+    uint32_t my_e = 0u, known = 0u;
+    Walker s{};
+    uint32_t moves = 0u, walks = 0u;
+    for (uint32_t T = 0u;; ++T) {
+        refill<INCR>(a, n_chunks, chunk, ce, lane, __ballot_sync(kFull, !active), &walks,
+                     [&](const ChunkEdge &x, uint32_t k) {
+                         s.walker = k;
+                         s.cur = x.src;
+                         s.tgt = x.tgt;
+                         s.we = x.we;
+                         s.c2 = x.c2;
+                         s.c3 = x.c3;
+                         s.rblk = 0xFFFFFFFFu;
+                         s.step = 1u;
+                         s.R = 0.f;
+                         s.prev = 0u;
+                         my_e = x.e;
+                         known = a.prune ? best_bits(a, x.e) : 0u;
+                         active = true;
+                     });
         if (!__any_sync(kFull, active)) break;
-        uint32_t fc = 0u;  // conductance bits of a walker that found its target now
-        // With four moves per iteration every walker enters an iteration at a
-        // step = 1 (mod 4) (walkers start at the top of an iteration and move
-        // four times in each one they stay in), so its Philox block for the
-        // iteration is drawn once, up front, and word mv serves move mv.
-        uint4 blk = make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-        for (int mv = 0; mv < (WEIGHTED ? 1 : MOVES); ++mv) {
-            int r = kContinue;
+#pragma unroll 1
+        for (uint32_t mv = 0; mv < 4u; ++mv) {
             bool moved = false;
             uint2 taken;
             uint32_t taken_at;
-            if constexpr (WEIGHTED) {
-                r = step_weighted_warp<INCR>(s, active, a.g, a.ix, a.max_steps, a.threshold, a.key,
-                                             s_seg + (threadIdx.x >> 5) * kSegs, lane, &moved,
-                                             &taken, &taken_at);
-            } else if (MOVES == 4 && active) {
-                const uint2 d = __ldg(a.g.desc + s.cur);
-                if (mv == 0)
-                    blk = philox4x32_10(make_uint4((s.step - 1u) >> 2, s.walker, s.c2, s.c3), a.key);
-                const uint32_t rd = mv == 0 ? blk.x : (mv == 1 ? blk.y : (mv == 2 ? blk.z : blk.w));
-                r = (s.step == 1u ? d.y == 0u : d.y <= 1u)
-                        ? kFail
-                        : move_uniform<INCR>(s, d, rd, a.g.slots, a.max_steps, a.threshold, &moved,
-                                             &taken, &taken_at);
-            } else if (active) {
-                r = step_once<INCR, false>(s, a.g.desc, a.g.slots, a.g.wts, a.max_steps,
-                                           a.threshold, a.key, &moved, &taken, &taken_at);
-            }
+            const int r = step_weighted_warp<INCR>(s, active, a.g, a.ix, a.max_steps, a.threshold, a.key,
+                                                   seg, lane, &moved, &taken, &taken_at);
             if (active) {
                 moves += moved ? 1u : 0u;
-                if (r != kContinue) {
-                    if (r == kFound) {
-                        const float cond = __frcp_rn(s.R);
-                        fc = __float_as_uint(cond);
-                        // published at once, so walkers of this edge in other
-                        // warps can stop early
-                        atomicMax(a.keys + my_e, pack_key(cond, s.walker, s.step));
-                    }
-                    active = false;
-                    ++walks;
-                }
+                if (r == kFound)
+                    atomicMax(a.keys + my_e, pack_key(__frcp_rn(s.R), s.walker, s.step));
+                if (r != kContinue || (known && below_best(s.R, __uint_as_float(known)))) active = false;
             }
+            if (!__any_sync(kFull, active)) break;
         }
-        if (a.prune) {
-            // R only grows along a walk and 1/R is monotone, so a walker whose
-            // 1/R is already below its edge's best success can neither win
-            // nor tie: stopping it leaves every result unchanged.
-            if (__any_sync(kFull, fc != 0u)) {
-                ce_best = max(ce_best, __reduce_max_sync(kFull, (fc && my_e == ce) ? fc : 0u));
-                pe_best = max(pe_best, __reduce_max_sync(kFull, (fc && my_e == pe) ? fc : 0u));
-            }
-            if (active) {
-                // the edge's best is read again every fourth move
-                constexpr uint32_t kEvery = MOVES >= 4 ? 1u : (MOVES == 2 ? 2u : 4u);
-                const uint32_t pm = kEvery * a.prune_every - 1u;
-                if ((T & pm) == pm)
-                    gbest = max(gbest, (uint32_t)(*(volatile unsigned long long *)(a.keys + my_e) >> 32));
-                const uint32_t known = max(gbest, (my_e == ce) ? ce_best
-                                                  : (my_e == pe ? pe_best : 0u));
-                if (known && below_best(s.R, __uint_as_float(known))) {
-                    active = false;
-                    ++walks;
-                }
-            }
+        if (active && a.prune && (T & (a.prune_every - 1u)) == a.prune_every - 1u) {
+            known = best_bits(a, my_e);
+            if (known && below_best(s.R, __uint_as_float(known))) active = false;
         }
-        ++T;
     }
-    const uint32_t wm = __reduce_add_sync(kFull, moves);
-    const uint32_t ww = __reduce_add_sync(kFull, walks);
-    if (lane == 0u) {
-        if (wm) atomicAdd(a.scalars + S_MOVES, (unsigned long long)wm);
-        if (ww) atomicAdd(a.scalars + S_WALKS, (unsigned long long)ww);
-    }
+    count_moves(a, moves, walks, lane);
 }
 
 // Replays the winner of each decremental edge and writes its path
@@ -956,61 +1022,32 @@ static uint32_t chunk_for(uint32_t walkers) {
     return c;
 }
 
-// Resident blocks per SM, cached per kernel instance (the instances share one
-// function type but not their launch bounds).
-template <bool INCR, bool WTD, int MOVES>
-static int persistent_blocks() {
-    static int per_sm = 0;
-    if (!per_sm) {
-        int nb = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_walk<INCR, WTD, MOVES>, kWalkThreads, 0);
-        per_sm = nb < 1 ? 1 : nb;
-    }
-    const uint32_t t = g_tune_bpsm.load();
-    const int b = (t && (int)t < per_sm) ? (int)t : per_sm;
-    return b * num_sms();
-}
-
-// Moves per warp iteration of the uniform walk: 4 by default (the warp's
-// refill, prune and loop bookkeeping then runs once per four moves; walk time
-// per step on the 100^3 mesh: 11.08 ms with one move, 9.99 with two, 9.64 with
-// four); DYG_WALK_MOVES = 1, 2 or 4 overrides it for tuning runs.  Results do
-// not depend on it.
-static int walk_moves() {
-    static int m = 0;
-    if (!m) {
-        const char *v = getenv("DYG_WALK_MOVES");
-        const int x = v ? atoi(v) : 4;
-        m = (x == 1 || x == 2) ? x : 4;
-    }
-    return m;
-}
-
-template <bool INCR, bool WTD>
+// The persistent grid: as many blocks as fit (or dyg_tune_set allows), but no
+// more warps than there are chunks, since each idle warp costs an atomic on
+// the chunk counter: a 32-edge batch has 512 chunks for 7,104 warps.
+template <auto Kernel>
 static void launch_walk_kernel(const WalkArgs &a, cudaStream_t st) {
-    if constexpr (!WTD) {
-        if (walk_moves() == 2) {
-            const int grid = persistent_blocks<INCR, WTD, 2>();
-            k_walk<INCR, WTD, 2><<<grid, kWalkThreads, 0, st>>>(a);
-            return;
-        }
-        if (walk_moves() == 4) {
-            const int grid = persistent_blocks<INCR, WTD, 4>();
-            k_walk<INCR, WTD, 4><<<grid, kWalkThreads, 0, st>>>(a);
-            return;
-        }
-    }
-    const int grid = persistent_blocks<INCR, WTD, 1>();
-    k_walk<INCR, WTD, 1><<<grid, kWalkThreads, 0, st>>>(a);
+    static const int per_sm = [] {
+        int nb = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, Kernel, kWalkThreads, 0);
+        return nb < 1 ? 1 : nb;
+    }();
+    const uint32_t t = g_tune_bpsm.load();
+    const uint64_t fit = (uint64_t)((t && (int)t < per_sm) ? (int)t : per_sm) * num_sms();
+    const uint64_t chunks = (uint64_t)a.job.n_host * (a.walkers / a.chunk);
+    // four chunks' warps to a block of eight while SMs are idle: half-empty
+    // blocks spread a small batch over more of them
+    const uint64_t want = (chunks + 3) / 4;
+    Kernel<<<(unsigned)(want < 1 ? 1 : (want < fit ? want : fit)), kWalkThreads, 0, st>>>(a);
 }
 
 static void launch_walk_any(const WalkArgs &a, bool incremental, bool wtd, cudaStream_t st) {
     if (incremental) {
-        if (wtd) launch_walk_kernel<true, true>(a, st);
-        else launch_walk_kernel<true, false>(a, st);
+        if (wtd) launch_walk_kernel<k_walk_weighted<true>>(a, st);
+        else launch_walk_kernel<k_walk_uniform<true>>(a, st);
     } else {
-        if (wtd) launch_walk_kernel<false, true>(a, st);
-        else launch_walk_kernel<false, false>(a, st);
+        if (wtd) launch_walk_kernel<k_walk_weighted<false>>(a, st);
+        else launch_walk_kernel<k_walk_uniform<false>>(a, st);
     }
 }
 

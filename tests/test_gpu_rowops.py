@@ -142,3 +142,17 @@ def test_records_beyond_those_fetched_ahead(dyg, oracle, k, room):  # noqa: F811
     assert np.array_equal(out[2][:m], rx[:m]) and np.array_equal(out[3][:m], ry[:m]) and np.array_equal(out[4][:m], rk[:m])
     same_graph(G, Go)
     same_graph(H, Ho)
+
+
+# the walk's remainder changes from the table to the general division at 256
+@pytest.mark.parametrize("leaves", [1, 2, 253, 254, 255, 256, 257, 2000])
+@pytest.mark.parametrize("steps", [1, 2, 4, 5, 40])
+def test_uniform_degrees_and_lengths(dyg, oracle, leaves, steps):  # noqa: F811
+    rng = np.random.default_rng(leaves + steps)
+    n = leaves + 30
+    hs, hd, hw = star(n, leaves, rng)
+    es = np.concatenate([np.zeros(8, np.int64), rng.integers(1, n, 24)]).astype(np.uint32)
+    ed = ((es + 1 + rng.integers(0, n - 1, 32)) % n).astype(np.uint32)
+    ew = rng.uniform(0.01, 0.05, 32).astype(np.float32)
+    p = dyg.WalkParams.make(threshold=10.0, walkers=96, max_steps=steps)
+    run_incr_both(dyg, oracle, n, hs, hd, hw, es, ed, ew, p, batch_size=20)
