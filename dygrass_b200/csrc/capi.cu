@@ -86,6 +86,8 @@ bool on_device(const void *p) {
 // 130 us of a 32-edge batch.  Larger arrays are copied one by one (staging
 // them would cost the host a pass over memory that the copies overlap).
 constexpr size_t kPackMax = 1u << 20;
+constexpr size_t kScalarPinned = 256;   // bytes of a handle's pinned mirror
+static_assert(kScalarBytes <= kScalarPinned, "the mirror holds scalars and counts");
 
 struct InArray {
     const char *name;
@@ -109,11 +111,11 @@ size_t align16(size_t b) { return (b + 15) & ~(size_t)15; }
 
 dyg_status ensure_pinned(Buf &b, size_t bytes) {
     if (b.bytes >= bytes) return DYG_OK;
-    if (b.p) cudaFreeHost(b.p);
+    host_free(b.p, b.bytes);
     b = Buf{};
     size_t want = 4096;
     while (want < bytes) want *= 2;
-    DYG_CUDA(cudaMallocHost(&b.p, want));
+    DYG_CUDA(host_alloc(&b.p, want));
     b.bytes = want;
     return DYG_OK;
 }
@@ -353,14 +355,14 @@ dyg_status graph_alloc_scalars(dyg_graph *G) {
     DYG_TRY(ensure(G->ws.scalars, kScalarBytes));
     DYG_CUDA(cudaMemset(G->ws.scalars.p, 0, kScalarBytes));
     G->ws.counts.p = ptr<unsigned long long>(G->ws.scalars) + S_NSCALARS;
-    DYG_CUDA(cudaMallocHost(&G->ws.host_scalars, kScalarBytes));
+    DYG_CUDA(host_alloc((void **)&G->ws.host_scalars, kScalarPinned));
     G->ws.host_counts = reinterpret_cast<uint32_t *>(G->ws.host_scalars + S_NSCALARS);
     G->g.top = ptr<unsigned long long>(G->ws.scalars) + S_TOP;
     return DYG_OK;
 }
 
 void free_buf(Buf &b) {
-    if (b.p) cudaFree(b.p);
+    dev_free(b.p);
     b.p = nullptr;
     b.bytes = 0;
 }
@@ -368,6 +370,7 @@ void free_buf(Buf &b) {
 void free_graph(dyg_graph *G) {
     if (!G) return;
     DeviceGuard dg(G->device);
+    cudaDeviceSynchronize();   // the blocks below may be handed out again at once
     Workspace &ws = G->ws;
     Buf *bufs[] = {&ws.keys, &ws.flags, &ws.pos, &ws.f_src, &ws.f_dst, &ws.f_idx, &ws.f_uid,
                    &ws.f_w, &ws.found, &ws.path_v, &ws.path_s, &ws.path_len, &ws.cand_x, &ws.cand_y,
@@ -377,13 +380,13 @@ void free_graph(dyg_graph *G) {
                    &ws.st_val, &ws.st_pos, &ws.st_wapp, &ws.big, &ws.s_uid, &ws.ix_base,
                    &ws.ix_list, &ws.ix_words, &ws.scalars, &ws.io_in, &ws.io_out};
     for (Buf *b : bufs) free_buf(*b);
-    if (ws.host_scalars) cudaFreeHost(ws.host_scalars);
-    if (ws.pin_in.p) cudaFreeHost(ws.pin_in.p);
-    if (ws.pin_out.p) cudaFreeHost(ws.pin_out.p);
-    if (G->g.desc) cudaFree(G->g.desc);
-    if (G->g.cap) cudaFree(G->g.cap);
-    if (G->g.slots) cudaFree(G->g.slots);
-    if (G->g.wts) cudaFree(G->g.wts);
+    host_free(ws.host_scalars, kScalarPinned);
+    host_free(ws.pin_in.p, ws.pin_in.bytes);
+    host_free(ws.pin_out.p, ws.pin_out.bytes);
+    dev_free(G->g.desc);
+    dev_free(G->g.cap);
+    dev_free(G->g.slots);
+    dev_free(G->g.wts);
     cudaGetLastError();
     delete G;
 }
@@ -409,10 +412,10 @@ dyg_status create_empty_graph(uint32_t n, uint64_t arena_slots, int device, uint
     G->g.arena_cap = arena_slots;
     dyg_status rc = graph_alloc_scalars(G);
     if (rc == DYG_OK &&
-        (cudaMalloc(&G->g.desc, sizeof(uint2) * (size_t)(n ? n : 1)) != cudaSuccess ||
-         cudaMalloc(&G->g.cap, sizeof(uint32_t) * (size_t)(n ? n : 1)) != cudaSuccess ||
-         cudaMalloc(&G->g.slots, sizeof(uint2) * (size_t)arena_slots) != cudaSuccess ||
-         cudaMalloc(&G->g.wts, sizeof(float) * (size_t)arena_slots) != cudaSuccess)) {
+        (dev_alloc(&G->g.desc, sizeof(uint2) * (size_t)(n ? n : 1)) != cudaSuccess ||
+         dev_alloc(&G->g.cap, sizeof(uint32_t) * (size_t)(n ? n : 1)) != cudaSuccess ||
+         dev_alloc(&G->g.slots, sizeof(uint2) * (size_t)arena_slots) != cudaSuccess ||
+         dev_alloc(&G->g.wts, sizeof(float) * (size_t)arena_slots) != cudaSuccess)) {
         cudaGetLastError();
         set_error("cudaMalloc of a pool graph failed");
         rc = DYG_ENOMEM;
@@ -491,50 +494,34 @@ dyg_status dyg_graph_create_from_edges(uint32_t n_vertices, uint64_t n_edges, co
         set_error("too many edges");
         return DYG_EINVAL;
     }
-    DYG_TRY(check_host_ids(src, n_edges, n_vertices, "src"));
-    DYG_TRY(check_host_ids(dst, n_edges, n_vertices, "dst"));
-    DYG_TRY(check_host_weights(w, n_edges));
+    // like a batch's, long lists are checked on the device, as they are read
+    if (n_edges <= kHostCheckMax) {
+        DYG_TRY(check_ids(src, n_edges, n_vertices, "src"));
+        DYG_TRY(check_ids(dst, n_edges, n_vertices, "dst"));
+        DYG_TRY(check_weights(w, n_edges));
+    }
     dyg_graph_opts o;
     dyg_graph_opts_default(&o);
     if (opts) o = *opts;
     int dev = o.device;
     if (dev < 0) DYG_CUDA(cudaGetDevice(&dev));
     DeviceGuard dg(dev);
-    // rows in file order (functions.cpp:130-232): count, prefix, fill
-    uint64_t *row_ptr = (uint64_t *)calloc((size_t)n_vertices + 1, sizeof(uint64_t));
-    uint32_t *col = (uint32_t *)malloc(sizeof(uint32_t) * (size_t)(2 * n_edges + 1));
-    float *ww = (float *)malloc(sizeof(float) * (size_t)(2 * n_edges + 1));
-    uint64_t *fill = (uint64_t *)calloc((size_t)n_vertices + 1, sizeof(uint64_t));
-    if (!row_ptr || !col || !ww || !fill) {
-        free(row_ptr); free(col); free(ww); free(fill);
-        set_error("host allocation failed");
-        return DYG_ENOMEM;
-    }
-    for (uint64_t i = 0; i < n_edges; ++i) {
-        row_ptr[src[i] + 1]++;
-        row_ptr[dst[i] + 1]++;
-    }
-    for (uint32_t v = 0; v < n_vertices; ++v) row_ptr[v + 1] += row_ptr[v];
-    for (uint64_t i = 0; i < n_edges; ++i) {
-        const uint32_t s = src[i], d = dst[i];
-        uint64_t ps = row_ptr[s] + fill[s]++;
-        col[ps] = d;
-        ww[ps] = w[i];
-        uint64_t pd = row_ptr[d] + fill[d]++;
-        col[pd] = s;
-        ww[pd] = w[i];
-    }
     dyg_graph *G = new dyg_graph();
     G->device = dev;
     G->slack = o.slack_per_row;
     G->headroom = o.arena_headroom > 0 ? o.arena_headroom : 0.0;
     dyg_status rc = graph_alloc_scalars(G);
-    if (rc == DYG_OK) rc = upload_graph(G, n_vertices, row_ptr, col, ww);
-    free(row_ptr); free(col); free(ww); free(fill);
-    if (rc != DYG_OK) {
-        free_graph(G);
-        return rc;
+    bool bad = false;
+    if (rc == DYG_OK) rc = build_graph(G, n_vertices, n_edges, src, dst, w, &bad);
+    if (rc != DYG_OK) free_graph(G);
+    if (bad) {
+        // the message names the first entry that failed the device's check
+        DYG_TRY(check_ids(src, n_edges, n_vertices, "src"));
+        DYG_TRY(check_ids(dst, n_edges, n_vertices, "dst"));
+        DYG_TRY(check_weights(w, n_edges));
+        set_error("an edge is not valid");
     }
+    if (rc != DYG_OK) return rc;
     *out = G;
     return DYG_OK;
 }
@@ -599,15 +586,16 @@ dyg_status dyg_graph_copy_from(dyg_graph *dst, const dyg_graph *src, dyg_stream_
         if (dst->g.arena_cap < s->ws.host_scalars[S_TOP]) {
             uint2 *ns = nullptr;
             float *nw = nullptr;
-            if (cudaMalloc(&ns, sizeof(uint2) * (size_t)src->g.arena_cap) != cudaSuccess ||
-                cudaMalloc(&nw, sizeof(float) * (size_t)src->g.arena_cap) != cudaSuccess) {
+            if (dev_alloc(&ns, sizeof(uint2) * (size_t)src->g.arena_cap) != cudaSuccess ||
+                dev_alloc(&nw, sizeof(float) * (size_t)src->g.arena_cap) != cudaSuccess) {
                 cudaGetLastError();
-                if (ns) cudaFree(ns);
+                if (ns) dev_free(ns);
                 set_error("cudaMalloc in copy_from failed");
                 return DYG_ENOMEM;
             }
-            DYG_CUDA(cudaFree(dst->g.slots));
-            DYG_CUDA(cudaFree(dst->g.wts));
+            DYG_CUDA(cudaDeviceSynchronize());
+            dev_free(dst->g.slots);
+            dev_free(dst->g.wts);
             dst->g.slots = ns;
             dst->g.wts = nw;
             dst->g.arena_cap = src->g.arena_cap;
@@ -635,10 +623,10 @@ dyg_status dyg_graph_clone(const dyg_graph *g, dyg_graph **out) {
     G->g.arena_cap = g->g.arena_cap;
     dyg_status rc = graph_alloc_scalars(G);
     if (rc == DYG_OK &&
-        (cudaMalloc(&G->g.desc, sizeof(uint2) * (size_t)(g->g.n ? g->g.n : 1)) != cudaSuccess ||
-         cudaMalloc(&G->g.cap, sizeof(uint32_t) * (size_t)(g->g.n ? g->g.n : 1)) != cudaSuccess ||
-         cudaMalloc(&G->g.slots, sizeof(uint2) * (size_t)g->g.arena_cap) != cudaSuccess ||
-         cudaMalloc(&G->g.wts, sizeof(float) * (size_t)g->g.arena_cap) != cudaSuccess)) {
+        (dev_alloc(&G->g.desc, sizeof(uint2) * (size_t)(g->g.n ? g->g.n : 1)) != cudaSuccess ||
+         dev_alloc(&G->g.cap, sizeof(uint32_t) * (size_t)(g->g.n ? g->g.n : 1)) != cudaSuccess ||
+         dev_alloc(&G->g.slots, sizeof(uint2) * (size_t)g->g.arena_cap) != cudaSuccess ||
+         dev_alloc(&G->g.wts, sizeof(float) * (size_t)g->g.arena_cap) != cudaSuccess)) {
         cudaGetLastError();
         set_error("cudaMalloc in clone failed");
         rc = DYG_ENOMEM;
@@ -672,26 +660,12 @@ dyg_status dyg_graph_info(const dyg_graph *g, uint32_t *n_vertices, uint64_t *n_
     }
     DeviceGuard dg(g->device);
     dyg_graph *G = const_cast<dyg_graph *>(g);
+    if (n_slots) DYG_TRY(count_slots_enqueue(G, nullptr));
     DYG_TRY(read_scalars(G, nullptr));
     if (n_vertices) *n_vertices = g->g.n;
     if (arena_used) *arena_used = G->ws.host_scalars[S_TOP];
     if (arena_cap) *arena_cap = g->g.arena_cap;
-    if (n_slots) {
-        uint2 *h = (uint2 *)malloc(sizeof(uint2) * (size_t)(g->g.n ? g->g.n : 1));
-        if (!h) {
-            set_error("host allocation failed");
-            return DYG_ENOMEM;
-        }
-        cudaError_t e = cudaMemcpy(h, g->g.desc, sizeof(uint2) * g->g.n, cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) {
-            free(h);
-            return cuda_fail(e, "info", __FILE__, __LINE__);
-        }
-        uint64_t s = 0;
-        for (uint32_t v = 0; v < g->g.n; ++v) s += h[v].y;
-        free(h);
-        *n_slots = s;
-    }
+    if (n_slots) *n_slots = G->ws.host_scalars[S_SLOTS];
     return DYG_OK;
 }
 
@@ -704,44 +678,12 @@ dyg_status dyg_graph_export(dyg_graph *g, uint64_t *row_ptr, uint32_t *col, floa
     }
     DeviceGuard dg(g->device);
     DYG_CUDA(cudaDeviceSynchronize());
-    DYG_TRY(read_scalars(g, nullptr));
-    const unsigned long long top = g->ws.host_scalars[S_TOP];
-    const uint32_t n = g->g.n;
-    uint2 *hd = (uint2 *)malloc(sizeof(uint2) * (size_t)(n ? n : 1));
-    uint2 *hs = (uint2 *)malloc(sizeof(uint2) * (size_t)(top ? top : 1));
-    float *hw = (float *)malloc(sizeof(float) * (size_t)(top ? top : 1));
-    if (!hd || !hs || !hw) {
-        free(hd); free(hs); free(hw);
-        set_error("host allocation failed");
-        return DYG_ENOMEM;
+    DYG_TRY(export_graph(g, row_ptr, col, w, slot_cap));
+    if (row_ptr[g->g.n] > slot_cap) {
+        set_error("slot_cap smaller than the number of slots");
+        return DYG_ERANGE;
     }
-    cudaError_t e = cudaMemcpy(hd, g->g.desc, sizeof(uint2) * n, cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess) e = cudaMemcpy(hs, g->g.slots, sizeof(uint2) * (size_t)top, cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess) e = cudaMemcpy(hw, g->g.wts, sizeof(float) * (size_t)top, cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) {
-        free(hd); free(hs); free(hw);
-        return cuda_fail(e, "export", __FILE__, __LINE__);
-    }
-    uint64_t o = 0;
-    dyg_status rc = DYG_OK;
-    for (uint32_t v = 0; v < n; ++v) {
-        row_ptr[v] = o;
-        for (uint32_t j = 0; j < hd[v].y; ++j) {
-            if (o + j < slot_cap) {
-                if (col) col[o + j] = hs[hd[v].x + j].x;
-                if (w) w[o + j] = hw[hd[v].x + j];
-            } else {
-                rc = DYG_ERANGE;
-            }
-        }
-        o += hd[v].y;
-    }
-    row_ptr[n] = o;
-    free(hd);
-    free(hs);
-    free(hw);
-    if (rc != DYG_OK) set_error("slot_cap smaller than the number of slots");
-    return rc;
+    return DYG_OK;
 }
 
 dyg_status dyg_graph_compact(dyg_graph *g, dyg_stream_t stream) {

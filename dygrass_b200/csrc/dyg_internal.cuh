@@ -224,8 +224,9 @@ enum Scalar : int {
     S_BAR = 15,       // grid barrier: arrivals (low word), generation (high word)
     S_ITEMS = 18,     // row operations: rows for a block (low word), for a warp (high word)
     S_IDX = 16,       // row index: next free word
+    S_SLOTS = 19,     // live slots, summed for dyg_graph_info
     S_IDXN = 17,      // row index: rows for a warp (low word), for a block (high word)
-    S_NSCALARS = 19
+    S_NSCALARS = 20
 };
 enum Count : int {
     C_FILTERED = 0,   // decremental: edges to walk
@@ -280,6 +281,22 @@ dyg_status cuda_fail(cudaError_t e, const char *what, const char *file, int line
         dyg_status _s = (call);            \
         if (_s != DYG_OK) return _s;       \
     } while (0)
+
+// --- memory.cu
+// Device memory from the current device's pool.  dev_free: the device has
+// finished with the block (or the caller has synchronized it).
+cudaError_t dev_alloc(void **out, size_t bytes);
+void dev_free(void *p);
+// Pinned host memory; host_free takes the size given to host_alloc, once the
+// device has finished with the block.
+cudaError_t host_alloc(void **out, size_t bytes);
+void host_free(void *p, size_t bytes);
+template <typename T>
+inline cudaError_t dev_alloc(T **out, size_t bytes) { return dev_alloc(reinterpret_cast<void **>(out), bytes); }
+// Unique id of the context current on this thread (cuCtxGetId, reached through
+// the runtime's driver entry points, so no libcuda link is needed); 0 when the
+// driver does not provide it.
+unsigned long long current_context_id();
 
 dyg_status ensure(Buf &b, size_t bytes);
 // Where a caller's pointer lives as seen from `device`: host memory (pageable
@@ -405,6 +422,16 @@ dyg_status stream_file_run(dyg_graph *G, dyg_graph *H, uint32_t op, const uint32
 // --- graph.cu
 dyg_status upload_graph(dyg_graph *G, uint32_t n, const uint64_t *row_ptr, const uint32_t *col,
                         const float *w);
+// The graph of an edge list (host arrays) with rows in list order, built on
+// the device; *bad is set, and nothing else happens, if an id or a weight is
+// not valid.
+dyg_status build_graph(dyg_graph *G, uint32_t n, uint64_t m, const uint32_t *src, const uint32_t *dst,
+                       const float *w, bool *bad);
+// Rows as a CSR into host arrays (col, w may be null); at most slot_cap slots
+// are copied.
+dyg_status export_graph(dyg_graph *G, uint64_t *row_ptr, uint32_t *col, float *w, uint64_t slot_cap);
+// Sums the degrees into S_SLOTS.
+dyg_status count_slots_enqueue(dyg_graph *G, cudaStream_t st);
 // Copies both graphs' scalars and counts to the host with one synchronize.
 dyg_status read_scalars2(dyg_graph *A, dyg_graph *B, cudaStream_t st);
 // Exclusive scan of in[0, m) into out; with m_dev, of in[0, min(m, *m_dev)).

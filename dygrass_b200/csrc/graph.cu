@@ -31,17 +31,18 @@ dyg_status ensure(Buf &b, size_t bytes) {
     if (bytes == 0) bytes = 16;
     if (b.bytes >= bytes) return DYG_OK;
     if (b.p) {
-        DYG_CUDA(cudaFree(b.p));
+        DYG_CUDA(cudaDeviceSynchronize());   // launches before may still use it
+        dev_free(b.p);
         b.p = nullptr;
         b.bytes = 0;
     }
     size_t want = bytes + bytes / 4;
     want = (want + 255) & ~(size_t)255;
-    cudaError_t e = cudaMalloc(&b.p, want);
+    cudaError_t e = dev_alloc(&b.p, want);
     if (e != cudaSuccess) {
         cudaGetLastError();
         b.p = nullptr;
-        set_error(std::string("cudaMalloc of ") + std::to_string(want) + " bytes failed: " +
+        set_error(std::string("allocation of ") + std::to_string(want) + " bytes failed: " +
                   cudaGetErrorString(e));
         return DYG_ENOMEM;
     }
@@ -117,10 +118,10 @@ dyg_status upload_graph(dyg_graph *G, uint32_t n, const uint64_t *row_ptr, const
     dyg_status rc = DYG_OK;
     G->g.n = n;
     G->g.arena_cap = arena;
-    if (cudaMalloc(&G->g.desc, sizeof(uint2) * (size_t)(n ? n : 1)) != cudaSuccess ||
-        cudaMalloc(&G->g.cap, sizeof(uint32_t) * (size_t)(n ? n : 1)) != cudaSuccess ||
-        cudaMalloc(&G->g.slots, sizeof(uint2) * (size_t)arena) != cudaSuccess ||
-        cudaMalloc(&G->g.wts, sizeof(float) * (size_t)arena) != cudaSuccess) {
+    if (dev_alloc(&G->g.desc, sizeof(uint2) * (size_t)(n ? n : 1)) != cudaSuccess ||
+        dev_alloc(&G->g.cap, sizeof(uint32_t) * (size_t)(n ? n : 1)) != cudaSuccess ||
+        dev_alloc(&G->g.slots, sizeof(uint2) * (size_t)arena) != cudaSuccess ||
+        dev_alloc(&G->g.wts, sizeof(float) * (size_t)arena) != cudaSuccess) {
         cudaGetLastError();
         set_error("cudaMalloc of the graph arena failed");
         rc = DYG_ENOMEM;
@@ -141,6 +142,358 @@ dyg_status upload_graph(dyg_graph *G, uint32_t n, const uint64_t *row_ptr, const
     return rc;
 }
 
+// ------------------------------------------------------------------ build
+// Rows of an edge list in list order (functions.cpp:130-232): half-edge
+// i = 2e enters row src[e] with column dst[e], i = 2e + 1 the other way.
+//   count   degrees, by one atomic per half-edge, with the input checks
+//   place   capacities scanned to row offsets; half-edge indices put into
+//           their rows in any order (again one atomic each)
+//   rows    each row's indices sorted, and its slots written from them
+// The host built the rows with two passes of dependent loads over the edges
+// and uploaded them with their padding; with the allocations 5 to 8 ms for the
+// 116,000 and the 324,000 edges of a 48^3 mesh's two graphs, now 0.24 and
+// 0.40.  Bound by the host's copy of the edges.
+
+namespace {
+
+__global__ void k_build_count(const uint32_t *src, const uint32_t *dst, const float *w, uint32_t m,
+                              uint32_t n, uint32_t *cnt, unsigned long long *err) {
+    for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < m; e += gridDim.x * blockDim.x) {
+        const uint32_t u = src[e], v = dst[e];
+        const float x = w[e];
+        if (u >= n || v >= n || !(x > 0.0f) || !isfinite(x)) {
+            atomicOr(err, (unsigned long long)kErrVertex);
+            continue;
+        }
+        atomicAdd(cnt + u, 1u);
+        atomicAdd(cnt + v, 1u);
+    }
+}
+
+// Row offsets; the counters start over for the placement.
+struct BuildScan {
+    uint32_t *cnt;
+    uint2 *desc;
+    uint32_t *cap;
+    uint32_t slack;
+    unsigned long long *long_flag, *top;
+    __device__ uint32_t load(uint32_t v) const { return cnt[v] + slack; }
+    __device__ void store(uint32_t v, uint32_t off, uint32_t c) const {
+        const uint32_t deg = c - slack;
+        desc[v] = make_uint2(off, deg);
+        cap[v] = c;
+        cnt[v] = 0u;
+        if (deg > kBigRow) *long_flag = 1ull;
+    }
+    __device__ void last(uint32_t total) const { *top = total; }
+};
+
+__global__ void k_build_place(const uint32_t *src, const uint32_t *dst, uint32_t m, const uint2 *desc,
+                              uint32_t *cnt, uint32_t *idx) {
+    for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < m; e += gridDim.x * blockDim.x) {
+        const uint32_t u = src[e], v = dst[e];
+        idx[desc[u].x + atomicAdd(cnt + u, 1u)] = 2u * e;
+        idx[desc[v].x + atomicAdd(cnt + v, 1u)] = 2u * e + 1u;
+    }
+}
+
+struct BuildList {
+    const uint32_t *src, *dst;
+    const float *w;
+};
+__device__ __forceinline__ void build_slot(const DevGraph &g, const BuildList &L, uint32_t at, uint32_t i) {
+    const float x = L.w[i >> 1];
+    g.slots[at] = make_uint2((i & 1u) ? L.src[i >> 1] : L.dst[i >> 1], __float_as_uint(__frcp_rn(x)));
+    g.wts[at] = x;
+}
+
+constexpr uint32_t kBuildLane = 8;       // rows up to this length are sorted by one lane
+constexpr uint32_t kBuildTile = 4096;    // indices a block sorts in shared memory at a time
+constexpr uint32_t kBuildThreads = 256;
+
+// Rows of up to kBigRow slots: by a lane, or by the warp 32 indices at a
+// time, each index's rank counted against the row's others.  Longer rows go
+// to `big` (n words) for k_build_big.
+__global__ void __launch_bounds__(kBuildThreads)
+k_build_rows(DevGraph g, BuildList L, const uint32_t *idx, uint32_t *big, unsigned long long *nbig) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint32_t vb = first - lane; vb < g.n; vb += gridDim.x * blockDim.x) {
+        const uint32_t v = vb + lane;
+        const uint2 d = v < g.n ? g.desc[v] : make_uint2(0u, 0u);
+        if (d.y <= kBuildLane) {
+            uint32_t i[kBuildLane];
+#pragma unroll
+            for (uint32_t u = 0; u < kBuildLane; ++u) i[u] = u < d.y ? idx[d.x + u] : ~0u;
+#pragma unroll
+            for (uint32_t u = 0; u < kBuildLane; ++u)
+                if (u < d.y) {
+                    uint32_t r = 0;
+#pragma unroll
+                    for (uint32_t q = 0; q < kBuildLane; ++q) r += i[q] < i[u] ? 1u : 0u;
+                    build_slot(g, L, d.x + r, i[u]);
+                }
+        } else if (d.y > kBigRow) {
+            big[atomicAdd(nbig, 1ull)] = v;
+        }
+        unsigned todo = __ballot_sync(kFull, d.y > kBuildLane && d.y <= kBigRow);
+        while (todo) {
+            const int src = __ffs(todo) - 1;
+            todo &= todo - 1u;
+            const uint32_t off = __shfl_sync(kFull, d.x, src), deg = __shfl_sync(kFull, d.y, src);
+            for (uint32_t j0 = 0; j0 < deg; j0 += 32u) {
+                const uint32_t mine = j0 + lane < deg ? idx[off + j0 + lane] : ~0u;
+                uint32_t r = 0;
+                for (uint32_t t0 = 0; t0 < deg; t0 += 32u) {
+                    const uint32_t other = t0 + lane < deg ? idx[off + t0 + lane] : ~0u;
+#pragma unroll
+                    for (uint32_t q = 0; q < 32u; ++q)
+                        r += __shfl_sync(kFull, other, q) < mine ? 1u : 0u;
+                }
+                if (mine != ~0u) build_slot(g, L, off + r, mine);
+            }
+        }
+    }
+}
+
+// Rows longer than kBigRow, one block each: sorted in shared memory a tile at
+// a time; an index of a row of several tiles then takes the place given by
+// its rank in every tile (binary searches: the indices are distinct).
+__global__ void __launch_bounds__(kBuildThreads)
+k_build_big(DevGraph g, BuildList L, uint32_t *idx, const uint32_t *big, const unsigned long long *nbig) {
+    __shared__ uint32_t s[kBuildTile];
+    const uint32_t nb = (uint32_t)*nbig;
+    for (uint32_t q = blockIdx.x; q < nb; q += gridDim.x) {
+        const uint2 d = g.desc[big[q]];
+        for (uint32_t t0 = 0; t0 < d.y; t0 += kBuildTile) {
+            const uint32_t c = min(kBuildTile, d.y - t0);
+            uint32_t N = 512u;
+            while (N < c) N <<= 1;
+            for (uint32_t j = threadIdx.x; j < N; j += blockDim.x) s[j] = j < c ? idx[d.x + t0 + j] : ~0u;
+            for (uint32_t k = 2u; k <= N; k <<= 1)
+                for (uint32_t h = k >> 1; h > 0u; h >>= 1) {
+                    __syncthreads();
+                    for (uint32_t p = threadIdx.x; p < N / 2u; p += blockDim.x) {
+                        const uint32_t i = 2u * p - (p & (h - 1u)), o = i + h;
+                        const uint32_t a = s[i], b = s[o];
+                        if ((a > b) == ((i & k) == 0u)) {
+                            s[i] = b;
+                            s[o] = a;
+                        }
+                    }
+                }
+            __syncthreads();
+            if (d.y <= kBuildTile)
+                for (uint32_t j = threadIdx.x; j < c; j += blockDim.x) build_slot(g, L, d.x + j, s[j]);
+            else
+                for (uint32_t j = threadIdx.x; j < c; j += blockDim.x) idx[d.x + t0 + j] = s[j];
+            __syncthreads();
+        }
+        if (d.y <= kBuildTile) continue;
+        for (uint32_t j = threadIdx.x; j < d.y; j += blockDim.x) {
+            const uint32_t i = idx[d.x + j], own = j / kBuildTile;
+            uint32_t r = j - own * kBuildTile;
+            for (uint32_t t = 0; t * kBuildTile < d.y; ++t) {
+                if (t == own) continue;
+                uint32_t lo = 0, hi = min(kBuildTile, d.y - t * kBuildTile);
+                while (lo < hi) {
+                    const uint32_t mid = (lo + hi) >> 1;
+                    if (idx[d.x + t * kBuildTile + mid] < i) lo = mid + 1u;
+                    else hi = mid;
+                }
+                r += lo;
+            }
+            build_slot(g, L, d.x + r, i);
+        }
+        __syncthreads();
+    }
+}
+
+// Device blocks of one call, freed when it leaves (after its work is done).
+struct Temps {
+    void *p[8];
+    int k = 0;
+    cudaError_t get(void **out, size_t bytes) {
+        const cudaError_t e = dev_alloc(out, bytes ? bytes : 16);
+        if (e == cudaSuccess) p[k++] = *out;
+        return e;
+    }
+    ~Temps() {
+        if (k) cudaStreamSynchronize(nullptr);
+        while (k) dev_free(p[--k]);
+    }
+};
+
+int grid_of(uint64_t items, uint32_t threads) {
+    const uint64_t b = (items + threads - 1) / threads, cap = (uint64_t)num_sms() * 16;
+    return (int)(b < 1 ? 1 : (b < cap ? b : cap));
+}
+
+}  // namespace
+
+dyg_status build_graph(dyg_graph *G, uint32_t n, uint64_t m, const uint32_t *src, const uint32_t *dst,
+                       const float *w, bool *bad) {
+    *bad = false;
+    const uint64_t used = 2 * m + (uint64_t)G->slack * n;
+    const uint64_t arena = used + (uint64_t)((double)(2 * m) * G->headroom) + 1024;
+    if (arena >= 0xFFFFFFFFull) {
+        set_error("graph too large for 32-bit slot offsets");
+        return DYG_EINVAL;
+    }
+    G->g.n = n;
+    G->g.arena_cap = arena;
+    const size_t nn = n ? n : 1;
+    Temps tmp;
+    void *d_src, *d_dst, *d_w, *d_cnt, *d_idx;
+    if (dev_alloc(&G->g.desc, sizeof(uint2) * nn) != cudaSuccess ||
+        dev_alloc(&G->g.cap, sizeof(uint32_t) * nn) != cudaSuccess ||
+        dev_alloc(&G->g.slots, sizeof(uint2) * (size_t)arena) != cudaSuccess ||
+        dev_alloc(&G->g.wts, sizeof(float) * (size_t)arena) != cudaSuccess ||
+        tmp.get(&d_src, sizeof(uint32_t) * m) != cudaSuccess ||
+        tmp.get(&d_dst, sizeof(uint32_t) * m) != cudaSuccess ||
+        tmp.get(&d_w, sizeof(float) * m) != cudaSuccess ||
+        tmp.get(&d_cnt, sizeof(uint32_t) * nn) != cudaSuccess ||
+        tmp.get(&d_idx, sizeof(uint32_t) * (size_t)(used + nn)) != cudaSuccess) {
+        cudaGetLastError();
+        set_error("cudaMalloc of the graph arena failed");
+        return DYG_ENOMEM;
+    }
+    cudaStream_t st = nullptr;
+    unsigned long long *sc = ptr<unsigned long long>(G->ws.scalars);
+    DYG_CUDA(cudaMemsetAsync(d_cnt, 0, sizeof(uint32_t) * nn, st));
+    DYG_CUDA(cudaMemcpyAsync(d_src, src, sizeof(uint32_t) * m, cudaMemcpyHostToDevice, st));
+    DYG_CUDA(cudaMemcpyAsync(d_dst, dst, sizeof(uint32_t) * m, cudaMemcpyHostToDevice, st));
+    DYG_CUDA(cudaMemcpyAsync(d_w, w, sizeof(float) * m, cudaMemcpyHostToDevice, st));
+    uint32_t *ds = (uint32_t *)d_src, *dd = (uint32_t *)d_dst, *cnt = (uint32_t *)d_cnt;
+    uint32_t *idx = (uint32_t *)d_idx, *big = idx + used;
+    if (m) {
+        k_build_count<<<grid_of(m, 256), 256, 0, st>>>(ds, dd, (float *)d_w, (uint32_t)m, n, cnt, sc + S_ERR);
+        count_launch();
+        DYG_CUDA(cudaGetLastError());
+        // nothing is placed by ids that were not checked
+        DYG_TRY(read_scalars(G, st));
+        if (G->ws.host_scalars[S_ERR]) {
+            *bad = true;
+            return DYG_EINVAL;
+        }
+    }
+    if (n) {
+        DYG_TRY(scan_op(G->ws, BuildScan{cnt, G->g.desc, G->g.cap, G->slack, sc + S_LONG, sc + S_TOP}, n,
+                        nullptr, nullptr, st));
+    }
+    if (m) {
+        const BuildList L{ds, dd, (float *)d_w};
+        k_build_place<<<grid_of(m, 256), 256, 0, st>>>(ds, dd, (uint32_t)m, G->g.desc, cnt, idx);
+        count_launch();
+        k_build_rows<<<grid_of(n, kBuildThreads), kBuildThreads, 0, st>>>(G->g, L, idx, big, sc + S_NBIG);
+        count_launch();
+        k_build_big<<<num_sms() * 4, kBuildThreads, 0, st>>>(G->g, L, idx, big, sc + S_NBIG);
+        count_launch();
+        DYG_CUDA(cudaGetLastError());
+        DYG_CUDA(cudaMemsetAsync(sc + S_NBIG, 0, sizeof(unsigned long long), st));
+    }
+    return read_scalars(G, st);   // synchronizes; picks up a long row
+}
+
+// ----------------------------------------------------------------- export
+
+namespace {
+
+struct DegreeScan {
+    const uint2 *desc;
+    unsigned long long *row_ptr;   // n + 1
+    uint32_t n;
+    __device__ uint32_t load(uint32_t v) const { return desc[v].y; }
+    __device__ void store(uint32_t v, uint32_t excl, uint32_t) const { row_ptr[v] = excl; }
+    __device__ void last(uint32_t total) const { row_ptr[n] = total; }
+};
+
+__global__ void k_count_slots(const uint2 *desc, uint32_t n, unsigned long long *sum) {
+    uint32_t mine = 0u;   // the slots of a graph fit 32 bits
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
+        mine += desc[v].y;
+    mine = __reduce_add_sync(kFull, mine);
+    if ((threadIdx.x & 31u) == 0u && mine) atomicAdd(sum, (unsigned long long)mine);
+}
+
+// Rows to their place in a CSR: a group of eight lanes per row, rows of a
+// lattice being shorter than that; rows over kBigRow by the whole warp.
+__global__ void __launch_bounds__(256)
+k_export_rows(DevGraph g, const unsigned long long *row_ptr, uint32_t *col, float *w) {
+    const uint32_t lane = threadIdx.x & 31u, sub = lane & 7u;
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t v0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 4u; v0 < g.n; v0 += 4u * warps) {
+        const uint32_t v = v0 + (lane >> 3);
+        const uint2 d = v < g.n ? g.desc[v] : make_uint2(0u, 0u);
+        const unsigned long long o = v < g.n ? row_ptr[v] : 0ull;
+        if (d.y <= kBigRow) {
+#pragma unroll 4
+            for (uint32_t j = sub; j < d.y; j += 8u) {
+                col[o + j] = g.slots[d.x + j].x;
+                w[o + j] = g.wts[d.x + j];
+            }
+        }
+        unsigned todo = __ballot_sync(kFull, sub == 0u && d.y > kBigRow);
+        while (todo) {
+            const int src = __ffs(todo) - 1;
+            todo &= todo - 1u;
+            const uint32_t off = __shfl_sync(kFull, d.x, src), deg = __shfl_sync(kFull, d.y, src);
+            const unsigned long long to = __shfl_sync(kFull, o, src);
+#pragma unroll 4
+            for (uint32_t j = lane; j < deg; j += 32u) {
+                col[to + j] = g.slots[off + j].x;
+                w[to + j] = g.wts[off + j];
+            }
+        }
+    }
+}
+
+}  // namespace
+
+dyg_status count_slots_enqueue(dyg_graph *G, cudaStream_t st) {
+    unsigned long long *sum = ptr<unsigned long long>(G->ws.scalars) + S_SLOTS;
+    DYG_CUDA(cudaMemsetAsync(sum, 0, sizeof(unsigned long long), st));
+    k_count_slots<<<grid_of(G->g.n, 256), 256, 0, st>>>(G->g.desc, G->g.n, sum);
+    count_launch();
+    DYG_CUDA(cudaGetLastError());
+    return DYG_OK;
+}
+
+dyg_status export_graph(dyg_graph *G, uint64_t *row_ptr, uint32_t *col, float *w, uint64_t slot_cap) {
+    const uint32_t n = G->g.n;
+    row_ptr[0] = 0;
+    if (n == 0) return DYG_OK;
+    cudaStream_t st = nullptr;
+    Temps tmp;
+    void *d_rp, *d_col = nullptr, *d_w = nullptr;
+    bool ok = tmp.get(&d_rp, sizeof(uint64_t) * ((size_t)n + 1)) == cudaSuccess;
+    if (ok) {
+        DYG_TRY(scan_op(G->ws, DegreeScan{G->g.desc, (unsigned long long *)d_rp, n}, n, nullptr, nullptr, st));
+        DYG_CUDA(cudaMemcpyAsync(row_ptr, d_rp, sizeof(uint64_t) * ((size_t)n + 1), cudaMemcpyDeviceToHost, st));
+        DYG_CUDA(cudaStreamSynchronize(st));
+        const uint64_t total = row_ptr[n], out = total < slot_cap ? total : slot_cap;
+        if (out && (col || w)) {
+            ok = tmp.get(&d_col, sizeof(uint32_t) * total) == cudaSuccess &&
+                 tmp.get(&d_w, sizeof(float) * total) == cudaSuccess;
+            if (ok) {
+                k_export_rows<<<grid_of((uint64_t)n * 8, 256), 256, 0, st>>>(
+                    G->g, (unsigned long long *)d_rp, (uint32_t *)d_col, (float *)d_w);
+                count_launch();
+                DYG_CUDA(cudaGetLastError());
+                if (col) DYG_CUDA(cudaMemcpyAsync(col, d_col, sizeof(uint32_t) * out, cudaMemcpyDeviceToHost, st));
+                if (w) DYG_CUDA(cudaMemcpyAsync(w, d_w, sizeof(float) * out, cudaMemcpyDeviceToHost, st));
+                DYG_CUDA(cudaStreamSynchronize(st));
+            }
+        }
+    }
+    if (!ok) {
+        cudaGetLastError();
+        set_error("device memory for the export is short");
+        return DYG_ENOMEM;
+    }
+    return DYG_OK;
+}
+
 dyg_status grow_arena(dyg_graph *G, uint64_t min_cap, cudaStream_t st) {
     uint64_t cap = G->g.arena_cap + G->g.arena_cap / 2;
     if (cap < min_cap + min_cap / 4 + 1024) cap = min_cap + min_cap / 4 + 1024;
@@ -151,11 +504,11 @@ dyg_status grow_arena(dyg_graph *G, uint64_t min_cap, cudaStream_t st) {
     }
     uint2 *ns = nullptr;
     float *nw = nullptr;
-    cudaError_t e = cudaMalloc(&ns, sizeof(uint2) * (size_t)cap);
-    if (e == cudaSuccess) e = cudaMalloc(&nw, sizeof(float) * (size_t)cap);
+    cudaError_t e = dev_alloc(&ns, sizeof(uint2) * (size_t)cap);
+    if (e == cudaSuccess) e = dev_alloc(&nw, sizeof(float) * (size_t)cap);
     if (e != cudaSuccess) {
         cudaGetLastError();
-        if (ns) cudaFree(ns);
+        if (ns) dev_free(ns);
         set_error("cudaMalloc while growing the arena failed");
         return DYG_ENOMEM;
     }
@@ -164,8 +517,8 @@ dyg_status grow_arena(dyg_graph *G, uint64_t min_cap, cudaStream_t st) {
     DYG_CUDA(cudaMemcpyAsync(ns, G->g.slots, sizeof(uint2) * (size_t)top, cudaMemcpyDeviceToDevice, st));
     DYG_CUDA(cudaMemcpyAsync(nw, G->g.wts, sizeof(float) * (size_t)top, cudaMemcpyDeviceToDevice, st));
     DYG_CUDA(cudaStreamSynchronize(st));
-    DYG_CUDA(cudaFree(G->g.slots));
-    DYG_CUDA(cudaFree(G->g.wts));
+    dev_free(G->g.slots);
+    dev_free(G->g.wts);
     G->g.slots = ns;
     G->g.wts = nw;
     G->g.arena_cap = cap;
@@ -311,11 +664,11 @@ dyg_status compact_graph(dyg_graph *G, cudaStream_t st) {
     if (cap >= 0xFFFFFFFFull) cap = 0xFFFFFFFEull;
     uint2 *ns = nullptr;
     float *nw = nullptr;
-    cudaError_t e = cudaMalloc(&ns, sizeof(uint2) * (size_t)cap);
-    if (e == cudaSuccess) e = cudaMalloc(&nw, sizeof(float) * (size_t)cap);
+    cudaError_t e = dev_alloc(&ns, sizeof(uint2) * (size_t)cap);
+    if (e == cudaSuccess) e = dev_alloc(&nw, sizeof(float) * (size_t)cap);
     if (e != cudaSuccess) {
         cudaGetLastError();
-        if (ns) cudaFree(ns);
+        if (ns) dev_free(ns);
         set_error("cudaMalloc during compaction failed");
         return DYG_ENOMEM;
     }
@@ -326,8 +679,8 @@ dyg_status compact_graph(dyg_graph *G, cudaStream_t st) {
     unsigned long long top = used;
     DYG_CUDA(cudaMemcpyAsync(G->g.top, &top, sizeof(top), cudaMemcpyHostToDevice, st));
     DYG_CUDA(cudaStreamSynchronize(st));
-    DYG_CUDA(cudaFree(G->g.slots));
-    DYG_CUDA(cudaFree(G->g.wts));
+    dev_free(G->g.slots);
+    dev_free(G->g.wts);
     G->g.slots = ns;
     G->g.wts = nw;
     G->g.arena_cap = cap;

@@ -1,0 +1,172 @@
+// memory.cu -- device memory of the graph handles.
+//
+// A handle owns some forty arrays that grow with the calls made on it, and a
+// cudaMalloc or cudaFree of a megabyte takes 0.3 to 0.7 ms (each maps or
+// unmaps pages and waits for the device): building two 110,592-vertex graphs,
+// one insertion and one deletion stream and closing them spent 12 of 27 ms
+// there.  Memory comes from one CUDA memory pool per device instead, which
+// keeps up to kPoolKeep bytes that no handle uses and gives what is above
+// back to the device at the next synchronize.  The pool is the driver's:
+// calls from any thread are safe.  Blocks are allocated and freed on a stream
+// of the pool's own; an allocation is complete when dev_alloc returns, and a
+// block is freed only when the device has finished with it, so blocks move
+// freely between handles, streams and threads.  Pinned host blocks (a handle's
+// scalar mirror and its packed arrays, in powers of two) are kept the same
+// way, at most 8 MB of them.
+#include <cuda.h>
+
+#include <mutex>
+#include <vector>
+
+#include "dyg_internal.cuh"
+
+namespace dyg {
+
+namespace {
+
+constexpr unsigned long long kPoolKeep = 256ull << 20;
+constexpr int kMaxDevices = 64;
+
+struct DevicePool {
+    cudaMemPool_t pool = nullptr;   // null: the device has no pools
+    cudaStream_t st = nullptr;
+    bool tried = false;
+    unsigned long long ctx = 0;
+};
+std::mutex g_pool_mu;
+DevicePool g_pools[kMaxDevices];
+
+// The pool of the current device, made on first use and again when the
+// device's context was replaced (cudaDeviceReset takes the pool with it).
+DevicePool current_pool() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return DevicePool{};
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    DevicePool &p = g_pools[dev];
+    const unsigned long long ctx = current_context_id();
+    if (p.tried && ctx == p.ctx) return p;
+    p = DevicePool{};
+    p.tried = true;
+    p.ctx = ctx;
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    unsigned long long keep = kPoolKeep;
+    if (cudaMemPoolCreate(&p.pool, &props) != cudaSuccess) p.pool = nullptr;
+    if (p.pool && (cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess ||
+                   cudaStreamCreateWithFlags(&p.st, cudaStreamNonBlocking) != cudaSuccess)) {
+        cudaMemPoolDestroy(p.pool);
+        p.pool = nullptr;
+    }
+    cudaGetLastError();
+    // the context may have been created by the calls above
+    p.ctx = current_context_id();
+    return p;
+}
+
+}  // namespace
+
+unsigned long long current_context_id() {
+    typedef CUresult (*GetCurrent)(CUcontext *);
+    typedef CUresult (*GetId)(CUcontext, unsigned long long *);
+    static GetCurrent get_current = nullptr;
+    static GetId get_id = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            get_current = reinterpret_cast<GetCurrent>(f);
+        f = nullptr;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            get_id = reinterpret_cast<GetId>(f);
+        cudaGetLastError();
+    });
+    if (!get_current || !get_id) return 0ull;
+    CUcontext c = nullptr;
+    unsigned long long id = 0ull;
+    if (get_current(&c) != CUDA_SUCCESS || !c || get_id(c, &id) != CUDA_SUCCESS) return 0ull;
+    return id;
+}
+
+cudaError_t dev_alloc(void **out, size_t bytes) {
+    *out = nullptr;
+    const DevicePool p = current_pool();
+    if (!p.pool) return cudaMalloc(out, bytes);
+    cudaError_t e = cudaMallocFromPoolAsync(out, bytes, p.pool, p.st);
+    if (e == cudaErrorMemoryAllocation) {
+        // what the pool holds in other sizes goes back first
+        cudaGetLastError();
+        cudaStreamSynchronize(p.st);
+        cudaMemPoolTrimTo(p.pool, 0);
+        e = cudaMallocFromPoolAsync(out, bytes, p.pool, p.st);
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(p.st);   // usable on any stream from here on
+    if (e != cudaSuccess) *out = nullptr;
+    return e;
+}
+
+void dev_free(void *ptr) {
+    if (!ptr) return;
+    const DevicePool p = current_pool();
+    if (!p.pool || cudaFreeAsync(ptr, p.st) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(ptr);
+    }
+    cudaGetLastError();
+}
+
+namespace {
+struct PinnedBlock {
+    void *p;
+    size_t bytes;
+    unsigned long long ctx;
+};
+std::mutex g_pinned_mu;
+std::vector<PinnedBlock> g_pinned;   // free blocks
+size_t g_pinned_bytes = 0;
+constexpr size_t kPinnedKeep = 8u << 20;
+}  // namespace
+
+cudaError_t host_alloc(void **out, size_t bytes) {
+    *out = nullptr;
+    const unsigned long long ctx = current_context_id();
+    {
+        std::lock_guard<std::mutex> lk(g_pinned_mu);
+        for (size_t i = g_pinned.size(); i-- > 0;) {
+            if (g_pinned[i].bytes != bytes || g_pinned[i].ctx != ctx) continue;
+            *out = g_pinned[i].p;
+            g_pinned_bytes -= bytes;
+            g_pinned[i] = g_pinned.back();
+            g_pinned.pop_back();
+            return cudaSuccess;
+        }
+    }
+    return cudaMallocHost(out, bytes);
+}
+
+void host_free(void *p, size_t bytes) {
+    if (!p) return;
+    const unsigned long long ctx = current_context_id();
+    {
+        std::lock_guard<std::mutex> lk(g_pinned_mu);
+        // blocks of a context that is gone went with it
+        for (size_t i = g_pinned.size(); ctx && i-- > 0;)
+            if (g_pinned[i].ctx != ctx) {
+                g_pinned_bytes -= g_pinned[i].bytes;
+                g_pinned[i] = g_pinned.back();
+                g_pinned.pop_back();
+            }
+        if (ctx && g_pinned_bytes + bytes <= kPinnedKeep) {
+            g_pinned.push_back(PinnedBlock{p, bytes, ctx});
+            g_pinned_bytes += bytes;
+            return;
+        }
+    }
+    cudaFreeHost(p);
+}
+
+}  // namespace dyg

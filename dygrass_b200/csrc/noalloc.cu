@@ -22,8 +22,6 @@
 // context; the address is cached together with the context's unique id and
 // looked up again when the id changes).  Make those calls before any stream
 // capture.
-#include <cuda.h>
-
 #include <mutex>
 
 #include "dyg_internal.cuh"
@@ -43,34 +41,6 @@ constexpr int kMaxDevices = 64;
 std::mutex g_setup_mu;
 unsigned long long *g_scratch_addr[kMaxDevices] = {nullptr};
 unsigned long long g_scratch_ctx[kMaxDevices] = {0};
-
-// Unique id of the context current on this thread (cuCtxGetId, reached through
-// the runtime's driver entry points, so no libcuda link is needed); 0 when the
-// driver does not provide it.
-unsigned long long current_context_id() {
-    typedef CUresult (*GetCurrent)(CUcontext *);
-    typedef CUresult (*GetId)(CUcontext, unsigned long long *);
-    static GetCurrent get_current = nullptr;
-    static GetId get_id = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void *f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_current = reinterpret_cast<GetCurrent>(f);
-        f = nullptr;
-        if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_id = reinterpret_cast<GetId>(f);
-        cudaGetLastError();
-    });
-    if (!get_current || !get_id) return 0ull;
-    CUcontext c = nullptr;
-    unsigned long long id = 0ull;
-    if (get_current(&c) != CUDA_SUCCESS || !c || get_id(c, &id) != CUDA_SUCCESS) return 0ull;
-    return id;
-}
 
 // Device address of g_noalloc_scratch on `dev` (which must be current).  In
 // host code the symbol's name is only a host-side stand-in, so the address is

@@ -494,7 +494,10 @@ dyg_status grow_keep(Buf &b, size_t bytes, size_t used, cudaStream_t st) {
         DYG_CUDA(cudaMemcpyAsync(nb.p, b.p, used, cudaMemcpyDeviceToDevice, st));
         DYG_CUDA(cudaStreamSynchronize(st));
     }
-    if (b.p) cudaFree(b.p);
+    if (b.p) {
+        if (!used) DYG_CUDA(cudaStreamSynchronize(st));
+        dev_free(b.p);
+    }
     b = nb;
     return DYG_OK;
 }

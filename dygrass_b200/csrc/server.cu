@@ -974,8 +974,9 @@ dyg_status dyg_server_destroy(dyg_server *s) {
     for (auto &kv : s->by_tag) delete kv.second;   // every request, queued or done
     {
         dyg::DevSet ds(s->H->device);
+        cudaDeviceSynchronize();
         for (dyg::Buf *b : {&s->d_src, &s->d_dst, &s->d_w, &s->d_uid, &s->d_out, &s->d_cond, &s->d_acc})
-            if (b->p) cudaFree(b->p);
+            dyg::dev_free(b->p);
         s->h_src.release();
         s->h_dst.release();
         s->h_rx.release();

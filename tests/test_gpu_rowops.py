@@ -156,3 +156,47 @@ def test_uniform_degrees_and_lengths(dyg, oracle, leaves, steps):  # noqa: F811
     ew = rng.uniform(0.01, 0.05, 32).astype(np.float32)
     p = dyg.WalkParams.make(threshold=10.0, walkers=96, max_steps=steps)
     run_incr_both(dyg, oracle, n, hs, hd, hw, es, ed, ew, p, batch_size=20)
+
+
+# rows built by a lane (8), a warp (256), in one shared-memory tile of a block
+# (4096) and in several; every row in edge-list order, as a stable sort gives it
+@pytest.mark.parametrize("leaves", [0, 7, 8, 31, 32, 33, 255, 256, 257, 4095, 4096, 9000])
+def test_build_and_export_rows(dyg, leaves):  # noqa: F811
+    rng = np.random.default_rng(leaves)
+    n = leaves + 50
+    s, d, w = star(n, leaves, rng)
+    # repeated edges, self-loops and an isolated last vertex
+    s = np.concatenate([s, s[:9], [3, 3]]).astype(np.uint32)
+    d = np.concatenate([d, d[:9], [3, 3]]).astype(np.uint32)
+    w = np.concatenate([w, w[:9] + 1, [5, 6]]).astype(np.float32)
+    g = dyg.Graph.from_edges(n + 1, s, d, w)
+    rows, cols = np.stack([s, d], 1).ravel(), np.stack([d, s], 1).ravel()
+    order = np.argsort(rows, kind="stable")
+    rp, col, ww = g.export()
+    assert np.array_equal(rp, np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=n + 1))]).astype(np.uint64))
+    assert np.array_equal(col, cols[order]) and np.array_equal(ww, np.repeat(w, 2)[order])
+    inf = g.info()
+    assert inf["n_slots"] == 2 * len(s) and inf["arena_used"] == 2 * len(s) + 2 * (n + 1)
+
+
+def test_build_long_list_is_checked(dyg):  # noqa: F811
+    """Lists over 65,536 edges are checked on the device."""
+    m = 70_000
+    s, d = np.arange(m, dtype=np.uint32), np.arange(1, m + 1, dtype=np.uint32)
+    w = np.ones(m, np.float32)
+    bad_w, bad_d = w.copy(), d.copy()
+    bad_w[69_000], bad_d[66_000] = np.inf, m + 1
+    for args in ((s, bad_d, w), (s, d, bad_w)):
+        with pytest.raises(dyg.DygError) as e:
+            dyg.Graph.from_edges(m + 1, *args)
+        assert e.value.status == dyg.DYG_EINVAL
+    assert dyg.Graph.from_edges(m + 1, s, d, w).info()["n_slots"] == 2 * m
+
+
+def test_export_short_buffer(dyg):  # noqa: F811
+    s, d, w = star(400, 300, np.random.default_rng(1))
+    g = dyg.Graph.from_edges(400, s, d, w)
+    rp0, col0, w0 = g.export()
+    rp, col, ww = np.zeros(401, np.uint64), np.zeros(50, np.uint32), np.zeros(50, np.float32)
+    assert dyg.lib().dyg_graph_export(g.handle, rp.ctypes.data, col.ctypes.data, ww.ctypes.data, 50) == 4
+    assert np.array_equal(rp, rp0) and np.array_equal(col, col0[:50]) and np.array_equal(ww, w0[:50])
