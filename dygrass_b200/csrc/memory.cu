@@ -25,6 +25,7 @@ namespace dyg {
 namespace {
 
 constexpr unsigned long long kPoolKeep = 256ull << 20;
+constexpr unsigned long long kScratchKeep = 256ull << 20;
 constexpr int kMaxDevices = 64;
 
 struct DevicePool {
@@ -117,6 +118,56 @@ void dev_free(void *ptr) {
         cudaFree(ptr);
     }
     cudaGetLastError();
+}
+
+namespace {
+// One scratch block per device, kept between the calls that borrow it.
+struct Scratch {
+    void *p = nullptr;
+    size_t bytes = 0;
+    unsigned long long ctx = 0;
+};
+std::mutex g_scratch_mu;
+Scratch g_scratch[kMaxDevices];
+}  // namespace
+
+cudaError_t scratch_borrow(Buf *b, size_t bytes) {
+    int dev = 0;
+    *b = Buf{};
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices) {
+        const unsigned long long ctx = current_context_id();
+        std::lock_guard<std::mutex> lk(g_scratch_mu);
+        Scratch &s = g_scratch[dev];
+        if (s.p && s.ctx != ctx) s = Scratch{};   // went with its context
+        if (s.p && s.bytes >= bytes) {
+            b->p = s.p;
+            b->bytes = s.bytes;
+            s = Scratch{};
+            return cudaSuccess;
+        }
+    }
+    const cudaError_t e = dev_alloc(&b->p, bytes);
+    b->bytes = e == cudaSuccess ? bytes : 0;
+    return e;
+}
+
+void scratch_return(Buf *b) {
+    if (!b->p) return;
+    int dev = 0;
+    Buf drop = *b;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices && b->bytes <= kScratchKeep) {
+        const unsigned long long ctx = current_context_id();
+        std::lock_guard<std::mutex> lk(g_scratch_mu);
+        Scratch &s = g_scratch[dev];
+        if (ctx && (!s.p || s.ctx != ctx || s.bytes < b->bytes)) {
+            drop = s.p && s.ctx == ctx ? Buf{s.p, s.bytes} : Buf{};
+            s.p = b->p;
+            s.bytes = b->bytes;
+            s.ctx = ctx;
+        }
+    }
+    dev_free(drop.p);
+    *b = Buf{};
 }
 
 namespace {

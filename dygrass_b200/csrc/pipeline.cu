@@ -108,6 +108,7 @@ struct DeleteArgs {
     uint32_t *f_src, *f_dst, *f_idx;
     unsigned long long *f_uid;
     unsigned long long *keys, *work;   // zeroed for the walks
+    uint32_t *rec_head;                // as well (may be null)
     uint32_t *blk, *counts;
     unsigned long long *err;
     const unsigned long long *halt;
@@ -126,6 +127,7 @@ __global__ void __launch_bounds__(kOpThreads, 2) k_delete(const __grid_constant_
         reinterpret_cast<uint16_t *>(a.fG)[e] = 0;
         reinterpret_cast<uint16_t *>(a.fH)[e] = 0;
         a.keys[e] = 0ull;
+        if (a.rec_head) a.rec_head[e] = 0u;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) *a.work = 0ull;
     if (!grid_sync(bar, [&] { *a.D.c.items = *a.D.items_h = 0ull; })) return;
@@ -217,10 +219,12 @@ __device__ __forceinline__ Fallback fallback_walk(const DevGraph &g, uint32_t s0
 
 // Walk results, recovery candidates and their commit in one launch.
 //   results    status and conductance of each walked deletion; path lengths
-//              and edges without a path summed per block
+//              (the winner's step count) and edges without a path summed per
+//              block
 //   candidates path edges of walk-list entry f at its scanned offset (one
-//              warp per path; each edge's weight from the G slot the replay
-//              took: G is unchanged since), then, after all path candidates,
+//              warp per path; each edge's vertices and weight from the G slots
+//              the winner took, as its record or its replay has them: G is
+//              unchanged since), then, after all path candidates,
 //              the fallback walks of the edges without a path
 //              (main.cu:400-408, 428-436); each enters the dedup table
 //   keep       candidate i is kept if it is the first occurrence of its edge
@@ -240,6 +244,7 @@ struct RecoverArgs {
     bool resume;   // the candidates are there: only their commit is missing
     unsigned long long *keys;   // winner keys of the walk list
     bool clear_keys;
+    PathRec rec;                // winners' paths: records, or (rec.heads null) replayed:
     const int32_t *plen;
     const uint32_t *pv, *ps;
     uint32_t stride, hw;
@@ -257,7 +262,7 @@ struct RecoverArgs {
     uint32_t *blk, *counts;
     unsigned long long *sc;   // G's scalars
     unsigned long long *halt;
-    unsigned long long code_records, code_arena;
+    unsigned long long code_records, code_arena, code_paths;
 };
 
 __device__ __forceinline__ void cand_put(const RecoverArgs &a, uint32_t i, uint32_t x, uint32_t y,
@@ -327,9 +332,8 @@ __global__ void __launch_bounds__(kOpThreads, 2) k_recover(const __grid_constant
         uint32_t len = 0u, none = 0u;
         for (uint32_t f = rg.x + threadIdx.x; f < rg.y; f += blockDim.x) {
             const uint32_t e = a.f_idx[f];
-            const int32_t L = a.plen[f];
             const unsigned long long k = a.keys[f];
-            if (a.clear_keys && k) a.keys[f] = 0ull;
+            const int32_t L = a.rec.heads ? key_found(k) : a.plen[f];
             a.status[e] = L > 0 ? L : DYG_DEL_NO_PATH;
             a.cond[e] = k ? __uint_as_float((uint32_t)(k >> 32)) : 0.f;
             if (L > 0) len += (uint32_t)L;
@@ -341,7 +345,25 @@ __global__ void __launch_bounds__(kOpThreads, 2) k_recover(const __grid_constant
             a.blk[blockIdx.x] = len;
             a.blk[kOpBlocksMax + blockIdx.x] = none;
         }
-        if (!grid_sync(bar)) return;
+        // path records that did not fit halt the batch before anything else of
+        // it changes; its walks are repeated with room for them
+        if (!grid_sync(bar, [&] {
+                if (!a.rec.heads) return;
+                const unsigned long long used = __ldcg(a.rec.cursor);
+                *a.rec.cursor = 0ull;
+                if (used > a.rec.cap) {
+                    a.sc[S_RECNEED] = used;
+                    *a.halt = a.code_paths;
+                }
+            }))
+            return;
+        if (*(volatile unsigned long long *)a.halt) {
+            for (uint32_t f = rg.x + threadIdx.x; f < rg.y; f += blockDim.x) {
+                a.rec.heads[f] = 0u;
+                if (a.clear_keys) a.keys[f] = 0ull;
+            }
+            return;
+        }
         const uint2 pl = blocks_before(a.blk, s.warp);
         const uint2 pn = blocks_before(a.blk + kOpBlocksMax, s.warp);
         n_path = pl.y;
@@ -354,7 +376,7 @@ __global__ void __launch_bounds__(kOpThreads, 2) k_recover(const __grid_constant
         uint32_t at = pl.x, nth = pn.x;
         for (uint32_t t = rg.x; t < rg.y; t += blockDim.x) {
             const uint32_t f = t + threadIdx.x;
-            const int32_t L = f < rg.y ? a.plen[f] : 0;
+            const int32_t L = f < rg.y ? (a.rec.heads ? key_found(a.keys[f]) : a.plen[f]) : 0;
             const uint32_t l = L > 0 ? (uint32_t)L : 0u, z = (f < rg.y && L <= 0) ? 1u : 0u;
             uint32_t tl, tz;
             const uint32_t ol = at + block_excl(l, s.warp, &tl), oz = nth + block_excl(z, s.warp, &tz);
@@ -367,10 +389,30 @@ __global__ void __launch_bounds__(kOpThreads, 2) k_recover(const __grid_constant
             for (uint32_t q = threadIdx.x >> 5; q < here; q += blockDim.x >> 5) {
                 const uint32_t base = s_off[q], n = s_len[q];
                 const uint32_t fq = t + q;
-                const uint32_t *v = a.pv + (size_t)fq * a.stride, *sl = a.ps + (size_t)fq * a.stride;
-                for (uint32_t j = lane; j < n; j += 32u)
-                    cand_put(a, base + j, v[j], v[j + 1], a.G.wts[sl[j + 1]], mask, true);
-                if (n) continue;
+                if (n && a.rec.heads) {
+                    const unsigned long long key = a.keys[fq];
+                    uint32_t r = a.rec.heads[fq];
+                    while (a.rec.words[r] != (uint32_t)key || a.rec.words[r + 1u] != (uint32_t)(key >> 32))
+                        r = a.rec.words[r - 1u];
+                    const uint32_t *sl = a.rec.words + r + 2u;
+                    for (uint32_t j = lane; j < n; j += 32u) {
+                        const uint32_t at = sl[j];
+                        const uint32_t x = j ? a.G.slots[sl[j - 1u]].x : a.job.src[fq];
+                        cand_put(a, base + j, x, a.G.slots[at].x, a.G.wts[at], mask, true);
+                    }
+                } else if (n) {
+                    const uint32_t *v = a.pv + (size_t)fq * a.stride, *sl = a.ps + (size_t)fq * a.stride;
+                    for (uint32_t j = lane; j < n; j += 32u)
+                        cand_put(a, base + j, v[j], v[j + 1], a.G.wts[sl[j + 1]], mask, true);
+                }
+                if (n) {
+                    __syncwarp();   // every lane has read the edge's key and list head
+                    if (lane == 0u) {
+                        if (a.rec.heads) a.rec.heads[fq] = 0u;
+                        if (a.clear_keys) a.keys[fq] = 0ull;
+                    }
+                    continue;
+                }
                 const unsigned long long uid = a.job.uid[fq];
                 for (uint32_t j = lane; j < 2u * a.hw; j += 32u) {
                     const Fallback r = fallback_walk(a.G, j < a.hw ? a.job.src[fq] : a.job.dst[fq], uid,
@@ -577,6 +619,7 @@ dyg_status decr_delete_enqueue(dyg_graph *G, dyg_graph *H, const uint32_t *src,
     a.f_uid = ptr<unsigned long long>(ws.f_uid);
     a.keys = ptr<unsigned long long>(ws.keys);
     a.work = sc + S_WORK;
+    a.rec_head = ws.rec_head.bytes >= sizeof(uint32_t) * (size_t)n ? ptr<uint32_t>(ws.rec_head) : nullptr;
     a.blk = ptr<uint32_t>(ws.blk);
     a.counts = ptr<uint32_t>(ws.counts);
     a.err = sc + S_ERR;
@@ -584,23 +627,70 @@ dyg_status decr_delete_enqueue(dyg_graph *G, dyg_graph *H, const uint32_t *src,
     return launch_phases<k_delete>(op_blocks(m, G->long_rows || H->long_rows), st, a, grid_bar(G));
 }
 
+dyg_status PathScratch::open(dyg_graph *G, uint32_t n, const dyg_walk_params &p, cudaStream_t stream) {
+    st = stream;
+    if (p.max_steps > kPathSteps || n == 0) return DYG_OK;
+    if (p.transition == DYG_TRANSITION_UNIFORM && (uint64_t)n * p.walkers > kPathWalkers) return DYG_OK;
+    Workspace &ws = G->ws;
+    const uint32_t threads = walk_threads(n, p);
+    const size_t hist_bytes = sizeof(uint32_t) * (size_t)threads * ((p.max_steps + 3u) & ~3u);
+    // some paths of a few moves per edge to begin with
+    const size_t words = sizeof(uint32_t) * ((size_t)n * 48u + 4096u);
+    if (scratch_borrow(&hist, hist_bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return DYG_OK;
+    }
+    DYG_TRY(ensure(ws.rec_head, sizeof(uint32_t) * (size_t)n));
+    DYG_TRY(ensure(ws.rec_words, words));
+    rec.heads = ptr<uint32_t>(ws.rec_head);
+    rec.words = ptr<uint32_t>(ws.rec_words);
+    rec.cap = (uint32_t)(ws.rec_words.bytes / sizeof(uint32_t) > 0xFFFFFF00u ? 0xFFFFFF00u
+                                                                             : ws.rec_words.bytes / sizeof(uint32_t));
+    rec.cursor = ptr<unsigned long long>(ws.scalars) + S_RECW;
+    rec.hist = ptr<uint32_t>(hist);
+    rec.threads = threads;
+    return DYG_OK;
+}
+
+dyg_status PathScratch::grow(dyg_graph *G) {
+    const unsigned long long need = G->ws.host_scalars[S_RECNEED] + G->ws.host_scalars[S_RECNEED] / 4;
+    if (need > 0xFFFFFF00ull) {
+        rec = PathRec{};   // replay the winners instead
+        return DYG_OK;
+    }
+    DYG_TRY(ensure(G->ws.rec_words, sizeof(uint32_t) * need));
+    rec.words = ptr<uint32_t>(G->ws.rec_words);
+    rec.cap = (uint32_t)need;
+    return DYG_OK;
+}
+
+PathScratch::~PathScratch() {
+    if (!hist.p) return;
+    cudaStreamSynchronize(st);
+    scratch_return(&hist);
+}
+
 // Walk-and-recover stage over walk-list entries [f0, f0 + nf) (nf a host
 // bound; F_dev, if given, is the device count of the whole list), from phase
-// `phase0` (0 = walks, 1 = recovery).
+// `phase0` (0 = walks, 1 = recovery, 2 = walks repeated with more room for
+// their paths: the deletions are done).
 dyg_status decr_walk_enqueue(dyg_graph *G, dyg_graph *H, uint32_t f0, uint32_t nf,
                              const uint32_t *F_dev, const dyg_walk_params &p,
                              unsigned long long *halt, uint32_t batch, uint32_t phase0,
                              int32_t *status, float *cond, cudaStream_t st, bool walk_ready,
-                             const unsigned long long *keys_given) {
+                             PathRec *rec, const unsigned long long *keys_given) {
     if (nf == 0) return DYG_OK;
     Workspace &ws = G->ws;
     const uint32_t n = nf;
     const uint32_t stride = p.max_steps > 2 ? p.max_steps : 2;
     const uint32_t hwk = p.heuristic_walkers;
     DYG_TRY(ensure(ws.keys, sizeof(unsigned long long) * n));
-    DYG_TRY(ensure(ws.path_v, sizeof(uint32_t) * (size_t)n * stride));
-    DYG_TRY(ensure(ws.path_s, sizeof(uint32_t) * (size_t)n * stride));
-    DYG_TRY(ensure(ws.path_len, sizeof(int32_t) * n));
+    const bool replay = keys_given || !rec || !rec->heads;
+    if (replay) {
+        DYG_TRY(ensure(ws.path_v, sizeof(uint32_t) * (size_t)n * stride));
+        DYG_TRY(ensure(ws.path_s, sizeof(uint32_t) * (size_t)n * stride));
+        DYG_TRY(ensure(ws.path_len, sizeof(int32_t) * n));
+    }
     // path candidates at [0, C_CANDS), then the fallback candidates
     const size_t n_path = (size_t)n * (stride - 1u), n_fb = (size_t)n * 4u * hwk, M = n_path + n_fb;
     DYG_TRY(ensure(ws.cand_x, sizeof(uint32_t) * M));
@@ -628,9 +718,10 @@ dyg_status decr_walk_enqueue(dyg_graph *G, dyg_graph *H, uint32_t f0, uint32_t n
     a.A.s[0] = append_side(H, ptr<uint32_t>(ws.cand_x), ptr<uint32_t>(ws.cand_y), ptr<float>(ws.cand_w));
     a.A.n = 1;
     a.job = job;
-    a.resume = phase0 > 0;
+    a.resume = phase0 == 1;
     a.keys = keys_given ? const_cast<unsigned long long *>(keys_given) : own;
     a.clear_keys = !keys_given;
+    if (!replay) a.rec = *rec;
     a.plen = ptr<int32_t>(ws.path_len);
     a.pv = ptr<uint32_t>(ws.path_v);
     a.ps = ptr<uint32_t>(ws.path_s);
@@ -655,15 +746,17 @@ dyg_status decr_walk_enqueue(dyg_graph *G, dyg_graph *H, uint32_t f0, uint32_t n
     a.halt = halt;
     a.code_records = halt_code(batch, (uint32_t)kHaltRecords, 1);
     a.code_arena = halt_code(batch, (uint32_t)kHaltArena, 1);
-    if (phase0 == 0) {
+    a.code_paths = halt_code(batch, (uint32_t)kHaltPaths, 2);
+    if (phase0 != 1) {
         // walks on the updated G (main.cu:392, 420)
         RowIndex ix{};   // of the walks, and of the replays of their winners
         DYG_TRY(index_enqueue(G, p, halt, &ix, st));
         if (!keys_given) {
             if (!walk_ready) DYG_CUDA(cudaMemsetAsync(own, 0, sizeof(unsigned long long) * n, st));
-            DYG_TRY(launch_walk(G, job, p, false, own, ix, st, walk_ready));
+            DYG_TRY(launch_walk(G, job, p, false, own, ix, st, walk_ready, replay ? nullptr : rec));
         }
-        DYG_TRY(launch_winner_paths(G, job, p, a.keys, n, stride, ptr<uint32_t>(ws.path_v),
+        if (replay)
+            DYG_TRY(launch_winner_paths(G, job, p, a.keys, n, stride, ptr<uint32_t>(ws.path_v),
                                     ptr<uint32_t>(ws.path_s), ptr<int32_t>(ws.path_len), ix, st));
     }
     // blocks for what a batch usually brings: a few candidates per deletion
@@ -674,13 +767,13 @@ dyg_status decr_walk_enqueue(dyg_graph *G, dyg_graph *H, uint32_t f0, uint32_t n
 // walks over the batch's whole walk list.
 static dyg_status decr_enqueue(dyg_graph *G, dyg_graph *H, const uint32_t *src, const uint32_t *dst,
                                uint32_t n, uint64_t uid0, const unsigned long long *uids,
-                               const dyg_walk_params &p,
+                               const dyg_walk_params &p, PathRec *rec,
                                unsigned long long *halt, uint32_t batch, uint32_t phase0,
                                int32_t *status, float *cond, cudaStream_t st) {
     if (phase0 == 0)
         DYG_TRY(decr_delete_enqueue(G, H, src, dst, n, uid0, uids, false, halt, status, cond, st));
     return decr_walk_enqueue(G, H, 0, n, ptr<uint32_t>(G->ws.counts) + C_FILTERED, p, halt, batch,
-                             phase0, status, cond, st, true);
+                             phase0, status, cond, st, true, rec);
 }
 
 // --------------------------------------------------------- stream drivers
@@ -767,12 +860,14 @@ dyg_status decremental_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, cons
     DYG_CUDA(cudaMemcpyAsync(sc + S_RECCNT, init, sizeof(init), cudaMemcpyHostToDevice, st));
     DYG_TRY(clear_halt(G, st));
     if (check_inputs) DYG_TRY(validate_enqueue(halt, sc + S_ERR, src, dst, nullptr, n, G->g.n, st));
+    PathScratch paths;
+    DYG_TRY(paths.open(G, B < n ? B : n, p, st));
     uint32_t b_start = 0, ph_start = 0;
     for (int round = 0; round < 64; ++round) {
         for (uint32_t b = b_start; (uint64_t)b * B < n; ++b) {
             const uint32_t b0 = b * B, nb = (n - b0 < B) ? n - b0 : B;
             DYG_TRY(decr_enqueue(G, H, src + b0, dst + b0, nb, uid_base + b0,
-                                 uids ? uids + b0 : nullptr, p, halt, b,
+                                 uids ? uids + b0 : nullptr, p, &paths.rec, halt, b,
                                  b == b_start ? ph_start : 0, status + b0, cond + b0, st));
         }
         if (during && round == 0) (*during)();
@@ -794,6 +889,8 @@ dyg_status decremental_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, cons
             cap = ncap;
             DYG_CUDA(cudaMemcpyAsync(sc + S_RECCAP, &cap, sizeof(cap), cudaMemcpyHostToDevice, st));
             DYG_CUDA(cudaStreamSynchronize(st));
+        } else if (hi.kind == kHaltPaths) {
+            DYG_TRY(paths.grow(G));
         } else {
             DYG_TRY(grow_arena(H, H->g.arena_cap * 2, st));
         }

@@ -296,7 +296,7 @@ dyg_status dyg_decremental_commit_keys(dyg_graph *G, dyg_graph *H, const dyg_wal
     for (; round < 64; ++round) {
         DYG_TRY(clear_halt_of(G, st));
         DYG_TRY(decr_walk_enqueue(G, H, 0, n_walk, nullptr, *p, halt, 0, phase, status,
-                                  conductance, st, false, (const unsigned long long *)keys));
+                                  conductance, st, false, nullptr, (const unsigned long long *)keys));
         DYG_TRY(read_scalars2(G, H, st));
         const unsigned long long h = ws.host_scalars[S_HALT];
         if (!h) {

@@ -587,6 +587,8 @@ dyg_status delete_file_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, cons
     DYG_TRY(clear_halt(G, st));
     if (check_inputs)
         DYG_TRY(validate_enqueue(halt, sc + S_ERR, src, dst, nullptr, n, G->g.n, st));
+    PathScratch paths;
+    DYG_TRY(paths.open(G, n, p, st));
     DYG_TRY(decr_delete_enqueue(G, H, src, dst, n, uid0, nullptr, true, halt, status, cond, st));
     const uint32_t nchunks = (uint32_t)(((uint64_t)n + chunk - 1) / chunk);
     uint32_t c_start = 0, ph_start = 0;
@@ -595,7 +597,7 @@ dyg_status delete_file_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, cons
             const uint32_t f0 = c * chunk;
             const uint32_t nc = n - f0 < chunk ? n - f0 : chunk;
             DYG_TRY(decr_walk_enqueue(G, H, f0, nc, ptr<uint32_t>(ws.counts) + C_FILTERED, p, halt,
-                                      c, c == c_start ? ph_start : 0, status, cond, st, true));
+                                      c, c == c_start ? ph_start : 0, status, cond, st, true, &paths.rec));
         }
         if (fetch) DYG_TRY((*fetch)());
         DYG_TRY(read_scalars2(G, H, st));
@@ -615,6 +617,8 @@ dyg_status delete_file_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, cons
             cap = ncap;
             DYG_CUDA(cudaMemcpyAsync(sc + S_RECCAP, &cap, sizeof(cap), cudaMemcpyHostToDevice, st));
             DYG_CUDA(cudaStreamSynchronize(st));
+        } else if (hi.kind == kHaltPaths) {
+            DYG_TRY(paths.grow(G));
         } else {
             DYG_TRY(grow_arena(H, H->g.arena_cap * 2, st));
         }

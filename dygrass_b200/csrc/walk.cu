@@ -86,6 +86,7 @@ struct WalkArgs {
     DevGraph g;
     WalkJob job;
     RowIndex ix;      // weighted walks
+    PathRec rec;      // decremental walks
     uint32_t walkers, max_steps;
     uint32_t prune;
     uint32_t prune_every;   // iterations between reads of the edge's best (a power of two)
@@ -736,6 +737,35 @@ __device__ __forceinline__ uint32_t best_bits(const WalkArgs &a, uint32_t e) {
     return *(reinterpret_cast<const volatile uint32_t *>(a.keys + e) + 1);
 }
 
+// Copies a walker's path of L moves to a record of edge e: its first `kept`
+// moves from the history (four = true: four moves to a uint4), the rest from
+// `last`.
+__device__ __forceinline__ void write_record(const PathRec &rec, uint32_t e, unsigned long long key,
+                                             uint32_t L, uint32_t tid, uint32_t nth, bool four,
+                                             uint32_t kept, const uint32_t (&last)[4]) {
+    const unsigned long long at = atomicAdd(rec.cursor, (unsigned long long)L + 3ull);
+    if (at + L + 3ull > rec.cap) return;   // the commit sees the cursor past the end
+    uint32_t *w = rec.words + at;
+    w[0] = atomicExch(rec.heads + e, (uint32_t)at + 1u);
+    w[1] = (uint32_t)key;
+    w[2] = (uint32_t)(key >> 32);
+    if (four) {
+        const uint4 *h = reinterpret_cast<const uint4 *>(rec.hist) + tid;
+        for (uint32_t j = 0; j < kept; j += 4u, h += nth) {
+            const uint4 q = *h;
+            w[3u + j] = q.x;
+            w[4u + j] = q.y;
+            w[5u + j] = q.z;
+            w[6u + j] = q.w;
+        }
+    } else {
+        for (uint32_t j = 0; j < kept; ++j) w[3u + j] = rec.hist[(size_t)j * nth + tid];
+    }
+#pragma unroll
+    for (uint32_t u = 0; u < 4u; ++u)
+        if (kept + u < L) w[3u + kept + u] = last[u];
+}
+
 // The uniform transition's walks.  Walks are short (5.8 moves on the mesh's
 // sparsifier: most end in a leaf), so the cost is shared between the moves and
 // what surrounds them; every iteration starts walkers in the free lanes and
@@ -752,8 +782,10 @@ __device__ __forceinline__ uint32_t best_bits(const WalkArgs &a, uint32_t e) {
 // and best per walker and the general remainder: insertions of the 100^3 mesh
 // 5.27 -> 4.43 ms, 24 random geometric graphs 1.14 -> 0.96 ms, deletions of
 // the mesh 2.28 -> 2.25 ms.
-template <bool INCR>
-__global__ void __launch_bounds__(kWalkThreads, 6) k_walk_uniform(WalkArgs a) {
+// REC: the walkers keep their paths (see PathRec), at five blocks of 48
+// registers, since six would spill.
+template <bool INCR, bool REC>
+__global__ void __launch_bounds__(kWalkThreads, REC ? 5 : 6) k_walk_uniform(WalkArgs a) {
     __shared__ uint32_t s_div[kDivTab];
     __shared__ ChunkEdge s_edge[kWalkThreads / 32];
     if (a.job.halt && *a.job.halt) return;
@@ -767,6 +799,7 @@ __global__ void __launch_bounds__(kWalkThreads, 6) k_walk_uniform(WalkArgs a) {
     uint32_t cur = 0u, prev = 0u, step = 0u, tgt = 0u, walker = 0u, c2 = 0u, c3 = 0u, my_e = 0u;
     float R = 0.f, we = 0.f;
     uint32_t moves = 0u, walks = 0u;
+    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;   // REC
     for (uint32_t T = 0u;; ++T) {
         refill<INCR>(a, n_chunks, chunk, ce, lane, __ballot_sync(kFull, !active), &walks,
                      [&](const ChunkEdge &x, uint32_t k) {
@@ -785,6 +818,8 @@ __global__ void __launch_bounds__(kWalkThreads, 6) k_walk_uniform(WalkArgs a) {
         if (active) {
             const uint4 blk = philox4x32_10(make_uint4((step - 1u) >> 2, walker, c2, c3), a.key);
             const uint32_t left = a.max_steps - step;   // the walk ends when its step reaches max_steps
+            uint32_t took[4] = {0u, 0u, 0u, 0u};        // slots of this iteration's moves (decremental)
+            uint32_t found = 0u;
 #pragma unroll
             for (uint32_t mv = 0; mv < 4u; ++mv) {
                 if (!active) break;
@@ -800,20 +835,26 @@ __global__ void __launch_bounds__(kWalkThreads, 6) k_walk_uniform(WalkArgs a) {
                 }
                 const uint32_t r = mv == 0u ? blk.x : (mv == 1u ? blk.y : (mv == 2u ? blk.z : blk.w));
                 const uint2 *row = a.g.slots + d.x;
-                uint2 sl = __ldg(row + rem_small(r, deg, s_div));
+                uint32_t at = rem_small(r, deg, s_div);
+                uint2 sl = __ldg(row + at);
                 if (!first) {
                     // loaded beside the drawn slot: some lane lands on its
                     // previous vertex in almost every move
                     const uint2 last = __ldg(row + deg);
-                    if (sl.x == prev) sl = last;
+                    if (sl.x == prev) {
+                        sl = last;
+                        at = deg;
+                    }
                 }
+                if (REC) took[mv] = d.x + at;
                 ++moves;
                 R = __fadd_rn(R, __uint_as_float(sl.y));
                 if (INCR && !first && __fmul_rn(R, we) >= a.threshold) {
                     active = false;
                 } else if (sl.x == tgt) {
                     // published at once, so the edge's other walkers can stop early
-                    atomicMax(a.keys + my_e, pack_key(__frcp_rn(R), walker, step + mv));
+                    if (REC) found = step + mv;
+                    else atomicMax(a.keys + my_e, pack_key(__frcp_rn(R), walker, step + mv));
                     active = false;
                 } else if (mv + 1u >= left) {
                     active = false;
@@ -821,6 +862,14 @@ __global__ void __launch_bounds__(kWalkThreads, 6) k_walk_uniform(WalkArgs a) {
                 prev = cur;
                 cur = sl.x;
             }
+            if (REC && found) {
+                const unsigned long long key = pack_key(__frcp_rn(R), walker, found);
+                const unsigned long long was = atomicMax(a.keys + my_e, key);
+                if (key > was) write_record(a.rec, my_e, key, found, tid, nth, true, step - 1u, took);
+            }
+            if (REC && active)
+                reinterpret_cast<uint4 *>(a.rec.hist)[(size_t)((step - 1u) >> 2) * nth + tid] =
+                    make_uint4(took[0], took[1], took[2], took[3]);
             step += 4u;
             if (active && a.prune && (T & (a.prune_every - 1u)) == a.prune_every - 1u) {
                 const uint32_t known = best_bits(a, my_e);
@@ -848,6 +897,7 @@ __global__ void __launch_bounds__(kWalkThreads, 3) k_walk_weighted(WalkArgs a) {
     uint32_t my_e = 0u, known = 0u;
     Walker s{};
     uint32_t moves = 0u, walks = 0u;
+    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
     for (uint32_t T = 0u;; ++T) {
         refill<INCR>(a, n_chunks, chunk, ce, lane, __ballot_sync(kFull, !active), &walks,
                      [&](const ChunkEdge &x, uint32_t k) {
@@ -875,8 +925,16 @@ __global__ void __launch_bounds__(kWalkThreads, 3) k_walk_weighted(WalkArgs a) {
                                                    seg, lane, &moved, &taken, &taken_at);
             if (active) {
                 moves += moved ? 1u : 0u;
-                if (r == kFound)
-                    atomicMax(a.keys + my_e, pack_key(__frcp_rn(s.R), s.walker, s.step));
+                if (r == kFound) {
+                    const unsigned long long key = pack_key(__frcp_rn(s.R), s.walker, s.step);
+                    const unsigned long long was = atomicMax(a.keys + my_e, key);
+                    if (!INCR && a.rec.heads && key > was) {
+                        const uint32_t took[4] = {taken_at, 0u, 0u, 0u};
+                        write_record(a.rec, my_e, key, s.step, tid, nth, false, s.step - 1u, took);
+                    }
+                } else if (!INCR && a.rec.heads && r == kContinue) {
+                    a.rec.hist[(size_t)(s.step - 2u) * nth + tid] = taken_at;   // the move just made
+                }
                 if (r != kContinue || (known && below_best(s.R, __uint_as_float(known)))) active = false;
             }
             if (!__any_sync(kFull, active)) break;
@@ -1026,7 +1084,7 @@ static uint32_t chunk_for(uint32_t walkers) {
 // more warps than there are chunks, since each idle warp costs an atomic on
 // the chunk counter: a 32-edge batch has 512 chunks for 7,104 warps.
 template <auto Kernel>
-static void launch_walk_kernel(const WalkArgs &a, cudaStream_t st) {
+static uint32_t walk_blocks(uint32_t n, uint32_t walkers, uint32_t chunk) {
     static const int per_sm = [] {
         int nb = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, Kernel, kWalkThreads, 0);
@@ -1034,20 +1092,34 @@ static void launch_walk_kernel(const WalkArgs &a, cudaStream_t st) {
     }();
     const uint32_t t = g_tune_bpsm.load();
     const uint64_t fit = (uint64_t)((t && (int)t < per_sm) ? (int)t : per_sm) * num_sms();
-    const uint64_t chunks = (uint64_t)a.job.n_host * (a.walkers / a.chunk);
     // four chunks' warps to a block of eight while SMs are idle: half-empty
     // blocks spread a small batch over more of them
-    const uint64_t want = (chunks + 3) / 4;
-    Kernel<<<(unsigned)(want < 1 ? 1 : (want < fit ? want : fit)), kWalkThreads, 0, st>>>(a);
+    const uint64_t want = ((uint64_t)n * (walkers / chunk) + 3) / 4;
+    return (uint32_t)(want < 1 ? 1 : (want < fit ? want : fit));
+}
+
+template <auto Kernel>
+static void launch_walk_kernel(const WalkArgs &a, cudaStream_t st) {
+    uint32_t blocks = walk_blocks<Kernel>(a.job.n_host, a.walkers, a.chunk);
+    if (a.rec.heads && blocks > a.rec.threads / kWalkThreads) blocks = a.rec.threads / kWalkThreads;
+    Kernel<<<blocks, kWalkThreads, 0, st>>>(a);
+}
+
+uint32_t walk_threads(uint32_t n, const dyg_walk_params &p) {
+    const uint32_t c = chunk_for(p.walkers);
+    return kWalkThreads * (p.transition == DYG_TRANSITION_WEIGHTED
+                               ? walk_blocks<k_walk_weighted<false>>(n, p.walkers, c)
+                               : walk_blocks<k_walk_uniform<false, true>>(n, p.walkers, c));
 }
 
 static void launch_walk_any(const WalkArgs &a, bool incremental, bool wtd, cudaStream_t st) {
     if (incremental) {
         if (wtd) launch_walk_kernel<k_walk_weighted<true>>(a, st);
-        else launch_walk_kernel<k_walk_uniform<true>>(a, st);
+        else launch_walk_kernel<k_walk_uniform<true, false>>(a, st);
     } else {
         if (wtd) launch_walk_kernel<k_walk_weighted<false>>(a, st);
-        else launch_walk_kernel<k_walk_uniform<false>>(a, st);
+        else if (a.rec.heads) launch_walk_kernel<k_walk_uniform<false, true>>(a, st);
+        else launch_walk_kernel<k_walk_uniform<false, false>>(a, st);
     }
 }
 
@@ -1087,10 +1159,11 @@ dyg_status index_enqueue(dyg_graph *G, const dyg_walk_params &p, const unsigned 
 
 dyg_status launch_walk(dyg_graph *G, const WalkJob &job, const dyg_walk_params &p, bool incremental,
                        unsigned long long *keys, const RowIndex &ix, cudaStream_t st,
-                       bool counter_zero) {
+                       bool counter_zero, const PathRec *rec) {
     WalkArgs a{};
     a.g = G->g;
     a.ix = ix;
+    if (rec) a.rec = *rec;
     a.job = job;
     a.walkers = p.walkers;
     a.max_steps = p.max_steps;

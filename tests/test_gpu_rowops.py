@@ -200,3 +200,34 @@ def test_export_short_buffer(dyg):  # noqa: F811
     rp, col, ww = np.zeros(401, np.uint64), np.zeros(50, np.uint32), np.zeros(50, np.float32)
     assert dyg.lib().dyg_graph_export(g.handle, rp.ctypes.data, col.ctypes.data, ww.ctypes.data, 50) == 4
     assert np.array_equal(rp, rp0) and np.array_equal(col, col0[:50]) and np.array_equal(ww, w0[:50])
+
+
+@pytest.mark.parametrize("transition", [0, 1])
+@pytest.mark.parametrize("steps", [3, 5, 100, 256, 257])
+def test_winner_paths_recorded_and_replayed(dyg, oracle, transition, steps):  # noqa: F811
+    """Winners of one to 200 moves, with walks that keep their paths (up to 256
+    steps) and walks whose winners are replayed; the long ones ask for more
+    room than a call starts with, so their walks are repeated."""
+    k, rng = 1000, np.random.default_rng(steps)
+    # cycles of 3..200 vertices with a few chords
+    sizes = np.where(np.arange(k) % 4 == 0, 200, rng.integers(3, 40, k))
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    base, L = np.repeat(off[:-1], sizes), np.repeat(sizes, sizes)
+    i = np.arange(off[-1]) - base
+    gs, gd = (base + i).astype(np.uint32), (base + (i + 1) % L).astype(np.uint32)
+    ch = np.flatnonzero(rng.random(len(gs)) < 0.02)
+    gs = np.concatenate([gs, gs[ch]])
+    gd = np.concatenate([gd, (base + (i + L // 2) % L)[ch]]).astype(np.uint32)
+    ok = gs != gd
+    gs, gd = gs[ok], gd[ok]
+    gw = rng.uniform(0.5, 2.0, len(gs)).astype(np.float32)
+    n, dele = int(off[-1]), off[:-1]
+    G, H = dyg.Graph.from_edges(n, gs, gd, gw), dyg.Graph.from_edges(n, gs[dele], gd[dele], gw[dele])
+    Go, Ho = oracle.OGraph(n, gs, gd, gw), oracle.OGraph(n, gs[dele], gd[dele], gw[dele])
+    p = dyg.WalkParams.make(walkers=64, max_steps=steps, transition=transition, heuristic_walkers=2)
+    r = dyg.decremental_stream(G, H, gs[dele], gd[dele], p, batch_size=400)
+    st, cd, rx, ry, rk, _ = oracle.decremental(Go, Ho, gs[dele], gd[dele], p, batch_size=400)
+    assert np.array_equal(r.status, st) and np.array_equal(r.conductance.view(np.uint32), cd.view(np.uint32))
+    assert np.array_equal(r.rec_src, rx) and np.array_equal(r.rec_dst, ry) and np.array_equal(r.rec_kind, rk)
+    same_graph(G, Go)
+    same_graph(H, Ho)
