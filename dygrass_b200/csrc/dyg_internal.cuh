@@ -92,16 +92,16 @@ __host__ __device__ __forceinline__ int32_t key_found(unsigned long long k) {
 
 // Fixed-point weight of the weight-proportional mode (exact w * 2^32,
 // truncated) so that prefix sums are associative and match the host: the
-// 24-bit significand shifted by the exponent.  Weights are positive; from
-// 2^32 on (infinity included) the value is all ones.
+// 24-bit significand m shifted by the exponent.  w = m * 2^(ex - 150), so
+// w * 2^32 = (m * 2^40) >> (158 - ex); m * 2^40 has an empty low word.
+// Weights are not negative; from 2^32 on (infinity included) the value is all
+// ones, and below 2^-32 (0 included) the shift leaves nothing.
 __device__ __forceinline__ unsigned long long wq(float w) {
-    const uint32_t b = __float_as_uint(w);
-    const uint32_t ex = b >> 23;   // sign bit 0
-    const unsigned long long m = (b & 0x7FFFFFu) | 0x800000u;
-    // w = m * 2^(ex - 150), so w * 2^32 = m * 2^(ex - 118); below 2^-32 it is 0
-    if (ex < 95u || (int)b < 0) return 0ull;
-    if (ex >= 159u) return 0xFFFFFFFFFFFFFFFFull;
-    return ex >= 118u ? m << (ex - 118u) : m >> (118u - ex);
+    const uint32_t b = __float_as_uint(w), ex = b >> 23;
+    const unsigned long long top = (unsigned long long)((b << 8) | 0x80000000u) << 32;
+    unsigned long long q;
+    asm("shr.u64 %0, %1, %2;" : "=l"(q) : "l"(top), "r"(158u - ex));   // shifts of 64 and more give 0
+    return ex >= 159u ? 0xFFFFFFFFFFFFFFFFull : q;
 }
 __device__ __forceinline__ unsigned long long mul_hi32(uint32_t r, unsigned long long total) {
     // floor(r * total / 2^32) for a 96-bit product

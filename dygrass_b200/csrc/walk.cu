@@ -150,37 +150,37 @@ constexpr uint32_t kPickGroup = 8;
 
 struct PickGroup {
     uint2 c[kPickGroup];
-    unsigned long long q[kPickGroup];   // 0 outside the row and for `ex`
+    unsigned long long p[kPickGroup];   // inclusive prefixes over the group
 };
-__device__ __forceinline__ void pick_load(PickGroup &p, const uint2 *__restrict__ slots,
+__device__ __forceinline__ void pick_load(PickGroup &g, const uint2 *__restrict__ slots,
                                           const float *__restrict__ wts, uint32_t lo,
                                           uint32_t left, uint32_t ex, bool has_ex) {
     float w[kPickGroup];
 #pragma unroll
     for (uint32_t u = 0; u < kPickGroup; ++u) {
-        p.c[u] = u < left ? __ldg(slots + lo + u) : make_uint2(0u, 0u);
+        g.c[u] = u < left ? __ldg(slots + lo + u) : make_uint2(0u, 0u);
         w[u] = u < left ? __ldg(wts + lo + u) : 0.f;
     }
-#pragma unroll
-    for (uint32_t u = 0; u < kPickGroup; ++u)
-        p.q[u] = (u >= left || (has_ex && p.c[u].x == ex)) ? 0ull : wq(w[u]);
-}
-// The group's first slot whose prefix exceeds target (~0u: none); *acc is
-// carried over the groups.
-__device__ __forceinline__ uint32_t pick_in_group(const PickGroup &p, unsigned long long target,
-                                                  unsigned long long *acc, uint2 *picked) {
-    uint32_t at = ~0u;
+    unsigned long long sum = 0ull;
 #pragma unroll
     for (uint32_t u = 0; u < kPickGroup; ++u) {
-        *acc += p.q[u];
-        // a slot of weight 0 never is the first: the prefix did not grow
-        // (after a wrap past 2^64 it could still exceed the target, and the
-        // slots that count as absent are skipped)
-        if (at == ~0u && p.q[u] != 0ull && *acc > target) {
-            at = u;
-            *picked = p.c[u];
-        }
+        if (has_ex && g.c[u].x == ex) w[u] = 0.f;   // counts as absent
+        sum += wq(w[u]);
+        g.p[u] = sum;
     }
+}
+// The group's first slot whose prefix (after `before`) exceeds target, ~0u if
+// none.  A slot that is absent or weighs nothing has its predecessor's prefix,
+// so it is never the first, whether or not the sums wrapped past 2^64.
+__device__ __forceinline__ uint32_t pick_in_group(const PickGroup &g, unsigned long long target,
+                                                  unsigned long long before, uint2 *picked) {
+    uint32_t at = ~0u;
+#pragma unroll
+    for (int u = (int)kPickGroup - 1; u >= 0; --u)
+        if (before + g.p[u] > target) {
+            at = (uint32_t)u;
+            *picked = g.c[u];
+        }
     return at;
 }
 
@@ -188,23 +188,25 @@ __device__ __forceinline__ uint32_t lane_pick_weighted(const uint2 *__restrict__
                                                        const float *__restrict__ wts, uint32_t lo,
                                                        uint32_t deg, uint32_t ex, bool has_ex,
                                                        uint32_t r, uint2 *picked) {
-    PickGroup p;
-    pick_load(p, slots, wts, lo, deg, ex, has_ex);
-    unsigned long long total = 0ull;
-#pragma unroll
-    for (uint32_t u = 0; u < kPickGroup; ++u) total += p.q[u];
+    PickGroup g;
+    pick_load(g, slots, wts, lo, deg, ex, has_ex);
+    unsigned long long total = g.p[kPickGroup - 1u];
+    if (deg <= kPickGroup) {
+        if (total == 0ull) return ~0u;
+        return lo + pick_in_group(g, mul_hi32(r, total), 0ull, picked);
+    }
     for (uint32_t j0 = kPickGroup; j0 < deg; j0 += kPickGroup) {
-        pick_load(p, slots, wts, lo + j0, deg - j0, ex, has_ex);
-#pragma unroll
-        for (uint32_t u = 0; u < kPickGroup; ++u) total += p.q[u];
+        pick_load(g, slots, wts, lo + j0, deg - j0, ex, has_ex);
+        total += g.p[kPickGroup - 1u];
     }
     if (total == 0ull) return ~0u;
     const unsigned long long target = mul_hi32(r, total);
-    unsigned long long acc = 0ull;
+    unsigned long long before = 0ull;
     for (uint32_t j0 = 0; j0 < deg; j0 += kPickGroup) {
-        if (deg > kPickGroup) pick_load(p, slots, wts, lo + j0, deg - j0, ex, has_ex);
-        const uint32_t u = pick_in_group(p, target, &acc, picked);
+        pick_load(g, slots, wts, lo + j0, deg - j0, ex, has_ex);
+        const uint32_t u = pick_in_group(g, target, before, picked);
         if (u != ~0u) return lo + j0 + u;
+        before += g.p[kPickGroup - 1u];
     }
     return ~0u;
 }
