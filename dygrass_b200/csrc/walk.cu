@@ -416,7 +416,7 @@ __device__ __forceinline__ uint32_t warp_pick_weighted(const uint2 *__restrict__
 // files 15.2 -> 4.4 ms).  It is built whenever the graph has hub rows (over
 // kBigRow slots): even a single edge's walkers scan more than it costs.  Rows with a repeated column, or whose sum
 // wraps past 2^64, get no index and are searched by the warp as before.
-constexpr uint32_t kIdxRow = 32;        // longer rows are indexed (kCoopRow: the lane scans up to it)
+constexpr uint32_t kIdxRow = kPickGroup;   // longer rows are indexed: the lane reads up to it at once
 constexpr uint32_t kIdxBlockRow = 1024; // ... by a whole block from here on
 constexpr uint32_t kIdxTile = 8;        // slots per thread of a block's tile
 
@@ -439,9 +439,11 @@ __device__ __forceinline__ uint32_t index_pick(const uint2 *__restrict__ slots,
         while (true) {
             const uint32_t t = __ldg(region + h);
             if (t == 0u) break;
-            if (__ldg(&slots[lo + t - 1u].x) == ex) {
+            const uint32_t col = __ldg(&slots[lo + t - 1u].x);
+            const float w = __ldg(wts + lo + t - 1u);   // beside the column, not after it
+            if (col == ex) {
                 pos = t - 1u;
-                e = wq(__ldg(wts + lo + pos));
+                e = wq(w);
                 break;
             }
             h = (h + 1u) & ((1u << bits) - 1u);
@@ -452,12 +454,20 @@ __device__ __forceinline__ uint32_t index_pick(const uint2 *__restrict__ slots,
     const unsigned long long target = mul_hi32(r, total);
     // first slot whose prefix without `ex` exceeds the target; the slot of
     // `ex` itself leaves that prefix as it was, so it is never the first
-    uint32_t a = 0u, b = deg - 1u;
-    while (a < b) {
-        const uint32_t mid = (a + b) >> 1;
-        const unsigned long long v = __ldg(pre + mid) - (mid >= pos ? e : 0ull);
-        if (v > target) b = mid;
-        else a = mid + 1u;
+    // (seven pivots at a time: each round of loads divides the range by eight)
+    uint32_t a = 0u, len = deg;   // the first is in [a, a + len)
+    while (len > 1u) {
+        const uint32_t step = (len + 7u) >> 3;
+        uint32_t below = 0u;   // pivots whose prefix does not exceed the target
+#pragma unroll
+        for (uint32_t u = 1u; u <= 7u; ++u) {
+            const uint32_t j = a + u * step - 1u;   // last slot of the u-th part
+            const bool in = u * step < len;
+            const unsigned long long v = in ? __ldg(pre + j) - (j >= pos ? e : 0ull) : ~0ull;
+            below += v <= target ? 1u : 0u;
+        }
+        a += below * step;
+        len = min(step, len - below * step);
     }
     return lo + a;
 }
@@ -617,11 +627,11 @@ __device__ __forceinline__ int step_weighted_warp(Walker &s, bool active, const 
     }
     uint32_t at = ~0u;
     uint2 sl = make_uint2(0u, 0u);
-    const bool own_row = pick && d.y <= kCoopRow;   // chosen by this lane, slot in hand
-    if (own_row) at = lane_pick_weighted(g.slots, g.wts, d.x, d.y, s.prev, !first, r, &sl);
     uint32_t base = 0u;
-    if (pick && !own_row && ix.rbase) base = __ldg(ix.rbase + s.cur);
+    if (pick && d.y > kIdxRow && ix.rbase) base = __ldg(ix.rbase + s.cur);
     if (base) at = index_pick(g.slots, g.wts, ix.words + base, d.x, d.y, s.prev, !first, r);
+    const bool own_row = pick && !base && d.y <= kCoopRow;   // chosen by this lane, slot in hand
+    if (own_row) at = lane_pick_weighted(g.slots, g.wts, d.x, d.y, s.prev, !first, r, &sl);
     unsigned coop = __ballot_sync(kFull, pick && !own_row && !base);
     while (coop) {
         const uint32_t L = __ffs(coop) - 1u;
