@@ -3,20 +3,25 @@
 //
 // A batch's commit is a chain of short passes, each needing the one before it
 // to be complete.  As separate launches a pass of a few thousand entries
-// costs 4-6 us, nearly all of it launch and drain; as phases of one
-// cooperative launch separated by a grid barrier it costs the barrier (1.5 us
-// with one block, 2-3 us with one block per SM) and its own loads.  Measured
-// on whole calls: 64 deletions with recovery, 24 launches -> 4, 301 -> 223 us;
+// costs 4-6 us, nearly all of it launch and drain; as phases of one launch
+// separated by a barrier it costs the barrier and its own loads.  Measured on
+// whole calls: 64 deletions with recovery, 24 launches -> 4, 301 -> 223 us;
 // 1,000 insertions in ten batches 652 -> 424 us; 297,000 deletions of a 100^3
-// mesh in ten batches 4.79 -> 3.82 ms; 12 stream files of 4,096 edges on an
-// R-MAT graph (hub rows) 8.3 -> 6.7 ms.
+// mesh in ten batches 4.79 -> 3.82 ms.
 //
-// The barrier counts arrivals on one word and publishes a generation on
-// another, both in the owning graph's scalars.  Every grid that uses it is
-// launched cooperatively (all its blocks are resident), so a waiting block's
-// peers run; the wait is bounded all the same, and a block that gives up
-// raises kErrBarrier (the call then fails) and leaves.
+// A list that one block holds needs no more than its own barrier.  Up to 16
+// blocks are launched as one thread-block cluster, scheduled together by the
+// hardware and meeting at its barrier: 10 us a launch less than a cooperative
+// grid of as many blocks (the thirteen batches of 4,999 insertions and 7,777
+// deletions on a 37 x 41 x 29 mesh: 1.58 -> 1.44 ms).  Larger grids are
+// launched cooperatively; their barrier counts arrivals on one word and
+// publishes a generation on another, both in the owning graph's scalars.  All
+// blocks of such a grid are resident, so a waiting block's peers run; the wait
+// is bounded all the same, and a block that gives up raises kErrBarrier (the
+// call then fails) and leaves.
 #pragma once
+
+#include <type_traits>
 
 #include "dyg_internal.cuh"
 
@@ -30,7 +35,18 @@ constexpr uint32_t kBarSpinLimit = 1u << 26;
 struct GridBar {
     uint32_t *count, *gen;
     unsigned long long *err;
+    bool cluster;   // the grid is one thread-block cluster
 };
+
+struct NoWork {
+    __device__ void operator()() const {}
+};
+
+// Every thread of the cluster arrives and waits; writes made before are
+// visible after, in global memory as well.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 
 // The last block to arrive runs `last` (one thread) before any block leaves.
 // Writes made before the barrier by any thread of the grid are visible after
@@ -38,6 +54,14 @@ struct GridBar {
 template <class F>
 __device__ __forceinline__ bool grid_sync(const GridBar &b, F last) {
     __shared__ uint32_t s_ok;
+    if (b.cluster) {
+        cluster_sync();
+        if (!std::is_same<F, NoWork>::value) {
+            if (blockIdx.x == 0u && threadIdx.x == 0u) last();
+            cluster_sync();
+        }
+        return true;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
         uint32_t ok = 1u;
@@ -72,7 +96,7 @@ __device__ __forceinline__ bool grid_sync(const GridBar &b, F last) {
     return s_ok != 0u;
 }
 __device__ __forceinline__ bool grid_sync(const GridBar &b) {
-    return grid_sync(b, [] {});
+    return grid_sync(b, NoWork{});
 }
 
 // This block's contiguous share of [0, m): whole warps, in block order, so
@@ -136,33 +160,50 @@ __device__ __forceinline__ uint2 blocks_before(const uint32_t *vals, uint32_t *s
 // Most blocks of a one-launch kernel (the per-block words are sized for it).
 constexpr uint32_t kOpBlocksMax = 1024;
 
-// Launches Kernel(args...) with at most `want` blocks of kOpThreads, no more
-// than fit the device at once; a single block needs no cooperative launch.
+// Most blocks of a grid that is launched as one cluster (16 needs the opt-in
+// that launch_phases makes).
+constexpr uint32_t kClusterMax = 16;
+
+// Launches Kernel(args..., bar) with `want` blocks of kOpThreads: a single
+// block as it is; up to kClusterMax blocks as one cluster, whose blocks are
+// scheduled together and meet at the hardware's barrier; more of them
+// cooperatively, no more than fit the device at once.
 template <auto Kernel, class... A>
-dyg_status launch_phases(uint32_t want, cudaStream_t st, const A &...args) {
+dyg_status launch_phases(uint32_t want, cudaStream_t st, GridBar bar, const A &...args) {
     count_launch();
-    if (want <= 1u) {
-        Kernel<<<1, kOpThreads, 0, st>>>(args...);
-        DYG_CUDA(cudaGetLastError());
-        return DYG_OK;
-    }
-    static const int per_sm = [] {
-        int nb = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, Kernel, kOpThreads, 0);
-        return nb < 1 ? 1 : nb;
-    }();
-    uint32_t fit = (uint32_t)per_sm * (uint32_t)num_sms();
-    if (fit > kOpBlocksMax) fit = kOpBlocksMax;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(want < fit ? want : fit);
     cfg.blockDim = dim3(kOpThreads);
     cfg.stream = st;
     cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeCooperative;
-    at.val.cooperative = 1;
     cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    DYG_CUDA(cudaLaunchKernelEx(&cfg, Kernel, args...));
+    if (want <= 1u) {
+        cfg.gridDim = dim3(1);
+    } else if (want <= kClusterMax) {
+        static const cudaError_t allowed =
+            cudaFuncSetAttribute(Kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        DYG_CUDA(allowed);
+        uint32_t k = 2u;
+        while (k < want) k <<= 1;
+        cfg.gridDim = dim3(k);
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = k;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.numAttrs = 1;
+        bar.cluster = true;
+    } else {
+        static const int per_sm = [] {
+            int nb = 0;
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, Kernel, kOpThreads, 0);
+            return nb < 1 ? 1 : nb;
+        }();
+        uint32_t fit = (uint32_t)per_sm * (uint32_t)num_sms();
+        if (fit > kOpBlocksMax) fit = kOpBlocksMax;
+        cfg.gridDim = dim3(want < fit ? want : fit);
+        at.id = cudaLaunchAttributeCooperative;
+        at.val.cooperative = 1;
+        cfg.numAttrs = 1;
+    }
+    DYG_CUDA(cudaLaunchKernelEx(&cfg, Kernel, args..., bar));
     return DYG_OK;
 }
 

@@ -624,7 +624,7 @@ dyg_status decr_delete_enqueue(dyg_graph *G, dyg_graph *H, const uint32_t *src,
     a.counts = ptr<uint32_t>(ws.counts);
     a.err = sc + S_ERR;
     a.halt = halt;
-    return launch_phases<k_delete>(op_blocks(m, G->long_rows || H->long_rows), st, a, grid_bar(G));
+    return launch_phases<k_delete>(op_blocks(m, G->long_rows || H->long_rows), st, grid_bar(G), a);
 }
 
 dyg_status PathScratch::open(dyg_graph *G, uint32_t n, const dyg_walk_params &p, cudaStream_t stream) {
@@ -760,7 +760,7 @@ dyg_status decr_walk_enqueue(dyg_graph *G, dyg_graph *H, uint32_t f0, uint32_t n
                                     ptr<uint32_t>(ws.path_s), ptr<int32_t>(ws.path_len), ix, st));
     }
     // blocks for what a batch usually brings: a few candidates per deletion
-    return launch_phases<k_recover>(op_blocks(4ull * n, H->long_rows), st, a, grid_bar(G));
+    return launch_phases<k_recover>(op_blocks(4ull * n, H->long_rows), st, grid_bar(G), a);
 }
 
 // Decremental batch `batch` of the standalone updater: deletion stage, then

@@ -737,8 +737,8 @@ __device__ __forceinline__ void del_listed_rows(const DevGraph &g, const DelList
 //   static constexpr bool kList       whether take's bit 0 also lists the edge
 template <class Op>
 __global__ void __launch_bounds__(kOpThreads, 2)
-k_append(const Op op, const __grid_constant__ AppSides A, GridBar bar, uint32_t *blk, unsigned long long *work,
-         unsigned long long *halt, unsigned long long code) {
+k_append(const Op op, const __grid_constant__ AppSides A, uint32_t *blk, unsigned long long *work,
+         unsigned long long *halt, unsigned long long code, GridBar bar) {
     __shared__ RowShared s;
     if (*halt) return;
     const uint32_t n = op.count();
@@ -799,7 +799,7 @@ dyg_status append_enqueue(const Op &op, uint32_t n_host, dyg_graph *GA, const Ed
         A.n = 2;
     }
     const bool hubs = GA->long_rows || (GB && GB->long_rows);
-    return launch_phases<k_append<Op>>(op_blocks(2ull * n_host, hubs), st, op, A, grid_bar(GA),
+    return launch_phases<k_append<Op>>(op_blocks(2ull * n_host, hubs), st, grid_bar(GA), op, A,
                                        ptr<uint32_t>(GA->ws.blk), work, halt, code);
 }
 

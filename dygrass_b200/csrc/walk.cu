@@ -1166,8 +1166,8 @@ dyg_status index_enqueue(dyg_graph *G, const dyg_walk_params &p, const unsigned 
     a.counts = sc + S_IDXN;
     a.halt = halt;
     uint32_t *bw = reinterpret_cast<uint32_t *>(sc + S_BAR);
-    const GridBar bar{bw, bw + 1, sc + S_ERR};
-    DYG_TRY(launch_phases<k_index>(2u * (uint32_t)num_sms(), st, a, bar));
+    const GridBar bar{bw, bw + 1, sc + S_ERR, false};
+    DYG_TRY(launch_phases<k_index>(2u * (uint32_t)num_sms(), st, bar, a));
     *out = RowIndex{a.rbase, a.words};
     return DYG_OK;
 }
