@@ -222,7 +222,7 @@ __device__ __forceinline__ Fallback fallback_walk(const DevGraph &g, uint32_t s0
 //              (the winner's step count) and edges without a path summed per
 //              block
 //   candidates path edges of walk-list entry f at its scanned offset (one
-//              warp per path; each edge's vertices and weight from the G slots
+//              thread per edge; each edge's vertices and weight from the G slots
 //              the winner took, as its record or its replay has them: G is
 //              unchanged since), then, after all path candidates,
 //              the fallback walks of the edges without a path
@@ -320,9 +320,8 @@ __device__ __forceinline__ bool cand_keep(const RecoverArgs &a, uint32_t i, uint
 __global__ void __launch_bounds__(kOpThreads, 2) k_recover(const __grid_constant__ RecoverArgs a,
                                                            GridBar bar) {
     __shared__ RowShared s;
-    __shared__ uint32_t s_off[kOpThreads], s_len[kOpThreads];
+    __shared__ uint32_t s_off[kOpThreads], s_rec[kOpThreads], s_none[kOpThreads];
     if (*a.halt) return;
-    const uint32_t lane = threadIdx.x & 31u;
     uint32_t n_path, M;
     uint32_t mask = 1023u;
     if (blockIdx.x == 0 && threadIdx.x == 0) a.sc[S_WORK] = 0ull;   // the next walk's chunk counter
@@ -375,53 +374,61 @@ __global__ void __launch_bounds__(kOpThreads, 2) k_recover(const __grid_constant
         while (mask + 1u < 2u * M) mask = 2u * mask + 1u;
         uint32_t at = pl.x, nth = pn.x;
         for (uint32_t t = rg.x; t < rg.y; t += blockDim.x) {
-            const uint32_t f = t + threadIdx.x;
-            const int32_t L = f < rg.y ? (a.rec.heads ? key_found(a.keys[f]) : a.plen[f]) : 0;
-            const uint32_t l = L > 0 ? (uint32_t)L : 0u, z = (f < rg.y && L <= 0) ? 1u : 0u;
+            // one thread per walked deletion finds its winner's path and where
+            // its candidates go ...
+            const uint32_t q = threadIdx.x, f = t + q;
+            uint32_t l = 0u, z = 0u;
+            if (f < rg.y) {
+                const unsigned long long key = a.keys[f];
+                const int32_t L = a.rec.heads ? key_found(key) : a.plen[f];
+                l = L > 0 ? (uint32_t)L : 0u;
+                z = l ? 0u : 1u;
+                if (a.rec.heads) {
+                    uint32_t r = a.rec.heads[f];
+                    a.rec.heads[f] = 0u;
+                    if (l)
+                        while (a.rec.words[r] != (uint32_t)key || a.rec.words[r + 1u] != (uint32_t)(key >> 32))
+                            r = a.rec.words[r - 1u];
+                    s_rec[q] = r + 2u;
+                }
+                if (a.clear_keys) a.keys[f] = 0ull;
+            }
             uint32_t tl, tz;
-            const uint32_t ol = at + block_excl(l, s.warp, &tl), oz = nth + block_excl(z, s.warp, &tz);
-            s_len[threadIdx.x] = l;
-            s_off[threadIdx.x] = l ? ol : n_path + oz * 4u * a.hw;
-            at += tl;
-            nth += tz;
+            const uint32_t ol = block_excl(l, s.warp, &tl), oz = block_excl(z, s.warp, &tz);
+            s_off[q] = ol;
+            if (z) s_none[oz] = q;
             __syncthreads();
-            const uint32_t here = min(blockDim.x, rg.y - t);
-            for (uint32_t q = threadIdx.x >> 5; q < here; q += blockDim.x >> 5) {
-                const uint32_t base = s_off[q], n = s_len[q];
-                const uint32_t fq = t + q;
-                if (n && a.rec.heads) {
-                    const unsigned long long key = a.keys[fq];
-                    uint32_t r = a.rec.heads[fq];
-                    while (a.rec.words[r] != (uint32_t)key || a.rec.words[r + 1u] != (uint32_t)(key >> 32))
-                        r = a.rec.words[r - 1u];
-                    const uint32_t *sl = a.rec.words + r + 2u;
-                    for (uint32_t j = lane; j < n; j += 32u) {
-                        const uint32_t at = sl[j];
-                        const uint32_t x = j ? a.G.slots[sl[j - 1u]].x : a.job.src[fq];
-                        cand_put(a, base + j, x, a.G.slots[at].x, a.G.wts[at], mask, true);
-                    }
-                } else if (n) {
+            // ... and one per candidate writes it
+            for (uint32_t c = threadIdx.x; c < tl; c += blockDim.x) {
+                uint32_t lo = 0u, hi = blockDim.x;   // the last path that starts at or before c
+                while (hi - lo > 1u) {
+                    const uint32_t mid = (lo + hi) >> 1;
+                    if (s_off[mid] <= c) lo = mid;
+                    else hi = mid;
+                }
+                const uint32_t fq = t + lo, j = c - s_off[lo];
+                if (a.rec.heads) {
+                    const uint32_t *sl = a.rec.words + s_rec[lo];
+                    const uint32_t slot = sl[j];
+                    const uint32_t x = j ? a.G.slots[sl[j - 1u]].x : a.job.src[fq];
+                    cand_put(a, at + c, x, a.G.slots[slot].x, a.G.wts[slot], mask, true);
+                } else {
                     const uint32_t *v = a.pv + (size_t)fq * a.stride, *sl = a.ps + (size_t)fq * a.stride;
-                    for (uint32_t j = lane; j < n; j += 32u)
-                        cand_put(a, base + j, v[j], v[j + 1], a.G.wts[sl[j + 1]], mask, true);
-                }
-                if (n) {
-                    __syncwarp();   // every lane has read the edge's key and list head
-                    if (lane == 0u) {
-                        if (a.rec.heads) a.rec.heads[fq] = 0u;
-                        if (a.clear_keys) a.keys[fq] = 0ull;
-                    }
-                    continue;
-                }
-                const unsigned long long uid = a.job.uid[fq];
-                for (uint32_t j = lane; j < 2u * a.hw; j += 32u) {
-                    const Fallback r = fallback_walk(a.G, j < a.hw ? a.job.src[fq] : a.job.dst[fq], uid,
-                                                     j, a.key);
-                    cand_put(a, base + 2u * j, r.x1 == ~0u ? ~0u : r.s0, r.x1, r.w1, mask, true);
-                    cand_put(a, base + 2u * j + 1u, r.x2 == ~0u ? ~0u : r.x1, r.x2, r.w2, mask, true);
+                    cand_put(a, at + c, v[j], v[j + 1], a.G.wts[sl[j + 1]], mask, true);
                 }
             }
-            __syncthreads();
+            const uint32_t per = 2u * a.hw;   // fallback walks of an edge without a path
+            for (uint32_t c = threadIdx.x; c < tz * per; c += blockDim.x) {
+                const uint32_t k = c / per, j = c - k * per, fq = t + s_none[k];
+                const uint32_t base = n_path + ((nth + k) * per + j) * 2u;
+                const Fallback r = fallback_walk(a.G, j < a.hw ? a.job.src[fq] : a.job.dst[fq], a.job.uid[fq],
+                                                 j, a.key);
+                cand_put(a, base, r.x1 == ~0u ? ~0u : r.s0, r.x1, r.w1, mask, true);
+                cand_put(a, base + 1u, r.x2 == ~0u ? ~0u : r.x1, r.x2, r.w2, mask, true);
+            }
+            at += tl;
+            nth += tz;
+            __syncthreads();   // the tile's shared arrays are written again by the next
         }
     } else {
         n_path = a.counts[C_CANDS];
