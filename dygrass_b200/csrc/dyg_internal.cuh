@@ -195,7 +195,6 @@ struct Workspace {
     Buf cand_x, cand_y, cand_w;               // recovery candidates
     Buf keep;                                 // u32 per candidate
     Buf htab_k, htab_v;                       // dedup hash table
-    Buf cub_tmp;
     Buf scan_status;                          // u64 per tile of the single-pass scan
     unsigned long long scan_tickets = 0;      // tile tickets handed out so far (S_SCAN)
     uint32_t scan_epoch = 0;                  // tags this workspace's scan statuses per call
@@ -206,7 +205,8 @@ struct Workspace {
     Buf rowcnt, rowhead;                      // row operations: per-row entries / last entry + 1
     Buf rowlist;                              // row operations: rows for warps and blocks
     Buf blk;                                  // row operations: per-block words
-    Buf st_key, st_val;                       // stream file: (min, max) keys and indices, sorted
+    Buf st_key, st_cnt;                       // stream file: table of (min, max) keys; counts, heads
+    Buf st_val;                               // stream file: chain links and table slots of the edges
     Buf st_pos;                               // stream file: uint4 slot positions in G and H
     Buf st_wapp;                              // stream file: G weight of each new edge
     Buf big;                                  // stream file: uint4 per long-row search
@@ -338,7 +338,7 @@ template <typename T>
 inline T *ptr(const Buf &b) { return static_cast<T *>(b.p); }
 
 int num_sms();
-// Counts launches of this library's own kernels (not cub's).
+// Counts launches of this library's kernels.
 void count_launch();
 
 // --- walk.cu

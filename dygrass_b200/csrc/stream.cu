@@ -4,10 +4,10 @@
 //
 // Insert file (gpu_graph.cuh:373-396, 620-643), all on the device:
 //   probe    every edge's slot positions in G and H (rows scanned by groups
-//            of 8 lanes, the shorter row first);
-//   sort     (min, max) keys with their file indices (stable radix sort), so
-//            the occurrences of one edge sit together in file order;
-//   merge    one thread per edge group: an edge already in G adds every
+//            of 8 lanes, the shorter row first); the occurrences of one edge
+//            chained under its (min, max) key in a hash table;
+//   merge    one thread per edge: its occurrences in file order; an edge
+//            already in G adds every
 //            occurrence's weight to G (and H) in file order; a new edge's
 //            first occurrence enters G with the later occurrences' weights
 //            folded in, and is listed for walking;
@@ -21,8 +21,6 @@
 // later kernel and the file resumes at the halted stage after the arena or
 // record buffers grew (nothing changed after the halt; the weight merges
 // come before any reservation and are not repeated).
-#include <cub/cub.cuh>
-
 #include "dyg_internal.cuh"
 #include "gridsync.cuh"
 #include "rowops.cuh"
@@ -95,16 +93,45 @@ __device__ __forceinline__ uint2 group_edge_short(const DevGraph &g, uint32_t a,
     return a_short ? make_uint2(ps, ~0u) : make_uint2(~0u, ps);
 }
 
-// One group of kProbeLanes lanes per edge: slot positions in G and H, the
-// sort key (min << nb | max) and index; self-loops and invalid endpoints get
-// key ~0 (sorted last, never merged or walked).  An edge with a row longer
+// The file's edges by (min, max) key: an open-addressing table of T >= 2n slots
+// (empty between files: key ~0, no occurrences) with a chain of occurrences
+// per key.
+struct EdgeTable {
+    unsigned long long *key;
+    uint32_t *cnt, *head;     // per slot: occurrences, last occurrence + 1
+    uint32_t mask;
+    uint32_t *nxt, *slot;     // per edge: previous occurrence + 1 (0: leader, ~0u: not in the
+                              // table); its slot
+};
+
+__device__ __forceinline__ unsigned long long pair_key(uint32_t a, uint32_t b) {
+    return ((unsigned long long)a << 32) | b;   // a < b
+}
+
+__device__ __forceinline__ void table_link(const EdgeTable &t, uint32_t i, unsigned long long k) {
+    unsigned long long h = k * 0x9E3779B97F4A7C15ull;
+    h ^= h >> 32;
+    uint32_t s = (uint32_t)h & t.mask;
+    while (true) {
+        const unsigned long long prev = atomicCAS(t.key + s, ~0ull, k);
+        if (prev == ~0ull || prev == k) break;
+        s = (s + 1u) & t.mask;
+    }
+    t.slot[i] = s;
+    t.nxt[i] = atomicExch(t.head + s, i + 1u);
+    atomicAdd(t.cnt + s, 1u);
+}
+
+// One group of kProbeLanes lanes per edge: slot positions in G and H, and the
+// edge's entry in the table; self-loops and invalid endpoints stay out of it
+// (never merged or walked).  An edge with a row longer
 // than kBigRow in G or H has its short rows searched here
 // (group_edge_short); if a long row remains to be searched it goes to the big
 // list for k_st_probe_big, with bit 0 (G) and bit 1 (H) of .w naming the
 // graphs whose search is open.
 __global__ void k_st_probe(const unsigned long long *halt, DevGraph G, DevGraph H,
-                           const uint32_t *src, const uint32_t *dst, uint32_t n, uint32_t nb,
-                           unsigned long long *key, uint32_t *val, uint4 *pos, uint32_t *nflag,
+                           const uint32_t *src, const uint32_t *dst, uint32_t n, EdgeTable tab,
+                           uint4 *pos, uint32_t *nflag,
                            int32_t *status, float *cond, uint4 *big, unsigned long long *nbig,
                            bool big_ok, unsigned long long *err) {
     if (HALTED(halt)) return;
@@ -123,8 +150,7 @@ __global__ void k_st_probe(const unsigned long long *halt, DevGraph G, DevGraph 
     if (a == b || b >= G.n) {
         if (lane == 0) {
             if (b >= G.n) atomicOr(err, (unsigned long long)kErrVertex);
-            key[i] = ~0ull;
-            val[i] = i;
+            tab.nxt[i] = ~0u;
             pos[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
             nflag[i] = 0;
             status[i] = DYG_INS_SELF_LOOP;
@@ -133,8 +159,7 @@ __global__ void k_st_probe(const unsigned long long *halt, DevGraph G, DevGraph 
         return;
     }
     if (lane == 0) {
-        key[i] = ((unsigned long long)a << nb) | b;
-        val[i] = i;
+        table_link(tab, i, pair_key(a, b));
         nflag[i] = 0;
     }
     if (big_ok && (long_rows(G, a, b) || long_rows(H, a, b))) {
@@ -201,61 +226,133 @@ __device__ __forceinline__ void set_weight(DevGraph &g, uint32_t slot, float w) 
     g.slots[slot].y = __float_as_uint(__frcp_rn(w));
 }
 
-// One thread per group of equal keys (dynamic_update/gpu_graph.cuh:373-396,
-// 452-465): weights are folded in file order, one float add per occurrence.
-__global__ void k_st_merge(const unsigned long long *halt, DevGraph G, DevGraph H,
-                           const unsigned long long *skey, const uint32_t *sval, uint32_t n,
-                           const uint4 *pos, const float *w, uint32_t *nflag, float *wapp,
-                           int32_t *status, float *cond) {
-    if (HALTED(halt)) return;
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const unsigned long long k = skey[j];
-    if (k == ~0ull || (j > 0 && skey[j - 1] == k)) return;
-    uint32_t e = j + 1;
-    while (e < n && skey[e] == k) ++e;
-    const uint32_t i0 = sval[j];
-    const uint4 p = pos[i0];
-    const bool inH = p.z != ~0u;
-    float ha = inH ? H.wts[p.z] : 0.f, hb = (inH && p.w != ~0u) ? H.wts[p.w] : 0.f;
-    if (p.x != ~0u) {
-        // already in G: every occurrence adds its weight to G and (if there) H
-        float ga = G.wts[p.x], gb = p.y != ~0u ? G.wts[p.y] : 0.f;
-        for (uint32_t q = j; q < e; ++q) {
-            const uint32_t i = sval[q];
-            const float wi = w[i];
-            ga = __fadd_rn(ga, wi);
-            gb = __fadd_rn(gb, wi);
-            if (inH) {
-                ha = __fadd_rn(ha, wi);
-                hb = __fadd_rn(hb, wi);
-            }
-            status[i] = DYG_INS_MERGED;
-            cond[i] = 0.f;
+// One edge's occurrences folded in file order, one float add each
+// (dynamic_update/gpu_graph.cuh:373-396, 452-465).
+struct Fold {
+    uint4 p;       // the first occurrence's slots
+    uint32_t i0;
+    bool first;
+    float ga, gb, ha, hb, wa;
+};
+struct MergeArgs {
+    DevGraph G, H;
+    const uint32_t *src, *dst;
+    const float *w;
+    uint32_t n;
+    EdgeTable tab;
+    const uint4 *pos;
+    uint32_t *nflag;
+    float *wapp;
+    int32_t *status;
+    float *cond;
+};
+
+__device__ __forceinline__ void fold_add(const MergeArgs &a, Fold &f, uint32_t i) {
+    const float wi = a.w[i];
+    if (f.first) {
+        f.first = false;
+        f.i0 = i;
+        f.p = a.pos[i];
+        f.ga = f.p.x != ~0u ? a.G.wts[f.p.x] : 0.f;
+        f.gb = f.p.y != ~0u ? a.G.wts[f.p.y] : 0.f;
+        f.ha = f.p.z != ~0u ? a.H.wts[f.p.z] : 0.f;
+        f.hb = (f.p.z != ~0u && f.p.w != ~0u) ? a.H.wts[f.p.w] : 0.f;
+        if (f.p.x == ~0u) {
+            // new: the first occurrence enters G and is walked; the later ones
+            // add their weights to its G copy (and to H's, if H has the edge)
+            f.wa = wi;
+            return;
         }
-        set_weight(G, p.x, ga);
-        if (p.y != ~0u) set_weight(G, p.y, gb);
-    } else {
-        // new: the first occurrence enters G and is walked; the later ones
-        // add their weights to its G copy (and to H's, if H has the edge)
-        float wa = w[i0];
-        for (uint32_t q = j + 1; q < e; ++q) {
-            const uint32_t i = sval[q];
-            const float wi = w[i];
-            wa = __fadd_rn(wa, wi);
-            if (inH) {
-                ha = __fadd_rn(ha, wi);
-                hb = __fadd_rn(hb, wi);
-            }
-            status[i] = DYG_INS_MERGED;
-            cond[i] = 0.f;
-        }
-        nflag[i0] = 1u;
-        wapp[i0] = wa;
     }
-    if (inH) {
-        set_weight(H, p.z, ha);
-        if (p.w != ~0u) set_weight(H, p.w, hb);
+    // already in G: every occurrence adds its weight to G and (if there) H
+    f.wa = __fadd_rn(f.wa, wi);
+    f.ga = __fadd_rn(f.ga, wi);
+    f.gb = __fadd_rn(f.gb, wi);
+    f.ha = __fadd_rn(f.ha, wi);
+    f.hb = __fadd_rn(f.hb, wi);
+    a.status[i] = DYG_INS_MERGED;
+    a.cond[i] = 0.f;
+}
+
+__device__ __forceinline__ void fold_end(MergeArgs &a, const Fold &f) {
+    if (f.p.x != ~0u) {
+        set_weight(a.G, f.p.x, f.ga);
+        if (f.p.y != ~0u) set_weight(a.G, f.p.y, f.gb);
+    } else {
+        a.nflag[f.i0] = 1u;
+        a.wapp[f.i0] = f.wa;
+    }
+    if (f.p.z != ~0u) {
+        set_weight(a.H, f.p.z, f.ha);
+        if (f.p.w != ~0u) set_weight(a.H, f.p.w, f.hb);
+    }
+}
+
+// One thread per edge: the leader of each key's chain empties its table slot
+// and folds its occurrences.  A chain of up to kFoldChain is followed and put
+// in file order; for a longer one the block scans the file, which meets them
+// in order, and one thread folds what each tile brings.
+constexpr uint32_t kFoldChain = 32;
+constexpr uint32_t kFoldThreads = 256;
+__global__ void __launch_bounds__(kFoldThreads) k_st_merge(const unsigned long long *halt, MergeArgs a) {
+    __shared__ unsigned long long s_key[kFoldThreads];
+    __shared__ uint32_t s_n, s_found[kFoldThreads], s_warp[kFoldThreads / 32 + 1];
+    if (HALTED(halt)) return;
+    if (threadIdx.x == 0) s_n = 0u;
+    __syncthreads();
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < a.n && a.tab.nxt[i] == 0u) {
+        const uint32_t s = a.tab.slot[i], c = a.tab.cnt[s];
+        uint32_t k = a.tab.head[s];
+        const unsigned long long key = a.tab.key[s];
+        a.tab.key[s] = ~0ull;
+        a.tab.cnt[s] = 0u;
+        a.tab.head[s] = 0u;
+        Fold f{};
+        f.first = true;
+        if (c == 1u) {
+            fold_add(a, f, i);
+            fold_end(a, f);
+        } else if (c <= kFoldChain) {
+            uint32_t idx[kFoldChain];
+            for (uint32_t u = 0; u < c; ++u) {   // insertion by file index
+                const uint32_t v = k - 1u;
+                k = a.tab.nxt[v];
+                uint32_t b = u;
+                while (b > 0u && idx[b - 1u] > v) {
+                    idx[b] = idx[b - 1u];
+                    --b;
+                }
+                idx[b] = v;
+            }
+            for (uint32_t u = 0; u < c; ++u) fold_add(a, f, idx[u]);
+            fold_end(a, f);
+        } else {
+            s_key[atomicAdd(&s_n, 1u)] = key;
+        }
+    }
+    __syncthreads();
+    const uint32_t nl = s_n;
+    for (uint32_t q = 0; q < nl; ++q) {
+        const unsigned long long key = s_key[q];
+        Fold f{};
+        f.first = true;
+        for (uint32_t t0 = 0; t0 < a.n; t0 += blockDim.x) {
+            const uint32_t e = t0 + threadIdx.x;
+            bool on = e < a.n && a.tab.nxt[e] != ~0u;
+            if (on) {
+                const uint32_t u = a.src[e], v = a.dst[e];
+                on = pair_key(min(u, v), max(u, v)) == key;
+            }
+            uint32_t total;
+            const uint32_t at = block_excl(on ? 1u : 0u, s_warp, &total);
+            if (on) s_found[at] = e;
+            __syncthreads();
+            if (threadIdx.x == 0)
+                for (uint32_t u = 0; u < total; ++u) fold_add(a, f, s_found[u]);
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) fold_end(a, f);
     }
 }
 
@@ -271,8 +368,13 @@ struct NewEdgeOp {
     float *f_w;
     unsigned long long *f_uid;
     uint32_t *f_idx, *counts;
+    unsigned long long *hkeys;   // zeroed for the first chunk's walks
+    uint32_t nkeys;
     __device__ uint32_t count() const { return n; }
-    __device__ uint32_t take(uint32_t i) const { return nflag[i]; }
+    __device__ uint32_t take(uint32_t i) const {
+        if (i < nkeys) hkeys[i] = 0ull;
+        return nflag[i];
+    }
     __device__ bool listed(uint32_t i) const { return nflag[i] != 0u; }
     __device__ void list(uint32_t i, uint32_t q) const {
         f_src[q] = src[i];
@@ -305,139 +407,31 @@ struct StAcceptOp {
     }
 };
 
-// Files of up to kSortSmall edges are grouped by one block: a bitonic sort of
-// words (key << 13 | file index), so equal keys stay in file order -- the
-// order the radix sort of larger files gives -- and self-loop keys (~0),
-// mapped to the largest 2nb-bit key, come last; in one launch instead of six.
-// Each thread holds kSortE consecutive words: partners closer than kSortE
-// are compared in registers, closer than 32 kSortE through warp shuffles,
-// and only the farther ones through shared memory.
-constexpr uint32_t kSortSmall = 8192;   // file indices fit 13 bits
-constexpr uint32_t kSortE = 8;
-
-__device__ __forceinline__ unsigned long long sort_keep(unsigned long long mine,
-                                                        unsigned long long other, uint32_t i,
-                                                        uint32_t j, uint32_t k) {
-    // element i keeps the smaller word when it is the lower one of an
-    // ascending pair or the upper one of a descending pair
-    return (((i & j) == 0u) == ((i & k) == 0u)) ? min(mine, other) : max(mine, other);
-}
-
-template <uint32_t J>
-__device__ __forceinline__ void sort_in_thread(unsigned long long (&v)[kSortE], uint32_t t,
-                                               uint32_t k) {
-#pragma unroll
-    for (uint32_t e = 0; e < kSortE; ++e) {
-        constexpr uint32_t kJ = J;
-        const uint32_t p = e ^ kJ;
-        if (p > e) {
-            const bool asc = ((t * kSortE + e) & k) == 0u;
-            const unsigned long long a = v[e], b = v[p];
-            if ((a > b) == asc) {
-                v[e] = b;
-                v[p] = a;
-            }
-        }
-    }
-}
-
-__global__ void __launch_bounds__(kSortSmall / kSortE)
-k_sort_small(const unsigned long long *key, uint32_t n, uint32_t N, uint32_t kbits,
-             unsigned long long *skey, uint32_t *sval) {
-    extern __shared__ unsigned long long s_w[];   // N words
-    const uint32_t t = threadIdx.x;
-    const unsigned long long kmax = (1ull << kbits) - 1ull;   // above every real key
-    for (uint32_t i = t; i < N; i += blockDim.x) {
-        unsigned long long w = ~0ull;   // padding sorts after every entry
-        if (i < n) {
-            const unsigned long long k = key[i];
-            w = ((k == ~0ull ? kmax : k) << 13) | i;
-        }
-        s_w[i] = w;
-    }
-    __syncthreads();
-    unsigned long long v[kSortE];
-#pragma unroll
-    for (uint32_t e = 0; e < kSortE; ++e) v[e] = s_w[t * kSortE + e];
-    for (uint32_t k = 2; k <= N; k <<= 1) {
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            if (j >= 32u * kSortE) {
-                __syncthreads();   // the last readers of s_w are done
-#pragma unroll
-                for (uint32_t e = 0; e < kSortE; ++e) s_w[t * kSortE + e] = v[e];
-                __syncthreads();
-#pragma unroll
-                for (uint32_t e = 0; e < kSortE; ++e) {
-                    const uint32_t i = t * kSortE + e;
-                    v[e] = sort_keep(v[e], s_w[i ^ j], i, j, k);
-                }
-            } else if (j >= kSortE) {
-                const uint32_t d = j / kSortE;   // partner lane offset
-#pragma unroll
-                for (uint32_t e = 0; e < kSortE; ++e) {
-                    const unsigned long long o = __shfl_xor_sync(0xFFFFFFFFu, v[e], d);
-                    v[e] = sort_keep(v[e], o, t * kSortE + e, j, k);
-                }
-            } else if (j == 4u) {
-                sort_in_thread<4>(v, t, k);
-            } else if (j == 2u) {
-                sort_in_thread<2>(v, t, k);
-            } else {
-                sort_in_thread<1>(v, t, k);
-            }
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (uint32_t e = 0; e < kSortE; ++e) s_w[t * kSortE + e] = v[e];
-    __syncthreads();
-    for (uint32_t i = t; i < n; i += blockDim.x) {
-        const unsigned long long w = s_w[i];
-        const unsigned long long k = w >> 13;
-        skey[i] = k == kmax ? ~0ull : k;
-        sval[i] = (uint32_t)(w & 0x1FFFu);
-    }
-}
-
-// The one-block sort applies to files of up to kSortSmall edges whose keys
-// (2 nb bits) and file indices (13 bits) fit one word below the padding.
-bool sort_small_fits(uint32_t n, uint32_t nb) { return n <= kSortSmall && 2u * nb + 13u <= 63u; }
-
-dyg_status sort_small_enqueue(const unsigned long long *key, uint32_t n, uint32_t nb,
-                              unsigned long long *skey, uint32_t *sval, cudaStream_t st) {
-    uint32_t N = 32u * kSortE;
-    while (N < n) N <<= 1;
-    const size_t bytes = (size_t)N * sizeof(unsigned long long);
-    if (bytes > 48u * 1024u)   // the attribute belongs to the current device
-        DYG_CUDA(cudaFuncSetAttribute(k_sort_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)bytes));
-    k_sort_small<<<1, N / kSortE, bytes, st>>>(key, n, N, 2u * nb, skey, sval);
-    count_launch();
-    DYG_CUDA(cudaGetLastError());
-    return DYG_OK;
-}
-
-uint32_t key_bits(uint32_t nv) {
-    uint32_t b = 1;
-    while (b < 32 && (nv - 1u) >> b) ++b;
-    return b;
-}
-
-// Probe, sort, merge and compact an insert file (no reservation: never halts).
+// Probe and merge an insert file (no reservation: never halts).
 dyg_status insert_prep_enqueue(dyg_graph *G, dyg_graph *H, const uint32_t *src,
                                const uint32_t *dst, const float *w, uint32_t n,
                                unsigned long long *halt, int32_t *status, float *cond,
                                cudaStream_t st) {
     Workspace &ws = G->ws;
-    const uint32_t nb = key_bits(G->g.n);
-    unsigned long long *key = ptr<unsigned long long>(ws.st_key), *skey = key + n;
-    uint32_t *val = ptr<uint32_t>(ws.st_val), *sval = val + n;
+    uint64_t T = 1024;
+    while (T < 2ull * n) T <<= 1;
+    if (ws.st_key.bytes < sizeof(unsigned long long) * T || ws.st_cnt.bytes < 2 * sizeof(uint32_t) * T) {
+        // empty when allocated, and left empty by every file
+        DYG_TRY(ensure(ws.st_key, sizeof(unsigned long long) * T));
+        DYG_TRY(ensure(ws.st_cnt, 2 * sizeof(uint32_t) * T));
+        DYG_CUDA(cudaMemsetAsync(ws.st_key.p, 0xFF, ws.st_key.bytes, st));
+        DYG_CUDA(cudaMemsetAsync(ws.st_cnt.p, 0, ws.st_cnt.bytes, st));
+    }
+    // counts and heads interleaved by halves of one allocation
+    uint32_t *cnt = ptr<uint32_t>(ws.st_cnt), *head = cnt + ws.st_cnt.bytes / (2 * sizeof(uint32_t));
+    uint32_t *nxt = ptr<uint32_t>(ws.st_val), *slot = nxt + n;
+    const EdgeTable tab{ptr<unsigned long long>(ws.st_key), cnt, head, (uint32_t)(T - 1), nxt, slot};
     uint32_t *nflag = ptr<uint32_t>(ws.flags);
     unsigned long long *sc = ptr<unsigned long long>(ws.scalars);
     const bool big_ok = G->long_rows || H->long_rows;
     if (big_ok) DYG_CUDA(cudaMemsetAsync(sc + S_NBIG, 0, sizeof(unsigned long long), st));
     k_st_probe<<<blocks((uint64_t)n * kProbeLanes, 256), 256, 0, st>>>(
-        halt, G->g, H->g, src, dst, n, nb, key, val, ptr<uint4>(ws.st_pos), nflag, status, cond,
+        halt, G->g, H->g, src, dst, n, tab, ptr<uint4>(ws.st_pos), nflag, status, cond,
         ptr<uint4>(ws.big), sc + S_NBIG, big_ok, sc + S_ERR);
     count_launch();
     if (big_ok) {
@@ -445,42 +439,28 @@ dyg_status insert_prep_enqueue(dyg_graph *G, dyg_graph *H, const uint32_t *src,
                                                               sc + S_NBIG, ptr<uint4>(ws.st_pos));
         count_launch();
     }
-    if (sort_small_fits(n, nb)) {
-        DYG_TRY(sort_small_enqueue(key, n, nb, skey, sval, st));   // values are file indices
-    } else {
-        size_t tmp = 0;
-        DYG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp, key, skey, val, sval, (int)n, 0,
-                                                 (int)(2 * nb), st));
-        DYG_TRY(ensure(ws.cub_tmp, tmp));
-        tmp = ws.cub_tmp.bytes;
-        // keys ~0 (self-loops) have all bits set: sorting on the low 2*nb
-        // bits still places them after every real key (each real key is
-        // < 2^(2nb) - 1)
-        DYG_CUDA(cub::DeviceRadixSort::SortPairs(ws.cub_tmp.p, tmp, key, skey, val, sval, (int)n, 0,
-                                                 (int)(2 * nb), st));
-    }
-    k_st_merge<<<blocks(n, 256), 256, 0, st>>>(halt, G->g, H->g, skey, sval, n,
-                                                ptr<uint4>(ws.st_pos), w, nflag,
-                                                ptr<float>(ws.st_wapp), status, cond);
+    const MergeArgs a{G->g, H->g, src, dst, w, n, tab, ptr<uint4>(ws.st_pos), nflag,
+                      ptr<float>(ws.st_wapp), status, cond};
+    k_st_merge<<<blocks(n, kFoldThreads), kFoldThreads, 0, st>>>(halt, a);
     count_launch();
     DYG_CUDA(cudaGetLastError());
     return DYG_OK;
 }
 
-dyg_status insert_gappend_enqueue(dyg_graph *G, const uint32_t *src, const uint32_t *dst,
-                                  const float *w, uint32_t n, uint64_t uid0,
-                                  unsigned long long *halt, cudaStream_t st) {
+dyg_status insert_gappend_enqueue(dyg_graph *G, dyg_graph *H, const uint32_t *src,
+                                  const uint32_t *dst, const float *w, uint32_t n, uint64_t uid0,
+                                  uint32_t nkeys, unsigned long long *halt, cudaStream_t st) {
     Workspace &ws = G->ws;
     const NewEdgeOp op{ptr<uint32_t>(ws.flags), src, dst, w, n, (unsigned long long)uid0,
                        ptr<uint32_t>(ws.f_src), ptr<uint32_t>(ws.f_dst), ptr<float>(ws.f_w),
                        ptr<unsigned long long>(ws.f_uid), ptr<uint32_t>(ws.f_idx),
-                       ptr<uint32_t>(ws.counts)};
+                       ptr<uint32_t>(ws.counts), ptr<unsigned long long>(H->ws.keys), nkeys};
     return append_enqueue(op, n, G, EdgeList{src, dst, ptr<float>(ws.st_wapp)}, nullptr, EdgeList{},
-                          nullptr, halt, halt_code(0, (uint32_t)kHaltArena, 1), st);
+                          ptr<unsigned long long>(H->ws.scalars) + S_WORK, halt, halt_code(0, (uint32_t)kHaltArena, 1), st);
 }
 
 // Walks chunk c (walk-list entries [c*chunk, c*chunk + nc)) on H and appends
-// its accepted edges to H.  walk_ready: the chunk before left H's keys and
+// its accepted edges to H.  walk_ready: the launch before left H's keys and
 // chunk counter zero.
 dyg_status insert_chunk_enqueue(dyg_graph *G, dyg_graph *H, uint32_t c, uint32_t chunk,
                                 uint32_t nc, const dyg_walk_params &p, unsigned long long *halt,
@@ -525,7 +505,6 @@ dyg_status insert_file_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, cons
     const uint32_t nc_max = n < chunk ? n : chunk;
     // every buffer at its final size before anything is enqueued: a resumed
     // stage finds the earlier stages' lists where they were left
-    DYG_TRY(ensure(wg.st_key, sizeof(unsigned long long) * (size_t)n * 2));
     DYG_TRY(ensure(wg.st_val, sizeof(uint32_t) * (size_t)n * 2));
     DYG_TRY(ensure(wg.st_pos, sizeof(uint4) * (size_t)n));
     DYG_TRY(ensure(wg.st_wapp, sizeof(float) * (size_t)n));
@@ -546,12 +525,12 @@ dyg_status insert_file_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, cons
     const uint32_t nchunks = (uint32_t)(((uint64_t)n + chunk - 1) / chunk);
     uint32_t start = 0;   // 0 = G append, c + 1 = chunk c
     for (int round = 0; round < 64; ++round) {
-        if (start == 0) DYG_TRY(insert_gappend_enqueue(G, src, dst, w, n, uid0, halt, st));
+        if (start == 0) DYG_TRY(insert_gappend_enqueue(G, H, src, dst, w, n, uid0, nc_max, halt, st));
         const uint32_t c0 = start ? start - 1 : 0;
         for (uint32_t c = c0; c < nchunks; ++c) {
             const uint32_t f0 = c * chunk;
             const uint32_t nc = n - f0 < chunk ? n - f0 : chunk;
-            DYG_TRY(insert_chunk_enqueue(G, H, c, chunk, nc, p, halt, status, cond, c > c0, st));
+            DYG_TRY(insert_chunk_enqueue(G, H, c, chunk, nc, p, halt, status, cond, start == 0 || c > c0, st));
         }
         if (fetch) DYG_TRY((*fetch)());
         DYG_TRY(read_scalars2(G, H, st));

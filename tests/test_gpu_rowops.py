@@ -231,3 +231,33 @@ def test_winner_paths_recorded_and_replayed(dyg, oracle, transition, steps):  # 
     assert np.array_equal(r.rec_src, rx) and np.array_equal(r.rec_dst, ry) and np.array_equal(r.rec_kind, rk)
     same_graph(G, Go)
     same_graph(H, Ho)
+
+
+# occurrences of one edge in a stream file: a single one, chains a lane folds
+# (up to 32) and ones the block scans the file for, for edges that are new, in
+# G only, and in both graphs
+@pytest.mark.parametrize("times", [1, 2, 31, 32, 33, 700])
+@pytest.mark.parametrize("more", [0, 300, 9000])
+def test_stream_repeats(dyg, oracle, times, more):  # noqa: F811
+    rng = np.random.default_rng(times + more)
+    n = 500
+    gs, gd, gw = star(n, 60, rng)
+    in_h = rng.random(len(gs)) < 0.6
+    hs, hd, hw = gs[in_h], gd[in_h], gw[in_h]
+    only_g = np.flatnonzero(~in_h)[0]
+    pick = [(gs[only_g], gd[only_g]), (hs[0], hd[0]), (5, 490), (7, 300)]
+    e = np.array(pick * times + [tuple(rng.integers(0, n, 2)) for _ in range(more)], np.uint32)
+    flip = rng.random(len(e)) < 0.5
+    e[flip] = e[flip][:, ::-1]
+    e = e[rng.permutation(len(e))]
+    w = rng.uniform(0.1, 1.0, len(e)).astype(np.float32)
+    G, H = dyg.Graph.from_edges(n, gs, gd, gw), dyg.Graph.from_edges(n, hs, hd, hw)
+    Go, Ho = oracle.OGraph(n, gs, gd, gw), oracle.OGraph(n, hs, hd, hw)
+    p = dyg.WalkParams.make(threshold=5.0, walkers=32, max_steps=20)
+    for k in range(2):   # the second file finds the table as the first left it
+        r = dyg.stream_file(G, H, 0, e[:, 0].copy(), e[:, 1].copy(), w, p, first_update_id=k * len(e))
+        st, cd, *_ = oracle.stream_file(Go, Ho, 0, e[:, 0].copy(), e[:, 1].copy(), w, p, first_uid=k * len(e))
+        assert np.array_equal(r.status, st)
+        assert np.array_equal(r.conductance.view(np.uint32), cd.view(np.uint32))
+        same_graph(G, Go)
+        same_graph(H, Ho)
