@@ -147,23 +147,26 @@ __device__ __forceinline__ int finish_move(Walker &s, uint2 sl, uint32_t at, boo
 // (8,000 insertions and 12,000 deletions on a 40^3 mesh: 8.99 -> 7.68 ms with
 // this and wq in integers, against groups of four read twice and wq in FP64.)
 constexpr uint32_t kPickGroup = 8;
+constexpr uint32_t kPickShort = 4;   // rows of a sparsifier: half the work of a group
 
+template <uint32_t U>
 struct PickGroup {
-    uint2 c[kPickGroup];
-    unsigned long long p[kPickGroup];   // inclusive prefixes over the group
+    uint2 c[U];
+    unsigned long long p[U];   // inclusive prefixes over the group
 };
-__device__ __forceinline__ void pick_load(PickGroup &g, const uint2 *__restrict__ slots,
+template <uint32_t U>
+__device__ __forceinline__ void pick_load(PickGroup<U> &g, const uint2 *__restrict__ slots,
                                           const float *__restrict__ wts, uint32_t lo,
                                           uint32_t left, uint32_t ex, bool has_ex) {
-    float w[kPickGroup];
+    float w[U];
 #pragma unroll
-    for (uint32_t u = 0; u < kPickGroup; ++u) {
+    for (uint32_t u = 0; u < U; ++u) {
         g.c[u] = u < left ? __ldg(slots + lo + u) : make_uint2(0u, 0u);
         w[u] = u < left ? __ldg(wts + lo + u) : 0.f;
     }
     unsigned long long sum = 0ull;
 #pragma unroll
-    for (uint32_t u = 0; u < kPickGroup; ++u) {
+    for (uint32_t u = 0; u < U; ++u) {
         if (has_ex && g.c[u].x == ex) w[u] = 0.f;   // counts as absent
         sum += wq(w[u]);
         g.p[u] = sum;
@@ -172,11 +175,12 @@ __device__ __forceinline__ void pick_load(PickGroup &g, const uint2 *__restrict_
 // The group's first slot whose prefix (after `before`) exceeds target, ~0u if
 // none.  A slot that is absent or weighs nothing has its predecessor's prefix,
 // so it is never the first, whether or not the sums wrapped past 2^64.
-__device__ __forceinline__ uint32_t pick_in_group(const PickGroup &g, unsigned long long target,
+template <uint32_t U>
+__device__ __forceinline__ uint32_t pick_in_group(const PickGroup<U> &g, unsigned long long target,
                                                   unsigned long long before, uint2 *picked) {
     uint32_t at = ~0u;
 #pragma unroll
-    for (int u = (int)kPickGroup - 1; u >= 0; --u)
+    for (int u = (int)U - 1; u >= 0; --u)
         if (before + g.p[u] > target) {
             at = (uint32_t)u;
             *picked = g.c[u];
@@ -184,18 +188,27 @@ __device__ __forceinline__ uint32_t pick_in_group(const PickGroup &g, unsigned l
     return at;
 }
 
+// A row of up to U slots.
+template <uint32_t U>
+__device__ __forceinline__ uint32_t lane_pick_short(const uint2 *__restrict__ slots,
+                                                    const float *__restrict__ wts, uint32_t lo,
+                                                    uint32_t deg, uint32_t ex, bool has_ex,
+                                                    uint32_t r, uint2 *picked) {
+    PickGroup<U> g;
+    pick_load(g, slots, wts, lo, deg, ex, has_ex);
+    const unsigned long long total = g.p[U - 1u];
+    if (total == 0ull) return ~0u;
+    return lo + pick_in_group(g, mul_hi32(r, total), 0ull, picked);
+}
+
 __device__ __forceinline__ uint32_t lane_pick_weighted(const uint2 *__restrict__ slots,
                                                        const float *__restrict__ wts, uint32_t lo,
                                                        uint32_t deg, uint32_t ex, bool has_ex,
                                                        uint32_t r, uint2 *picked) {
-    PickGroup g;
-    pick_load(g, slots, wts, lo, deg, ex, has_ex);
-    unsigned long long total = g.p[kPickGroup - 1u];
-    if (deg <= kPickGroup) {
-        if (total == 0ull) return ~0u;
-        return lo + pick_in_group(g, mul_hi32(r, total), 0ull, picked);
-    }
-    for (uint32_t j0 = kPickGroup; j0 < deg; j0 += kPickGroup) {
+    if (deg <= kPickGroup) return lane_pick_short<kPickGroup>(slots, wts, lo, deg, ex, has_ex, r, picked);
+    PickGroup<kPickGroup> g;
+    unsigned long long total = 0ull;
+    for (uint32_t j0 = 0; j0 < deg; j0 += kPickGroup) {
         pick_load(g, slots, wts, lo + j0, deg - j0, ex, has_ex);
         total += g.p[kPickGroup - 1u];
     }
@@ -631,7 +644,14 @@ __device__ __forceinline__ int step_weighted_warp(Walker &s, bool active, const 
     if (pick && d.y > kIdxRow && ix.rbase) base = __ldg(ix.rbase + s.cur);
     if (base) at = index_pick(g.slots, g.wts, ix.words + base, d.x, d.y, s.prev, !first, r);
     const bool own_row = pick && !base && d.y <= kCoopRow;   // chosen by this lane, slot in hand
-    if (own_row) at = lane_pick_weighted(g.slots, g.wts, d.x, d.y, s.prev, !first, r, &sl);
+    // insertion walks are on a sparsifier, whose rows are short (their walks on
+    // a weighted 40^3 mesh 1.52 -> 1.36 ms); one width for the whole warp: two
+    // in turn would cost more than the wider
+    if (!INCR || __any_sync(kFull, own_row && d.y > kPickShort)) {
+        if (own_row) at = lane_pick_weighted(g.slots, g.wts, d.x, d.y, s.prev, !first, r, &sl);
+    } else if (own_row) {
+        at = lane_pick_short<kPickShort>(g.slots, g.wts, d.x, d.y, s.prev, !first, r, &sl);
+    }
     unsigned coop = __ballot_sync(kFull, pick && !own_row && !base);
     while (coop) {
         const uint32_t L = __ffs(coop) - 1u;
