@@ -803,8 +803,8 @@ __device__ __forceinline__ void write_record(const PathRec &rec, uint32_t e, uns
 // what surrounds them; every iteration starts walkers in the free lanes and
 // then moves each walker four times, so that a walker enters every iteration
 // at a step 1 mod 4 and draws one Philox block for it, and the step counter
-// advances once per iteration.  The edge's best is read once per iteration,
-// after the moves, by the walkers still alive: R only grows along a walk and
+// advances once per iteration.  The edge's best is read once per iteration
+// and applied after the moves to the walkers still alive: R only grows along a walk and
 // 1/R is monotone, so a walker whose 1/R is below it can neither win nor tie,
 // and stopping it leaves every result unchanged.
 // 40 registers: six blocks (48 warps) per SM; eight blocks spill (insertions
@@ -849,6 +849,11 @@ __global__ void __launch_bounds__(kWalkThreads, REC ? 5 : 6) k_walk_uniform(Walk
         if (!__any_sync(kFull, active)) break;
         if (active) {
             const uint4 blk = philox4x32_10(make_uint4((step - 1u) >> 2, walker, c2, c3), a.key);
+            // insertion walks read the edge's best before the moves, whose
+            // latency hides it; few of their edges ever have one, so its age
+            // matters little (insertion rounds 2-6 % faster; deletion walks
+            // prune on the latest)
+            const uint32_t early = INCR && a.prune ? best_bits(a, my_e) : 0u;
             const uint32_t left = a.max_steps - step;   // the walk ends when its step reaches max_steps
             uint32_t took[4] = {0u, 0u, 0u, 0u};        // slots of this iteration's moves (decremental)
             uint32_t found = 0u;
@@ -904,7 +909,7 @@ __global__ void __launch_bounds__(kWalkThreads, REC ? 5 : 6) k_walk_uniform(Walk
                     make_uint4(took[0], took[1], took[2], took[3]);
             step += 4u;
             if (active && a.prune && (T & (a.prune_every - 1u)) == a.prune_every - 1u) {
-                const uint32_t known = best_bits(a, my_e);
+                const uint32_t known = INCR ? early : best_bits(a, my_e);
                 if (known && below_best(R, __uint_as_float(known))) active = false;
             }
         }
@@ -1089,8 +1094,15 @@ k_winner_paths_weighted(DevGraph g, WalkJob job, RowIndex ix, uint32_t max_steps
 
 // Walkers handed to a warp at a time: 32 by default, so that the 512 walks
 // of an edge nobody connects spread over 16 warps instead of running as 16
-// waves on one.  DYG_WALK_CHUNK (a multiple of 32 dividing the walker count)
-// overrides it for tuning sweeps.
+// waves on one; 64 for uniform insertion batches of 2M walkers and more, and
+// deletion batches of 4M (a part of which is walked), which fill the device
+// many times over, so that half as many chunks are fetched (uniform
+// walks with 32 and 64, ms a call: 200,000 insertions of the 100^3 mesh in ten
+// batches 4.45 and 4.07, in batches of 5,000 0.68 and 0.63 per 25,000; 297,000
+// deletions 2.29 and 1.91; but rounds of 2,400 insertions 0.93 and 1.08, of
+// 100 insertions 0.22 and 0.30).  DYG_WALK_CHUNK (a multiple of 32 dividing
+// the walker count) overrides it for tuning sweeps.
+constexpr uint64_t kBigChunkWalkers = 2u << 20;
 // Launch shape of the walk kernel, process-wide (dyg_tune_set); 0 = default.
 static std::atomic<uint32_t> g_tune_chunk{0}, g_tune_bpsm{0}, g_tune_prune{0};
 
@@ -1103,7 +1115,7 @@ static uint32_t prune_every() {
 // Weighted deletion walks take 16: their walks are long-tailed, and a warp
 // with fewer of them waits less for its slowest (12,000 deletions of a 40^3
 // mesh 2.47 -> 2.16 ms of walks; insertions 1.51 -> 1.59).
-static uint32_t chunk_for(uint32_t walkers, bool weighted, bool incremental) {
+static uint32_t chunk_for(uint32_t n, uint32_t walkers, bool weighted, bool incremental) {
     static int env = -1;
     if (env < 0) {
         const char *v = getenv("DYG_WALK_CHUNK");
@@ -1111,6 +1123,8 @@ static uint32_t chunk_for(uint32_t walkers, bool weighted, bool incremental) {
     }
     const uint32_t want = g_tune_chunk.load() ? g_tune_chunk.load() : (uint32_t)(env > 0 ? env : 0);
     uint32_t c = weighted && !incremental ? 16u : 32u;
+    if (!weighted && walkers % 64u == 0u && (uint64_t)n * walkers >= kBigChunkWalkers * (incremental ? 1u : 2u))
+        c = 64u;
     if (want > 0 && want % 32 == 0 && walkers % want == 0) c = want;
     return c;
 }
@@ -1141,7 +1155,7 @@ static void launch_walk_kernel(const WalkArgs &a, cudaStream_t st) {
 }
 
 uint32_t walk_threads(uint32_t n, const dyg_walk_params &p) {
-    const uint32_t c = chunk_for(p.walkers, p.transition == DYG_TRANSITION_WEIGHTED, false);
+    const uint32_t c = chunk_for(n, p.walkers, p.transition == DYG_TRANSITION_WEIGHTED, false);
     return kWalkThreads * (p.transition == DYG_TRANSITION_WEIGHTED
                                ? walk_blocks<k_walk_weighted<false>>(n, p.walkers, c)
                                : walk_blocks<k_walk_uniform<false, true>>(n, p.walkers, c));
@@ -1204,7 +1218,7 @@ dyg_status launch_walk(dyg_graph *G, const WalkJob &job, const dyg_walk_params &
     a.max_steps = p.max_steps;
     a.prune = (p.flags & DYG_FLAG_EXHAUSTIVE) ? 0u : 1u;
     a.prune_every = prune_every();
-    a.chunk = chunk_for(p.walkers, p.transition == DYG_TRANSITION_WEIGHTED, incremental);
+    a.chunk = chunk_for(job.n_host, p.walkers, p.transition == DYG_TRANSITION_WEIGHTED, incremental);
     a.threshold = p.threshold;
     a.key = make_uint2((uint32_t)p.seed, (uint32_t)(p.seed >> 32));
     a.keys = keys;
@@ -1230,7 +1244,7 @@ dyg_status launch_walk_scalars(const DevGraph &g, const WalkJob &job, const dyg_
     a.max_steps = p.max_steps;
     a.prune = (p.flags & DYG_FLAG_EXHAUSTIVE) ? 0u : 1u;
     a.prune_every = prune_every();
-    a.chunk = chunk_for(p.walkers, p.transition == DYG_TRANSITION_WEIGHTED, incremental);
+    a.chunk = chunk_for(job.n_host, p.walkers, p.transition == DYG_TRANSITION_WEIGHTED, incremental);
     a.threshold = p.threshold;
     a.key = make_uint2((uint32_t)p.seed, (uint32_t)(p.seed >> 32));
     a.keys = keys;
