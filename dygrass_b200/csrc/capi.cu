@@ -423,6 +423,10 @@ dyg_status create_empty_graph(uint32_t n, uint64_t arena_slots, int device, uint
     if (rc == DYG_OK && (cudaMemset(G->g.desc, 0, sizeof(uint2) * (size_t)(n ? n : 1)) != cudaSuccess ||
                          cudaMemset(G->g.cap, 0, sizeof(uint32_t) * (size_t)(n ? n : 1)) != cudaSuccess))
         rc = cuda_fail(cudaGetLastError(), "cudaMemset", __FILE__, __LINE__);
+    // the first call on the graph may come on a stream that the default one
+    // does not wait for
+    if (rc == DYG_OK && cudaDeviceSynchronize() != cudaSuccess)
+        rc = cuda_fail(cudaGetLastError(), "cudaDeviceSynchronize", __FILE__, __LINE__);
     if (rc != DYG_OK) {
         free_graph(G);
         return rc;

@@ -176,14 +176,24 @@ dyg_status launch_phases(uint32_t want, cudaStream_t st, GridBar bar, const A &.
     cfg.stream = st;
     cudaLaunchAttribute at{};
     cfg.attrs = &at;
+    // the largest cluster of this kernel that the device can place
+    static const uint32_t cluster_max = [] {
+        cudaLaunchConfig_t c{};
+        c.gridDim = dim3(kClusterMax);
+        c.blockDim = dim3(kOpThreads);
+        int most = 0;
+        if (cudaFuncSetAttribute(Kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+            cudaOccupancyMaxPotentialClusterSize(&most, Kernel, &c) != cudaSuccess) {
+            cudaGetLastError();
+            most = 0;
+        }
+        return most < (int)kClusterMax ? (uint32_t)(most < 0 ? 0 : most) : kClusterMax;
+    }();
+    uint32_t k = 2u;
+    while (k < want) k <<= 1;
     if (want <= 1u) {
         cfg.gridDim = dim3(1);
-    } else if (want <= kClusterMax) {
-        static const cudaError_t allowed =
-            cudaFuncSetAttribute(Kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        DYG_CUDA(allowed);
-        uint32_t k = 2u;
-        while (k < want) k <<= 1;
+    } else if (k <= cluster_max) {
         cfg.gridDim = dim3(k);
         at.id = cudaLaunchAttributeClusterDimension;
         at.val.clusterDim.x = k;

@@ -597,8 +597,8 @@ dyg_status decr_delete_enqueue(dyg_graph *G, dyg_graph *H, const uint32_t *src,
                                cudaStream_t st) {
     Workspace &ws = G->ws;
     const uint64_t m = 2ull * n;
-    DYG_TRY(rowops_ensure(G, m));
-    DYG_TRY(rowops_ensure(H, m));
+    DYG_TRY(rowops_ensure(G, m, st));
+    DYG_TRY(rowops_ensure(H, m, st));
     DYG_TRY(ensure(ws.dtmp, sizeof(uint32_t) * (size_t)m * 2));
     DYG_TRY(ensure(ws.found, (size_t)m * 2));
     DYG_TRY(ensure(ws.keys, sizeof(unsigned long long) * n));
@@ -713,8 +713,8 @@ dyg_status decr_walk_enqueue(dyg_graph *G, dyg_graph *H, uint32_t f0, uint32_t n
         DYG_CUDA(cudaMemsetAsync(ws.htab_k.p, 0xFF, ws.htab_k.bytes, st));
         DYG_CUDA(cudaMemsetAsync(ws.htab_v.p, 0xFF, ws.htab_v.bytes, st));
     }
-    DYG_TRY(rowops_ensure(G, 1));
-    DYG_TRY(rowops_ensure(H, 2ull * M));
+    DYG_TRY(rowops_ensure(G, 1, st));
+    DYG_TRY(rowops_ensure(H, 2ull * M, st));
     unsigned long long *sc = ptr<unsigned long long>(ws.scalars);
     WalkJob job{halt, ptr<uint32_t>(ws.f_src) + f0, ptr<uint32_t>(ws.f_dst) + f0, nullptr,
                 ptr<unsigned long long>(ws.f_uid) + f0, 0ull, F_dev, n, kDomainDecr, f0};

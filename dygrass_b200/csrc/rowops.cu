@@ -3,7 +3,7 @@
 
 namespace dyg {
 
-dyg_status rowops_ensure(dyg_graph *G, uint64_t m) {
+dyg_status rowops_ensure(dyg_graph *G, uint64_t m, cudaStream_t st) {
     Workspace &ws = G->ws;
     DYG_TRY(ensure(ws.nxt, sizeof(uint32_t) * (size_t)(m ? m : 1)));
     DYG_TRY(ensure(ws.rowlist, sizeof(uint32_t) * (size_t)(m ? m : 1)));
@@ -12,8 +12,8 @@ dyg_status rowops_ensure(dyg_graph *G, uint64_t m) {
         const size_t bytes = sizeof(uint32_t) * (size_t)(G->g.n ? G->g.n : 1);
         DYG_TRY(ensure(ws.rowcnt, bytes));
         DYG_TRY(ensure(ws.rowhead, bytes));
-        DYG_CUDA(cudaMemset(ws.rowcnt.p, 0, ws.rowcnt.bytes));
-        DYG_CUDA(cudaMemset(ws.rowhead.p, 0, ws.rowhead.bytes));
+        DYG_CUDA(cudaMemsetAsync(ws.rowcnt.p, 0, ws.rowcnt.bytes, st));
+        DYG_CUDA(cudaMemsetAsync(ws.rowhead.p, 0, ws.rowhead.bytes, st));
     }
     return DYG_OK;
 }

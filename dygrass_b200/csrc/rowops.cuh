@@ -779,8 +779,8 @@ k_append(const Op op, const __grid_constant__ AppSides A, uint32_t *blk, unsigne
     app_commit(A, 2u * n, bar, halt, code, s, [] {});
 }
 
-// Workspace of a row operation on up to m half-edges.
-dyg_status rowops_ensure(dyg_graph *G, uint64_t m);
+// Workspace of a row operation on up to m half-edges (cleared on st).
+dyg_status rowops_ensure(dyg_graph *G, uint64_t m, cudaStream_t st);
 GridBar grid_bar(dyg_graph *G);
 AppSide append_side(dyg_graph *G, const uint32_t *src, const uint32_t *dst, const float *w);
 
@@ -789,12 +789,12 @@ dyg_status append_enqueue(const Op &op, uint32_t n_host, dyg_graph *GA, const Ed
                           dyg_graph *GB, const EdgeList &EB, unsigned long long *work,
                           unsigned long long *halt, unsigned long long code, cudaStream_t st) {
     if (n_host == 0) return DYG_OK;
-    DYG_TRY(rowops_ensure(GA, 2ull * n_host));
+    DYG_TRY(rowops_ensure(GA, 2ull * n_host, st));
     AppSides A{};
     A.s[0] = append_side(GA, EA.src, EA.dst, EA.w);
     A.n = 1;
     if (GB) {
-        DYG_TRY(rowops_ensure(GB, 2ull * n_host));
+        DYG_TRY(rowops_ensure(GB, 2ull * n_host, st));
         A.s[1] = append_side(GB, EB.src, EB.dst, EB.w);
         A.n = 2;
     }

@@ -261,3 +261,24 @@ def test_stream_repeats(dyg, oracle, times, more):  # noqa: F811
         assert np.array_equal(r.conductance.view(np.uint32), cd.view(np.uint32))
         same_graph(G, Go)
         same_graph(H, Ho)
+
+
+def test_fresh_handles_on_a_stream_of_the_caller(dyg, oracle):  # noqa: F811
+    """The first calls of new handles on a stream that the default stream does
+    not wait for: workspaces are cleared on the stream that uses them."""
+    import torch
+    import dygrass_b200.workloads as wl
+    W = wl.mesh_3d(12, inserts=400)
+    Go, Ho = oracle.OGraph(W.n, W.g_src, W.g_dst, W.g_w), oracle.OGraph(W.n, W.h_src, W.h_dst, W.h_w)
+    oracle.incremental(Ho, W.ins_src, W.ins_dst, W.ins_w, W.params, G=Go)
+    st, cd, rx, ry, rk, _ = oracle.decremental(Go, Ho, W.del_src, W.del_dst, W.dparams)
+    for _ in range(4):
+        s = torch.cuda.Stream()
+        G, H = dyg.Graph.from_edges(W.n, W.g_src, W.g_dst, W.g_w), dyg.Graph.from_edges(W.n, W.h_src, W.h_dst, W.h_w)
+        dyg.incremental_stream(H, W.ins_src, W.ins_dst, W.ins_w, W.params, G=G, stream=s.cuda_stream)
+        r = dyg.decremental_stream(G, H, W.del_src, W.del_dst, W.dparams, stream=s.cuda_stream)
+        assert np.array_equal(r.status, st) and np.array_equal(r.rec_src, rx) and np.array_equal(r.rec_dst, ry)
+        same_graph(G, Go)
+        same_graph(H, Ho)
+        G.close()
+        H.close()
