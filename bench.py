@@ -327,7 +327,7 @@ def dom_is_decr(prof):
 
 
 def dom_name(prof):
-    return "k_walk<0,0>" if dom_is_decr(prof) else "k_walk<1,0>"
+    return "k_walk_uniform<0>" if dom_is_decr(prof) else "k_walk_uniform<1>"
 
 
 def dom_bytes(prof, incr_moves, decr_moves, steps):
@@ -343,8 +343,10 @@ def dom_ms(prof):
     return prof["incr_walk_ms"] / max(prof["incr_walk_launches"], 1)
 
 
-KERNEL_DESC = {"k_walk<0,0>": "k_walk<0,0> (decremental walk on G)",
-               "k_walk<1,0>": "k_walk<1,0> (incremental walk on H)"}
+KERNEL_DESC = {"k_walk_uniform<0>": "k_walk_uniform<0> (decremental walk on G)",
+               "k_walk_uniform<1>": "k_walk_uniform<1> (incremental walk on H)",
+               "k_walk_weighted<0>": "k_walk_weighted<0> (decremental walk on G)",
+               "k_walk_weighted<1>": "k_walk_weighted<1> (incremental walk on H)"}
 
 
 def run_ours(args, rank, world, local_rank):
@@ -864,7 +866,7 @@ def run_many(args, rank, world, local_rank):
         "walk_ms_per_step": prof["incr_walk_ms"] / args.steps,
         "walk_launches": prof["incr_walk_launches"], "prof": prof,
         "launches_per_step": launches / args.steps, "clocks": clk, "e2e": e2e,
-        "dom_kernel": "k_walk<1,0>",
+        "dom_kernel": "k_walk_uniform<1>",
         "dom_bytes_per_launch": dom_bytes(prof, incr_moves, 0.0, args.steps),
         "dom_ms_per_launch": dom_ms(prof),
         "plain_ms_per_step": plain_ms,
@@ -1453,6 +1455,8 @@ def main():
     hbm = peaks.get("hbm_gbs")
     peak_note = "measured" if hbm else "fallback"
     hbm = hbm or 6650.0
+    if args.transition == "weighted":
+        res["dom_kernel"] = res["dom_kernel"].replace("uniform", "weighted")
     achieved = res["dom_bytes_per_launch"] / (res["dom_ms_per_launch"] / 1e3) / 1e9
     traffic, traffic_src, l2_bytes = None, None, None
     tpath = os.path.join(ROOT, "profiles", "roofline_traffic.json")

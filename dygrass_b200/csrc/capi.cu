@@ -1,15 +1,10 @@
 // capi.cu -- the extern "C" boundary (include/dyg.h): graph handles and the
 // incremental / decremental batch and stream entry points.
 //
-// Batch flow, incremental (one iteration of random_walk_incremental/main.cu:314-340):
-//   stage inputs -> walk H (persistent kernel, per-edge winner keys) ->
-//   decode flags -> exclusive scan of the accept flags (input order) ->
-//   append accepted half-edges to H [-> append every half-edge to G].
-// Batch flow, decremental (random_walk_decremental/main.cu:413-444):
-//   delete from G and H in input order -> compact the edges found in both ->
-//   walk G -> replay winners for their paths -> dedup path edges, drop those
-//   in H, append the rest in order -> 2-step fallback walks for the edges
-//   without a path, same dedup and append.
+// The batch flows themselves are in pipeline.cu.  This file places the
+// caller's arrays: host inputs of up to kPackMax bytes in all are packed into
+// one page-locked block and copied once, results come back the same way, and
+// device arrays are used where they are.
 #include <math.h>
 #include <string.h>
 

@@ -7,16 +7,17 @@
 // max_steps walks), so instead of the reference's one-block-per-edge with a
 // 512-thread barrier tree, each warp of a persistent grid keeps its 32 lanes
 // busy: a lane whose walker ends takes the next walker of the warp's current
-// chunk, and the warp pulls a new chunk (32 walkers of an edge) from a global
-// counter when that is handed out.  The per-edge winner (max 1/R, lowest
+// chunk, and the warp pulls a new chunk (16, 32 or 64 walkers of an edge, see
+// chunk_for) from a global counter when that is handed out.  The per-edge winner (max 1/R, lowest
 // walker id) is a 64-bit key reduced with atomicMax, so no barrier and no
 // global scratch arrays are needed.  Lanes refill in step with one another
 // (every four moves), so the random-number blocks are drawn by whole warps.
 //
 // Draw d of walker k of update u is word d&3 of
-// Philox4x32-10({d>>2, k, u_lo, u_hi | domain<<24}, seed): any walker can be
-// replayed, which is how the decremental winner's path is recovered without
-// the reference's per-thread path[100] arrays.
+// Philox4x32-10({d>>2, k, u_lo, u_hi | domain<<24}, seed).  The decremental
+// winner's path comes from the record its walker left (PathRec) or, in the
+// batches that keep none, from a replay of that walker: any walker can be
+// replayed.  Neither needs the reference's per-thread path[100] arrays.
 #include <stdlib.h>
 
 #include <mutex>
@@ -813,7 +814,8 @@ __device__ __forceinline__ void write_record(const PathRec &rec, uint32_t e, uns
 // throughput (70 %) on the dense graph.  Against one lane-private edge read
 // and best per walker and the general remainder: insertions of the 100^3 mesh
 // 5.27 -> 4.43 ms, 24 random geometric graphs 1.14 -> 0.96 ms, deletions of
-// the mesh 2.28 -> 2.25 ms.
+// the mesh 2.28 -> 2.25 ms.  With chunks of 64 and the edge's best read before the
+// moves (insertions), the two mesh walks take 4.0 and 1.9 ms.
 // REC: the walkers keep their paths (see PathRec), at five blocks of 48
 // registers, since six would spill.
 template <bool INCR, bool REC>
