@@ -647,8 +647,8 @@ dyg_status PathScratch::open(dyg_graph *G, uint32_t n, const dyg_walk_params &p,
         cudaGetLastError();
         return DYG_OK;
     }
-    DYG_TRY(ensure(ws.rec_head, sizeof(uint32_t) * (size_t)n));
-    DYG_TRY(ensure(ws.rec_words, words));
+    if (ensure(ws.rec_head, sizeof(uint32_t) * (size_t)n) != DYG_OK || ensure(ws.rec_words, words) != DYG_OK)
+        return DYG_OK;
     rec.heads = ptr<uint32_t>(ws.rec_head);
     rec.words = ptr<uint32_t>(ws.rec_words);
     rec.cap = (uint32_t)(ws.rec_words.bytes / sizeof(uint32_t) > 0xFFFFFF00u ? 0xFFFFFF00u
@@ -661,11 +661,10 @@ dyg_status PathScratch::open(dyg_graph *G, uint32_t n, const dyg_walk_params &p,
 
 dyg_status PathScratch::grow(dyg_graph *G) {
     const unsigned long long need = G->ws.host_scalars[S_RECNEED] + G->ws.host_scalars[S_RECNEED] / 4;
-    if (need > 0xFFFFFF00ull) {
+    if (need > 0xFFFFFF00ull || ensure(G->ws.rec_words, sizeof(uint32_t) * need) != DYG_OK) {
         rec = PathRec{};   // replay the winners instead
         return DYG_OK;
     }
-    DYG_TRY(ensure(G->ws.rec_words, sizeof(uint32_t) * need));
     rec.words = ptr<uint32_t>(G->ws.rec_words);
     rec.cap = (uint32_t)need;
     return DYG_OK;

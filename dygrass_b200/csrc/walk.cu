@@ -1187,9 +1187,11 @@ dyg_status index_enqueue(dyg_graph *G, const dyg_walk_params &p, const unsigned 
     const uint32_t n = G->g.n;
     uint64_t words = 6ull * G->g.arena_cap + 2ull;
     if (words > kIdxWordsMax) words = kIdxWordsMax;
-    DYG_TRY(ensure(ws.ix_base, sizeof(uint32_t) * (size_t)n));
-    DYG_TRY(ensure(ws.ix_list, sizeof(uint32_t) * (size_t)n));
-    DYG_TRY(ensure(ws.ix_words, sizeof(uint32_t) * (size_t)words));
+    // where memory is short, the walks search their long rows without an index
+    if (ensure(ws.ix_base, sizeof(uint32_t) * (size_t)n) != DYG_OK ||
+        ensure(ws.ix_list, sizeof(uint32_t) * (size_t)n) != DYG_OK ||
+        ensure(ws.ix_words, sizeof(uint32_t) * (size_t)words) != DYG_OK)
+        return DYG_OK;
     unsigned long long *sc = ptr<unsigned long long>(ws.scalars);
     DYG_CUDA(cudaMemsetAsync(sc + S_IDX, 0, 2 * sizeof(unsigned long long), st));
     IndexArgs a{};
