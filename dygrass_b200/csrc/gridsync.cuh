@@ -21,6 +21,8 @@
 // call then fails) and leaves.
 #pragma once
 
+#include <atomic>
+
 #include <type_traits>
 
 #include "dyg_internal.cuh"
@@ -176,19 +178,30 @@ dyg_status launch_phases(uint32_t want, cudaStream_t st, GridBar bar, const A &.
     cfg.stream = st;
     cudaLaunchAttribute at{};
     cfg.attrs = &at;
-    // the largest cluster of this kernel that the device can place
-    static const uint32_t cluster_max = [] {
-        cudaLaunchConfig_t c{};
-        c.gridDim = dim3(kClusterMax);
-        c.blockDim = dim3(kOpThreads);
-        int most = 0;
-        if (cudaFuncSetAttribute(Kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-            cudaOccupancyMaxPotentialClusterSize(&most, Kernel, &c) != cudaSuccess) {
-            cudaGetLastError();
-            most = 0;
+    // the largest cluster of this kernel that the device can place, asked for
+    // (and allowed, which a context keeps) once in each device's context
+    constexpr int kDevs = 64;
+    static std::atomic<unsigned long long> placed[kDevs];   // context, 1 + the size; 0: not asked yet
+    uint32_t cluster_max = 0;
+    int dev = -1;
+    if (want > 1u && cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kDevs) {
+        const unsigned long long ctx = current_context_id() << 8;
+        unsigned long long known = placed[dev].load(std::memory_order_acquire);
+        if (!known || (known & ~0xFFull) != ctx) {
+            cudaLaunchConfig_t c{};
+            c.gridDim = dim3(kClusterMax);
+            c.blockDim = dim3(kOpThreads);
+            int most = 0;
+            if (cudaFuncSetAttribute(Kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+                cudaOccupancyMaxPotentialClusterSize(&most, Kernel, &c) != cudaSuccess || most < 0) {
+                cudaGetLastError();
+                most = 0;
+            }
+            known = ctx | (1u + (most < (int)kClusterMax ? (uint32_t)most : kClusterMax));
+            placed[dev].store(known, std::memory_order_release);
         }
-        return most < (int)kClusterMax ? (uint32_t)(most < 0 ? 0 : most) : kClusterMax;
-    }();
+        cluster_max = (uint32_t)(known & 0xFFull) - 1u;
+    }
     uint32_t k = 2u;
     while (k < want) k <<= 1;
     if (want <= 1u) {
