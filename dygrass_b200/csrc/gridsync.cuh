@@ -45,9 +45,11 @@ struct NoWork {
 };
 
 // Every thread of the cluster arrives and waits; writes made before are
-// visible after, in global memory as well.
+// visible after, in global memory as well.  Not the .aligned forms: a phase
+// ends in loops of different lengths and in branches of one thread, and
+// nothing makes the lanes of a warp come back together before they get here.
 __device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 
 // The last block to arrive runs `last` (one thread) before any block leaves.
