@@ -333,11 +333,6 @@ dyg_status check_device_errors(dyg_graph *G, cudaStream_t st) {
             set_error("a prefix scan tile timed out waiting for its predecessor");
             return DYG_ESTATE;
         }
-        if (err & kErrBarrier) {
-            DYG_CUDA(cudaMemset(ptr<unsigned long long>(G->ws.scalars) + S_BAR, 0, sizeof(unsigned long long)));
-            set_error("a block timed out waiting at a grid barrier; the graphs are no longer consistent");
-            return DYG_ESTATE;
-        }
         set_error("internal consistency check failed (device error bits " + std::to_string(err) + ")");
         return DYG_ESTATE;
     }
@@ -604,6 +599,7 @@ dyg_status dyg_graph_copy_from(dyg_graph *dst, const dyg_graph *src, dyg_stream_
     dst->slack = src->slack;
     dst->headroom = src->headroom;
     dst->long_rows = src->long_rows;
+    dst->broken = src->broken;
     return DYG_OK;
 }
 

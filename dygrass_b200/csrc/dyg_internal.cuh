@@ -261,10 +261,15 @@ constexpr unsigned long long kHaltArena = 1;    // an arena reservation did not 
 constexpr unsigned long long kHaltRecords = 2;  // the recovered-edge buffers are full
 constexpr unsigned long long kHaltInvalid = 3;  // a device-resident batch failed its input check
 constexpr unsigned long long kHaltPaths = 4;    // the path records did not fit (the walks are repeated)
+constexpr unsigned long long kHaltBroken = 5;   // a block gave up at a grid barrier (nothing resumes)
 __host__ __device__ __forceinline__ unsigned long long halt_code(uint32_t batch, uint32_t kind,
                                                                  uint32_t phase) {
     return ((unsigned long long)(batch + 1) << 8) | (kind << 4) | phase;
 }
+
+// Reads of a grid barrier's word before a block gives up: a phase may rightly
+// last a while (a block rewriting hub rows), so about a minute.
+constexpr uint32_t kBarSpinLimit = 1u << 26;
 
 }  // namespace dyg
 
@@ -282,6 +287,11 @@ struct dyg_graph {
     // then spread their entries over every SM, and stream files search such
     // rows with whole blocks (the results do not depend on it).
     bool long_rows = false;
+    // A launch that updated the graph was cut short (kErrBarrier): its rows may
+    // hold part of a batch.  Updates are refused until a whole graph is copied
+    // over it.
+    bool broken = false;
+    uint32_t bar_limit = dyg::kBarSpinLimit;   // GridBar::limit
 };
 
 namespace dyg {
@@ -371,8 +381,9 @@ dyg_status launch_walk_scalars(const DevGraph &g, const WalkJob &job, const dyg_
                                bool incremental, unsigned long long *keys,
                                unsigned long long *scalars, cudaStream_t st);
 // The row index for weighted walks on G as it is now; empty for a uniform
-// transition or a graph without hub rows.
-dyg_status index_enqueue(dyg_graph *G, const dyg_walk_params &p, const unsigned long long *halt,
+// transition or a graph without hub rows.  The walks that use it test the same
+// halt word: an index whose launch was cut short must not be read.
+dyg_status index_enqueue(dyg_graph *G, const dyg_walk_params &p, unsigned long long *halt,
                          RowIndex *out, cudaStream_t st);
 dyg_status launch_winner_paths(dyg_graph *G, const WalkJob &job, const dyg_walk_params &p,
                                const unsigned long long *keys, uint32_t n_max, uint32_t path_stride,
@@ -482,7 +493,11 @@ dyg_status export_graph(dyg_graph *G, uint64_t *row_ptr, uint32_t *col, float *w
 // Sums the degrees into S_SLOTS.
 dyg_status count_slots_enqueue(dyg_graph *G, cudaStream_t st);
 // Copies both graphs' scalars and counts to the host with one synchronize.
+// DYG_ESTATE if a launch on either was cut short at a grid barrier: both are
+// then marked broken, their workspaces as new.
 dyg_status read_scalars2(dyg_graph *A, dyg_graph *B, cudaStream_t st);
+// DYG_ESTATE for a broken graph (B may be null).
+dyg_status check_usable(const dyg_graph *A, const dyg_graph *B);
 // Exclusive scan of in[0, m) into out; with m_dev, of in[0, min(m, *m_dev)).
 dyg_status exclusive_scan_u32(Workspace &ws, const uint32_t *in, uint32_t *out, uint32_t m,
                               cudaStream_t st, const uint32_t *m_dev = nullptr);

@@ -50,6 +50,25 @@ dyg_status ensure(Buf &b, size_t bytes) {
     return DYG_OK;
 }
 
+// The workspace of a graph whose update was cut short: what the operations
+// expect to find as the one before left it (chains, hash tables, counters) is
+// made as new.
+static dyg_status recover_workspace(dyg_graph *G) {
+    Workspace &ws = G->ws;
+    DYG_CUDA(cudaDeviceSynchronize());
+    for (Buf *b : {&ws.rowcnt, &ws.rowhead, &ws.htab_k, &ws.htab_v, &ws.st_key, &ws.st_cnt}) {
+        dev_free(b->p);
+        *b = Buf{};
+    }
+    for (int s : {S_NEED, S_CURSOR, S_KEPT, S_NBIG, S_TMPCUR, S_ERR, S_WORK, S_HALT, S_BAR, S_RECW, S_ITEMS}) {
+        DYG_CUDA(cudaMemset(ptr<unsigned long long>(ws.scalars) + s, 0, sizeof(unsigned long long)));
+        ws.host_scalars[s] = 0ull;
+    }
+    DYG_CUDA(cudaDeviceSynchronize());
+    G->bar_limit = kBarSpinLimit;
+    return DYG_OK;
+}
+
 dyg_status read_scalars(dyg_graph *G, cudaStream_t st) { return read_scalars2(G, nullptr, st); }
 
 dyg_status read_scalars2(dyg_graph *A, dyg_graph *B, cudaStream_t st) {
@@ -59,9 +78,26 @@ dyg_status read_scalars2(dyg_graph *A, dyg_graph *B, cudaStream_t st) {
             DYG_CUDA(cudaMemcpyAsync(G->ws.host_scalars, G->ws.scalars.p, kScalarBytes,
                                      cudaMemcpyDeviceToHost, st));
     DYG_CUDA(cudaStreamSynchronize(st));
+    unsigned long long err = 0ull;
     for (dyg_graph *G : {A, B})
-        if (G && G->ws.host_scalars[S_LONG]) G->long_rows = true;
-    return DYG_OK;
+        if (G) {
+            if (G->ws.host_scalars[S_LONG]) G->long_rows = true;
+            err |= G->ws.host_scalars[S_ERR];
+        }
+    if (!(err & kErrBarrier)) return DYG_OK;
+    for (dyg_graph *G : {A, B})
+        if (G) {
+            G->broken = true;
+            DYG_TRY(recover_workspace(G));
+        }
+    set_error("a block timed out waiting at a grid barrier: the graphs hold part of an update");
+    return DYG_ESTATE;
+}
+
+dyg_status check_usable(const dyg_graph *A, const dyg_graph *B) {
+    if (!A->broken && (!B || !B->broken)) return DYG_OK;
+    set_error("an earlier call was cut short and the graph holds part of its update; copy a whole graph over it");
+    return DYG_ESTATE;
 }
 
 // ------------------------------------------------------------------ upload

@@ -17,8 +17,16 @@
 // launched cooperatively; their barrier counts arrivals on one word and
 // publishes a generation on another, both in the owning graph's scalars.  All
 // blocks of such a grid are resident, so a waiting block's peers run; the wait
-// is bounded all the same, and a block that gives up raises kErrBarrier (the
-// call then fails) and leaves.
+// is bounded all the same, and a block that gives up raises kErrBarrier, halts
+// the call (every later launch of it returns at once) and leaves.  What the
+// kernel was doing stays half done: read_scalars2 reports it as DYG_ESTATE and
+// marks the graphs (see recover_workspace).
+//
+// A block may give up while others of its grid go on to the next phase (the
+// late arrival that it did not wait for opens the barrier), so the halt word
+// can change under a running phase.  A kernel that asks whether *it* halted
+// therefore compares the word with its own code; the word is only set when it
+// is zero, so that such a code stays.
 #pragma once
 
 #include <atomic>
@@ -30,14 +38,12 @@
 namespace dyg {
 
 constexpr uint32_t kOpThreads = 512;
-// Reads of the generation word before a block gives up: a phase may rightly
-// last a while (a block rewriting hub rows), so about a minute.
-constexpr uint32_t kBarSpinLimit = 1u << 26;
 
 struct GridBar {
     uint32_t *count, *gen;
-    unsigned long long *err;
-    bool cluster;   // the grid is one thread-block cluster
+    unsigned long long *err, *halt;
+    uint32_t limit;   // reads of the generation word before a block gives up
+    bool cluster;     // the grid is one thread-block cluster
 };
 
 struct NoWork {
@@ -85,8 +91,9 @@ __device__ __forceinline__ bool grid_sync(const GridBar &b, F last) {
                 uint32_t spins = 0;
                 while (*vg == g) {
                     if (++spins > 4096u) __nanosleep(256);
-                    if (spins > kBarSpinLimit) {
+                    if (spins > b.limit) {
                         atomicOr(b.err, (unsigned long long)kErrBarrier);
+                        atomicCAS(b.halt, 0ull, halt_code(0, (uint32_t)kHaltBroken, 0));
                         ok = 0u;
                         break;
                     }

@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(kOpThreads, 2) k_recover(const __grid_constant
                 }
             }))
             return;
-        if (*(volatile unsigned long long *)a.halt) {
+        if (*(volatile unsigned long long *)a.halt == a.code_paths) {
             for (uint32_t f = rg.x + threadIdx.x; f < rg.y; f += blockDim.x) {
                 a.rec.heads[f] = 0u;
                 if (a.clear_keys) a.keys[f] = 0ull;
@@ -480,7 +480,7 @@ __global__ void __launch_bounds__(kOpThreads, 2) k_recover(const __grid_constant
         a.tk[i] = ~0ull;
         a.tv[i] = ~0u;
     }
-    if (*(volatile unsigned long long *)a.halt) return;
+    if (*(volatile unsigned long long *)a.halt == a.code_records) return;
     const uint2 pk = blocks_before(a.blk, s.warp);
     const unsigned long long rec0 = a.sc[S_RECCNT];
     uint32_t base = pk.x;
@@ -631,7 +631,7 @@ dyg_status decr_delete_enqueue(dyg_graph *G, dyg_graph *H, const uint32_t *src,
     a.counts = ptr<uint32_t>(ws.counts);
     a.err = sc + S_ERR;
     a.halt = halt;
-    return launch_phases<k_delete>(op_blocks(m, G->long_rows || H->long_rows), st, grid_bar(G), a);
+    return launch_phases<k_delete>(op_blocks(m, G->long_rows || H->long_rows), st, grid_bar(G, halt), a);
 }
 
 dyg_status PathScratch::open(dyg_graph *G, uint32_t n, const dyg_walk_params &p, cudaStream_t stream) {
@@ -766,7 +766,7 @@ dyg_status decr_walk_enqueue(dyg_graph *G, dyg_graph *H, uint32_t f0, uint32_t n
                                     ptr<uint32_t>(ws.path_s), ptr<int32_t>(ws.path_len), ix, st));
     }
     // blocks for what a batch usually brings: a few candidates per deletion
-    return launch_phases<k_recover>(op_blocks(4ull * n, H->long_rows), st, grid_bar(G), a);
+    return launch_phases<k_recover>(op_blocks(4ull * n, H->long_rows), st, grid_bar(G, halt), a);
 }
 
 // Decremental batch `batch` of the standalone updater: deletion stage, then
@@ -816,6 +816,7 @@ dyg_status incremental_run(dyg_graph *H, dyg_graph *G, const uint32_t *src, cons
                            const std::function<dyg_status()> *fetch) {
     unsigned long long *sc = ptr<unsigned long long>(H->ws.scalars);
     unsigned long long *halt = sc + S_HALT;
+    DYG_TRY(check_usable(H, G));
     DYG_TRY(clear_halt(H, st));
     if (check_inputs) DYG_TRY(validate_enqueue(halt, sc + S_ERR, src, dst, w, n, H->g.n, st));
     // no batch is larger than the first, so the keys it clears are clear for
@@ -854,6 +855,7 @@ dyg_status decremental_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, cons
     Workspace &ws = G->ws;
     unsigned long long *sc = ptr<unsigned long long>(ws.scalars);
     unsigned long long *halt = sc + S_HALT;
+    DYG_TRY(check_usable(G, H));
     // record buffers: start at 4 per deletion, grown on demand (halt + resume)
     const uint64_t want = (uint64_t)n * 4 + 1024;
     DYG_TRY(ensure(ws.rx2, sizeof(uint32_t) * want));

@@ -18,10 +18,10 @@ dyg_status rowops_ensure(dyg_graph *G, uint64_t m, cudaStream_t st) {
     return DYG_OK;
 }
 
-GridBar grid_bar(dyg_graph *G) {
+GridBar grid_bar(dyg_graph *G, unsigned long long *halt) {
     unsigned long long *sc = ptr<unsigned long long>(G->ws.scalars);
     uint32_t *words = reinterpret_cast<uint32_t *>(sc + S_BAR);
-    return GridBar{words, words + 1, sc + S_ERR, false};
+    return GridBar{words, words + 1, sc + S_ERR, halt, G->bar_limit, false};
 }
 
 AppSide append_side(dyg_graph *G, const uint32_t *src, const uint32_t *dst, const float *w) {

@@ -386,7 +386,7 @@ __device__ __forceinline__ bool app_commit(const AppSides &A, uint32_t m, const 
             if (reserve_moves(A, halt, code)) on_reserve();
         }))
         return false;
-    const bool halted = *(volatile unsigned long long *)halt != 0ull;
+    const bool halted = *(volatile unsigned long long *)halt == code;
     for (uint32_t k = 0; k < A.n; ++k) app_rows(A.s[k], m, halted, s);
     return true;
 }
@@ -781,7 +781,7 @@ k_append(const Op op, const __grid_constant__ AppSides A, uint32_t *blk, unsigne
 
 // Workspace of a row operation on up to m half-edges (cleared on st).
 dyg_status rowops_ensure(dyg_graph *G, uint64_t m, cudaStream_t st);
-GridBar grid_bar(dyg_graph *G);
+GridBar grid_bar(dyg_graph *G, unsigned long long *halt);
 AppSide append_side(dyg_graph *G, const uint32_t *src, const uint32_t *dst, const float *w);
 
 template <class Op>
@@ -799,7 +799,7 @@ dyg_status append_enqueue(const Op &op, uint32_t n_host, dyg_graph *GA, const Ed
         A.n = 2;
     }
     const bool hubs = GA->long_rows || (GB && GB->long_rows);
-    return launch_phases<k_append<Op>>(op_blocks(2ull * n_host, hubs), st, grid_bar(GA), op, A,
+    return launch_phases<k_append<Op>>(op_blocks(2ull * n_host, hubs), st, grid_bar(GA, halt), op, A,
                                        ptr<uint32_t>(GA->ws.blk), work, halt, code);
 }
 

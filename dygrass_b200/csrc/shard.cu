@@ -77,6 +77,7 @@ dyg_status dyg_walk_keys(dyg_graph *X, const uint32_t *src, const uint32_t *dst,
         return DYG_EINVAL;
     }
     DYG_TRY(check_walk(p));
+    DYG_TRY(check_usable(X, nullptr));
     if (lo == hi) return DYG_OK;
     Guard g(X->device);
     if (!dev_ptr(keys)) {
@@ -110,7 +111,7 @@ dyg_status dyg_walk_keys(dyg_graph *X, const uint32_t *src, const uint32_t *dst,
                 (unsigned long long)(first_update_id + lo), nullptr, hi - lo,
                 incremental ? kDomainIncr : kDomainDecr};
     RowIndex ix{};
-    DYG_TRY(index_enqueue(X, *p, job.halt, &ix, st));
+    DYG_TRY(index_enqueue(X, *p, sc + S_HALT, &ix, st));
     DYG_TRY(launch_walk(X, job, *p, incremental != 0, k, ix, st));
     DYG_TRY(read_scalars(X, st));
     if (ws.host_scalars[S_HALT]) return rejected_inputs(X, st);
@@ -131,6 +132,7 @@ dyg_status dyg_incremental_commit_keys(dyg_graph *H, dyg_graph *G, const uint32_
         set_error("G and H must be two handles with the same vertex count and device");
         return DYG_EINVAL;
     }
+    DYG_TRY(check_usable(H, G));
     if (n == 0) return DYG_OK;
     Guard gd(H->device);
     const bool outs_dev = (!found_at || dev_ptr(found_at)) && (!conductance || dev_ptr(conductance)) &&
@@ -185,6 +187,7 @@ dyg_status dyg_decremental_delete(dyg_graph *G, dyg_graph *H, const uint32_t *sr
         return DYG_EINVAL;
     }
     *n_walk = 0;
+    DYG_TRY(check_usable(G, H));
     if (n == 0) return DYG_OK;
     Guard gd(G->device);
     if (!dev_ptr(status) || !dev_ptr(conductance)) {
@@ -229,6 +232,7 @@ dyg_status dyg_decremental_walk_keys(dyg_graph *G, uint32_t lo, uint32_t hi,
         return DYG_EINVAL;
     }
     DYG_TRY(check_walk(p));
+    DYG_TRY(check_usable(G, nullptr));
     if (lo == hi) return DYG_OK;
     Guard gd(G->device);
     Workspace &ws = G->ws;
@@ -244,13 +248,14 @@ dyg_status dyg_decremental_walk_keys(dyg_graph *G, uint32_t lo, uint32_t hi,
     cudaStream_t st = (cudaStream_t)stream;
     unsigned long long *k = (unsigned long long *)keys + lo;
     DYG_CUDA(cudaMemsetAsync(k, 0, sizeof(unsigned long long) * (hi - lo), st));
-    WalkJob job{nullptr, ptr<uint32_t>(ws.f_src) + lo, ptr<uint32_t>(ws.f_dst) + lo, nullptr,
+    unsigned long long *halt = ptr<unsigned long long>(ws.scalars) + S_HALT;
+    DYG_TRY(clear_halt_of(G, st));
+    WalkJob job{halt, ptr<uint32_t>(ws.f_src) + lo, ptr<uint32_t>(ws.f_dst) + lo, nullptr,
                 ptr<unsigned long long>(ws.f_uid) + lo, 0ull, nullptr, hi - lo, kDomainDecr};
     RowIndex ix{};
-    DYG_TRY(index_enqueue(G, *p, nullptr, &ix, st));
+    DYG_TRY(index_enqueue(G, *p, halt, &ix, st));
     DYG_TRY(launch_walk(G, job, *p, false, k, ix, st));
-    DYG_CUDA(cudaStreamSynchronize(st));
-    return DYG_OK;
+    return read_scalars(G, st);
 }
 
 dyg_status dyg_decremental_commit_keys(dyg_graph *G, dyg_graph *H, const dyg_walk_params *p,
@@ -265,6 +270,7 @@ dyg_status dyg_decremental_commit_keys(dyg_graph *G, dyg_graph *H, const dyg_wal
     }
     DYG_TRY(check_walk(p));
     if (n_rec) *n_rec = 0;
+    DYG_TRY(check_usable(G, H));
     if (n_walk == 0) return DYG_OK;
     Guard gd(G->device);
     if (!dev_ptr(keys) || !dev_ptr(status) || !dev_ptr(conductance)) {

@@ -622,6 +622,7 @@ dyg_status stream_file_run(dyg_graph *G, dyg_graph *H, uint32_t op, const uint32
                            uint64_t *n_rec, cudaStream_t st, bool check_inputs,
                            const std::function<dyg_status()> *fetch) {
     *n_rec = 0;
+    DYG_TRY(check_usable(G, H));
     if (chunk == 0) chunk = stream_default_chunk(G->g.n);
     if (op == DYG_STREAM_INSERT)
         return insert_file_run(G, H, src, dst, w, n, uid0, chunk, p, status, cond, st,

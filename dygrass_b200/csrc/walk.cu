@@ -27,6 +27,7 @@
 
 #include "dyg_internal.cuh"
 #include "gridsync.cuh"
+#include "rowops.cuh"
 
 namespace dyg {
 
@@ -450,7 +451,7 @@ __device__ __forceinline__ uint32_t index_pick(const uint2 *__restrict__ slots,
     uint32_t pos = deg;
     if (has_ex) {
         uint32_t h = idx_hash(ex, bits);
-        while (true) {
+        for (uint32_t left = 1u << bits; left > 0u; --left) {   // half of the table is empty
             const uint32_t t = __ldg(region + h);
             if (t == 0u) break;
             const uint32_t col = __ldg(&slots[lo + t - 1u].x);
@@ -510,7 +511,7 @@ __device__ __forceinline__ bool idx_insert(const IndexArgs &a, uint32_t *tab, ui
 __global__ void __launch_bounds__(kOpThreads, 2) k_index(const __grid_constant__ IndexArgs a, GridBar bar) {
     __shared__ unsigned long long s_sum[kOpThreads / 32];
     __shared__ uint32_t s_bad;
-    if (a.halt && *a.halt) return;
+    if (*a.halt) return;
     const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
     // regions, and the lists of rows: for a warp from the front, for a block
     // from the back
@@ -1179,7 +1180,7 @@ static void launch_walk_any(const WalkArgs &a, bool incremental, bool wtd, cudaS
 // rows that do not fit stay without an index.
 constexpr uint64_t kIdxWordsMax = 1ull << 29;
 
-dyg_status index_enqueue(dyg_graph *G, const dyg_walk_params &p, const unsigned long long *halt,
+dyg_status index_enqueue(dyg_graph *G, const dyg_walk_params &p, unsigned long long *halt,
                          RowIndex *out, cudaStream_t st) {
     *out = RowIndex{};
     if (p.transition != DYG_TRANSITION_WEIGHTED || !G->long_rows) return DYG_OK;
@@ -1203,9 +1204,7 @@ dyg_status index_enqueue(dyg_graph *G, const dyg_walk_params &p, const unsigned 
     a.cursor = sc + S_IDX;
     a.counts = sc + S_IDXN;
     a.halt = halt;
-    uint32_t *bw = reinterpret_cast<uint32_t *>(sc + S_BAR);
-    const GridBar bar{bw, bw + 1, sc + S_ERR, false};
-    DYG_TRY(launch_phases<k_index>(2u * (uint32_t)num_sms(), st, bar, a));
+    DYG_TRY(launch_phases<k_index>(2u * (uint32_t)num_sms(), st, grid_bar(G, halt), a));
     *out = RowIndex{a.rbase, a.words};
     return DYG_OK;
 }

@@ -46,7 +46,10 @@
  * an endpoint >= |V| or a weight that is not finite and > 0, in host or
  * device memory, makes the call return DYG_EINVAL with G and H unchanged.
  * With host outputs the call returns after the results are on the
- * host.  A handle is not thread-safe; distinct handles are.  Calls are
+ * host.  A call that ends with DYG_ESTATE because a launch of it was cut
+ * short may have applied part of its update; its graphs then refuse updates
+ * (DYG_ESTATE) until dyg_graph_copy_from copies a whole graph over them.
+ * A handle is not thread-safe; distinct handles are.  Calls are
  * ordered on the given CUDA stream (NULL = legacy default stream).
  * No torch types cross this boundary.
  */
