@@ -94,6 +94,19 @@ dyg_status read_scalars2(dyg_graph *A, dyg_graph *B, cudaStream_t st) {
     return DYG_ESTATE;
 }
 
+// After a scan on G and read_scalars: DYG_ESTATE if a tile of it gave up, so
+// that nothing is placed or copied by its results.
+static dyg_status check_scan(dyg_graph *G) {
+    Workspace &ws = G->ws;
+    if (!(ws.host_scalars[S_ERR] & kErrScan)) return DYG_OK;
+    ws.host_scalars[S_ERR] &= ~(unsigned long long)kErrScan;
+    DYG_CUDA(cudaMemcpy(ptr<unsigned long long>(ws.scalars) + S_ERR, ws.host_scalars + S_ERR,
+                        sizeof(unsigned long long), cudaMemcpyHostToDevice));
+    ws.scan_tickets = ws.host_scalars[S_SCAN];   // in step again
+    set_error("a prefix scan tile timed out waiting for its predecessor");
+    return DYG_ESTATE;
+}
+
 dyg_status check_usable(const dyg_graph *A, const dyg_graph *B) {
     if (!A->broken && (!B || !B->broken)) return DYG_OK;
     set_error("an earlier call was cut short and the graph holds part of its update; copy a whole graph over it");
@@ -224,8 +237,11 @@ struct BuildScan {
     __device__ void last(uint32_t total) const { *top = total; }
 };
 
+// With an error of the scan before it, the offsets are not to be used: the
+// rows are left alone, and the call fails.
 __global__ void k_build_place(const uint32_t *src, const uint32_t *dst, uint32_t m, const uint2 *desc,
-                              uint32_t *cnt, uint32_t *idx) {
+                              uint32_t *cnt, uint32_t *idx, const unsigned long long *err) {
+    if (*err) return;
     for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < m; e += gridDim.x * blockDim.x) {
         const uint32_t u = src[e], v = dst[e];
         idx[desc[u].x + atomicAdd(cnt + u, 1u)] = 2u * e;
@@ -251,7 +267,9 @@ constexpr uint32_t kBuildThreads = 256;
 // time, each index's rank counted against the row's others.  Longer rows go
 // to `big` (n words) for k_build_big.
 __global__ void __launch_bounds__(kBuildThreads)
-k_build_rows(DevGraph g, BuildList L, const uint32_t *idx, uint32_t *big, unsigned long long *nbig) {
+k_build_rows(DevGraph g, BuildList L, const uint32_t *idx, uint32_t *big, unsigned long long *nbig,
+             const unsigned long long *err) {
+    if (*err) return;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x;
     for (uint32_t vb = first - lane; vb < g.n; vb += gridDim.x * blockDim.x) {
@@ -419,16 +437,17 @@ dyg_status build_graph(dyg_graph *G, uint32_t n, uint64_t m, const uint32_t *src
     }
     if (m) {
         const BuildList L{ds, dd, (float *)d_w};
-        k_build_place<<<grid_of(m, 256), 256, 0, st>>>(ds, dd, (uint32_t)m, G->g.desc, cnt, idx);
+        k_build_place<<<grid_of(m, 256), 256, 0, st>>>(ds, dd, (uint32_t)m, G->g.desc, cnt, idx, sc + S_ERR);
         count_launch();
-        k_build_rows<<<grid_of(n, kBuildThreads), kBuildThreads, 0, st>>>(G->g, L, idx, big, sc + S_NBIG);
+        k_build_rows<<<grid_of(n, kBuildThreads), kBuildThreads, 0, st>>>(G->g, L, idx, big, sc + S_NBIG, sc + S_ERR);
         count_launch();
         k_build_big<<<num_sms() * 4, kBuildThreads, 0, st>>>(G->g, L, idx, big, sc + S_NBIG);
         count_launch();
         DYG_CUDA(cudaGetLastError());
         DYG_CUDA(cudaMemsetAsync(sc + S_NBIG, 0, sizeof(unsigned long long), st));
     }
-    return read_scalars(G, st);   // synchronizes; picks up a long row
+    DYG_TRY(read_scalars(G, st));   // synchronizes; picks up a long row
+    return check_scan(G);
 }
 
 // ----------------------------------------------------------------- export
@@ -506,7 +525,8 @@ dyg_status export_graph(dyg_graph *G, uint64_t *row_ptr, uint32_t *col, float *w
     if (ok) {
         DYG_TRY(scan_op(G->ws, DegreeScan{G->g.desc, (unsigned long long *)d_rp, n}, n, nullptr, nullptr, st));
         DYG_CUDA(cudaMemcpyAsync(row_ptr, d_rp, sizeof(uint64_t) * ((size_t)n + 1), cudaMemcpyDeviceToHost, st));
-        DYG_CUDA(cudaStreamSynchronize(st));
+        DYG_TRY(read_scalars(G, st));
+        DYG_TRY(check_scan(G));
         const uint64_t total = row_ptr[n], out = total < slot_cap ? total : slot_cap;
         if (out && (col || w)) {
             ok = tmp.get(&d_col, sizeof(uint32_t) * total) == cudaSuccess &&
@@ -693,7 +713,8 @@ dyg_status compact_graph(dyg_graph *G, cudaStream_t st) {
     uint32_t last_off = 0, last_cap = 0;
     DYG_CUDA(cudaMemcpyAsync(&last_off, ptr<uint32_t>(ws.pos) + n - 1, 4, cudaMemcpyDeviceToHost, st));
     DYG_CUDA(cudaMemcpyAsync(&last_cap, ptr<uint32_t>(ws.flags) + n - 1, 4, cudaMemcpyDeviceToHost, st));
-    DYG_CUDA(cudaStreamSynchronize(st));
+    DYG_TRY(read_scalars(G, st));
+    DYG_TRY(check_scan(G));
     const uint64_t used = (uint64_t)last_off + last_cap;
     uint64_t cap = used + (uint64_t)((double)used * G->headroom) + 1024;
     if (cap < G->g.arena_cap / 2) cap = G->g.arena_cap / 2 > used ? G->g.arena_cap / 2 : cap;

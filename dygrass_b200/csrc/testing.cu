@@ -13,3 +13,8 @@ extern "C" dyg_status dyg_testing_stall_barrier(dyg_graph *g, uint32_t spin_limi
     g->bar_limit = spin_limit;
     return DYG_OK;
 }
+
+extern "C" dyg_status dyg_testing_stall_scan(dyg_graph *g) {
+    g->ws.scan_tickets -= 1;
+    return DYG_OK;
+}

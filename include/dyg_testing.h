@@ -15,6 +15,10 @@ extern "C" {
  * give up after spin_limit reads (> 4096; the default is about a minute's). */
 dyg_status dyg_testing_stall_barrier(dyg_graph *g, uint32_t spin_limit);
 
+/* The next prefix scan on g (an export, a compaction) misses its first tile:
+ * the others wait for it until their limit. */
+dyg_status dyg_testing_stall_scan(dyg_graph *g);
+
 #ifdef __cplusplus
 }
 #endif

@@ -130,3 +130,23 @@ def test_split_calls_report_it(dyg):  # noqa: F811
     assert [c() for c in (walk, commit)] == [0, 0]
     restored()
     assert [c() for c in (delete, dwalk, dcommit)] == [0, 0, 0]
+
+
+@pytest.mark.parametrize("n", [10, 5000])
+@pytest.mark.parametrize("call", ["export", "compact"])
+def test_scan_that_runs_out(dyg, oracle, n, call):  # noqa: F811
+    """Row offsets that were not all computed are not used: the call says so,
+    and the next one works."""
+    rng = np.random.default_rng(n)
+    gs, gd, gw = hub_and_path(n, 3, rng)
+    g, go = dyg.Graph.from_edges(n, gs, gd, gw), oracle.OGraph(n, gs, gd, gw)
+    f = dyg.lib().dyg_testing_stall_scan
+    f.argtypes, f.restype = [C.c_void_p], C.c_int
+    for _ in range(2):
+        assert f(g.handle) == 0
+        with pytest.raises(dyg.DygError) as e:
+            g.export() if call == "export" else g.compact()
+        assert e.value.status == ESTATE
+        same_graph(g, go)
+        g.compact()
+        same_graph(g, go)
