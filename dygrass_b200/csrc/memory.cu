@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "dyg_internal.cuh"
+#include "pinned_cache.h"
 
 namespace dyg {
 
@@ -171,51 +172,35 @@ void scratch_return(Buf *b) {
 }
 
 namespace {
-struct PinnedBlock {
-    void *p;
-    size_t bytes;
-    unsigned long long ctx;
-};
-std::mutex g_pinned_mu;
-std::vector<PinnedBlock> g_pinned;   // free blocks
-size_t g_pinned_bytes = 0;
 constexpr size_t kPinnedKeep = 8u << 20;
+std::mutex g_pinned_mu;
+PinnedCache g_pinned(kPinnedKeep);
+
+// The current device, if its context can be told from one that replaced it.
+bool current_place(int *dev, unsigned long long *ctx) {
+    *ctx = current_context_id();
+    return *ctx && cudaGetDevice(dev) == cudaSuccess;
+}
 }  // namespace
 
 cudaError_t host_alloc(void **out, size_t bytes) {
+    int dev = 0;
+    unsigned long long ctx = 0;
     *out = nullptr;
-    const unsigned long long ctx = current_context_id();
-    {
+    if (current_place(&dev, &ctx)) {
         std::lock_guard<std::mutex> lk(g_pinned_mu);
-        for (size_t i = g_pinned.size(); i-- > 0;) {
-            if (g_pinned[i].bytes != bytes || g_pinned[i].ctx != ctx) continue;
-            *out = g_pinned[i].p;
-            g_pinned_bytes -= bytes;
-            g_pinned[i] = g_pinned.back();
-            g_pinned.pop_back();
-            return cudaSuccess;
-        }
+        *out = g_pinned.take(dev, ctx, bytes);
     }
-    return cudaMallocHost(out, bytes);
+    return *out ? cudaSuccess : cudaMallocHost(out, bytes);
 }
 
 void host_free(void *p, size_t bytes) {
+    int dev = 0;
+    unsigned long long ctx = 0;
     if (!p) return;
-    const unsigned long long ctx = current_context_id();
-    {
+    if (current_place(&dev, &ctx)) {
         std::lock_guard<std::mutex> lk(g_pinned_mu);
-        // blocks of a context that is gone went with it
-        for (size_t i = g_pinned.size(); ctx && i-- > 0;)
-            if (g_pinned[i].ctx != ctx) {
-                g_pinned_bytes -= g_pinned[i].bytes;
-                g_pinned[i] = g_pinned.back();
-                g_pinned.pop_back();
-            }
-        if (ctx && g_pinned_bytes + bytes <= kPinnedKeep) {
-            g_pinned.push_back(PinnedBlock{p, bytes, ctx});
-            g_pinned_bytes += bytes;
-            return;
-        }
+        if (g_pinned.keep(dev, ctx, p, bytes)) return;
     }
     cudaFreeHost(p);
 }
