@@ -322,6 +322,9 @@ void dev_free(void *p);
 struct Buf;
 cudaError_t scratch_borrow(Buf *b, size_t bytes);
 void scratch_return(Buf *b);
+// For tests: this thread's next `pass` allocations go through, the `fail` after
+// them do not.
+void fail_allocations(uint32_t pass, uint32_t fail);
 // Pinned host memory; host_free takes the size given to host_alloc, once the
 // device has finished with the block.
 cudaError_t host_alloc(void **out, size_t bytes);

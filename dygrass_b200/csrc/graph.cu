@@ -5,7 +5,9 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstring>
+#include <new>
 #include <vector>
 
 #include "dyg_internal.cuh"
@@ -372,10 +374,11 @@ struct Temps {
         if (e == cudaSuccess) p[k++] = *out;
         return e;
     }
-    ~Temps() {
+    void release() {
         if (k) cudaStreamSynchronize(nullptr);
         while (k) dev_free(p[--k]);
     }
+    ~Temps() { release(); }
 };
 
 int grid_of(uint64_t items, uint32_t threads) {
@@ -384,6 +387,47 @@ int grid_of(uint64_t items, uint32_t threads) {
 }
 
 }  // namespace
+
+// The rows as the device makes them, by the host: for lists whose copy and
+// half-edge indices (20 bytes an edge beside the graph's 36) do not fit the
+// device.
+static dyg_status build_on_host(dyg_graph *G, uint32_t n, uint64_t m, const uint32_t *src,
+                                const uint32_t *dst, const float *w, bool *bad) {
+    for (uint64_t e = 0; e < m; ++e)
+        if (src[e] >= n || dst[e] >= n || !(w[e] > 0.0f) || !std::isfinite(w[e])) {
+            *bad = true;
+            return DYG_EINVAL;
+        }
+    std::vector<uint64_t> row_ptr, fill;
+    std::vector<uint32_t> col;
+    std::vector<float> ww;
+    try {
+        row_ptr.assign((size_t)n + 1, 0);
+        fill.resize(n);
+        col.resize(2 * m + 1);
+        ww.resize(2 * m + 1);
+    } catch (const std::bad_alloc &) {
+        set_error("host allocation failed");
+        return DYG_ENOMEM;
+    }
+    for (uint64_t e = 0; e < m; ++e) {
+        row_ptr[src[e] + 1]++;
+        row_ptr[dst[e] + 1]++;
+    }
+    for (uint32_t v = 0; v < n; ++v) {
+        row_ptr[v + 1] += row_ptr[v];
+        fill[v] = row_ptr[v];
+    }
+    for (uint64_t e = 0; e < m; ++e) {
+        const uint64_t ps = fill[src[e]]++;
+        col[ps] = dst[e];
+        ww[ps] = w[e];
+        const uint64_t pd = fill[dst[e]]++;
+        col[pd] = src[e];
+        ww[pd] = w[e];
+    }
+    return upload_graph(G, n, row_ptr.data(), col.data(), ww.data());
+}
 
 dyg_status build_graph(dyg_graph *G, uint32_t n, uint64_t m, const uint32_t *src, const uint32_t *dst,
                        const float *w, bool *bad) {
@@ -397,20 +441,31 @@ dyg_status build_graph(dyg_graph *G, uint32_t n, uint64_t m, const uint32_t *src
     G->g.n = n;
     G->g.arena_cap = arena;
     const size_t nn = n ? n : 1;
-    Temps tmp;
-    void *d_src, *d_dst, *d_w, *d_cnt, *d_idx;
     if (dev_alloc(&G->g.desc, sizeof(uint2) * nn) != cudaSuccess ||
         dev_alloc(&G->g.cap, sizeof(uint32_t) * nn) != cudaSuccess ||
         dev_alloc(&G->g.slots, sizeof(uint2) * (size_t)arena) != cudaSuccess ||
-        dev_alloc(&G->g.wts, sizeof(float) * (size_t)arena) != cudaSuccess ||
-        tmp.get(&d_src, sizeof(uint32_t) * m) != cudaSuccess ||
-        tmp.get(&d_dst, sizeof(uint32_t) * m) != cudaSuccess ||
-        tmp.get(&d_w, sizeof(float) * m) != cudaSuccess ||
-        tmp.get(&d_cnt, sizeof(uint32_t) * nn) != cudaSuccess ||
-        tmp.get(&d_idx, sizeof(uint32_t) * (size_t)(used + nn)) != cudaSuccess) {
+        dev_alloc(&G->g.wts, sizeof(float) * (size_t)arena) != cudaSuccess) {
         cudaGetLastError();
         set_error("cudaMalloc of the graph arena failed");
         return DYG_ENOMEM;
+    }
+    Temps tmp;
+    void *d_src, *d_dst, *d_w, *d_cnt, *d_idx;
+    if (tmp.get(&d_src, sizeof(uint32_t) * m) != cudaSuccess ||
+        tmp.get(&d_dst, sizeof(uint32_t) * m) != cudaSuccess ||
+        tmp.get(&d_w, sizeof(float) * m) != cudaSuccess ||
+        tmp.get(&d_cnt, sizeof(uint32_t) * nn) != cudaSuccess ||
+        tmp.get(&d_idx, sizeof(uint32_t) * (size_t)(used + nn)) != cudaSuccess ||
+        scan_ensure(G->ws, n, nullptr) != DYG_OK) {
+        cudaGetLastError();
+        set_error("");
+        tmp.release();
+        for (void *p : {(void *)G->g.desc, (void *)G->g.cap, (void *)G->g.slots, (void *)G->g.wts}) dev_free(p);
+        G->g.desc = nullptr;
+        G->g.cap = nullptr;
+        G->g.slots = nullptr;
+        G->g.wts = nullptr;
+        return build_on_host(G, n, m, src, dst, w, bad);
     }
     cudaStream_t st = nullptr;
     unsigned long long *sc = ptr<unsigned long long>(G->ws.scalars);
@@ -514,6 +569,38 @@ dyg_status count_slots_enqueue(dyg_graph *G, cudaStream_t st) {
     return DYG_OK;
 }
 
+// The rows by the host from a copy of the arena, for when the device has no
+// room for them twice.
+static dyg_status export_on_host(dyg_graph *G, uint64_t *row_ptr, uint32_t *col, float *w, uint64_t slot_cap) {
+    const uint32_t n = G->g.n;
+    DYG_TRY(read_scalars(G, nullptr));
+    const size_t top = (size_t)G->ws.host_scalars[S_TOP];
+    std::vector<uint2> desc, slots;
+    std::vector<float> wts;
+    try {
+        desc.resize(n);
+        slots.resize(col ? top : 0);
+        wts.resize(w ? top : 0);
+    } catch (const std::bad_alloc &) {
+        set_error("host allocation failed");
+        return DYG_ENOMEM;
+    }
+    DYG_CUDA(cudaMemcpy(desc.data(), G->g.desc, sizeof(uint2) * n, cudaMemcpyDeviceToHost));
+    if (!slots.empty()) DYG_CUDA(cudaMemcpy(slots.data(), G->g.slots, sizeof(uint2) * top, cudaMemcpyDeviceToHost));
+    if (!wts.empty()) DYG_CUDA(cudaMemcpy(wts.data(), G->g.wts, sizeof(float) * top, cudaMemcpyDeviceToHost));
+    uint64_t o = 0;
+    for (uint32_t v = 0; v < n; ++v) {
+        row_ptr[v] = o;
+        for (uint32_t j = 0; j < desc[v].y && o + j < slot_cap; ++j) {
+            if (col) col[o + j] = slots[desc[v].x + j].x;
+            if (w) w[o + j] = wts[desc[v].x + j];
+        }
+        o += desc[v].y;
+    }
+    row_ptr[n] = o;
+    return DYG_OK;
+}
+
 dyg_status export_graph(dyg_graph *G, uint64_t *row_ptr, uint32_t *col, float *w, uint64_t slot_cap) {
     const uint32_t n = G->g.n;
     row_ptr[0] = 0;
@@ -523,31 +610,34 @@ dyg_status export_graph(dyg_graph *G, uint64_t *row_ptr, uint32_t *col, float *w
     void *d_rp, *d_col = nullptr, *d_w = nullptr;
     bool ok = tmp.get(&d_rp, sizeof(uint64_t) * ((size_t)n + 1)) == cudaSuccess;
     if (ok) {
-        DYG_TRY(scan_op(G->ws, DegreeScan{G->g.desc, (unsigned long long *)d_rp, n}, n, nullptr, nullptr, st));
+        const dyg_status rc =
+            scan_op(G->ws, DegreeScan{G->g.desc, (unsigned long long *)d_rp, n}, n, nullptr, nullptr, st);
+        ok = rc == DYG_OK;
+        if (!ok && rc != DYG_ENOMEM) return rc;
+    }
+    if (ok) {
         DYG_CUDA(cudaMemcpyAsync(row_ptr, d_rp, sizeof(uint64_t) * ((size_t)n + 1), cudaMemcpyDeviceToHost, st));
         DYG_TRY(read_scalars(G, st));
         DYG_TRY(check_scan(G));
         const uint64_t total = row_ptr[n], out = total < slot_cap ? total : slot_cap;
-        if (out && (col || w)) {
-            ok = tmp.get(&d_col, sizeof(uint32_t) * total) == cudaSuccess &&
-                 tmp.get(&d_w, sizeof(float) * total) == cudaSuccess;
-            if (ok) {
-                k_export_rows<<<grid_of((uint64_t)n * 8, 256), 256, 0, st>>>(
-                    G->g, (unsigned long long *)d_rp, (uint32_t *)d_col, (float *)d_w);
-                count_launch();
-                DYG_CUDA(cudaGetLastError());
-                if (col) DYG_CUDA(cudaMemcpyAsync(col, d_col, sizeof(uint32_t) * out, cudaMemcpyDeviceToHost, st));
-                if (w) DYG_CUDA(cudaMemcpyAsync(w, d_w, sizeof(float) * out, cudaMemcpyDeviceToHost, st));
-                DYG_CUDA(cudaStreamSynchronize(st));
-            }
+        if (!out || (!col && !w)) return DYG_OK;
+        ok = tmp.get(&d_col, sizeof(uint32_t) * total) == cudaSuccess &&
+             tmp.get(&d_w, sizeof(float) * total) == cudaSuccess;
+        if (ok) {
+            k_export_rows<<<grid_of((uint64_t)n * 8, 256), 256, 0, st>>>(
+                G->g, (unsigned long long *)d_rp, (uint32_t *)d_col, (float *)d_w);
+            count_launch();
+            DYG_CUDA(cudaGetLastError());
+            if (col) DYG_CUDA(cudaMemcpyAsync(col, d_col, sizeof(uint32_t) * out, cudaMemcpyDeviceToHost, st));
+            if (w) DYG_CUDA(cudaMemcpyAsync(w, d_w, sizeof(float) * out, cudaMemcpyDeviceToHost, st));
+            DYG_CUDA(cudaStreamSynchronize(st));
         }
     }
-    if (!ok) {
-        cudaGetLastError();
-        set_error("device memory for the export is short");
-        return DYG_ENOMEM;
-    }
-    return DYG_OK;
+    if (ok) return DYG_OK;
+    cudaGetLastError();
+    set_error("");   // a scan's status words that did not fit either
+    tmp.release();
+    return export_on_host(G, row_ptr, col, w, slot_cap);
 }
 
 dyg_status grow_arena(dyg_graph *G, uint64_t min_cap, cudaStream_t st) {

@@ -94,20 +94,43 @@ unsigned long long current_context_id() {
     return id;
 }
 
-cudaError_t dev_alloc(void **out, size_t bytes) {
+namespace {
+// Allocations of this thread that are still to succeed, and to fail after
+// them (dyg_testing_fail_allocations).
+thread_local uint32_t t_pass = 0, t_fail = 0;
+
+cudaError_t alloc_once(const DevicePool &p, void **out, size_t bytes) {
     *out = nullptr;
-    const DevicePool p = current_pool();
+    if (t_fail) {
+        if (t_pass == 0) {
+            --t_fail;
+            return cudaErrorMemoryAllocation;
+        }
+        --t_pass;
+    }
     if (!p.pool) return cudaMalloc(out, bytes);
     cudaError_t e = cudaMallocFromPoolAsync(out, bytes, p.pool, p.st);
-    if (e == cudaErrorMemoryAllocation) {
+    if (e == cudaSuccess) e = cudaStreamSynchronize(p.st);   // usable on any stream from here on
+    if (e != cudaSuccess) *out = nullptr;
+    return e;
+}
+}  // namespace
+
+void fail_allocations(uint32_t pass, uint32_t fail) {
+    t_pass = pass;
+    t_fail = fail;
+}
+
+cudaError_t dev_alloc(void **out, size_t bytes) {
+    const DevicePool p = current_pool();
+    cudaError_t e = alloc_once(p, out, bytes);
+    if (e == cudaErrorMemoryAllocation && p.pool) {
         // what the pool holds in other sizes goes back first
         cudaGetLastError();
         cudaStreamSynchronize(p.st);
         cudaMemPoolTrimTo(p.pool, 0);
-        e = cudaMallocFromPoolAsync(out, bytes, p.pool, p.st);
+        e = alloc_once(p, out, bytes);
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(p.st);   // usable on any stream from here on
-    if (e != cudaSuccess) *out = nullptr;
     return e;
 }
 

@@ -142,16 +142,22 @@ k_scan_op(Op op, uint32_t m, const uint32_t *m_dev, ScanCtl c) {
     }
 }
 
+// Status words for a scan of m elements.
+inline dyg_status scan_ensure(Workspace &ws, uint32_t m, cudaStream_t st) {
+    const size_t bytes = sizeof(unsigned long long) * ((m + (size_t)kScanTile - 1) / kScanTile);
+    if (ws.scan_status.bytes >= bytes) return DYG_OK;
+    DYG_TRY(ensure(ws.scan_status, bytes));
+    DYG_CUDA(cudaMemsetAsync(ws.scan_status.p, 0, ws.scan_status.bytes, st));
+    return DYG_OK;
+}
+
 // Enqueues the scan of [0, m) (of [0, min(m, *m_dev)) with a device count).
 template <class Op>
 dyg_status scan_op(Workspace &ws, const Op &op, uint32_t m, const uint32_t *m_dev,
                    const unsigned long long *halt, cudaStream_t st) {
     if (m == 0) return DYG_OK;
-    const uint32_t tiles = (m + kScanTile - 1) / kScanTile;
-    if (ws.scan_status.bytes < sizeof(unsigned long long) * tiles) {
-        DYG_TRY(ensure(ws.scan_status, sizeof(unsigned long long) * tiles));
-        DYG_CUDA(cudaMemsetAsync(ws.scan_status.p, 0, ws.scan_status.bytes, st));
-    }
+    const uint32_t tiles = (uint32_t)(((uint64_t)m + kScanTile - 1) / kScanTile);
+    DYG_TRY(scan_ensure(ws, m, st));
     ws.scan_epoch = ws.scan_epoch + 1u == 0x40000000u ? 1u : ws.scan_epoch + 1u;
     unsigned long long *sc = ptr<unsigned long long>(ws.scalars);
     const ScanCtl c{ptr<unsigned long long>(ws.scan_status), sc + S_SCAN, ws.scan_tickets,

@@ -14,6 +14,8 @@ extern "C" dyg_status dyg_testing_stall_barrier(dyg_graph *g, uint32_t spin_limi
     return DYG_OK;
 }
 
+extern "C" void dyg_testing_fail_allocations(uint32_t pass, uint32_t fail) { fail_allocations(pass, fail); }
+
 extern "C" dyg_status dyg_testing_stall_scan(dyg_graph *g) {
     g->ws.scan_tickets -= 1;
     return DYG_OK;

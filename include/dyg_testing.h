@@ -19,6 +19,11 @@ dyg_status dyg_testing_stall_barrier(dyg_graph *g, uint32_t spin_limit);
  * the others wait for it until their limit. */
 dyg_status dyg_testing_stall_scan(dyg_graph *g);
 
+/* Device memory runs short on this host thread: its next `pass` allocations
+ * succeed, the `fail` after them do not (an allocation that must not fail is
+ * tried twice).  (0, 0) ends it. */
+void dyg_testing_fail_allocations(uint32_t pass, uint32_t fail);
+
 #ifdef __cplusplus
 }
 #endif
