@@ -191,7 +191,8 @@ struct Workspace {
     Buf found;                                // u8 per half-edge
     Buf path_v, path_s;                       // replayed winner paths: vertices, taken slots
     Buf path_len;                             // i32 per filtered edge
-    Buf rec_head, rec_words;                  // path records of the walks
+    Buf rec_head;                             // path records of the walks: last of each edge
+    uint64_t rec_words = 0;                   // words they took in an earlier call that ran short
     Buf cand_x, cand_y, cand_w;               // recovery candidates
     Buf keep;                                 // u32 per candidate
     Buf htab_k, htab_v;                       // dedup hash table
@@ -211,7 +212,6 @@ struct Workspace {
     Buf st_wapp;                              // stream file: G weight of each new edge
     Buf big;                                  // stream file: uint4 per long-row search
     Buf s_uid;                                // staged per-edge update ids
-    Buf ix_base, ix_list, ix_words;           // row index of the weighted walks
     Buf scalars;                              // u64 scalars (see Scalar)
     Buf counts;                               // u32 counts (see Count), behind the scalars
     unsigned long long *host_scalars = nullptr;   // pinned mirror of scalars and counts
@@ -316,12 +316,14 @@ dyg_status cuda_fail(cudaError_t e, const char *what, const char *file, int line
 // finished with the block (or the caller has synchronized it).
 cudaError_t dev_alloc(void **out, size_t bytes);
 void dev_free(void *p);
-// Scratch for one call: the device's kept block if it is free and large enough,
-// else a new one; returned once the device has finished with it (one block of
-// at most 256 MB per device is kept).
+// Scratch that a call can do without: a kept block of the device if one is free
+// and large enough, else a new one; returned once the device has finished with
+// it (at most 256 MB per device are kept).  scratch_drop frees what is kept;
+// an allocation that does not fit otherwise does so first.
 struct Buf;
 cudaError_t scratch_borrow(Buf *b, size_t bytes);
 void scratch_return(Buf *b);
+void scratch_drop();
 // For tests: this thread's next `pass` allocations go through, the `fail` after
 // them do not.
 void fail_allocations(uint32_t pass, uint32_t fail);
@@ -386,8 +388,9 @@ dyg_status launch_walk_scalars(const DevGraph &g, const WalkJob &job, const dyg_
 // The row index for weighted walks on G as it is now; empty for a uniform
 // transition or a graph without hub rows.  The walks that use it test the same
 // halt word: an index whose launch was cut short must not be read.
+struct WalkScratch;
 dyg_status index_enqueue(dyg_graph *G, const dyg_walk_params &p, unsigned long long *halt,
-                         RowIndex *out, cudaStream_t st);
+                         WalkScratch &scratch, RowIndex *out, cudaStream_t st);
 dyg_status launch_winner_paths(dyg_graph *G, const WalkJob &job, const dyg_walk_params &p,
                                const unsigned long long *keys, uint32_t n_max, uint32_t path_stride,
                                uint32_t *path_v, uint32_t *path_s, int32_t *path_len, const RowIndex &ix,
@@ -431,6 +434,11 @@ dyg_status decremental_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, cons
                            const std::function<void()> *during = nullptr,
                            const std::function<dyg_status()> *fetch = nullptr);
 
+struct WalkScratch;
+// The buffers that the deletion stage of n edges and the walks and recoveries
+// of n walked ones cannot do without.
+dyg_status decr_delete_ensure(dyg_graph *G, dyg_graph *H, uint32_t n, cudaStream_t st);
+dyg_status decr_walk_ensure(dyg_graph *G, dyg_graph *H, uint32_t n, const dyg_walk_params &p, cudaStream_t st);
 dyg_status decr_delete_enqueue(dyg_graph *G, dyg_graph *H, const uint32_t *src,
                                const uint32_t *dst, uint32_t n, uint64_t uid0,
                                const unsigned long long *uids, bool file_orient,
@@ -443,11 +451,9 @@ dyg_status decr_walk_enqueue(dyg_graph *G, dyg_graph *H, uint32_t f0, uint32_t n
                              const uint32_t *F_dev, const dyg_walk_params &p,
                              unsigned long long *halt, uint32_t batch, uint32_t phase0,
                              int32_t *status, float *cond, cudaStream_t st, bool walk_ready,
-                             PathRec *rec, const unsigned long long *keys_given = nullptr);
-// The walks' path records for calls of up to n walked deletions; left empty
-// (rec->heads null: winners are replayed) for walks longer than
-// kPathSteps, for more than kPathWalkers uniform ones, or when memory is short.
-// Borrowed for one call.  Replays last as long as one longest path whatever the
+                             WalkScratch &scratch, const unsigned long long *keys_given = nullptr);
+// Path records are kept for walks of up to kPathSteps steps and for up to
+// kPathWalkers uniform ones.  Replays last as long as one longest path whatever the
 // batch; keeping paths costs the uniform walk nothing while it is bound by the
 // latency of its longest walks, and a sixth of its time once it is bound by
 // throughput: 1,013 deletions of a 37 x 41 x 29 mesh (160 walkers) take 57 us
@@ -456,14 +462,35 @@ dyg_status decr_walk_enqueue(dyg_graph *G, dyg_graph *H, uint32_t f0, uint32_t n
 // much that keeping its slot is nothing.
 constexpr uint32_t kPathSteps = 256;
 constexpr uint64_t kPathWalkers = 2u << 20;
-struct PathScratch {
-    PathRec rec{};
-    Buf hist;
-    cudaStream_t st = nullptr;
-    dyg_status open(dyg_graph *G, uint32_t n, const dyg_walk_params &p, cudaStream_t stream);
+// What the walks of one call borrow and can do without: path records (else
+// winners are replayed) and the row index (else the warp searches the rows).
+// Asked for after what the call needs; given back when the call ends, or
+// earlier if something that it needs does not fit otherwise.
+struct WalkScratch {
+    cudaStream_t st;
+    PathRec rec{};      // heads null: replay
+    Buf hist, words;
+    Buf index;
+    bool index_tried = false;
+    explicit WalkScratch(cudaStream_t stream) : st(stream) {}
+    WalkScratch(const WalkScratch &) = delete;
+    WalkScratch &operator=(const WalkScratch &) = delete;
+    ~WalkScratch() { release(); }
+    // Records for calls of up to n walked deletions.
+    void open_paths(dyg_graph *G, uint32_t n, const dyg_walk_params &p);
     // After a kHaltPaths halt (scalars just read): room for what was asked for.
-    dyg_status grow(dyg_graph *G);
-    ~PathScratch();
+    void grow_paths(dyg_graph *G);
+    // Waits for the stream and gives everything back; false: there was nothing.
+    bool release();
+    // Runs f, and once more without the scratch if memory was short.
+    template <class F>
+    dyg_status with_room(F f) {
+        dyg_status rc = f();
+        if (rc != DYG_ENOMEM || !release()) return rc;
+        scratch_drop();
+        set_error("");
+        return f();
+    }
 };
 // The commit reads keys; clear_keys zeroes them behind it for the next walk.
 dyg_status incr_commit_enqueue(dyg_graph *H, dyg_graph *G, const uint32_t *src,

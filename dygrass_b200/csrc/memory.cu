@@ -117,6 +117,7 @@ cudaError_t alloc_once(const DevicePool &p, void **out, size_t bytes) {
 }  // namespace
 
 void fail_allocations(uint32_t pass, uint32_t fail) {
+    scratch_drop();   // what is kept would be handed out without an allocation
     t_pass = pass;
     t_fail = fail;
 }
@@ -124,11 +125,14 @@ void fail_allocations(uint32_t pass, uint32_t fail) {
 cudaError_t dev_alloc(void **out, size_t bytes) {
     const DevicePool p = current_pool();
     cudaError_t e = alloc_once(p, out, bytes);
-    if (e == cudaErrorMemoryAllocation && p.pool) {
-        // what the pool holds in other sizes goes back first
+    if (e == cudaErrorMemoryAllocation) {
+        // the kept scratch and what the pool holds in other sizes go back first
         cudaGetLastError();
-        cudaStreamSynchronize(p.st);
-        cudaMemPoolTrimTo(p.pool, 0);
+        scratch_drop();
+        if (p.pool) {
+            cudaStreamSynchronize(p.st);
+            cudaMemPoolTrimTo(p.pool, 0);
+        }
         e = alloc_once(p, out, bytes);
     }
     return e;
@@ -145,53 +149,98 @@ void dev_free(void *ptr) {
 }
 
 namespace {
-// One scratch block per device, kept between the calls that borrow it.
+// Scratch blocks of each device, kept between the calls that borrow them.
 struct Scratch {
-    void *p = nullptr;
-    size_t bytes = 0;
+    std::vector<Buf> blocks;
+    size_t total = 0;
     unsigned long long ctx = 0;
 };
 std::mutex g_scratch_mu;
 Scratch g_scratch[kMaxDevices];
+
+// The current device's, as of its present context (g_scratch_mu held).
+Scratch *current_scratch() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
+    const unsigned long long ctx = current_context_id();
+    if (!ctx) return nullptr;
+    Scratch &s = g_scratch[dev];
+    if (s.ctx != ctx) {   // the blocks went with their context
+        s = Scratch{};
+        s.ctx = ctx;
+    }
+    return &s;
+}
+
+Buf take_scratch(Scratch &s, size_t i) {
+    const Buf b = s.blocks[i];
+    s.total -= b.bytes;
+    s.blocks[i] = s.blocks.back();
+    s.blocks.pop_back();
+    return b;
+}
 }  // namespace
 
-cudaError_t scratch_borrow(Buf *b, size_t bytes) {
-    int dev = 0;
-    *b = Buf{};
-    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices) {
-        const unsigned long long ctx = current_context_id();
+void scratch_drop() {
+    std::vector<Buf> drop;
+    {
         std::lock_guard<std::mutex> lk(g_scratch_mu);
-        Scratch &s = g_scratch[dev];
-        if (s.p && s.ctx != ctx) s = Scratch{};   // went with its context
-        if (s.p && s.bytes >= bytes) {
-            b->p = s.p;
-            b->bytes = s.bytes;
-            s = Scratch{};
+        Scratch *s = current_scratch();
+        if (!s) return;
+        drop.swap(s->blocks);
+        s->total = 0;
+    }
+    for (Buf &b : drop) dev_free(b.p);
+}
+
+cudaError_t scratch_borrow(Buf *b, size_t bytes) {
+    *b = Buf{};
+    {
+        std::lock_guard<std::mutex> lk(g_scratch_mu);
+        Scratch *s = current_scratch();
+        size_t best = s ? s->blocks.size() : 0;   // the smallest that is large enough
+        for (size_t i = 0; s && i < s->blocks.size(); ++i)
+            if (s->blocks[i].bytes >= bytes && (best == s->blocks.size() || s->blocks[i].bytes < s->blocks[best].bytes))
+                best = i;
+        if (s && best < s->blocks.size()) {
+            *b = take_scratch(*s, best);
             return cudaSuccess;
         }
     }
-    const cudaError_t e = dev_alloc(&b->p, bytes);
-    b->bytes = e == cudaSuccess ? bytes : 0;
+    const size_t want = (bytes + bytes / 8 + 0xFFFF) & ~(size_t)0xFFFF;
+    const DevicePool p = current_pool();
+    cudaError_t e = alloc_once(p, &b->p, want);
+    if (e == cudaErrorMemoryAllocation) {
+        // the kept blocks, all too small, go first; the pool stays as it is:
+        // the caller can do without
+        cudaGetLastError();
+        scratch_drop();
+        e = alloc_once(p, &b->p, want);
+    }
+    b->bytes = e == cudaSuccess ? want : 0;
     return e;
 }
 
 void scratch_return(Buf *b) {
     if (!b->p) return;
-    int dev = 0;
-    Buf drop = *b;
-    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices && b->bytes <= kScratchKeep) {
-        const unsigned long long ctx = current_context_id();
+    std::vector<Buf> drop{*b};
+    *b = Buf{};
+    {
         std::lock_guard<std::mutex> lk(g_scratch_mu);
-        Scratch &s = g_scratch[dev];
-        if (ctx && (!s.p || s.ctx != ctx || s.bytes < b->bytes)) {
-            drop = s.p && s.ctx == ctx ? Buf{s.p, s.bytes} : Buf{};
-            s.p = b->p;
-            s.bytes = b->bytes;
-            s.ctx = ctx;
+        Scratch *s = current_scratch();
+        if (s && drop[0].bytes <= kScratchKeep) {
+            s->blocks.push_back(drop[0]);
+            s->total += drop[0].bytes;
+            drop.clear();
+            while (s->total > kScratchKeep) {   // the smallest go: any borrower can use the larger
+                size_t k = 0;
+                for (size_t i = 1; i < s->blocks.size(); ++i)
+                    if (s->blocks[i].bytes < s->blocks[k].bytes) k = i;
+                drop.push_back(take_scratch(*s, k));
+            }
         }
     }
-    dev_free(drop.p);
-    *b = Buf{};
+    for (Buf &d : drop) dev_free(d.p);
 }
 
 namespace {

@@ -108,7 +108,7 @@ struct DeleteArgs {
     uint32_t *f_src, *f_dst, *f_idx;
     unsigned long long *f_uid;
     unsigned long long *keys, *work;   // zeroed for the walks
-    uint32_t *rec_head;                // as well (may be null)
+    uint32_t *rec_head;                // as well
     uint32_t *blk, *counts;
     unsigned long long *err;
     const unsigned long long *halt;
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(kOpThreads, 2) k_delete(const __grid_constant_
         reinterpret_cast<uint16_t *>(a.fG)[e] = 0;
         reinterpret_cast<uint16_t *>(a.fH)[e] = 0;
         a.keys[e] = 0ull;
-        if (a.rec_head) a.rec_head[e] = 0u;
+        a.rec_head[e] = 0u;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) *a.work = 0ull;
     if (!grid_sync(bar, [&] { *a.D.c.items = *a.D.items_h = 0ull; })) return;
@@ -574,14 +574,29 @@ static dyg_status incr_enqueue(dyg_graph *H, dyg_graph *G, const uint32_t *src, 
                                const float *w, uint32_t n, uint64_t uid0,
                                const unsigned long long *uids, const dyg_walk_params &p,
                                unsigned long long *halt, uint32_t batch, int32_t *found, float *cond,
-                               uint8_t *acc, cudaStream_t st, bool walk_ready) {
+                               uint8_t *acc, cudaStream_t st, bool walk_ready, WalkScratch &scratch) {
     unsigned long long *keys = ptr<unsigned long long>(H->ws.keys);
     if (!walk_ready) DYG_CUDA(cudaMemsetAsync(keys, 0, sizeof(unsigned long long) * n, st));
     WalkJob job{halt, src, dst, w, uids, (unsigned long long)uid0, nullptr, n, kDomainIncr, 0u};
     RowIndex ix{};
-    DYG_TRY(index_enqueue(H, p, halt, &ix, st));
+    DYG_TRY(index_enqueue(H, p, halt, scratch, &ix, st));
     DYG_TRY(launch_walk(H, job, p, true, keys, ix, st, walk_ready));
     return incr_commit_enqueue(H, G, src, dst, w, n, keys, true, halt, batch, found, cond, acc, st);
+}
+
+dyg_status decr_delete_ensure(dyg_graph *G, dyg_graph *H, uint32_t n, cudaStream_t st) {
+    Workspace &ws = G->ws;
+    const uint64_t m = 2ull * n;
+    DYG_TRY(rowops_ensure(G, m, st));
+    DYG_TRY(rowops_ensure(H, m, st));
+    DYG_TRY(ensure(ws.dtmp, sizeof(uint32_t) * (size_t)m * 2));
+    DYG_TRY(ensure(ws.found, (size_t)m * 2));
+    DYG_TRY(ensure(ws.keys, sizeof(unsigned long long) * n));
+    DYG_TRY(ensure(ws.f_src, sizeof(uint32_t) * n));
+    DYG_TRY(ensure(ws.f_dst, sizeof(uint32_t) * n));
+    DYG_TRY(ensure(ws.f_idx, sizeof(uint32_t) * n));
+    DYG_TRY(ensure(ws.f_uid, sizeof(unsigned long long) * n));
+    return ensure(ws.rec_head, sizeof(uint32_t) * n);
 }
 
 // Deletion stage of a decremental batch: delete every edge from G (swap with
@@ -597,15 +612,7 @@ dyg_status decr_delete_enqueue(dyg_graph *G, dyg_graph *H, const uint32_t *src,
                                cudaStream_t st) {
     Workspace &ws = G->ws;
     const uint64_t m = 2ull * n;
-    DYG_TRY(rowops_ensure(G, m, st));
-    DYG_TRY(rowops_ensure(H, m, st));
-    DYG_TRY(ensure(ws.dtmp, sizeof(uint32_t) * (size_t)m * 2));
-    DYG_TRY(ensure(ws.found, (size_t)m * 2));
-    DYG_TRY(ensure(ws.keys, sizeof(unsigned long long) * n));
-    DYG_TRY(ensure(ws.f_src, sizeof(uint32_t) * n));
-    DYG_TRY(ensure(ws.f_dst, sizeof(uint32_t) * n));
-    DYG_TRY(ensure(ws.f_idx, sizeof(uint32_t) * n));
-    DYG_TRY(ensure(ws.f_uid, sizeof(unsigned long long) * n));
+    DYG_TRY(decr_delete_ensure(G, H, n, st));
     unsigned long long *sc = ptr<unsigned long long>(ws.scalars);
     DeleteArgs a{};
     a.G = G->g;
@@ -626,7 +633,7 @@ dyg_status decr_delete_enqueue(dyg_graph *G, dyg_graph *H, const uint32_t *src,
     a.f_uid = ptr<unsigned long long>(ws.f_uid);
     a.keys = ptr<unsigned long long>(ws.keys);
     a.work = sc + S_WORK;
-    a.rec_head = ws.rec_head.bytes >= sizeof(uint32_t) * (size_t)n ? ptr<uint32_t>(ws.rec_head) : nullptr;
+    a.rec_head = ptr<uint32_t>(ws.rec_head);
     a.blk = ptr<uint32_t>(ws.blk);
     a.counts = ptr<uint32_t>(ws.counts);
     a.err = sc + S_ERR;
@@ -634,71 +641,59 @@ dyg_status decr_delete_enqueue(dyg_graph *G, dyg_graph *H, const uint32_t *src,
     return launch_phases<k_delete>(op_blocks(m, G->long_rows || H->long_rows), st, grid_bar(G, halt), a);
 }
 
-dyg_status PathScratch::open(dyg_graph *G, uint32_t n, const dyg_walk_params &p, cudaStream_t stream) {
-    st = stream;
-    if (p.max_steps > kPathSteps || n == 0) return DYG_OK;
-    if (p.transition == DYG_TRANSITION_UNIFORM && (uint64_t)n * p.walkers > kPathWalkers) return DYG_OK;
+void WalkScratch::open_paths(dyg_graph *G, uint32_t n, const dyg_walk_params &p) {
+    if (p.max_steps > kPathSteps || n == 0) return;
+    if (p.transition == DYG_TRANSITION_UNIFORM && (uint64_t)n * p.walkers > kPathWalkers) return;
     Workspace &ws = G->ws;
     const uint32_t threads = walk_threads(n, p);
     const size_t hist_bytes = sizeof(uint32_t) * (size_t)threads * ((p.max_steps + 3u) & ~3u);
     // some paths of a few moves per edge to begin with
-    const size_t words = sizeof(uint32_t) * ((size_t)n * 48u + 4096u);
-    if (scratch_borrow(&hist, hist_bytes) != cudaSuccess) {
+    uint64_t want = (uint64_t)n * 48u + 4096u;
+    if (want < ws.rec_words) want = ws.rec_words;
+    if (scratch_borrow(&hist, hist_bytes) != cudaSuccess ||
+        scratch_borrow(&words, sizeof(uint32_t) * want) != cudaSuccess) {
         cudaGetLastError();
-        return DYG_OK;
+        scratch_return(&hist);   // nothing has used it
+        return;
     }
-    if (ensure(ws.rec_head, sizeof(uint32_t) * (size_t)n) != DYG_OK || ensure(ws.rec_words, words) != DYG_OK)
-        return DYG_OK;
+    const uint64_t room = words.bytes / sizeof(uint32_t);
     rec.heads = ptr<uint32_t>(ws.rec_head);
-    rec.words = ptr<uint32_t>(ws.rec_words);
-    rec.cap = (uint32_t)(ws.rec_words.bytes / sizeof(uint32_t) > 0xFFFFFF00u ? 0xFFFFFF00u
-                                                                             : ws.rec_words.bytes / sizeof(uint32_t));
+    rec.words = ptr<uint32_t>(words);
+    rec.cap = (uint32_t)(room > 0xFFFFFF00u ? 0xFFFFFF00u : room);
     rec.cursor = ptr<unsigned long long>(ws.scalars) + S_RECW;
     rec.hist = ptr<uint32_t>(hist);
     rec.threads = threads;
-    return DYG_OK;
 }
 
-dyg_status PathScratch::grow(dyg_graph *G) {
+void WalkScratch::grow_paths(dyg_graph *G) {
     const unsigned long long need = G->ws.host_scalars[S_RECNEED] + G->ws.host_scalars[S_RECNEED] / 4;
-    if (need > 0xFFFFFF00ull || ensure(G->ws.rec_words, sizeof(uint32_t) * need) != DYG_OK) {
+    scratch_return(&words);   // the stream was waited for
+    if (need > 0xFFFFFF00ull || scratch_borrow(&words, sizeof(uint32_t) * need) != cudaSuccess) {
+        cudaGetLastError();
         rec = PathRec{};   // replay the winners instead
-        return DYG_OK;
+        return;
     }
-    rec.words = ptr<uint32_t>(G->ws.rec_words);
+    G->ws.rec_words = need;
+    rec.words = ptr<uint32_t>(words);
     rec.cap = (uint32_t)need;
-    return DYG_OK;
 }
 
-PathScratch::~PathScratch() {
-    if (!hist.p) return;
+bool WalkScratch::release() {
+    if (!hist.p && !words.p && !index.p) return false;
     cudaStreamSynchronize(st);
-    scratch_return(&hist);
+    for (Buf *b : {&hist, &words, &index}) scratch_return(b);
+    rec = PathRec{};
+    return true;
 }
 
-// Walk-and-recover stage over walk-list entries [f0, f0 + nf) (nf a host
-// bound; F_dev, if given, is the device count of the whole list), from phase
-// `phase0` (0 = walks, 1 = recovery, 2 = walks repeated with more room for
-// their paths: the deletions are done).
-dyg_status decr_walk_enqueue(dyg_graph *G, dyg_graph *H, uint32_t f0, uint32_t nf,
-                             const uint32_t *F_dev, const dyg_walk_params &p,
-                             unsigned long long *halt, uint32_t batch, uint32_t phase0,
-                             int32_t *status, float *cond, cudaStream_t st, bool walk_ready,
-                             PathRec *rec, const unsigned long long *keys_given) {
-    if (nf == 0) return DYG_OK;
+static uint32_t path_stride(const dyg_walk_params &p) { return p.max_steps > 2 ? p.max_steps : 2; }
+
+dyg_status decr_walk_ensure(dyg_graph *G, dyg_graph *H, uint32_t n, const dyg_walk_params &p, cudaStream_t st) {
     Workspace &ws = G->ws;
-    const uint32_t n = nf;
-    const uint32_t stride = p.max_steps > 2 ? p.max_steps : 2;
-    const uint32_t hwk = p.heuristic_walkers;
     DYG_TRY(ensure(ws.keys, sizeof(unsigned long long) * n));
-    const bool replay = keys_given || !rec || !rec->heads;
-    if (replay) {
-        DYG_TRY(ensure(ws.path_v, sizeof(uint32_t) * (size_t)n * stride));
-        DYG_TRY(ensure(ws.path_s, sizeof(uint32_t) * (size_t)n * stride));
-        DYG_TRY(ensure(ws.path_len, sizeof(int32_t) * n));
-    }
     // path candidates at [0, C_CANDS), then the fallback candidates
-    const size_t n_path = (size_t)n * (stride - 1u), n_fb = (size_t)n * 4u * hwk, M = n_path + n_fb;
+    const size_t n_path = (size_t)n * (path_stride(p) - 1u), n_fb = (size_t)n * 4u * p.heuristic_walkers,
+                 M = n_path + n_fb;
     DYG_TRY(ensure(ws.cand_x, sizeof(uint32_t) * M));
     DYG_TRY(ensure(ws.cand_y, sizeof(uint32_t) * M));
     DYG_TRY(ensure(ws.cand_w, sizeof(float) * M));
@@ -713,7 +708,30 @@ dyg_status decr_walk_enqueue(dyg_graph *G, dyg_graph *H, uint32_t f0, uint32_t n
         DYG_CUDA(cudaMemsetAsync(ws.htab_v.p, 0xFF, ws.htab_v.bytes, st));
     }
     DYG_TRY(rowops_ensure(G, 1, st));
-    DYG_TRY(rowops_ensure(H, 2ull * M, st));
+    return rowops_ensure(H, 2ull * M, st);
+}
+
+// Walk-and-recover stage over walk-list entries [f0, f0 + nf) (nf a host
+// bound; F_dev, if given, is the device count of the whole list), from phase
+// `phase0` (0 = walks, 1 = recovery, 2 = walks repeated with more room for
+// their paths: the deletions are done).
+dyg_status decr_walk_enqueue(dyg_graph *G, dyg_graph *H, uint32_t f0, uint32_t nf,
+                             const uint32_t *F_dev, const dyg_walk_params &p,
+                             unsigned long long *halt, uint32_t batch, uint32_t phase0,
+                             int32_t *status, float *cond, cudaStream_t st, bool walk_ready,
+                             WalkScratch &scratch, const unsigned long long *keys_given) {
+    if (nf == 0) return DYG_OK;
+    Workspace &ws = G->ws;
+    const uint32_t n = nf;
+    const uint32_t stride = path_stride(p);
+    const uint32_t hwk = p.heuristic_walkers;
+    DYG_TRY(decr_walk_ensure(G, H, n, p, st));
+    const bool replay = keys_given || !scratch.rec.heads;
+    if (replay) {
+        DYG_TRY(ensure(ws.path_v, sizeof(uint32_t) * (size_t)n * stride));
+        DYG_TRY(ensure(ws.path_s, sizeof(uint32_t) * (size_t)n * stride));
+        DYG_TRY(ensure(ws.path_len, sizeof(int32_t) * n));
+    }
     unsigned long long *sc = ptr<unsigned long long>(ws.scalars);
     WalkJob job{halt, ptr<uint32_t>(ws.f_src) + f0, ptr<uint32_t>(ws.f_dst) + f0, nullptr,
                 ptr<unsigned long long>(ws.f_uid) + f0, 0ull, F_dev, n, kDomainDecr, f0};
@@ -727,7 +745,7 @@ dyg_status decr_walk_enqueue(dyg_graph *G, dyg_graph *H, uint32_t f0, uint32_t n
     a.resume = phase0 == 1;
     a.keys = keys_given ? const_cast<unsigned long long *>(keys_given) : own;
     a.clear_keys = !keys_given;
-    if (!replay) a.rec = *rec;
+    if (!replay) a.rec = scratch.rec;
     a.plen = ptr<int32_t>(ws.path_len);
     a.pv = ptr<uint32_t>(ws.path_v);
     a.ps = ptr<uint32_t>(ws.path_s);
@@ -756,10 +774,10 @@ dyg_status decr_walk_enqueue(dyg_graph *G, dyg_graph *H, uint32_t f0, uint32_t n
     if (phase0 != 1) {
         // walks on the updated G (main.cu:392, 420)
         RowIndex ix{};   // of the walks, and of the replays of their winners
-        DYG_TRY(index_enqueue(G, p, halt, &ix, st));
+        DYG_TRY(index_enqueue(G, p, halt, scratch, &ix, st));
         if (!keys_given) {
             if (!walk_ready) DYG_CUDA(cudaMemsetAsync(own, 0, sizeof(unsigned long long) * n, st));
-            DYG_TRY(launch_walk(G, job, p, false, own, ix, st, walk_ready, replay ? nullptr : rec));
+            DYG_TRY(launch_walk(G, job, p, false, own, ix, st, walk_ready, replay ? nullptr : &scratch.rec));
         }
         if (replay)
             DYG_TRY(launch_winner_paths(G, job, p, a.keys, n, stride, ptr<uint32_t>(ws.path_v),
@@ -773,13 +791,13 @@ dyg_status decr_walk_enqueue(dyg_graph *G, dyg_graph *H, uint32_t f0, uint32_t n
 // walks over the batch's whole walk list.
 static dyg_status decr_enqueue(dyg_graph *G, dyg_graph *H, const uint32_t *src, const uint32_t *dst,
                                uint32_t n, uint64_t uid0, const unsigned long long *uids,
-                               const dyg_walk_params &p, PathRec *rec,
+                               const dyg_walk_params &p, WalkScratch &scratch,
                                unsigned long long *halt, uint32_t batch, uint32_t phase0,
                                int32_t *status, float *cond, cudaStream_t st) {
     if (phase0 == 0)
         DYG_TRY(decr_delete_enqueue(G, H, src, dst, n, uid0, uids, false, halt, status, cond, st));
     return decr_walk_enqueue(G, H, 0, n, ptr<uint32_t>(G->ws.counts) + C_FILTERED, p, halt, batch,
-                             phase0, status, cond, st, true, rec);
+                             phase0, status, cond, st, true, scratch);
 }
 
 // --------------------------------------------------------- stream drivers
@@ -800,12 +818,6 @@ dyg_status clear_halt(dyg_graph *D, cudaStream_t st) {
     return DYG_OK;
 }
 
-dyg_status grow_for_halt(dyg_graph *A, dyg_graph *B, cudaStream_t st) {
-    DYG_TRY(grow_arena(A, A->g.arena_cap * 2, st));
-    if (B) DYG_TRY(grow_arena(B, B->g.arena_cap * 2, st));
-    return DYG_OK;
-}
-
 }  // namespace
 
 dyg_status incremental_run(dyg_graph *H, dyg_graph *G, const uint32_t *src, const uint32_t *dst,
@@ -821,7 +833,11 @@ dyg_status incremental_run(dyg_graph *H, dyg_graph *G, const uint32_t *src, cons
     if (check_inputs) DYG_TRY(validate_enqueue(halt, sc + S_ERR, src, dst, w, n, H->g.n, st));
     // no batch is larger than the first, so the keys it clears are clear for
     // the later ones
-    DYG_TRY(ensure(H->ws.keys, sizeof(unsigned long long) * (B < n ? B : n)));
+    const uint32_t b_max = B < n ? B : n;
+    DYG_TRY(ensure(H->ws.keys, sizeof(unsigned long long) * b_max));
+    DYG_TRY(rowops_ensure(H, 2ull * b_max, st));
+    if (G) DYG_TRY(rowops_ensure(G, 2ull * b_max, st));
+    WalkScratch scratch(st);
     uint32_t b_start = 0;
     for (int round = 0; round < 64; ++round) {
         for (uint32_t b = b_start; (uint64_t)b * B < n; ++b) {
@@ -829,7 +845,7 @@ dyg_status incremental_run(dyg_graph *H, dyg_graph *G, const uint32_t *src, cons
             DYG_TRY(incr_enqueue(H, G, src + b0, dst + b0, w + b0, nb, uid_base + b0,
                                  uids ? uids + b0 : nullptr, p, halt, b,
                                  found ? found + b0 : nullptr, cond ? cond + b0 : nullptr,
-                                 acc ? acc + b0 : nullptr, st, b > b_start));
+                                 acc ? acc + b0 : nullptr, st, b > b_start, scratch));
         }
         if (during && round == 0) (*during)();
         if (fetch) DYG_TRY((*fetch)());
@@ -838,7 +854,8 @@ dyg_status incremental_run(dyg_graph *H, dyg_graph *G, const uint32_t *src, cons
         if (!h) return DYG_OK;
         const HaltInfo hi = decode_halt(h);
         if (hi.kind == kHaltInvalid) return rejected_inputs(H, st);
-        DYG_TRY(grow_for_halt(H, G, st));
+        for (dyg_graph *X : {H, G})
+            if (X) DYG_TRY(scratch.with_room([&] { return grow_arena(X, X->g.arena_cap * 2, st); }));
         DYG_TRY(clear_halt(H, st));
         b_start = hi.batch;   // nothing of the halted batch changed: redo it whole
     }
@@ -868,14 +885,17 @@ dyg_status decremental_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, cons
     DYG_CUDA(cudaMemcpyAsync(sc + S_RECCNT, init, sizeof(init), cudaMemcpyHostToDevice, st));
     DYG_TRY(clear_halt(G, st));
     if (check_inputs) DYG_TRY(validate_enqueue(halt, sc + S_ERR, src, dst, nullptr, n, G->g.n, st));
-    PathScratch paths;
-    DYG_TRY(paths.open(G, B < n ? B : n, p, st));
+    const uint32_t b_max = B < n ? B : n;
+    DYG_TRY(decr_delete_ensure(G, H, b_max, st));
+    DYG_TRY(decr_walk_ensure(G, H, b_max, p, st));
+    WalkScratch scratch(st);
+    scratch.open_paths(G, b_max, p);
     uint32_t b_start = 0, ph_start = 0;
     for (int round = 0; round < 64; ++round) {
         for (uint32_t b = b_start; (uint64_t)b * B < n; ++b) {
             const uint32_t b0 = b * B, nb = (n - b0 < B) ? n - b0 : B;
             DYG_TRY(decr_enqueue(G, H, src + b0, dst + b0, nb, uid_base + b0,
-                                 uids ? uids + b0 : nullptr, p, &paths.rec, halt, b,
+                                 uids ? uids + b0 : nullptr, p, scratch, halt, b,
                                  b == b_start ? ph_start : 0, status + b0, cond + b0, st));
         }
         if (during && round == 0) (*during)();
@@ -891,16 +911,18 @@ dyg_status decremental_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, cons
         if (hi.kind == kHaltRecords) {
             const uint64_t used = ws.host_scalars[S_RECCNT];
             const uint64_t ncap = cap * 2;
-            DYG_TRY(grow_keep(ws.rx2, sizeof(uint32_t) * ncap, sizeof(uint32_t) * used, st));
-            DYG_TRY(grow_keep(ws.ry2, sizeof(uint32_t) * ncap, sizeof(uint32_t) * used, st));
-            DYG_TRY(grow_keep(ws.rk2, ncap, used, st));
+            DYG_TRY(scratch.with_room([&] {
+                DYG_TRY(grow_keep(ws.rx2, sizeof(uint32_t) * ncap, sizeof(uint32_t) * used, st));
+                DYG_TRY(grow_keep(ws.ry2, sizeof(uint32_t) * ncap, sizeof(uint32_t) * used, st));
+                return grow_keep(ws.rk2, ncap, used, st);
+            }));
             cap = ncap;
             DYG_CUDA(cudaMemcpyAsync(sc + S_RECCAP, &cap, sizeof(cap), cudaMemcpyHostToDevice, st));
             DYG_CUDA(cudaStreamSynchronize(st));
         } else if (hi.kind == kHaltPaths) {
-            DYG_TRY(paths.grow(G));
+            scratch.grow_paths(G);
         } else {
-            DYG_TRY(grow_arena(H, H->g.arena_cap * 2, st));
+            DYG_TRY(scratch.with_room([&] { return grow_arena(H, H->g.arena_cap * 2, st); }));
         }
         DYG_TRY(clear_halt(G, st));
         b_start = hi.batch;

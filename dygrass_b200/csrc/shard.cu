@@ -111,7 +111,8 @@ dyg_status dyg_walk_keys(dyg_graph *X, const uint32_t *src, const uint32_t *dst,
                 (unsigned long long)(first_update_id + lo), nullptr, hi - lo,
                 incremental ? kDomainIncr : kDomainDecr};
     RowIndex ix{};
-    DYG_TRY(index_enqueue(X, *p, sc + S_HALT, &ix, st));
+    WalkScratch scratch(st);
+    DYG_TRY(index_enqueue(X, *p, sc + S_HALT, scratch, &ix, st));
     DYG_TRY(launch_walk(X, job, *p, incremental != 0, k, ix, st));
     DYG_TRY(read_scalars(X, st));
     if (ws.host_scalars[S_HALT]) return rejected_inputs(X, st);
@@ -253,7 +254,8 @@ dyg_status dyg_decremental_walk_keys(dyg_graph *G, uint32_t lo, uint32_t hi,
     WalkJob job{halt, ptr<uint32_t>(ws.f_src) + lo, ptr<uint32_t>(ws.f_dst) + lo, nullptr,
                 ptr<unsigned long long>(ws.f_uid) + lo, 0ull, nullptr, hi - lo, kDomainDecr};
     RowIndex ix{};
-    DYG_TRY(index_enqueue(G, *p, halt, &ix, st));
+    WalkScratch scratch(st);
+    DYG_TRY(index_enqueue(G, *p, halt, scratch, &ix, st));
     DYG_TRY(launch_walk(G, job, *p, false, k, ix, st));
     return read_scalars(G, st);
 }
@@ -298,11 +300,12 @@ dyg_status dyg_decremental_commit_keys(dyg_graph *G, dyg_graph *H, const dyg_wal
     uint32_t phase = 0;
     uint64_t total = 0;
     int round = 0;
+    WalkScratch scratch(st);   // the winners are replayed: their walks kept no records
     G->last_rec = 0;
     for (; round < 64; ++round) {
         DYG_TRY(clear_halt_of(G, st));
         DYG_TRY(decr_walk_enqueue(G, H, 0, n_walk, nullptr, *p, halt, 0, phase, status,
-                                  conductance, st, false, nullptr, (const unsigned long long *)keys));
+                                  conductance, st, false, scratch, (const unsigned long long *)keys));
         DYG_TRY(read_scalars2(G, H, st));
         const unsigned long long h = ws.host_scalars[S_HALT];
         if (!h) {
@@ -314,14 +317,16 @@ dyg_status dyg_decremental_commit_keys(dyg_graph *G, dyg_graph *H, const dyg_wal
         if (kind == kHaltRecords) {
             const uint64_t used = ws.host_scalars[S_RECCNT];
             const uint64_t ncap = cap * 2;
-            DYG_TRY(grow_keep(ws.rx2, sizeof(uint32_t) * ncap, sizeof(uint32_t) * used, st));
-            DYG_TRY(grow_keep(ws.ry2, sizeof(uint32_t) * ncap, sizeof(uint32_t) * used, st));
-            DYG_TRY(grow_keep(ws.rk2, ncap, used, st));
+            DYG_TRY(scratch.with_room([&] {
+                DYG_TRY(grow_keep(ws.rx2, sizeof(uint32_t) * ncap, sizeof(uint32_t) * used, st));
+                DYG_TRY(grow_keep(ws.ry2, sizeof(uint32_t) * ncap, sizeof(uint32_t) * used, st));
+                return grow_keep(ws.rk2, ncap, used, st);
+            }));
             cap = ncap;
             DYG_CUDA(cudaMemcpyAsync(sc + S_RECCAP, &cap, sizeof(cap), cudaMemcpyHostToDevice, st));
             DYG_CUDA(cudaStreamSynchronize(st));
         } else {
-            DYG_TRY(grow_arena(H, H->g.arena_cap * 2, st));
+            DYG_TRY(scratch.with_room([&] { return grow_arena(H, H->g.arena_cap * 2, st); }));
         }
     }
     if (round == 64) {

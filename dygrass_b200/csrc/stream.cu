@@ -464,7 +464,8 @@ dyg_status insert_gappend_enqueue(dyg_graph *G, dyg_graph *H, const uint32_t *sr
 // chunk counter zero.
 dyg_status insert_chunk_enqueue(dyg_graph *G, dyg_graph *H, uint32_t c, uint32_t chunk,
                                 uint32_t nc, const dyg_walk_params &p, unsigned long long *halt,
-                                int32_t *status, float *cond, bool walk_ready, cudaStream_t st) {
+                                int32_t *status, float *cond, bool walk_ready, WalkScratch &scratch,
+                                cudaStream_t st) {
     Workspace &wg = G->ws, &wh = H->ws;
     const uint32_t f0 = c * chunk;
     const uint32_t *fsrc = ptr<uint32_t>(wg.f_src) + f0, *fdst = ptr<uint32_t>(wg.f_dst) + f0;
@@ -474,7 +475,7 @@ dyg_status insert_chunk_enqueue(dyg_graph *G, dyg_graph *H, uint32_t c, uint32_t
     const WalkJob job{halt, fsrc, fdst, fw, ptr<unsigned long long>(wg.f_uid) + f0, 0ull,
                       ptr<uint32_t>(wg.counts) + C_WALKLIST, nc, kDomainIncr, f0};
     RowIndex ix{};
-    DYG_TRY(index_enqueue(H, p, halt, &ix, st));
+    DYG_TRY(index_enqueue(H, p, halt, scratch, &ix, st));
     DYG_TRY(launch_walk(H, job, p, true, keys, ix, st, walk_ready));
     const StAcceptOp op{job, keys, ptr<uint32_t>(wg.f_idx) + f0, status, cond};
     return append_enqueue(op, nc, H, EdgeList{fsrc, fdst, fw}, nullptr, EdgeList{},
@@ -516,6 +517,9 @@ dyg_status insert_file_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, cons
     DYG_TRY(ensure(wg.f_uid, sizeof(unsigned long long) * (size_t)n));
     DYG_TRY(ensure(wg.f_idx, sizeof(uint32_t) * (size_t)n));
     DYG_TRY(ensure(wh.keys, sizeof(unsigned long long) * (size_t)nc_max));
+    DYG_TRY(rowops_ensure(G, 2ull * n, st));
+    DYG_TRY(rowops_ensure(H, 2ull * nc_max, st));
+    WalkScratch scratch(st);
     unsigned long long *halt = ptr<unsigned long long>(wg.scalars) + S_HALT;
     DYG_TRY(clear_halt(G, st));
     if (check_inputs)
@@ -530,7 +534,7 @@ dyg_status insert_file_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, cons
         for (uint32_t c = c0; c < nchunks; ++c) {
             const uint32_t f0 = c * chunk;
             const uint32_t nc = n - f0 < chunk ? n - f0 : chunk;
-            DYG_TRY(insert_chunk_enqueue(G, H, c, chunk, nc, p, halt, status, cond, start == 0 || c > c0, st));
+            DYG_TRY(insert_chunk_enqueue(G, H, c, chunk, nc, p, halt, status, cond, start == 0 || c > c0, scratch, st));
         }
         if (fetch) DYG_TRY((*fetch)());
         DYG_TRY(read_scalars2(G, H, st));
@@ -539,7 +543,7 @@ dyg_status insert_file_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, cons
         const HaltInfo hi = decode_halt(h);
         if (hi.kind == kHaltInvalid) return rejected_inputs(G, st);
         dyg_graph *grow = hi.batch == 0 ? G : H;
-        DYG_TRY(grow_arena(grow, grow->g.arena_cap * 2, st));
+        DYG_TRY(scratch.with_room([&] { return grow_arena(grow, grow->g.arena_cap * 2, st); }));
         DYG_TRY(clear_halt(G, st));
         start = hi.batch;
     }
@@ -566,8 +570,10 @@ dyg_status delete_file_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, cons
     DYG_TRY(clear_halt(G, st));
     if (check_inputs)
         DYG_TRY(validate_enqueue(halt, sc + S_ERR, src, dst, nullptr, n, G->g.n, st));
-    PathScratch paths;
-    DYG_TRY(paths.open(G, n, p, st));
+    DYG_TRY(decr_delete_ensure(G, H, n, st));
+    DYG_TRY(decr_walk_ensure(G, H, n < chunk ? n : chunk, p, st));
+    WalkScratch scratch(st);
+    scratch.open_paths(G, n, p);
     DYG_TRY(decr_delete_enqueue(G, H, src, dst, n, uid0, nullptr, true, halt, status, cond, st));
     const uint32_t nchunks = (uint32_t)(((uint64_t)n + chunk - 1) / chunk);
     uint32_t c_start = 0, ph_start = 0;
@@ -576,7 +582,7 @@ dyg_status delete_file_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, cons
             const uint32_t f0 = c * chunk;
             const uint32_t nc = n - f0 < chunk ? n - f0 : chunk;
             DYG_TRY(decr_walk_enqueue(G, H, f0, nc, ptr<uint32_t>(ws.counts) + C_FILTERED, p, halt,
-                                      c, c == c_start ? ph_start : 0, status, cond, st, true, &paths.rec));
+                                      c, c == c_start ? ph_start : 0, status, cond, st, true, scratch));
         }
         if (fetch) DYG_TRY((*fetch)());
         DYG_TRY(read_scalars2(G, H, st));
@@ -590,16 +596,18 @@ dyg_status delete_file_run(dyg_graph *G, dyg_graph *H, const uint32_t *src, cons
         if (hi.kind == kHaltRecords) {
             const uint64_t used = ws.host_scalars[S_RECCNT];
             const uint64_t ncap = cap * 2;
-            DYG_TRY(grow_keep(ws.rx2, sizeof(uint32_t) * ncap, sizeof(uint32_t) * used, st));
-            DYG_TRY(grow_keep(ws.ry2, sizeof(uint32_t) * ncap, sizeof(uint32_t) * used, st));
-            DYG_TRY(grow_keep(ws.rk2, ncap, used, st));
+            DYG_TRY(scratch.with_room([&] {
+                DYG_TRY(grow_keep(ws.rx2, sizeof(uint32_t) * ncap, sizeof(uint32_t) * used, st));
+                DYG_TRY(grow_keep(ws.ry2, sizeof(uint32_t) * ncap, sizeof(uint32_t) * used, st));
+                return grow_keep(ws.rk2, ncap, used, st);
+            }));
             cap = ncap;
             DYG_CUDA(cudaMemcpyAsync(sc + S_RECCAP, &cap, sizeof(cap), cudaMemcpyHostToDevice, st));
             DYG_CUDA(cudaStreamSynchronize(st));
         } else if (hi.kind == kHaltPaths) {
-            DYG_TRY(paths.grow(G));
+            scratch.grow_paths(G);
         } else {
-            DYG_TRY(grow_arena(H, H->g.arena_cap * 2, st));
+            DYG_TRY(scratch.with_room([&] { return grow_arena(H, H->g.arena_cap * 2, st); }));
         }
         DYG_TRY(clear_halt(G, st));
         c_start = hi.batch;

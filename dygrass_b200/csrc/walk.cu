@@ -1181,26 +1181,30 @@ static void launch_walk_any(const WalkArgs &a, bool incremental, bool wtd, cudaS
 constexpr uint64_t kIdxWordsMax = 1ull << 29;
 
 dyg_status index_enqueue(dyg_graph *G, const dyg_walk_params &p, unsigned long long *halt,
-                         RowIndex *out, cudaStream_t st) {
+                         WalkScratch &scratch, RowIndex *out, cudaStream_t st) {
     *out = RowIndex{};
     if (p.transition != DYG_TRANSITION_WEIGHTED || !G->long_rows) return DYG_OK;
     Workspace &ws = G->ws;
     const uint32_t n = G->g.n;
-    uint64_t words = 6ull * G->g.arena_cap + 2ull;
-    if (words > kIdxWordsMax) words = kIdxWordsMax;
+    const size_t rows = ((size_t)n + 1) & ~(size_t)1;   // words before the index's, which are read in pairs
+    if (!scratch.index_tried) {
+        uint64_t words = 6ull * G->g.arena_cap + 2ull;
+        if (words > kIdxWordsMax) words = kIdxWordsMax;
+        scratch.index_tried = true;
+        if (scratch_borrow(&scratch.index, sizeof(uint32_t) * (2 * rows + (size_t)words)) != cudaSuccess)
+            cudaGetLastError();
+    }
     // where memory is short, the walks search their long rows without an index
-    if (ensure(ws.ix_base, sizeof(uint32_t) * (size_t)n) != DYG_OK ||
-        ensure(ws.ix_list, sizeof(uint32_t) * (size_t)n) != DYG_OK ||
-        ensure(ws.ix_words, sizeof(uint32_t) * (size_t)words) != DYG_OK)
-        return DYG_OK;
+    if (!scratch.index.p) return DYG_OK;
+    const uint64_t room = scratch.index.bytes / sizeof(uint32_t) - 2 * rows;
     unsigned long long *sc = ptr<unsigned long long>(ws.scalars);
     DYG_CUDA(cudaMemsetAsync(sc + S_IDX, 0, 2 * sizeof(unsigned long long), st));
     IndexArgs a{};
     a.g = G->g;
-    a.rbase = ptr<uint32_t>(ws.ix_base);
-    a.list = ptr<uint32_t>(ws.ix_list);
-    a.words = ptr<uint32_t>(ws.ix_words);
-    a.cap = (uint32_t)words;
+    a.rbase = ptr<uint32_t>(scratch.index);
+    a.list = a.rbase + rows;
+    a.words = a.list + rows;
+    a.cap = (uint32_t)(room < kIdxWordsMax ? room : kIdxWordsMax);
     a.cursor = sc + S_IDX;
     a.counts = sc + S_IDXN;
     a.halt = halt;

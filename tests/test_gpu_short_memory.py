@@ -78,3 +78,80 @@ def test_export(dyg, fail, cap):  # noqa: F811
         assert rc == (0 if cap is None else 4)
         assert np.array_equal(rp, rp0) and np.array_equal(col[:k], col0[:k]) and np.array_equal(w[:k], w0[:k])
         assert not col[k:].any() and not w[k:].any()
+
+
+def cycles(k, rng):
+    """k cycles of 3..200 vertices, whose deleted edges have winners of up to 199
+    moves: more records than a call starts with room for."""
+    sizes = np.where(np.arange(k) % 4 == 0, 200, rng.integers(3, 40, k))
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    base, L = np.repeat(off[:-1], sizes), np.repeat(sizes, sizes)
+    i = np.arange(off[-1]) - base
+    # and a row of 400 slots: weighted walks have an index
+    leaf = np.arange(400)
+    s = np.concatenate([base + i, np.full(400, off[-1])]).astype(np.uint32)
+    d = np.concatenate([base + (i + 1) % L, off[-1] + 1 + leaf]).astype(np.uint32)
+    return int(off[-1]) + 401, off[:-1], s, d, rng.uniform(0.5, 2.0, len(s)).astype(np.float32)
+
+
+@pytest.mark.parametrize("fail", [1, 2, 3, 100])
+@pytest.mark.parametrize("transition", [0, 1])
+@pytest.mark.parametrize("call", ["delete", "insert", "file_delete", "file_insert"])
+def test_updates(dyg, oracle, call, transition, fail):  # noqa: F811
+    """Every allocation of a call on fresh handles fails in turn.  With one
+    failure the call goes on (a second try, or without the scratch); with more it
+    goes on or says DYG_ENOMEM; and the handles work afterwards."""
+    rng = np.random.default_rng(3)
+    k = 300
+    n, first, gs, gd, gw = cycles(k, rng)
+    kw = dict(slack_per_row=0, arena_headroom=0.0)   # insertions and recoveries grow the arenas
+    G0 = dyg.Graph.from_edges(n, gs, gd, gw, **kw)
+    H0 = dyg.Graph.from_edges(n, *(a[np.r_[first, -400:0]] for a in (gs, gd, gw)), **kw)
+    es = rng.integers(0, n, 3000).astype(np.uint32)
+    ed = ((es + 1 + rng.integers(0, n - 1, 3000)) % n).astype(np.uint32)
+    ew = rng.uniform(0.01, 0.5, 3000).astype(np.float32)
+    p = dyg.WalkParams.make(threshold=10.0, walkers=64, max_steps=220, transition=transition, heuristic_walkers=2)
+    dele = first
+    Go, Ho = oracle.OGraph(n, gs, gd, gw), oracle.OGraph(n, *(a[np.r_[first, -400:0]] for a in (gs, gd, gw)))
+    if call == "delete":
+        want = oracle.decremental(Go, Ho, gs[dele], gd[dele], p, batch_size=200)[:5]
+    elif call == "insert":
+        want = oracle.incremental(Ho, es, ed, ew, p, batch_size=1500, G=Go)[:3]
+    elif call == "file_delete":
+        want = oracle.stream_file(Go, Ho, 1, gs[dele], gd[dele], None, p, chunk=200)[:5]
+    else:
+        want = oracle.stream_file(Go, Ho, 0, es, ed, ew, p, chunk=1500)[:2]
+
+    def go(G, H):
+        if call == "delete":
+            r = dyg.decremental_stream(G, H, gs[dele], gd[dele], p, batch_size=200)
+        elif call == "insert":
+            r = dyg.incremental_stream(H, es, ed, ew, p, 1500, G=G)
+            return r.found_at, r.conductance, r.accepted
+        elif call == "file_delete":
+            r = dyg.stream_file(G, H, 1, gs[dele], gd[dele], None, p, chunk=200)
+        else:
+            r = dyg.stream_file(G, H, 0, es, ed, ew, p, chunk=1500)
+            return r.status, r.conductance
+        return r.status, r.conductance, r.rec_src, r.rec_dst, r.rec_kind
+
+    def right(got, G, H):
+        for a, b in zip(got, want):
+            assert np.array_equal(np.asarray(a).view(np.uint8), np.asarray(b).astype(a.dtype).view(np.uint8))
+        same_graph(G, Go)
+        same_graph(H, Ho)
+
+    for skip in list(range(0, 60, 1 if fail in (1, 2) else 3)):
+        G, H = G0.clone(), H0.clone()
+        try:
+            with failing(dyg, skip, fail):
+                got = go(G, H)
+                assert dyg.lib().dyg_last_error_string() == b""
+        except dyg.DygError as e:
+            assert e.status == ENOMEM and fail > 1, (skip, str(e))
+            G.copy_from(G0)
+            H.copy_from(H0)
+            got = go(G, H)
+        right(got, G, H)
+        G.close()
+        H.close()
