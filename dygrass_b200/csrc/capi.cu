@@ -348,6 +348,8 @@ dyg_status graph_alloc_scalars(dyg_graph *G) {
     DYG_CUDA(host_alloc((void **)&G->ws.host_scalars, kScalarPinned));
     G->ws.host_counts = reinterpret_cast<uint32_t *>(G->ws.host_scalars + S_NSCALARS);
     G->g.top = ptr<unsigned long long>(G->ws.scalars) + S_TOP;
+    G->counted = true;
+    scratch_handles(G->device, 1);
     return DYG_OK;
 }
 
@@ -361,6 +363,7 @@ void free_graph(dyg_graph *G) {
     if (!G) return;
     DeviceGuard dg(G->device);
     cudaDeviceSynchronize();   // the blocks below may be handed out again at once
+    if (G->counted) scratch_handles(G->device, -1);
     Workspace &ws = G->ws;
     Buf *bufs[] = {&ws.keys, &ws.flags, &ws.pos, &ws.f_src, &ws.f_dst, &ws.f_idx, &ws.f_uid,
                    &ws.f_w, &ws.found, &ws.path_v, &ws.path_s, &ws.path_len, &ws.rec_head, &ws.cand_x, &ws.cand_y,

@@ -291,6 +291,7 @@ struct dyg_graph {
     // hold part of a batch.  Updates are refused until a whole graph is copied
     // over it.
     bool broken = false;
+    bool counted = false;   // among its device's handles
     uint32_t bar_limit = dyg::kBarSpinLimit;   // GridBar::limit
 };
 
@@ -318,12 +319,14 @@ cudaError_t dev_alloc(void **out, size_t bytes);
 void dev_free(void *p);
 // Scratch that a call can do without: a kept block of the device if one is free
 // and large enough, else a new one; returned once the device has finished with
-// it (at most 256 MB per device are kept).  scratch_drop frees what is kept;
-// an allocation that does not fit otherwise does so first.
+// it.  A device keeps at most 3 GB of it, 256 MB once it has no handles
+// (scratch_handles counts them; the device is current).  scratch_drop frees
+// what is kept; an allocation that does not fit otherwise does so first.
 struct Buf;
 cudaError_t scratch_borrow(Buf *b, size_t bytes);
 void scratch_return(Buf *b);
 void scratch_drop();
+void scratch_handles(int dev, int change);
 // For tests: this thread's next `pass` allocations go through, the `fail` after
 // them do not.
 void fail_allocations(uint32_t pass, uint32_t fail);

@@ -26,7 +26,12 @@ namespace dyg {
 namespace {
 
 constexpr unsigned long long kPoolKeep = 256ull << 20;
-constexpr unsigned long long kScratchKeep = 256ull << 20;
+// Kept scratch of a device: all that one call may borrow while the device has
+// handles (the row index is up to 2.3 GB, and allocating and freeing 0.3 GB in
+// each call took 5 to 15 ms of a weighted file on an R-MAT graph of scale 18,
+// of which the rest took 1), a little of it when the last is closed.
+constexpr unsigned long long kScratchKeep = 3ull << 30;
+constexpr unsigned long long kScratchIdle = 256ull << 20;
 constexpr int kMaxDevices = 64;
 
 struct DevicePool {
@@ -154,6 +159,7 @@ struct Scratch {
     std::vector<Buf> blocks;
     size_t total = 0;
     unsigned long long ctx = 0;
+    int handles = 0;
 };
 std::mutex g_scratch_mu;
 Scratch g_scratch[kMaxDevices];
@@ -166,7 +172,8 @@ Scratch *current_scratch() {
     if (!ctx) return nullptr;
     Scratch &s = g_scratch[dev];
     if (s.ctx != ctx) {   // the blocks went with their context
-        s = Scratch{};
+        s.blocks.clear();
+        s.total = 0;
         s.ctx = ctx;
     }
     return &s;
@@ -179,19 +186,34 @@ Buf take_scratch(Scratch &s, size_t i) {
     s.blocks.pop_back();
     return b;
 }
-}  // namespace
-
-void scratch_drop() {
+// Frees the smallest kept blocks (any borrower can use the larger) until at
+// most `keep` bytes are left.
+void shrink_scratch(size_t keep) {
     std::vector<Buf> drop;
     {
         std::lock_guard<std::mutex> lk(g_scratch_mu);
         Scratch *s = current_scratch();
-        if (!s) return;
-        drop.swap(s->blocks);
-        s->total = 0;
+        while (s && s->total > keep) {
+            size_t k = 0;
+            for (size_t i = 1; i < s->blocks.size(); ++i)
+                if (s->blocks[i].bytes < s->blocks[k].bytes) k = i;
+            drop.push_back(take_scratch(*s, k));
+        }
     }
     for (Buf &b : drop) dev_free(b.p);
 }
+}  // namespace
+
+void scratch_handles(int dev, int change) {
+    int left = 1;
+    if (dev >= 0 && dev < kMaxDevices) {
+        std::lock_guard<std::mutex> lk(g_scratch_mu);
+        left = g_scratch[dev].handles += change;
+    }
+    if (left == 0) shrink_scratch(kScratchIdle);
+}
+
+void scratch_drop() { shrink_scratch(0); }
 
 cudaError_t scratch_borrow(Buf *b, size_t bytes) {
     *b = Buf{};
@@ -223,24 +245,24 @@ cudaError_t scratch_borrow(Buf *b, size_t bytes) {
 
 void scratch_return(Buf *b) {
     if (!b->p) return;
-    std::vector<Buf> drop{*b};
-    *b = Buf{};
+    bool kept = false;
+    size_t keep = 0;
     {
         std::lock_guard<std::mutex> lk(g_scratch_mu);
         Scratch *s = current_scratch();
-        if (s && drop[0].bytes <= kScratchKeep) {
-            s->blocks.push_back(drop[0]);
-            s->total += drop[0].bytes;
-            drop.clear();
-            while (s->total > kScratchKeep) {   // the smallest go: any borrower can use the larger
-                size_t k = 0;
-                for (size_t i = 1; i < s->blocks.size(); ++i)
-                    if (s->blocks[i].bytes < s->blocks[k].bytes) k = i;
-                drop.push_back(take_scratch(*s, k));
+        if (s) {
+            keep = s->handles > 0 ? kScratchKeep : kScratchIdle;
+            if (b->bytes <= keep) {
+                s->blocks.push_back(*b);
+                s->total += b->bytes;
+                kept = true;
+                if (s->total <= keep) keep = 0;
             }
         }
     }
-    for (Buf &d : drop) dev_free(d.p);
+    if (!kept) dev_free(b->p);
+    else if (keep) shrink_scratch(keep);
+    *b = Buf{};
 }
 
 namespace {

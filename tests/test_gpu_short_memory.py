@@ -155,3 +155,34 @@ def test_updates(dyg, oracle, call, transition, fail):  # noqa: F811
         right(got, G, H)
         G.close()
         H.close()
+
+
+def test_large_scratch_is_kept_for_the_handles(dyg):  # noqa: F811
+    """A row index of 0.6 GB stays with the device while it has handles, is lent
+    to one after the other, and goes when the last is closed."""
+    import gc
+    import torch
+    rng = np.random.default_rng(4)
+    n, m = 1 << 20, 8_000_000
+    s, d = rng.integers(0, n, m).astype(np.uint32), rng.integers(0, n, m).astype(np.uint32)
+    s[:400], d[:400] = 7, 100 + np.arange(400)
+    w = np.ones(m, np.float32)
+    p = dyg.WalkParams.make(threshold=10.0, walkers=32, max_steps=8, transition=1)
+
+    def free():
+        torch.cuda.synchronize()   # the pool gives back what is above its share then
+        return torch.cuda.mem_get_info()[0]
+
+    gc.collect()
+    before = free()
+    H = dyg.Graph.from_edges(n, s, d, w)
+    H2 = H.clone()
+    dyg.incremental_batch(H, s[:8], d[1:9], w[:8], p)
+    held = free()
+    for X in (H2, H, H2):
+        dyg.incremental_batch(X, s[:8], d[1:9], w[:8], p)
+        assert abs(free() - held) < 64 << 20
+    H.close()
+    H2.close()
+    # the pool and the scratch keep 256 MB each
+    assert before - free() < 560 << 20
