@@ -238,13 +238,14 @@ enum Scalar : int {
     S_LONG = 13,      // set by an append that made a row longer than kBigRow
     S_SCAN = 14,      // tile tickets of the single-pass scan (accumulating)
     S_BAR = 15,       // grid barrier: arrivals (low word), generation (high word)
-    S_ITEMS = 18,     // row operations: rows for a block (low word), for a warp (high word)
     S_IDX = 16,       // row index: next free word
+    S_IDXN = 17,      // row index: rows for a warp (low word), for a block (high word)
+    S_IDXSUM = 18,    // row index: slots of rows a lane can search (low word), of longer ones (high word)
     S_SLOTS = 19,     // live slots, summed for dyg_graph_info
     S_RECW = 20,      // path records: words asked for (zero between walks)
     S_RECNEED = 21,   // path records: words a halted walk asked for
-    S_IDXN = 17,      // row index: rows for a warp (low word), for a block (high word)
-    S_NSCALARS = 22
+    S_ITEMS = 22,     // row operations: rows for a block (low word), for a warp (high word)
+    S_NSCALARS = 23
 };
 enum Count : int {
     C_FILTERED = 0,   // decremental: edges to walk
@@ -388,12 +389,12 @@ uint32_t walk_threads(uint32_t n, const dyg_walk_params &p);
 dyg_status launch_walk_scalars(const DevGraph &g, const WalkJob &job, const dyg_walk_params &p,
                                bool incremental, unsigned long long *keys,
                                unsigned long long *scalars, cudaStream_t st);
-// The row index for weighted walks on G as it is now; empty for a uniform
-// transition or a graph without hub rows.  The walks that use it test the same
-// halt word: an index whose launch was cut short must not be read.
+// The row index for weighted walks from up to n edges on G as it is now; empty
+// for a uniform transition or a graph without hub rows.  The walks that use it
+// test the same halt word: an index whose launch was cut short must not be read.
 struct WalkScratch;
-dyg_status index_enqueue(dyg_graph *G, const dyg_walk_params &p, unsigned long long *halt,
-                         WalkScratch &scratch, RowIndex *out, cudaStream_t st);
+dyg_status index_enqueue(dyg_graph *G, uint32_t n, const dyg_walk_params &p, bool incremental,
+                         unsigned long long *halt, WalkScratch &scratch, RowIndex *out, cudaStream_t st);
 dyg_status launch_winner_paths(dyg_graph *G, const WalkJob &job, const dyg_walk_params &p,
                                const unsigned long long *keys, uint32_t n_max, uint32_t path_stride,
                                uint32_t *path_v, uint32_t *path_s, int32_t *path_len, const RowIndex &ix,

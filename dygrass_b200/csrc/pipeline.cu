@@ -579,7 +579,7 @@ static dyg_status incr_enqueue(dyg_graph *H, dyg_graph *G, const uint32_t *src, 
     if (!walk_ready) DYG_CUDA(cudaMemsetAsync(keys, 0, sizeof(unsigned long long) * n, st));
     WalkJob job{halt, src, dst, w, uids, (unsigned long long)uid0, nullptr, n, kDomainIncr, 0u};
     RowIndex ix{};
-    DYG_TRY(index_enqueue(H, p, halt, scratch, &ix, st));
+    DYG_TRY(index_enqueue(H, n, p, true, halt, scratch, &ix, st));
     DYG_TRY(launch_walk(H, job, p, true, keys, ix, st, walk_ready));
     return incr_commit_enqueue(H, G, src, dst, w, n, keys, true, halt, batch, found, cond, acc, st);
 }
@@ -774,7 +774,7 @@ dyg_status decr_walk_enqueue(dyg_graph *G, dyg_graph *H, uint32_t f0, uint32_t n
     if (phase0 != 1) {
         // walks on the updated G (main.cu:392, 420)
         RowIndex ix{};   // of the walks, and of the replays of their winners
-        DYG_TRY(index_enqueue(G, p, halt, scratch, &ix, st));
+        DYG_TRY(index_enqueue(G, n, p, false, halt, scratch, &ix, st));
         if (!keys_given) {
             if (!walk_ready) DYG_CUDA(cudaMemsetAsync(own, 0, sizeof(unsigned long long) * n, st));
             DYG_TRY(launch_walk(G, job, p, false, own, ix, st, walk_ready, replay ? nullptr : &scratch.rec));

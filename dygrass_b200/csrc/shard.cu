@@ -112,7 +112,7 @@ dyg_status dyg_walk_keys(dyg_graph *X, const uint32_t *src, const uint32_t *dst,
                 incremental ? kDomainIncr : kDomainDecr};
     RowIndex ix{};
     WalkScratch scratch(st);
-    DYG_TRY(index_enqueue(X, *p, sc + S_HALT, scratch, &ix, st));
+    DYG_TRY(index_enqueue(X, hi - lo, *p, incremental != 0, sc + S_HALT, scratch, &ix, st));
     DYG_TRY(launch_walk(X, job, *p, incremental != 0, k, ix, st));
     DYG_TRY(read_scalars(X, st));
     if (ws.host_scalars[S_HALT]) return rejected_inputs(X, st);
@@ -255,7 +255,7 @@ dyg_status dyg_decremental_walk_keys(dyg_graph *G, uint32_t lo, uint32_t hi,
                 ptr<unsigned long long>(ws.f_uid) + lo, 0ull, nullptr, hi - lo, kDomainDecr};
     RowIndex ix{};
     WalkScratch scratch(st);
-    DYG_TRY(index_enqueue(G, *p, halt, scratch, &ix, st));
+    DYG_TRY(index_enqueue(G, hi - lo, *p, false, halt, scratch, &ix, st));
     DYG_TRY(launch_walk(G, job, *p, false, k, ix, st));
     return read_scalars(G, st);
 }

@@ -475,7 +475,7 @@ dyg_status insert_chunk_enqueue(dyg_graph *G, dyg_graph *H, uint32_t c, uint32_t
     const WalkJob job{halt, fsrc, fdst, fw, ptr<unsigned long long>(wg.f_uid) + f0, 0ull,
                       ptr<uint32_t>(wg.counts) + C_WALKLIST, nc, kDomainIncr, f0};
     RowIndex ix{};
-    DYG_TRY(index_enqueue(H, p, halt, scratch, &ix, st));
+    DYG_TRY(index_enqueue(H, nc, p, true, halt, scratch, &ix, st));
     DYG_TRY(launch_walk(H, job, p, true, keys, ix, st, walk_ready));
     const StAcceptOp op{job, keys, ptr<uint32_t>(wg.f_idx) + f0, status, cond};
     return append_enqueue(op, nc, H, EdgeList{fsrc, fdst, fw}, nullptr, EdgeList{},

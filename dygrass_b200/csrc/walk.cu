@@ -423,15 +423,30 @@ __device__ __forceinline__ uint32_t warp_pick_weighted(const uint2 *__restrict__
 // reading such a row for one lane after another bounds the walk: 9.87 ms for
 // the deletion walks of a 1,000-edge R-MAT file (scale 13).  A walker needs
 // two things of the row: the position and weight of the column it came from,
-// and the first prefix sum above its target.  k_index tabulates both for
-// every row longer than kIdxRow, once per launch of walks (the rows do not
-// change while they walk), and each lane then chooses by itself: one hash
-// lookup and one binary search.  Its cost is a pass over the long rows (40 us
-// a launch there, of which the walk was 9.87 ms and is 1.15 ms; the whole six
-// files 15.2 -> 4.4 ms).  It is built whenever the graph has hub rows (over
-// kBigRow slots): even a single edge's walkers scan more than it costs.  Rows with a repeated column, or whose sum
-// wraps past 2^64, get no index and are searched by the warp as before.
+// and the first prefix sum above its target.  k_index tabulates both, once per
+// launch of walks (the rows do not change while they walk), and each lane then
+// chooses by itself: one hash lookup and one search of the prefixes.  Rows with
+// a repeated column, or whose sum wraps past 2^64, get no index and are searched
+// by the warp as before.
+//
+// It is built whenever the graph has hub rows (over kBigRow slots), of the rows
+// that the warp would search (over kCoopRow): even a single edge's 256 walkers
+// scan more than it costs.  Stream files on R-MAT graphs, us a file with the
+// index and without (and with the rows read slot by slot as before either):
+//   scale 13, 204,000 slots      1 deletion 287, 627 (1,408)    1,000: 1,826, 18,300 (28,600)
+//   scale 18, 7.6 M slots        1 deletion 2,021, 13,210 (28,400)  1,000: 5,170, 68,500 (76,200)
+//   scale 20, 31 M slots         1 deletion 2,570, 2,290 (4,530)    1,000: 11,200, 137,000 (149,000)
+// The rows of kIdxRow + 1 to kCoopRow slots, which a lane can search, are
+// indexed as well where that at most doubles the index (the R-MAT graphs: a few
+// per cent slower without) or where there are enough walks: their index costs as
+// a pass over their slots, and each walk saves some scans of such rows.  On a
+// random geometric graph of 200,000 vertices and 3.2 M slots with one hub, us a
+// batch with and without them (as before): 1 insertion 889, 557 (878); 32: 959,
+// 698 (1,038); 1,000: 2,490, 3,260 (3,540); 4,096 deletions 669, 502 (628),
+// 1,000: 513, 301 (377).  The lines lie at 16 slots a walk for insertions, whose
+// walks are long, and at one for deletions, most of which walk a few moves.
 constexpr uint32_t kIdxRow = kPickGroup;   // longer rows are indexed: the lane reads up to it at once
+constexpr uint32_t kIdxInsertSlots = 16;   // slots a walk is worth
 constexpr uint32_t kIdxBlockRow = 1024; // ... by a whole block from here on
 constexpr uint32_t kIdxTile = 8;        // slots per thread of a block's tile
 
@@ -493,6 +508,9 @@ struct IndexArgs {
     uint32_t cap;                    // words
     unsigned long long *cursor;      // next free word (from 2 on: 0 means no region)
     unsigned long long *counts;      // S_IDXN
+    unsigned long long *sums;        // S_IDXSUM
+    unsigned long long budget;       // slots of short rows that the walks are worth
+    bool all;                        // the budget covers any graph: nothing to count
     const unsigned long long *halt;
 };
 
@@ -513,12 +531,28 @@ __global__ void __launch_bounds__(kOpThreads, 2) k_index(const __grid_constant__
     __shared__ uint32_t s_bad;
     if (*a.halt) return;
     const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    uint32_t shortest = kIdxRow;
+    if (!a.all) {
+        uint32_t mid = 0u, lng = 0u;   // a graph's slots fit 32 bits
+        for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < a.g.n; v += gridDim.x * blockDim.x) {
+            const uint32_t deg = a.g.desc[v].y;
+            if (deg > kCoopRow) lng += deg;
+            else if (deg > kIdxRow) mid += deg;
+        }
+        __syncwarp();
+        mid = __reduce_add_sync(kFull, mid);
+        lng = __reduce_add_sync(kFull, lng);
+        if (lane == 0u && (mid | lng)) atomicAdd(a.sums, ((unsigned long long)lng << 32) + mid);
+        if (!grid_sync(bar)) return;
+        const unsigned long long both = __ldcg(a.sums);
+        if ((both & 0xFFFFFFFFull) > (both >> 32) + a.budget) shortest = kCoopRow;
+    }
     // regions, and the lists of rows: for a warp from the front, for a block
     // from the back
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < a.g.n; v += gridDim.x * blockDim.x) {
         const uint32_t deg = a.g.desc[v].y;
         uint32_t base = 0u;
-        if (deg > kIdxRow) {
+        if (deg > shortest) {
             const unsigned long long want = (1ull << idx_bits(deg)) + 2ull * deg;
             const unsigned long long at = atomicAdd(a.cursor, want) + 2ull;
             if (at + want <= a.cap) {
@@ -620,9 +654,9 @@ __global__ void __launch_bounds__(kOpThreads, 2) k_index(const __grid_constant__
     }
 }
 
-// One move of every active lane's walker, with rows longer than kCoopRow
-// chosen through their index or, without one, searched by the whole warp (all
-// 32 lanes call this).  Returns the move's result for active lanes.
+// One move of every active lane's walker: in a row with an index through it,
+// in another of up to kCoopRow slots by the lane, in a longer one by the whole
+// warp (all 32 lanes call this).  Returns the move's result for active lanes.
 template <bool INCR>
 __device__ __forceinline__ int step_weighted_warp(Walker &s, bool active, const DevGraph &g,
                                                   const RowIndex &ix, uint32_t max_steps, float thr, uint2 key,
@@ -1180,8 +1214,8 @@ static void launch_walk_any(const WalkArgs &a, bool incremental, bool wtd, cudaS
 // rows that do not fit stay without an index.
 constexpr uint64_t kIdxWordsMax = 1ull << 29;
 
-dyg_status index_enqueue(dyg_graph *G, const dyg_walk_params &p, unsigned long long *halt,
-                         WalkScratch &scratch, RowIndex *out, cudaStream_t st) {
+dyg_status index_enqueue(dyg_graph *G, uint32_t edges, const dyg_walk_params &p, bool incremental,
+                         unsigned long long *halt, WalkScratch &scratch, RowIndex *out, cudaStream_t st) {
     *out = RowIndex{};
     if (p.transition != DYG_TRANSITION_WEIGHTED || !G->long_rows) return DYG_OK;
     Workspace &ws = G->ws;
@@ -1198,7 +1232,7 @@ dyg_status index_enqueue(dyg_graph *G, const dyg_walk_params &p, unsigned long l
     if (!scratch.index.p) return DYG_OK;
     const uint64_t room = scratch.index.bytes / sizeof(uint32_t) - 2 * rows;
     unsigned long long *sc = ptr<unsigned long long>(ws.scalars);
-    DYG_CUDA(cudaMemsetAsync(sc + S_IDX, 0, 2 * sizeof(unsigned long long), st));
+    DYG_CUDA(cudaMemsetAsync(sc + S_IDX, 0, 3 * sizeof(unsigned long long), st));
     IndexArgs a{};
     a.g = G->g;
     a.rbase = ptr<uint32_t>(scratch.index);
@@ -1207,6 +1241,9 @@ dyg_status index_enqueue(dyg_graph *G, const dyg_walk_params &p, unsigned long l
     a.cap = (uint32_t)(room < kIdxWordsMax ? room : kIdxWordsMax);
     a.cursor = sc + S_IDX;
     a.counts = sc + S_IDXN;
+    a.sums = sc + S_IDXSUM;
+    a.budget = (unsigned long long)edges * p.walkers * (incremental ? kIdxInsertSlots : 1u);
+    a.all = a.budget >= G->g.arena_cap;
     a.halt = halt;
     DYG_TRY(launch_phases<k_index>(2u * (uint32_t)num_sms(), st, grid_bar(G, halt), a));
     *out = RowIndex{a.rbase, a.words};
