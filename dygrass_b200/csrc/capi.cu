@@ -369,7 +369,7 @@ void free_graph(dyg_graph *G) {
                    &ws.f_w, &ws.found, &ws.path_v, &ws.path_s, &ws.path_len, &ws.rec_head, &ws.cand_x, &ws.cand_y,
                    &ws.cand_w, &ws.keep, &ws.htab_k, &ws.htab_v, &ws.scan_status,
                    &ws.s_src, &ws.s_dst, &ws.s_w, &ws.s_o1, &ws.s_o2, &ws.s_o3, &ws.rx2, &ws.ry2,
-                   &ws.rk2, &ws.nxt, &ws.dtmp, &ws.rowcnt, &ws.rowhead, &ws.rowlist, &ws.blk, &ws.st_key,
+                   &ws.rk2, &ws.nxt, &ws.runs, &ws.rowcnt, &ws.rowhead, &ws.rowlist, &ws.blk, &ws.st_key,
                    &ws.st_cnt, &ws.st_val, &ws.st_pos, &ws.st_wapp, &ws.big, &ws.s_uid, &ws.scalars, &ws.io_in, &ws.io_out};
     for (Buf *b : bufs) free_buf(*b);
     host_free(ws.host_scalars, kScalarPinned);

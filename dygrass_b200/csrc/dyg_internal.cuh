@@ -202,7 +202,7 @@ struct Workspace {
     Buf s_src, s_dst, s_w, s_o1, s_o2, s_o3;  // whole-stream staging
     Buf rx2, ry2;                             // recovered edges of a whole stream
     Buf rk2;
-    Buf nxt, dtmp;                            // row operations: per-entry chain link / ordered run
+    Buf nxt, runs;                            // row operations: per-entry chain link / ordered entries
     Buf rowcnt, rowhead;                      // row operations: per-row entries / last entry + 1
     Buf rowlist;                              // row operations: rows for warps and blocks
     Buf blk;                                  // row operations: per-block words
@@ -226,7 +226,7 @@ enum Scalar : int {
     S_CURSOR = 1,     // arena cursor of the moves of that append
     S_KEPT = 2,       // recovery candidates kept so far (zero between recoveries)
     S_NBIG = 3,       // stream file: entries on the long-row list
-    S_TMPCUR = 4,     // scratch cursor of a delete (zero between deletes)
+    S_RUNS = 4,       // row operations: next free word of the runs (low word), runs to fill (high word)
     S_ERR = 5,        // device error bits (kErr*)
     S_MOVES = 6,      // walker moves (accumulating)
     S_WALKS = 7,      // walks finished (accumulating)

@@ -130,20 +130,25 @@ __global__ void __launch_bounds__(kOpThreads, 2) k_delete(const __grid_constant_
         a.rec_head[e] = 0u;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) *a.work = 0ull;
-    if (!grid_sync(bar, [&] { *a.D.c.items = *a.D.items_h = 0ull; })) return;
+    if (!grid_sync(bar, [&] { *a.D.c.items = *a.D.items_h = *a.D.c.cursor = 0ull; })) return;
     const uint32_t m = 2u * a.n;
     del_list(a.G, a.H, a.D, m);
     __syncthreads();   // the marks of this block's entries are set
     del_lane_rows(a.G, a.D, m, 1u, nullptr, a.fG, false);
     if (!grid_sync(bar)) return;
-    const unsigned long long items_g = __ldcg(a.D.c.items), items_h = __ldcg(a.D.items_h);
+    const unsigned long long items_g = __ldcg(a.D.c.items), items_h = __ldcg(a.D.items_h),
+                             runs = __ldcg(a.D.c.cursor);
+    if (runs >> 32) {
+        fill_runs(a.D.c, m, [&](uint32_t i) { return del_row(a.D, i); });
+        if (!grid_sync(bar)) return;
+    }
     if (items_g) {
-        del_listed_rows(a.G, a.D, a.D.c.list, items_g, m, nullptr, a.fG, false, s);
+        del_listed_rows(a.G, a.D, a.D.c.list, items_g, m, false, nullptr, a.fG, false, s);
         if (!grid_sync(bar)) return;
     }
     del_lane_rows(a.H, a.D, m, 2u, a.fG, a.fH, true);
-    del_listed_rows(a.H, a.D, a.D.list_h, items_h, m, a.fG, a.fH, true, s);
-    if (!grid_sync(bar, [&] { *a.D.cursor = 0ull; })) return;
+    del_listed_rows(a.H, a.D, a.D.list_h, items_h, m, true, a.fG, a.fH, true, s);
+    if (!grid_sync(bar)) return;
     uint32_t mine = 0u;
     for (uint32_t e = rg.x + threadIdx.x; e < rg.y; e += blockDim.x) {
         const bool inG = a.fG[2 * e] && a.fG[2 * e + 1];
@@ -472,7 +477,7 @@ __global__ void __launch_bounds__(kOpThreads, 2) k_recover(const __grid_constant
     if (!grid_sync(bar, [&] {
             const unsigned long long k = __ldcg(a.sc + S_KEPT);
             a.sc[S_KEPT] = 0ull;
-            *a.A.s[0].c.items = 0ull;
+            *a.A.s[0].c.items = *a.A.s[0].c.cursor = 0ull;
             if (a.sc[S_RECCNT] + k > a.sc[S_RECCAP]) *a.halt = a.code_records;
         }))
         return;
@@ -589,7 +594,6 @@ dyg_status decr_delete_ensure(dyg_graph *G, dyg_graph *H, uint32_t n, cudaStream
     const uint64_t m = 2ull * n;
     DYG_TRY(rowops_ensure(G, m, st));
     DYG_TRY(rowops_ensure(H, m, st));
-    DYG_TRY(ensure(ws.dtmp, sizeof(uint32_t) * (size_t)m * 2));
     DYG_TRY(ensure(ws.found, (size_t)m * 2));
     DYG_TRY(ensure(ws.keys, sizeof(unsigned long long) * n));
     DYG_TRY(ensure(ws.f_src, sizeof(uint32_t) * n));
@@ -617,8 +621,7 @@ dyg_status decr_delete_enqueue(dyg_graph *G, dyg_graph *H, const uint32_t *src,
     DeleteArgs a{};
     a.G = G->g;
     a.H = H->g;
-    a.D = DelList{append_side(G, src, dst, nullptr).c, src, dst, ptr<uint32_t>(ws.dtmp), sc + S_TMPCUR,
-                  ptr<uint32_t>(H->ws.rowlist), ptr<unsigned long long>(H->ws.scalars) + S_ITEMS};
+    a.D = DelList{append_side(G, src, dst, nullptr).c, src, dst, ptr<uint32_t>(H->ws.rowlist), ptr<unsigned long long>(H->ws.scalars) + S_ITEMS};
     a.n = n;
     a.file_orient = file_orient;
     a.uid0 = uid0;

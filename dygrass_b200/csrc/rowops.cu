@@ -7,6 +7,7 @@ dyg_status rowops_ensure(dyg_graph *G, uint64_t m, cudaStream_t st) {
     Workspace &ws = G->ws;
     DYG_TRY(ensure(ws.nxt, sizeof(uint32_t) * (size_t)(m ? m : 1)));
     DYG_TRY(ensure(ws.rowlist, sizeof(uint32_t) * (size_t)(m ? m : 1)));
+    DYG_TRY(ensure(ws.runs, sizeof(uint32_t) * (size_t)(m ? m : 1)));
     DYG_TRY(ensure(ws.blk, sizeof(uint32_t) * kOpBlocksMax * 2));
     if (!ws.rowcnt.p || !ws.rowhead.p) {
         const size_t bytes = sizeof(uint32_t) * (size_t)(G->g.n ? G->g.n : 1);
@@ -29,7 +30,7 @@ AppSide append_side(dyg_graph *G, const uint32_t *src, const uint32_t *dst, cons
     unsigned long long *sc = ptr<unsigned long long>(ws.scalars);
     return AppSide{G->g,
                    Chains{ptr<uint32_t>(ws.rowcnt), ptr<uint32_t>(ws.rowhead), ptr<uint32_t>(ws.nxt),
-                          ptr<uint32_t>(ws.rowlist), sc + S_ITEMS},
+                          ptr<uint32_t>(ws.rowlist), sc + S_ITEMS, ptr<uint32_t>(ws.runs), sc + S_RUNS},
                    EdgeList{src, dst, w}, G->slack, sc};
 }
 
