@@ -245,7 +245,8 @@ enum Scalar : int {
     S_RECW = 20,      // path records: words asked for (zero between walks)
     S_RECNEED = 21,   // path records: words a halted walk asked for
     S_ITEMS = 22,     // row operations: rows for a block (low word), for a warp (high word)
-    S_NSCALARS = 23
+    S_FOLD = 23,      // stream file: words of the often repeated edges' runs (low word), such edges (high word)
+    S_NSCALARS = 24
 };
 enum Count : int {
     C_FILTERED = 0,   // decremental: edges to walk

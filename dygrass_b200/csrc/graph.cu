@@ -62,7 +62,7 @@ static dyg_status recover_workspace(dyg_graph *G) {
         dev_free(b->p);
         *b = Buf{};
     }
-    for (int s : {S_NEED, S_CURSOR, S_KEPT, S_NBIG, S_RUNS, S_ERR, S_WORK, S_HALT, S_BAR, S_RECW, S_ITEMS}) {
+    for (int s : {S_NEED, S_CURSOR, S_KEPT, S_NBIG, S_RUNS, S_ERR, S_WORK, S_HALT, S_BAR, S_RECW, S_ITEMS, S_FOLD}) {
         DYG_CUDA(cudaMemset(ptr<unsigned long long>(ws.scalars) + s, 0, sizeof(unsigned long long)));
         ws.host_scalars[s] = 0ull;
     }

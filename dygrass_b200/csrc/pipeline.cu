@@ -64,7 +64,7 @@ __global__ void k_validate(unsigned long long *halt, const uint32_t *src, const 
 // to G.  With `clear` the key is zeroed behind the decode, so that the next
 // batch's walks need no memset.
 struct IncrOp {
-    static constexpr bool kList = false;
+    static constexpr bool kList = false, kPrep = false;
     unsigned long long *keys;
     int32_t *found;
     float *cond;

@@ -930,12 +930,20 @@ __device__ __forceinline__ void del_listed_rows(const DevGraph &g, const DelList
 //   uint32_t count()                  edges (device or host count)
 //   uint32_t take(uint32_t e)
 //   static constexpr bool kList       whether take's bit 0 also lists the edge
+//   static constexpr bool kPrep       whether something may come before all this:
+//   bool pending()                    what, read beside the halt word; if so
+//   bool prep(bar, s)                 every thread of the grid does it (false: the
+//                                     barrier gave up)
 template <class Op>
 __global__ void __launch_bounds__(kOpThreads, 2)
-k_append(const Op op, const __grid_constant__ AppSides A, uint32_t *blk, unsigned long long *work,
+k_append(const __grid_constant__ Op op, const __grid_constant__ AppSides A, uint32_t *blk, unsigned long long *work,
          unsigned long long *halt, unsigned long long code, GridBar bar) {
     __shared__ RowShared s;
+    bool pending = false;
+    if constexpr (Op::kPrep) pending = op.pending();
     if (*halt) return;
+    if constexpr (Op::kPrep)
+        if (pending && !op.prep(bar, s)) return;
     const uint32_t n = op.count();
     const uint2 rg = block_range(n);
     uint32_t mine = 0u;

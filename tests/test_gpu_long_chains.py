@@ -71,3 +71,38 @@ def test_delete(dyg, oracle, rows, each, others, more):  # noqa: F811
         assert np.array_equal(r.rec_src, rx) and np.array_equal(r.rec_dst, ry) and np.array_equal(r.rec_kind, rk)
         same_graph(G, Go)
         same_graph(H, Ho)
+
+
+@pytest.mark.parametrize("keys,times,others", [(4, 32, 100), (4, 33, 100), (300, 40, 0), (300, 40, 9000), (60, 255, 0),
+                                               (60, 256, 0), (60, 257, 0), (6, 4095, 0), (6, 4096, 0), (6, 4097, 0),
+                                               (2, 9000, 3000)])
+@pytest.mark.parametrize("tight", [False, True])
+def test_file_repeats(dyg, oracle, keys, times, others, tight):  # noqa: F811
+    """Edges repeated many times in a stream file: new ones, ones in G, ones in
+    both graphs; `tight`: the new edges make G's arena grow, after the weights
+    were added."""
+    rng = np.random.default_rng(keys * times + others)
+    n = 4000
+    gs, gd = np.arange(n - 1, dtype=np.uint32), np.arange(1, n, dtype=np.uint32)
+    gw = rng.uniform(0.5, 2.0, n - 1).astype(np.float32)
+    in_h = rng.random(n - 1) < 0.5
+    known = rng.choice(n - 1, keys, replace=False)
+    pick = [(gs[k], gd[k]) if i % 3 else (rng.integers(0, n // 2), n // 2 + rng.integers(0, n // 2))
+            for i, k in enumerate(known)]
+    e = np.concatenate([np.repeat(np.array(pick, np.int64).reshape(-1, 2), times, 0), rng.integers(0, n, (others, 2))])
+    flip = rng.random(len(e)) < 0.5
+    e[flip] = e[flip][:, ::-1]
+    e = e[rng.permutation(len(e))].astype(np.uint32)
+    w = rng.uniform(0.1, 1.0, len(e)).astype(np.float32)
+    kw = dict(slack_per_row=0, arena_headroom=0.0) if tight else {}
+    G = dyg.Graph.from_edges(n, gs, gd, gw, **kw)
+    H = dyg.Graph.from_edges(n, gs[in_h], gd[in_h], gw[in_h], **kw)
+    Go, Ho = oracle.OGraph(n, gs, gd, gw), oracle.OGraph(n, gs[in_h], gd[in_h], gw[in_h])
+    p = dyg.WalkParams.make(threshold=5.0, walkers=32, max_steps=10)
+    for k in range(2):   # the second file finds the table as the first left it
+        r = dyg.stream_file(G, H, 0, e[:, 0].copy(), e[:, 1].copy(), w, p, first_update_id=k * len(e))
+        st, cd, *_ = oracle.stream_file(Go, Ho, 0, e[:, 0].copy(), e[:, 1].copy(), w, p, first_uid=k * len(e))
+        assert np.array_equal(r.status, st)
+        assert np.array_equal(r.conductance.view(np.uint32), cd.view(np.uint32))
+        same_graph(G, Go)
+        same_graph(H, Ho)
