@@ -1149,9 +1149,14 @@ static uint32_t prune_every() {
     return (t == 2u || t == 4u) ? t : 1u;
 }
 
-// Weighted deletion walks take 16: their walks are long-tailed, and a warp
-// with fewer of them waits less for its slowest (12,000 deletions of a 40^3
-// mesh 2.47 -> 2.16 ms of walks; insertions 1.51 -> 1.59).
+// Weighted deletion walks take 16 in batches of up to 2M walkers: their walks
+// are long-tailed, and a warp with fewer of them waits less for its slowest
+// (12,000 deletions of a 40^3 mesh in ten batches 2.47 -> 2.16 ms of walks;
+// insertions 1.51 -> 1.59).  Where the batch fills the device many times over,
+// fetching twice as many chunks costs more (calls of one batch, 512 walkers, us
+// with 16 and 32: random geometric graph of 400,000 vertices, 1,000 deletions 504
+// and 503, 4,000 765 and 735, 8,000 1,093 and 1,016, 16,000 1,902 and 1,732; 100^3
+// mesh 430 and 494, 847 and 861, 1,378 and 1,359, 2,408 and 2,344).
 static uint32_t chunk_for(uint32_t n, uint32_t walkers, bool weighted, bool incremental) {
     static int env = -1;
     if (env < 0) {
@@ -1159,9 +1164,9 @@ static uint32_t chunk_for(uint32_t n, uint32_t walkers, bool weighted, bool incr
         env = v ? atoi(v) : 0;
     }
     const uint32_t want = g_tune_chunk.load() ? g_tune_chunk.load() : (uint32_t)(env > 0 ? env : 0);
-    uint32_t c = weighted && !incremental ? 16u : 32u;
-    if (!weighted && walkers % 64u == 0u && (uint64_t)n * walkers >= kBigChunkWalkers * (incremental ? 1u : 2u))
-        c = 64u;
+    const uint64_t all = (uint64_t)n * walkers;
+    uint32_t c = weighted && !incremental && all < kBigChunkWalkers ? 16u : 32u;
+    if (!weighted && walkers % 64u == 0u && all >= kBigChunkWalkers * (incremental ? 1u : 2u)) c = 64u;
     if (want > 0 && want % 32 == 0 && walkers % want == 0) c = want;
     return c;
 }
