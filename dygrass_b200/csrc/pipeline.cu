@@ -270,6 +270,17 @@ struct RecoverArgs {
     unsigned long long code_records, code_arena, code_paths;
 };
 
+// Mask of the dedup table for M candidates: 2M slots at least, 1,024 at least, as
+// the host sizes it.  In 64 bits: 2M does not fit 32 from M = 2^31 on, and the
+// doubling would not end from 2^30 + 1 on.
+__host__ __device__ constexpr uint32_t dedup_mask(uint32_t M) {
+    uint64_t T = 1024;
+    while (T < 2ull * M) T <<= 1;
+    return (uint32_t)(T - 1);
+}
+static_assert(dedup_mask(0) == 1023u && dedup_mask(512) == 1023u && dedup_mask(513) == 2047u, "sizes");
+static_assert(dedup_mask(1u << 30) == 0x7FFFFFFFu && dedup_mask((1u << 30) + 1u) == 0xFFFFFFFFu, "sizes");
+
 __device__ __forceinline__ void cand_put(const RecoverArgs &a, uint32_t i, uint32_t x, uint32_t y,
                                          float w, uint32_t mask, bool store) {
     if (store) {
@@ -328,7 +339,7 @@ __global__ void __launch_bounds__(kOpThreads, 2) k_recover(const __grid_constant
     __shared__ uint32_t s_off[kOpThreads], s_rec[kOpThreads], s_none[kOpThreads];
     if (*a.halt) return;
     uint32_t n_path, M;
-    uint32_t mask = 1023u;
+    uint32_t mask;
     if (blockIdx.x == 0 && threadIdx.x == 0) a.sc[S_WORK] = 0ull;   // the next walk's chunk counter
     if (!a.resume) {
         const uint32_t F = job_count(a.job);
@@ -376,7 +387,7 @@ __global__ void __launch_bounds__(kOpThreads, 2) k_recover(const __grid_constant
             a.counts[C_CANDS] = n_path;
             a.counts[C_CANDS_ALL] = M;
         }
-        while (mask + 1u < 2u * M) mask = 2u * mask + 1u;
+        mask = dedup_mask(M);
         uint32_t at = pl.x, nth = pn.x;
         for (uint32_t t = rg.x; t < rg.y; t += blockDim.x) {
             // one thread per walked deletion finds its winner's path and where
@@ -438,7 +449,7 @@ __global__ void __launch_bounds__(kOpThreads, 2) k_recover(const __grid_constant
     } else {
         n_path = a.counts[C_CANDS];
         M = a.counts[C_CANDS_ALL];
-        while (mask + 1u < 2u * M) mask = 2u * mask + 1u;
+        mask = dedup_mask(M);
         GSTRIDE(i, M) cand_put(a, i, a.cx[i], a.cy[i], 0.f, mask, false);
     }
     if (!grid_sync(bar)) return;
@@ -481,8 +492,8 @@ __global__ void __launch_bounds__(kOpThreads, 2) k_recover(const __grid_constant
             if (a.sc[S_RECCNT] + k > a.sc[S_RECCAP]) *a.halt = a.code_records;
         }))
         return;
-    GSTRIDE(i, mask + 1u) {   // the table as it was found
-        a.tk[i] = ~0ull;
+    for (uint64_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= mask; i += gridDim.x * blockDim.x) {
+        a.tk[i] = ~0ull;   // the table as it was found
         a.tv[i] = ~0u;
     }
     if (*(volatile unsigned long long *)a.halt == a.code_records) return;
@@ -702,7 +713,7 @@ dyg_status decr_walk_ensure(dyg_graph *G, dyg_graph *H, uint32_t n, const dyg_wa
     DYG_TRY(ensure(ws.cand_w, sizeof(float) * M));
     DYG_TRY(ensure(ws.keep, sizeof(uint32_t) * M));
     uint64_t T = 1024;
-    while (T < 2u * (uint64_t)M) T <<= 1;
+    while (T < 2ull * M) T <<= 1;
     if (ws.htab_k.bytes < sizeof(unsigned long long) * T || ws.htab_v.bytes < sizeof(uint32_t) * T) {
         // empty when allocated, and left empty by every recovery
         DYG_TRY(ensure(ws.htab_k, sizeof(unsigned long long) * T));
