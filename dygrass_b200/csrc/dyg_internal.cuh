@@ -151,12 +151,11 @@ __device__ __forceinline__ uint32_t block_find(const uint2 *slots, uint32_t off,
 }
 
 // ------------------------------------------------------------- workspace
-// Device scratch owned by a graph handle, grown on demand.
-// Lookup index of a graph's rows longer than kIdxRow for the weight-proportional
-// walks (k_index, walk.cu), rebuilt for every launch: rbase[v] is the word
-// offset of row v's region in `words`, 0 for a row without one.  A region is a
-// hash table of 2^k >= 2 deg words (position + 1 of a column, 0 empty) and the
-// row's deg inclusive prefix sums of wq (two words each).
+// Lookup index of a graph's long rows for the weight-proportional walks (k_index,
+// walk.cu), rebuilt for every launch: rbase[v] is the word offset of row v's
+// region in `words`, 0 for a row without one.  A region is a hash table of
+// 2^k >= 2 deg words (position + 1 of a column, 0 empty) and the row's deg
+// inclusive prefix sums of wq (two words each).
 struct RowIndex {
     const uint32_t *rbase;   // null: no row has an index
     const uint32_t *words;
@@ -182,6 +181,7 @@ struct PathRec {
     uint32_t threads;             // most threads a walk may have
 };
 
+// Device scratch owned by a graph handle, grown on demand.
 struct Workspace {
     Buf keys;                                 // u64 per edge
     Buf flags, pos;                           // u32 per edge / per vertex (compaction)
@@ -533,9 +533,9 @@ dyg_status count_slots_enqueue(dyg_graph *G, cudaStream_t st);
 dyg_status read_scalars2(dyg_graph *A, dyg_graph *B, cudaStream_t st);
 // DYG_ESTATE for a broken graph (B may be null).
 dyg_status check_usable(const dyg_graph *A, const dyg_graph *B);
-// Exclusive scan of in[0, m) into out; with m_dev, of in[0, min(m, *m_dev)).
+// Exclusive scan of in[0, m) into out.
 dyg_status exclusive_scan_u32(Workspace &ws, const uint32_t *in, uint32_t *out, uint32_t m,
-                              cudaStream_t st, const uint32_t *m_dev = nullptr);
+                              cudaStream_t st);
 dyg_status compact_graph(dyg_graph *G, cudaStream_t st);
 // src's rows, capacities and arena top into dst, whose arena holds them.
 dyg_status copy_graph_enqueue(dyg_graph *dst, const dyg_graph *src, cudaStream_t st);

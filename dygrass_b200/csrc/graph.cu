@@ -1,6 +1,6 @@
 // graph.cu -- device-resident dynamic CSR: upload, arena growth, compaction
 // and the small shared helpers (allocation, scans, scalar read-back).  Row
-// updates live in rowops.cu.  Row moves (capacity exceeded) take space from a
+// updates live in rowops.cuh.  Row moves (capacity exceeded) take space from a
 // bump arena: offsets differ from run to run but contents never do.
 
 #include <algorithm>
@@ -488,7 +488,7 @@ dyg_status build_graph(dyg_graph *G, uint32_t n, uint64_t m, const uint32_t *src
     }
     if (n) {
         DYG_TRY(scan_op(G->ws, BuildScan{cnt, G->g.desc, G->g.cap, G->slack, sc + S_LONG, sc + S_TOP}, n,
-                        nullptr, nullptr, st));
+                        st));
     }
     if (m) {
         const BuildList L{ds, dd, (float *)d_w};
@@ -611,7 +611,7 @@ dyg_status export_graph(dyg_graph *G, uint64_t *row_ptr, uint32_t *col, float *w
     bool ok = tmp.get(&d_rp, sizeof(uint64_t) * ((size_t)n + 1)) == cudaSuccess;
     if (ok) {
         const dyg_status rc =
-            scan_op(G->ws, DegreeScan{G->g.desc, (unsigned long long *)d_rp, n}, n, nullptr, nullptr, st);
+            scan_op(G->ws, DegreeScan{G->g.desc, (unsigned long long *)d_rp, n}, n, st);
         ok = rc == DYG_OK;
         if (!ok && rc != DYG_ENOMEM) return rc;
     }
@@ -733,8 +733,8 @@ struct CopyScan {
 }  // namespace
 
 dyg_status exclusive_scan_u32(Workspace &ws, const uint32_t *in, uint32_t *out, uint32_t m,
-                              cudaStream_t st, const uint32_t *m_dev) {
-    return scan_op(ws, CopyScan{in, out}, m, m_dev, nullptr, st);
+                              cudaStream_t st) {
+    return scan_op(ws, CopyScan{in, out}, m, st);
 }
 
 // -------------------------------------------------------------- compaction

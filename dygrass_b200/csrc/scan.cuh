@@ -20,9 +20,6 @@
 //                                             exclusive prefix of element i
 //   void last(uint32_t total)                 once, with the sum of [0, m)
 // so a flag pass, the scan and the compaction that follows it are one launch.
-// With a device count m_dev, the scan covers [0, min(m, *m_dev)); the tiles
-// past it leave after their ticket (no tile that stays looks back at them).
-// A halted stream (*halt != 0) makes every tile leave after its ticket.
 #pragma once
 
 #include "dyg_internal.cuh"
@@ -40,7 +37,6 @@ struct ScanCtl {
     unsigned long long base;      // tickets handed out before this launch
     uint32_t epoch;
     unsigned long long *err;      // scalars + S_ERR
-    const unsigned long long *halt;
 };
 
 __device__ __forceinline__ unsigned long long scan_word(uint32_t epoch, uint32_t flag, uint32_t v) {
@@ -49,7 +45,7 @@ __device__ __forceinline__ unsigned long long scan_word(uint32_t epoch, uint32_t
 
 template <class Op>
 __global__ void __launch_bounds__(kScanThreads)
-k_scan_op(Op op, uint32_t m, const uint32_t *m_dev, ScanCtl c) {
+k_scan_op(Op op, uint32_t m, ScanCtl c) {
     __shared__ uint32_t s_tile, s_prefix;
     __shared__ uint32_t s_warp[kScanThreads / 32];
     if (threadIdx.x == 0) {
@@ -60,9 +56,6 @@ k_scan_op(Op op, uint32_t m, const uint32_t *m_dev, ScanCtl c) {
     __syncthreads();
     const uint32_t tile = s_tile;
     if (tile == ~0u) return;
-    if (c.halt && *c.halt) return;
-    if (m_dev) m = min(m, *m_dev);
-    if ((uint64_t)tile * kScanTile >= m) return;
     const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
     const uint64_t i0 = (uint64_t)tile * kScanTile + (uint64_t)threadIdx.x * kScanItems;
     uint32_t v[kScanItems];
@@ -151,18 +144,17 @@ inline dyg_status scan_ensure(Workspace &ws, uint32_t m, cudaStream_t st) {
     return DYG_OK;
 }
 
-// Enqueues the scan of [0, m) (of [0, min(m, *m_dev)) with a device count).
+// Enqueues the scan of [0, m).
 template <class Op>
-dyg_status scan_op(Workspace &ws, const Op &op, uint32_t m, const uint32_t *m_dev,
-                   const unsigned long long *halt, cudaStream_t st) {
+dyg_status scan_op(Workspace &ws, const Op &op, uint32_t m, cudaStream_t st) {
     if (m == 0) return DYG_OK;
     const uint32_t tiles = (uint32_t)(((uint64_t)m + kScanTile - 1) / kScanTile);
     DYG_TRY(scan_ensure(ws, m, st));
     ws.scan_epoch = ws.scan_epoch + 1u == 0x40000000u ? 1u : ws.scan_epoch + 1u;
     unsigned long long *sc = ptr<unsigned long long>(ws.scalars);
     const ScanCtl c{ptr<unsigned long long>(ws.scan_status), sc + S_SCAN, ws.scan_tickets,
-                    ws.scan_epoch, sc + S_ERR, halt};
-    k_scan_op<Op><<<tiles, kScanThreads, 0, st>>>(op, m, m_dev, c);
+                    ws.scan_epoch, sc + S_ERR};
+    k_scan_op<Op><<<tiles, kScanThreads, 0, st>>>(op, m, c);
     count_launch();
     DYG_CUDA(cudaGetLastError());
     ws.scan_tickets += tiles;   // every launched tile takes one ticket

@@ -260,30 +260,21 @@ __device__ __forceinline__ int move_uniform(Walker &s, uint2 d, uint32_t r,
     return finish_move<INCR>(s, sl, at, first, max_steps, thr, moved, taken, taken_at);
 }
 
-// One move of one walker, mirroring the reference loop body:
+// One uniform move of one walker, mirroring the reference loop body:
 //   step 1:  any neighbour, r % deg                    (main.cu:99-106)
 //   step >1: dead end if deg == 1; r % (deg - 1) and the last slot when the
 //            draw lands on the previous vertex          (main.cu:118-137)
 // then finish_move.  *moved is set when a neighbour was drawn; *taken
-// receives its slot.  WEIGHTED rows are scanned by this thread alone (the
-// walk kernel searches long rows with the whole warp instead).
-template <bool INCR, bool WEIGHTED>
-__device__ __forceinline__ int step_once(Walker &s, const uint2 *__restrict__ desc,
-                                         const uint2 *__restrict__ slots,
-                                         const float *__restrict__ wts, uint32_t max_steps,
-                                         float thr, uint2 key, bool *moved, uint2 *taken,
-                                         uint32_t *taken_at) {
+// receives its slot.
+template <bool INCR>
+__device__ __forceinline__ int step_uniform(Walker &s, const uint2 *__restrict__ desc,
+                                            const uint2 *__restrict__ slots, uint32_t max_steps,
+                                            float thr, uint2 key, bool *moved, uint2 *taken,
+                                            uint32_t *taken_at) {
     *moved = false;
     const uint2 d = __ldg(desc + s.cur);
-    const uint32_t deg = d.y;
-    const bool first = (s.step == 1u);
-    if (first ? (deg == 0u) : (deg <= 1u)) return kFail;
-    const uint32_t r = draw_next(s, key);
-    if (!WEIGHTED) return move_uniform<INCR>(s, d, r, slots, max_steps, thr, moved, taken, taken_at);
-    uint2 sl;
-    const uint32_t at = lane_pick_weighted(slots, wts, d.x, deg, s.prev, !first, r, &sl);
-    if (at == ~0u) return kFail;
-    return finish_move<INCR>(s, sl, at, first, max_steps, thr, moved, taken, taken_at);
+    if (s.step == 1u ? (d.y == 0u) : (d.y <= 1u)) return kFail;
+    return move_uniform<INCR>(s, d, draw_next(s, key), slots, max_steps, thr, moved, taken, taken_at);
 }
 
 // ------------------------------------------------ weighted, warp-cooperative
@@ -854,9 +845,10 @@ __device__ __forceinline__ void write_record(const PathRec &rec, uint32_t e, uns
 // 1/R is monotone, so a walker whose 1/R is below it can neither win nor tie,
 // and stopping it leaves every result unchanged.
 // 40 registers: six blocks (48 warps) per SM; eight blocks spill (insertions
-// of the 100^3 mesh 4.43 -> 6.43 ms).  Bound by instruction issue on a
-// sparsifier (65-70 % of cycles) and by gather latency and the L1's
-// throughput (70 %) on the dense graph.  Against one lane-private edge read
+// of the 100^3 mesh 4.43 -> 6.43 ms).  Bound by the L1's gathers on a sparsifier
+// (88 % of its throughput, 66 % of issue cycles, 71 % of the warps, third insertion
+// batch of a 60^3 mesh) and by gather latency and the last long walks on the dense
+// graph (57 %, 29 %, 42 %, its third deletion batch).  Against one lane-private edge read
 // and best per walker and the general remainder: insertions of the 100^3 mesh
 // 5.27 -> 4.43 ms, 24 random geometric graphs 1.14 -> 0.96 ms, deletions of
 // the mesh 2.28 -> 2.25 ms.  With chunks of 64 and the edge's best read before the
@@ -1031,10 +1023,9 @@ __global__ void __launch_bounds__(kWalkThreads, 3) k_walk_weighted(WalkArgs a) {
     count_moves(a, moves, walks, lane);
 }
 
-// Replays the winner of each decremental edge and writes its path
-// (random_walk_decremental/main.cu:206-217 writes the same vertices from a
+// Replays the winner of each edge of uniform decremental walks and writes its
+// path (random_walk_decremental/main.cu:206-217 writes the same vertices from a
 // per-thread local array).
-template <bool WEIGHTED>
 __global__ void k_winner_paths(DevGraph g, WalkJob job, uint32_t max_steps, uint2 key,
                                const unsigned long long *keys, uint32_t stride, uint32_t *pv,
                                uint32_t *ps, int32_t *plen, unsigned long long *scalars) {
@@ -1069,8 +1060,7 @@ __global__ void k_winner_paths(DevGraph g, WalkJob job, uint32_t max_steps, uint
         bool moved;
         uint2 taken;
         uint32_t taken_at;
-        r = step_once<false, WEIGHTED>(s, g.desc, g.slots, g.wts, max_steps, 0.f, key, &moved,
-                                       &taken, &taken_at);
+        r = step_uniform<false>(s, g.desc, g.slots, max_steps, 0.f, key, &moved, &taken, &taken_at);
         if (moved && at < stride) {   // no load: a store waiting on one would stall the chain
             row_v[at] = taken.x;
             row_s[at] = taken_at;
@@ -1329,7 +1319,7 @@ dyg_status launch_winner_paths(dyg_graph *G, const WalkJob &job, const dyg_walk_
                                   kReplayThreads, 0, st>>>(G->g, job, ix, p.max_steps, key, keys, stride,
                                                            path_v, path_s, path_len, sc);
     else
-        k_winner_paths<false><<<grid, threads, 0, st>>>(G->g, job, p.max_steps, key, keys, stride,
+        k_winner_paths<<<grid, threads, 0, st>>>(G->g, job, p.max_steps, key, keys, stride,
                                                         path_v, path_s, path_len, sc);
     count_launch();
     DYG_CUDA(cudaGetLastError());

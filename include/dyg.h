@@ -42,7 +42,9 @@
  * Conventions: the caller owns every host buffer; the library owns device
  * graph state.  Array arguments may be host or device pointers (detected per
  * call); device pointers must be memory of the graph's own GPU (or managed
- * memory), else DYG_EINVAL.  Inputs are checked before anything changes:
+ * memory), else DYG_EINVAL.  A call on a dense graph G and a sparsifier H
+ * takes two different handles (one for both: DYG_EINVAL).  Inputs are
+ * checked before anything changes:
  * an endpoint >= |V| or a weight that is not finite and > 0, in host or
  * device memory, makes the call return DYG_EINVAL with G and H unchanged.
  * With host outputs the call returns after the results are on the
@@ -273,7 +275,8 @@ dyg_status dyg_decremental_commit_keys(dyg_graph *G, dyg_graph *H, const dyg_wal
 
 /* Launch shape of the walk kernel for this process (an autotuner's knobs;
  * results do not depend on them): walkers each warp takes per fetch (a
- * multiple of 32 dividing the walker count; 0 = 32) and resident blocks per
+ * multiple of 32 dividing the walker count; 0 = 16, 32 or 64, by the kind and
+ * size of the batch) and resident blocks per
  * SM (0 or more than fit = as many as fit).  Replaces the reference's fixed
  * one-block-per-edge launch (random_walk_incremental/main.cu:316). */
 void dyg_tune_set(uint32_t walk_chunk, uint32_t blocks_per_sm);
@@ -338,7 +341,7 @@ dyg_status dyg_incremental_walk_noalloc(const dyg_graph *H, const uint32_t *src,
 typedef struct dyg_profile {
     double incr_walk_ms;
     double decr_walk_ms;
-    double other_walk_ms;      /* winner replays and fallback walks */
+    double other_walk_ms;      /* winner replays (fallback walks are part of the commit) */
     uint64_t incr_walk_launches;
     uint64_t decr_walk_launches;
     uint64_t other_walk_launches;
