@@ -192,7 +192,7 @@ struct Workspace {
     Buf path_v, path_s;                       // replayed winner paths: vertices, taken slots
     Buf path_len;                             // i32 per filtered edge
     Buf rec_head;                             // path records of the walks: last of each edge
-    uint64_t rec_words = 0;                   // words they took in an earlier call that ran short
+    uint32_t rec_each = 48;                   // words to begin with for each edge: as a call came to need
     Buf cand_x, cand_y, cand_w;               // recovery candidates
     Buf keep;                                 // u32 per candidate
     Buf htab_k, htab_v;                       // dedup hash table
@@ -475,6 +475,7 @@ struct WalkScratch {
     cudaStream_t st;
     PathRec rec{};      // heads null: replay
     Buf hist, words;
+    uint32_t edges = 0;   // that records were opened for
     Buf index;
     bool index_tried = false;
     explicit WalkScratch(cudaStream_t stream) : st(stream) {}

@@ -662,8 +662,8 @@ void WalkScratch::open_paths(dyg_graph *G, uint32_t n, const dyg_walk_params &p)
     const uint32_t threads = walk_threads(n, p);
     const size_t hist_bytes = sizeof(uint32_t) * (size_t)threads * ((p.max_steps + 3u) & ~3u);
     // some paths of a few moves per edge to begin with
-    uint64_t want = (uint64_t)n * 48u + 4096u;
-    if (want < ws.rec_words) want = ws.rec_words;
+    const uint64_t want = (uint64_t)n * ws.rec_each + 4096u;
+    edges = n;
     if (scratch_borrow(&hist, hist_bytes) != cudaSuccess ||
         scratch_borrow(&words, sizeof(uint32_t) * want) != cudaSuccess) {
         cudaGetLastError();
@@ -687,7 +687,9 @@ void WalkScratch::grow_paths(dyg_graph *G) {
         rec = PathRec{};   // replay the winners instead
         return;
     }
-    G->ws.rec_words = need;
+    // the next call begins with as much, within reason: its edges may be others
+    const unsigned long long each = need / edges + 1u;
+    if (each > G->ws.rec_each) G->ws.rec_each = each < kPathSteps ? (uint32_t)each : kPathSteps;
     rec.words = ptr<uint32_t>(words);
     rec.cap = (uint32_t)need;
 }
