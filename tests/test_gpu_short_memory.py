@@ -186,3 +186,50 @@ def test_large_scratch_is_kept_for_the_handles(dyg):  # noqa: F811
     H2.close()
     # the pool and the scratch keep 256 MB each
     assert before - free() < 560 << 20
+
+
+def test_scratch_lent_to_threads(dyg, oracle):  # noqa: F811
+    """Calls on four threads, each with handles and a stream of its own, borrow
+    scratch side by side: every result is the oracle's."""
+    import threading
+    import torch
+    rng = np.random.default_rng(6)
+    n, first, gs, gd, gw = cycles(200, rng)
+    hub = np.r_[first, -400:0]
+    es = rng.integers(0, n, 800).astype(np.uint32)
+    ed = ((es + 1 + rng.integers(0, n - 1, 800)) % n).astype(np.uint32)
+    ew = rng.uniform(0.01, 0.5, 800).astype(np.float32)
+    want = {}
+    for tr in (0, 1):
+        p = dyg.WalkParams.make(threshold=10.0, walkers=64, max_steps=220, transition=tr, heuristic_walkers=2)
+        Go, Ho = oracle.OGraph(n, gs, gd, gw), oracle.OGraph(n, gs[hub], gd[hub], gw[hub])
+        fo, co, _, _ = oracle.incremental(Ho, es, ed, ew, p, batch_size=400, G=Go)
+        st, cd, rx, ry, _, _ = oracle.decremental(Go, Ho, gs[first], gd[first], p, batch_size=100)
+        want[tr] = (fo, co, st, cd, rx, ry)
+    G0, H0 = dyg.Graph.from_edges(n, gs, gd, gw), dyg.Graph.from_edges(n, gs[hub], gd[hub], gw[hub])
+    wrong = []
+
+    def work(tr):
+        try:
+            p = dyg.WalkParams.make(threshold=10.0, walkers=64, max_steps=220, transition=tr, heuristic_walkers=2)
+            s = torch.cuda.Stream()
+            G, H = G0.clone(), H0.clone()
+            for _ in range(8):
+                G.copy_from(G0, stream=s.cuda_stream)
+                H.copy_from(H0, stream=s.cuda_stream)
+                a = dyg.incremental_stream(H, es, ed, ew, p, 400, G=G, stream=s.cuda_stream)
+                b = dyg.decremental_stream(G, H, gs[first], gd[first], p, batch_size=100, stream=s.cuda_stream)
+                got = (a.found_at, a.conductance, b.status, b.conductance, b.rec_src, b.rec_dst)
+                for x, y in zip(got, want[tr]):
+                    assert np.array_equal(np.asarray(x).view(np.uint8), np.asarray(y).astype(x.dtype).view(np.uint8))
+            G.close()
+            H.close()
+        except BaseException as e:   # reported by the test's thread
+            wrong.append(e)
+
+    threads = [threading.Thread(target=work, args=(k % 2,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong, wrong
