@@ -37,6 +37,8 @@
 
 namespace dyg {
 
+// Two blocks of this size an SM leave 64 registers a thread: k_append spills 24 to
+// 36 bytes, k_recover 36, k_delete 8.
 constexpr uint32_t kOpThreads = 512;
 
 struct GridBar {

@@ -295,7 +295,7 @@ __device__ __forceinline__ void fold_end(const MergeArgs &a, const Fold &f) {
 
 // One thread per edge: the leader of each key's chain empties its table slot
 // and folds its occurrences.  A chain of up to kFoldChain is followed and put
-// in file order; a longer one is left to fold_often.
+// in file order, in a local array of 128 bytes; a longer one is left to fold_often.
 constexpr uint32_t kFoldChain = 32;
 constexpr uint32_t kFoldThreads = 256;
 __global__ void __launch_bounds__(kFoldThreads) k_st_merge(const unsigned long long *halt, MergeArgs a) {
